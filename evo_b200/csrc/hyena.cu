@@ -15,7 +15,10 @@
 // falls out for free, arbitrary L (8193!) costs nothing, and the algorithmic HBM traffic is
 // 8 B per token per channel (read 3 bf16, write 1 bf16).
 //
-// Parallelisation: one thread per channel, sequential along L inside a segment; the grid is
+// Kernels: hyena_tc.cuh (heads of 128, all but short sequences: the convolution by blocks on the tensor cores), hyena_ms.cuh (short ones: the recurrence as a
+// scan fed by TMA), hyena_tma.cuh (its predecessor, for comparisons) and the generic scan below; make_plan() chooses.
+//
+// Parallelisation of the scans: one thread per channel, sequential along L inside a segment; the grid is
 // (channel blocks) x (batch) x (L segments).  With more than one segment a first pass
 // computes each segment's zero-start end state (reads x1, v only) and the output pass
 // starts every segment from the exactly combined carry  S_j = p^len S_{j-1} + E_{j-1}.
@@ -27,6 +30,7 @@
 #include <algorithm>
 #include "hyena_tma.cuh"
 #include "hyena_ms.cuh"
+#include "hyena_tc.cuh"
 #include <stdlib.h>
 
 using namespace evo;
@@ -310,18 +314,95 @@ int pick_segments(const evo_hyena_params* p) {
 
 }  // namespace
 
-extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) {
-  if (p->L <= 0) return 0;
-  int nseg = pick_segments(p);
-  if (nseg <= 1 && !p->state_only) return 0;
-  return (size_t)p->B * nseg * p->D * NS * 2 * sizeof(float);
+// Which kernel, how many blocks per row (tensor-core path) and how many segments.
+struct HyenaPlan { bool tc; int R, nseg; long long seg_len; };
+
+// The tensor-core path does the work of 256 R tokens x 32 channels per tile and item in a time that hardly depends on how many of the tokens exist, and computes its
+// constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 64: scan 14.9, tensor
+// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 46; 4 x 1000: 123 / 78; 8 x 300: 44 / 76; 8 x 8193: 953 / 832.  The smaller estimate decides; both sides are in us.
+// Few items (narrow models, one sequence) are cut into segments: a pass over x1 and v then finds the states between them, at about half the price of the output pass.
+HyenaPlan make_plan(const evo_hyena_params* p) {
+  const long long L = p->L;
+  const int sms = device_sm_count();
+  HyenaPlan best = {false, 0, pick_segments(p), 0};
+  best.seg_len = (L + best.nseg - 1) / best.nseg;
+  best.nseg = (int)((L + best.seg_len - 1) / best.seg_len);
+  const char* env_v = getenv("EVO_B200_HYENA_VARIANT");      // comparisons: 0, 1 = the modal scans, 2 = tensor cores; read per call
+  const int variant = env_v ? atoi(env_v) : -1;
+  // taps, biases and carried inputs are read four channels at a time
+  const bool can = use_tma_path(p) && (((uintptr_t)p->fir_w | (uintptr_t)p->fir_b | (uintptr_t)p->halo) & 7) == 0;
+  if (!can || variant == 0 || variant == 1) return best;
+  const long long scan_ctas = (long long)p->D / evo_hy2::CH_PER_CTA * p->B * best.nseg;
+  double cost = variant == 2 ? 1e30 : 7.0 + 0.116 * best.seg_len * (best.nseg > 1 ? 1.6 : std::max(1.0, (double)scan_ctas / sms));
+  const char* env_r = getenv("EVO_B200_HYENA_R");
+  const double per_tile[3] = {5.7, 8.0, 14.4}, fill[3] = {6.0, 9.0, 9.0};
+  const long long items = (long long)p->D / evo_hytc::CH * p->B;
+  for (int r = 0; r < 3; ++r) {
+    const int R = 1 << r;
+    if (env_r && atoi(env_r) != R) continue;
+    const long long tile = 256 * R;
+    const long long most = p->force_segments > 0 ? 1 : std::max<long long>(1, sms / items);
+    for (long long n = 1; n <= most; n = n == most ? most + 1 : most) {
+      long long nseg, len;
+      if (p->force_segments > 0) { nseg = std::min<long long>(p->force_segments, std::max<long long>(1, L)); len = (L + nseg - 1) / nseg; }
+      else { nseg = n; len = ((L + nseg - 1) / nseg + tile - 1) / tile * tile; }
+      nseg = (L + len - 1) / len;
+      const long long tiles = (std::min(len, L) + tile - 1) / tile, rounds = (items * nseg + sms - 1) / sms;
+      double c = 8.0 + fill[r] + rounds * tiles * per_tile[r];
+      if (nseg > 1) c += 4.0 + 0.5 * ((items * (nseg - 1) + sms - 1) / sms) * tiles * per_tile[r];
+      if (c < cost) { cost = c; best = {true, R, (int)nseg, len}; }
+    }
+  }
+  return best;
 }
 
-// segment geometry: equal segments, none empty
-static void segment_geometry(const evo_hyena_params* p, int& nseg, long long& seg_len) {
-  nseg = pick_segments(p);
-  seg_len = (p->L + nseg - 1) / nseg;
-  nseg = (int)((p->L + seg_len - 1) / seg_len);
+static size_t segment_bytes(const evo_hyena_params* p, int nseg) {
+  return nseg <= 1 && !p->state_only ? 0 : (size_t)p->B * nseg * p->D * NS * 2 * sizeof(float);
+}
+
+extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) {
+  if (p->L <= 0) return 0;
+  const HyenaPlan plan = make_plan(p);
+  // the tensor-core path keeps its channels' constants behind the segment states, on the next multiple of 256 bytes
+  return segment_bytes(p, plan.nseg) + (plan.tc ? 256 + evo_hytc::table_bytes(p->D) : 0);
+}
+
+// evo_hytc: constants, then (more than one segment) the segments' end states, then the output
+template <int R>
+static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, void* workspace, cudaStream_t st) {
+  using namespace evo_hytc;
+  int rc;
+  evo_hytc::Args a;
+  a.z = (const bf16*)p->z; a.y = (bf16*)p->y;
+  a.fir_w = (const bf16*)p->fir_w; a.fir_b = (const bf16*)p->fir_b; a.Dskip = (const bf16*)p->Dskip;
+  a.poles = p->poles; a.residues = p->residues; a.halo = (const bf16*)p->halo; a.state_in = p->state_in; a.state_out = p->state_out;
+  a.seg_states = (float*)workspace;
+  uint8_t* consts = (uint8_t*)(((uintptr_t)workspace + segment_bytes(p, nseg) + 255) & ~(uintptr_t)255);
+  float2* seg_pow = (float2*)(consts + (size_t)p->D * CONST_BYTES);
+  a.consts = consts; a.seg_pow = seg_pow;
+  a.B = p->B; a.D = p->D; a.nseg = nseg; a.L = p->L; a.seg_len = seg_len;
+  a.y_wide = ((uintptr_t)p->y & 7) == 0;
+  CUtensorMap tmZ;
+  uint64_t dims[3] = {(uint64_t)3 * p->D, (uint64_t)p->L, (uint64_t)p->B};
+  uint64_t str[2] = {(uint64_t)3 * p->D * 2, (uint64_t)p->L * 3 * p->D * 2};
+  uint32_t box[3] = {CH, (uint32_t)STAGE + 2, 1};
+  if ((rc = make_tmap_nd_bf16(&tmZ, p->z, 3, dims, str, box, false))) return rc;
+  constexpr int smem = evo_hytc::smem_bytes(R);
+  static unsigned long long done_s = 0, done_o = 0;
+  if ((rc = ensure_dyn_smem(hyena_tc_kernel<R, true>, smem, done_s))) return rc;
+  if ((rc = ensure_dyn_smem(hyena_tc_kernel<R, false>, smem, done_o))) return rc;
+  hyena_tc_constants_kernel<<<p->D / PREP_WARPS, PREP_WARPS * 32, 0, st>>>(p->poles, p->residues, consts, seg_pow, p->D, R, nseg > 1 ? seg_len : 0);
+  if ((rc = check_launch("hyena_tc_constants"))) return rc;
+  const int per_seg = p->D / CH * p->B, sms = device_sm_count();
+  if (p->state_only || (nseg > 1 && !p->reuse_segment_states)) {
+    a.items = per_seg * (p->state_only ? nseg : nseg - 1);
+    hyena_tc_kernel<R, true><<<std::min(a.items, sms), evo_hytc::THREADS, smem, st>>>(tmZ, a);
+    if ((rc = check_launch("hyena_tc<state>"))) return rc;
+  }
+  if (p->state_only) return 0;
+  a.items = per_seg * nseg;
+  hyena_tc_kernel<R, false><<<std::min(a.items, sms), evo_hytc::THREADS, smem, st>>>(tmZ, a);
+  return check_launch("hyena_tc<out>");
 }
 
 extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -330,14 +411,18 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
   EVO_REQUIRE(p->B > 0 && p->B <= 65535, "evo_hyena_fwd: bad batch %d", p->B);
   if (p->L == 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  int nseg; long long seg_len;
-  segment_geometry(p, nseg, seg_len);
+  const HyenaPlan plan = make_plan(p);
+  const int nseg = plan.nseg;
+  const long long seg_len = plan.seg_len;
   size_t need = evo_hyena_fwd_workspace(p);
   EVO_REQUIRE(workspace_bytes >= need && (need == 0 || workspace), "evo_hyena_fwd: workspace too small (%zu < %zu)", workspace_bytes, need);
   if (p->state_only) EVO_REQUIRE(p->state_out != nullptr, "evo_hyena_fwd: state_only needs state_out");
   else EVO_REQUIRE(p->y != nullptr, "evo_hyena_fwd: y is NULL");
   int rc;
-  if (use_tma_path(p)) {
+  if (plan.tc) {
+    const int R = plan.R;
+    if ((rc = R == 4 ? launch_tc<4>(p, nseg, seg_len, workspace, st) : (R == 2 ? launch_tc<2>(p, nseg, seg_len, workspace, st) : launch_tc<1>(p, nseg, seg_len, workspace, st)))) return rc;
+  } else if (use_tma_path(p)) {
     using namespace evo_hy2;
     CUtensorMap tmZ;
     uint64_t dims[3] = {(uint64_t)3 * p->D, (uint64_t)p->L, (uint64_t)p->B};
@@ -354,14 +439,14 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     if ((rc = ensure_dyn_smem(hyena_scan_tma_kernel<false>, smem_bytes(STAGES), done_o))) return rc;
     // 1 (default) = mode-split kernel (hyena_ms.cuh: 8 compute warps, 4 modal states per thread); 0 = round-1 kernel
     // (4 compute warps, 8 states per thread), kept for A/B timing and as a second implementation in the parity tests
-    const char* env_v = getenv("EVO_B200_HYENA_VARIANT");      // read per call: experiments flip it inside one process
+    const char* env_v = getenv("EVO_B200_HYENA_VARIANT");
     const int variant = env_v ? atoi(env_v) : 1;
     static unsigned long long done_ms = 0, done_mo = 0;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<true>, smem_bytes(STAGES), done_ms))) return rc;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<false>, smem_bytes(STAGES), done_mo))) return rc;
-    dim3 grid(p->D / CH_PER_CTA, p->B, nseg), block(variant == 1 ? evo_hy3::THREADS : evo_hy2::THREADS);
-    auto k_state = variant == 1 ? evo_hy3::hyena_scan_ms_kernel<true> : hyena_scan_tma_kernel<true>;
-    auto k_out = variant == 1 ? evo_hy3::hyena_scan_ms_kernel<false> : hyena_scan_tma_kernel<false>;
+    dim3 grid(p->D / CH_PER_CTA, p->B, nseg), block(variant != 0 ? evo_hy3::THREADS : evo_hy2::THREADS);
+    auto k_state = variant != 0 ? evo_hy3::hyena_scan_ms_kernel<true> : hyena_scan_tma_kernel<true>;
+    auto k_out = variant != 0 ? evo_hy3::hyena_scan_ms_kernel<false> : hyena_scan_tma_kernel<false>;
     // ring depth 4 (96 KB): two CTAs can co-reside and hide each other's latency when the grid exceeds the SM count.
     // An 8-deep ring for single-CTA-per-SM grids was measured and did not help (1.21 vs 1.06-1.13 ms at B=8, L=8193).
     a.nst = 4;
