@@ -29,6 +29,7 @@
 // The per-channel decay is the state-space loop with one decay per state row, staged beside the (key, query) pairs, and the delta rule's
 // epilogue; evo_low_rank_decay computes the decays sigmoid(A2 u + b)^(1/tau) of all rows and channels beforehand, in fp32.
 // The single-token step is the same kernel with L == 1.
+// The delta rule's prompts in bf16 (heads of 64 or 128 key channels, 32 tokens or more) go by blocks on the tensor cores instead: delta_block.cu.
 #include "common.cuh"
 #include <stdlib.h>
 #include "../../include/evo_b200.h"
@@ -39,6 +40,8 @@ using namespace evo;
 
 namespace evo {
 int decay_scan_recurrent(const evo_decay_scan_params* p, cudaStream_t st);      // called by linear_attention.cu
+size_t delta_block_workspace(const evo_gated_delta_params* p);                   // delta_block.cu: prompts by blocks (0: not taken)
+int delta_block_fwd(const evo_gated_delta_params* p, void* ws, size_t bytes, cudaStream_t st);
 }
 
 namespace {
@@ -530,6 +533,7 @@ int dispatch(ScanArgs a, void* workspace, size_t workspace_bytes, cudaStream_t s
 }  // namespace
 
 extern "C" size_t evo_gated_delta_workspace(const evo_gated_delta_params* p) {
+  if (const size_t n = delta_block_workspace(p)) return n;
   const Plan pl = plan(p->dk, p->dv, (int64_t)p->B * p->H, p->L);
   return pl.chunks > 1 ? sizeof(float) * (size_t)p->B * p->L * p->H * p->dv : 0;
 }
@@ -539,6 +543,7 @@ extern "C" int evo_gated_delta_fwd(const evo_gated_delta_params* p, void* worksp
   EVO_REQUIRE(p->B >= 0 && p->L >= 0 && p->H > 0 && p->G > 0 && p->H % p->G == 0 && p->dk > 0 && p->dv > 0 && p->ldo >= (int64_t)p->H * p->dv,
               "evo_gated_delta_fwd: bad shape");
   if (p->B == 0 || p->L == 0) return 0;
+  if (delta_block_workspace(p)) return delta_block_fwd(p, workspace, workspace_bytes, (cudaStream_t)stream);
   ScanArgs a = {};
   a.kk = p->k; a.qq = p->q; a.vv = p->v; a.ld = p->ld;
   a.s0 = p->b; a.s1 = p->a; a.lds = p->ldz;
