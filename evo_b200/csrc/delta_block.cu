@@ -10,10 +10,10 @@
 //   one product are then, lane by lane, the first operand of the next, so the 16 x dk piece of the state stays in the warp's registers and warps exchange nothing:
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
 //   S, W, U are fp32 and enter as three bf16 parts; K and Q are bf16 as they stand (their norms scale the sums); T, P have three parts and meet W, U in the six products
-//   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by cp.async while one is in work.
+//   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work.
 // delta_norm_kernel: head norm, weight and SiLU gate of the fp32 read-outs.
-// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 739 us (token by token 2774), of which the scan 417, bound by the tensor pipe (816 mma of 8.7 cycles per block and
-// warp, one warp per scheduler: 7.1 k of 12.4 k cycles) and the splits between its products; 1 x 777 tokens, 32 heads: 134 us (516).
+// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 590 us (token by token 2774), of which the scan 395, bound by the tensor pipe (816 mma of 8.7 cycles per block and
+// warp, one warp per scheduler: 7.1 k of 10.4 k cycles) and the splits between its products; 1 x 777 tokens, 32 heads: 110 us (516).
 // A block in which W or U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
 #include "common.cuh"
 #include "mma_sync.cuh"
@@ -65,6 +65,18 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool on) {       // zero-filled when off
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
+// global -> shared memory, bytes and both addresses multiples of 16
+__device__ __forceinline__ void bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+// an mbarrier wait with a limit; one that runs out is counted and the kernel ends
+__device__ unsigned int delta_lost_waits;
+__device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < (1 << 22); ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  atomicAdd(&delta_lost_waits, 1u);
+  return false;
+}
 __device__ __forceinline__ void mma_np(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {       // free to be scheduled
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -73,15 +85,16 @@ __device__ __forceinline__ void mma_np(float* d, const uint32_t* a, uint32_t b0,
 __device__ __forceinline__ float softplus_f(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // ------------------------------------------------------------------------------------------------ what does not depend on the state
+__host__ __device__ constexpr int prepare_rows_bytes(int dk) { return 2 * BT * (2 * dk + 16) > 2 * BT * (BT + 4) * 4 ? 2 * BT * (2 * dk + 16) : 2 * BT * (BT + 4) * 4; }
 template <int DK>
 __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
-  constexpr int PITCH = 2 * DK + 16, AP = BT + 1;            // bytes of a key row; floats of a row of A (one column per thread reads rows: broadcasts)
+  constexpr int PITCH = 2 * DK + 16, AP = BT + 4;            // bytes of a key row; floats of a row of A (16-byte pieces)
   extern __shared__ __align__(16) uint8_t sm[];
   uint8_t* ks = sm;
   uint8_t* qs = ks + BT * PITCH;
-  float* As = reinterpret_cast<float*>(qs + BT * PITCH);     // [BT][AP] A, then T diag(beta)
+  float* As = reinterpret_cast<float*>(sm);                  // [BT][AP] A, then T, in the place of the keys and queries once they are multiplied
   float* Ps = As + BT * AP;                                  // [BT][AP]
-  float* rk = Ps + BT * AP;
+  float* rk = reinterpret_cast<float*>(sm + prepare_rows_bytes(DK));
   float* rq = rk + BT;
   float* beta = rq + BT;
   float* lh = beta + BT;                                     // running log decay, high and low float
@@ -148,7 +161,6 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
     sk += __shfl_xor_sync(0xffffffffu, sk, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 1);
     if (!(lane & 1)) { rk[t] = 1.0f / sqrtf(sk + p.unit_eps); rq[t] = p.q_scale / sqrtf(sq + p.unit_eps); }
   }
-  for (int e = tid; e < BT * AP; e += 128) As[e] = 0.f;
   __syncthreads();
   // ---- k . k and q . k: warp = 16 rows i, tiles of 8 columns j up to the diagonal
   {
@@ -175,6 +187,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
         }
       }
     }
+    __syncthreads();
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       if (n / 2 > warp) continue;
@@ -190,22 +203,29 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
     }
   }
   __syncthreads();
-  // ---- T = (1 + A)^-1: thread j solves for column j, T_ij = -sum_{j<=k<i} A_ik T_kj (rows above j stay zero), in four interleaved sums
+  // ---- T = (1 + A)^-1 in fp32: the two diagonal blocks of 32 by forward substitution, one column per thread; then T21 = -T22 (A21 T11), with the
+  // inner product in the unused upper right block (one block of 64 would be 2016 multiply-adds in a row, an instruction stream no cache holds)
   uint8_t* out = p.blocks + (((int64_t)b * p.H + h) * p.n_blocks + blk) * BLOCK_BYTES;
   float* vec = reinterpret_cast<float*>(out + 2 * TRI_BYTES);
   if (tid < BT) {
-    float T[BT];
+    const int d = tid & 32, c = tid & 31;
+    const float* Ad = As + d * AP + d;
+    float T[32];
 #pragma unroll
-    for (int i = 0; i < BT; ++i) {
+    for (int i = 0; i < 32; ++i) {
       float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int k = 0; k < i; ++k) s[k & 3] = fmaf(As[i * AP + k], T[k], s[k & 3]);
-      T[i] = i < tid ? 0.f : (i == tid ? 1.f : -((s[0] + s[1]) + (s[2] + s[3])));
-    }
-    asm volatile("bar.sync 1, 64;" ::: "memory");                       // all rows of A are read
-    const float bj = beta[tid];
+      for (int k = 0; k < i; k += 4) {
+        const float4 r = *reinterpret_cast<const float4*>(Ad + i * AP + k);          // (what lies on and above the diagonal is not used)
+        const float rv[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-    for (int i = 0; i < BT; ++i) As[i * AP + tid] = i < tid ? 0.f : T[i] * bj;
+        for (int u = 0; u < 4; ++u) if (k + u < i) s[u] = fmaf(rv[u], T[k + u], s[u]);
+      }
+      T[i] = i < c ? 0.f : (i == c ? 1.f : -((s[0] + s[1]) + (s[2] + s[3])));
+    }
+    __syncwarp();                                                       // a diagonal block is read and replaced by one warp
+#pragma unroll
+    for (int i = 0; i < 32; ++i) As[(d + i) * AP + d + c] = T[i];
   } else {
     const int t = tid - BT;
     const float G = expf(lh[t] + ll[t]);
@@ -214,6 +234,31 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
     vec[V_CK * BT + t] = expf((lh[BT - 1] - lh[t]) + (ll[BT - 1] - ll[t])) * rk[t];
     vec[V_RK * BT + t] = rk[t]; vec[V_RQ * BT + t] = rq[t]; vec[V_BETA * BT + t] = beta[t];
     if (t == BT - 1) vec[V_ROWS * BT] = G;
+  }
+  __syncthreads();
+  {
+    const int r = tid >> 2, c = (tid & 3) * 8;
+    // acc[0..7] = sum_k left[k] * right[k][c ..]
+    auto row_times = [&](const float* left, const float* right, float (&acc)[8]) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < 32; ++k) {
+        const float l = left[k];
+        const float4 x = *reinterpret_cast<const float4*>(right + k * AP + c), y = *reinterpret_cast<const float4*>(right + k * AP + c + 4);
+        acc[0] = fmaf(l, x.x, acc[0]); acc[1] = fmaf(l, x.y, acc[1]); acc[2] = fmaf(l, x.z, acc[2]); acc[3] = fmaf(l, x.w, acc[3]);
+        acc[4] = fmaf(l, y.x, acc[4]); acc[5] = fmaf(l, y.y, acc[5]); acc[6] = fmaf(l, y.z, acc[6]); acc[7] = fmaf(l, y.w, acc[7]);
+      }
+    };
+    float acc[8];
+    row_times(As + (32 + r) * AP, As, acc);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) As[r * AP + 32 + c + u] = acc[u];
+    __syncthreads();
+    row_times(As + (32 + r) * AP + 32, As + 32, acc);
+    // (A21 was read before the barrier)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) As[(32 + r) * AP + c + u] = -acc[u];
   }
   __syncthreads();
   // ---- as second operands: column n = token i, k = token j; lane (g, tq) of tile (kt, nt): i = 8 nt + g, j = 16 kt + 2 tq + {0, 1} | + 8
@@ -226,7 +271,9 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int jj = j + 8 * u;
-      split3(jj <= i ? src[i * AP + jj] : 0.f, jj + 1 <= i ? src[i * AP + jj + 1] : 0.f, w[u][0], w[u][1], w[u][2]);
+      const float2 x = *reinterpret_cast<const float2*>(src + i * AP + jj);
+      const float f0 = e < TILES ? beta[jj] : 1.f, f1 = e < TILES ? beta[jj + 1] : 1.f;
+      split3(jj <= i ? x.x * f0 : 0.f, jj + 1 <= i ? x.y * f1 : 0.f, w[u][0], w[u][1], w[u][2]);
     }
     uint2* dst = reinterpret_cast<uint2*>(out + (e < TILES ? 0 : TRI_BYTES) + (e % TILES) * 3 * PART_BYTES) + lane;
 #pragma unroll
@@ -236,36 +283,34 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
 
 // ------------------------------------------------------------------------------------------------ the recurrence
 template <int DK>
-__global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
-  constexpr int PITCH = 2 * DK + 16, KT = DK / 16;
-  extern __shared__ __align__(16) uint8_t sm[];
+__global__ void __launch_bounds__(256, 1) delta_scan_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmV, const Args p) {
+  constexpr int KT = DK / 16, BOX = BT * 128, ROWS_BYTES = DK / 64 * BOX;      // keys and queries: boxes of 64 columns, 16-byte pieces of a row swizzled by row & 7
+  extern __shared__ __align__(16) uint8_t sm_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t arrived[2];
   const int nw = blockDim.x >> 5, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-  const int vpitch = nw * 32 + 16, stage_bytes = 2 * BT * PITCH + BT * vpitch + BLOCK_BYTES;
+  const int vpitch = nw * 32, stage_bytes = 2 * ROWS_BYTES + BT * vpitch + BLOCK_BYTES;
   const int h = blockIdx.x, b = blockIdx.y, g = h / (p.H / p.G), dv = p.dv;
   const int c0 = blockIdx.z * nw * 16, cw = c0 + warp * 16;            // the CTA's and the warp's first value channel
   const int64_t rowb = (int64_t)b * p.L + p.first * BT, left = p.L - p.first * BT;       // the slab's first row; tokens from there
   const uint8_t* blocks = p.blocks + ((int64_t)b * p.H + h) * p.n_blocks * (int64_t)BLOCK_BYTES;
 
+  // a block's rows of K, Q, V (rows behind the last token arrive as zeros) and its T, P and vectors: one lane
   auto fetch = [&](int blk) {
     uint8_t* st = sm + (blk & 1) * stage_bytes;
-    const int64_t t0 = (int64_t)blk * BT;
-    for (int e = tid; e < BT * (DK / 8); e += blockDim.x) {
-      const int r = e / (DK / 8), c = e % (DK / 8);
-      const bool on = t0 + r < left;
-      const int64_t off = (rowb + (on ? t0 + r : 0)) * p.ld + (int64_t)g * DK + c * 8;
-      cp16(smem_u32(st + r * PITCH + c * 16), p.k + off, on);
-      cp16(smem_u32(st + BT * PITCH + r * PITCH + c * 16), p.q + off, on);
+    uint64_t* bar = &arrived[blk & 1];
+    const int t0 = (int)(p.first + blk) * BT;
+    mbar_arrive_expect_tx(bar, stage_bytes);
+#pragma unroll
+    for (int i = 0; i < DK / 64; ++i) {
+      tma_load_3d(st + i * BOX, &tmK, bar, g * DK + i * 64, t0, b);
+      tma_load_3d(st + ROWS_BYTES + i * BOX, &tmQ, bar, g * DK + i * 64, t0, b);
     }
-    for (int e = tid; e < BT * nw * 2; e += blockDim.x) {
-      const int r = e / (nw * 2), c = e % (nw * 2);
-      const bool on = t0 + r < left && c0 + c * 8 < dv;
-      cp16(smem_u32(st + 2 * BT * PITCH + r * vpitch + c * 16), p.v + (on ? (rowb + t0 + r) * p.ld + (int64_t)h * dv + c0 + c * 8 : 0), on);
-    }
-    const uint8_t* src = blocks + (int64_t)blk * BLOCK_BYTES;
-    uint8_t* dst = st + 2 * BT * PITCH + BT * vpitch;
-    for (int e = tid; e < BLOCK_BYTES / 16; e += blockDim.x) cp16(smem_u32(dst + e * 16), src + e * 16, true);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    tma_load_3d(st + 2 * ROWS_BYTES, &tmV, bar, h * dv + c0, t0, b);
+    bulk(st + 2 * ROWS_BYTES + BT * vpitch, blocks + (int64_t)blk * BLOCK_BYTES, BLOCK_BYTES, bar);
   };
+  if (tid == 0) { mbar_init(&arrived[0], 1); mbar_init(&arrived[1], 1); fence_barrier_init(); }
+  __syncthreads();
 
   // ---- S^T: rows = value channels cw + gq (+ 8), columns = state rows: S[n][..] covers state rows 8 n + 2 tq, + 1
   float S[2 * KT][4];
@@ -277,15 +322,14 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
     for (int e = 0; e < 4; ++e)
       S[n][e] = (p.zero_start || !live) ? 0.f : Sg[(int64_t)(8 * n + 2 * tq + (e & 1)) * dv + cw + gq + (e >> 1) * 8];
 
-  fetch(0);
+  if (tid == 0) fetch(0);
   for (int blk = 0; blk < p.n_blocks; ++blk) {
-    if (blk + 1 < p.n_blocks) fetch(blk + 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
+    if (tid == 0 && blk + 1 < p.n_blocks) fetch(blk + 1);
     const uint8_t* ks = sm + (blk & 1) * stage_bytes;
-    const uint8_t* qs = ks + BT * PITCH;
-    const uint8_t* vs = qs + BT * PITCH;
+    const bool here = wait_or_give_up(&arrived[blk & 1], (blk >> 1) & 1);
+    if (__syncthreads_or(!here)) break;
+    const uint8_t* qs = ks + ROWS_BYTES;
+    const uint8_t* vs = qs + ROWS_BYTES;
     const uint8_t* tri = vs + BT * vpitch;
     const float* vec = reinterpret_cast<const float*>(tri + 2 * TRI_BYTES);
     const int nt = (int)min((int64_t)BT, left - (int64_t)blk * BT);
@@ -296,10 +340,10 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
       for (int n = 0; n < 8; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) W[n][e] = O[n][e] = 0.f;
-      const int brow = (lane & 7) + ((lane >> 4) << 3), bcol = ((lane >> 3) & 1) * 16;
-      const uint32_t kb = smem_u32(ks) + brow * PITCH + bcol, qb = smem_u32(qs) + brow * PITCH + bcol;
+      const uint32_t brow = ((lane & 7) + ((lane >> 4) << 3)) * 128, piece = (lane >> 3) & 1, turn = lane & 7;
 #pragma unroll
       for (int kt = 0; kt < KT; ++kt) {
+        const uint32_t at = (kt >> 2) * BOX + brow + (((2 * (kt & 3) + piece) ^ turn) << 4), kb = smem_u32(ks) + at, qb = smem_u32(qs) + at;
         uint32_t a[3][4];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -309,8 +353,8 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
 #pragma unroll
         for (int n2 = 0; n2 < 4; ++n2) {
           uint32_t bk[4], bq[4];
-          ldmatrix_x4_at(bk, kb + n2 * 16 * PITCH + kt * 32);
-          ldmatrix_x4_at(bq, qb + n2 * 16 * PITCH + kt * 32);
+          ldmatrix_x4_at(bk, kb + n2 * 16 * 128);
+          ldmatrix_x4_at(bq, qb + n2 * 16 * 128);
 #pragma unroll
           for (int s = 2; s >= 0; --s) {
             mma_np(W[2 * n2], a[s], bk[0], bk[1]); mma_np(W[2 * n2 + 1], a[s], bk[2], bk[3]);
@@ -349,15 +393,19 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
             split3(X[2 * kt + u][2], X[2 * kt + u][3], a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
           }
 #pragma unroll
-          for (int n = 2 * kt; n < 8; ++n) {
-            const uint2* t = reinterpret_cast<const uint2*>(base + tile_index(kt, n) * 3 * PART_BYTES) + lane;
-            const uint2 t0 = t[0], t1 = t[32], t2 = t[64];
-            mma_np(Y[n], a[0], t2.x, t2.y);
-            mma_np(Y[n], a[2], t0.x, t0.y);
-            mma_np(Y[n], a[1], t1.x, t1.y);
-            mma_np(Y[n], a[0], t1.x, t1.y);
-            mma_np(Y[n], a[1], t0.x, t0.y);
-            mma_np(Y[n], a[0], t0.x, t0.y);
+          for (int n0 = 2 * kt; n0 < 8; n0 += 4) {                       // four sums at a time: a sum's next mma is four later (23 cycles of latency, 8.7 of issue)
+            uint2 t[4][3];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (n0 + c < 8)
+#pragma unroll
+                for (int s = 0; s < 3; ++s) t[c][s] = (reinterpret_cast<const uint2*>(base + tile_index(kt, n0 + c) * 3 * PART_BYTES) + lane)[s * 32];
+            const int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};       // small products first
+#pragma unroll
+            for (int m = 0; m < 6; ++m)
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                if (n0 + c < 8) mma_np(Y[n0 + c], a[pa[m]], t[c][pb[m]].x, t[c][pb[m]].y);
           }
         }
       };
@@ -386,7 +434,7 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
         for (int n = 0; n < 2 * KT; ++n)
 #pragma unroll
           for (int e = 0; e < 4; ++e) S[n][e] *= G;
-        const uint32_t kt_b = smem_u32(ks) + ((lane & 7) + (((lane >> 3) & 1) << 3)) * PITCH + (lane >> 4) * 16;
+        const uint32_t kt_b = smem_u32(ks) + ((lane & 7) + (((lane >> 3) & 1) << 3)) * 128;
 #pragma unroll
         for (int kt = 0; kt < 4; ++kt) {
           uint32_t a[3][4];
@@ -398,11 +446,14 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
             split3(U[n][2] * ck.x, U[n][3] * ck.y, a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
           }
 #pragma unroll
-          for (int n2 = 0; n2 < KT; ++n2) {
-            uint32_t bk[4];
-            ldmatrix_x4_trans_at(bk, kt_b + kt * 16 * PITCH + n2 * 32);
+          for (int n2 = 0; n2 < KT; n2 += 2) {
+            uint32_t bk[8];
+            ldmatrix_x4_trans_at(bk, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + (lane >> 4)) ^ turn) << 4));
+            ldmatrix_x4_trans_at(bk + 4, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + 2 + (lane >> 4)) ^ turn) << 4));
 #pragma unroll
-            for (int s = 2; s >= 0; --s) { mma_np(S[2 * n2], a[s], bk[0], bk[1]); mma_np(S[2 * n2 + 1], a[s], bk[2], bk[3]); }
+            for (int s = 2; s >= 0; --s)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) mma_np(S[2 * n2 + c], a[s], bk[2 * c], bk[2 * c + 1]);
           }
         }
       } else {
@@ -412,7 +463,7 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
           float pk[2] = {0.f, 0.f}, po[2] = {0.f, 0.f}, kq = 0.f;
 #pragma unroll
           for (int n = 0; n < 2 * KT; ++n) {
-            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + t * PITCH + 16 * n + 4 * tq), qw = *reinterpret_cast<const uint32_t*>(qs + t * PITCH + 16 * n + 4 * tq);
+            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq), qw = *reinterpret_cast<const uint32_t*>(qs + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
             const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk, q0 = bf_lo(qw) * nq, q1 = bf_hi(qw) * nq;
             kq = fmaf(k1, q1, fmaf(k0, q0, kq));
 #pragma unroll
@@ -432,7 +483,7 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
           }
 #pragma unroll
           for (int n = 0; n < 2 * KT; ++n) {
-            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + t * PITCH + 16 * n + 4 * tq);
+            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
             const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk;
 #pragma unroll
             for (int u = 0; u < 2; ++u) { S[n][2 * u] = fmaf(k0, pk[u], S[n][2 * u]); S[n][2 * u + 1] = fmaf(k1, pk[u], S[n][2 * u + 1]); }
@@ -442,7 +493,6 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const Args p) {
     }
     __syncthreads();                                                    // the stage may be filled again
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (p.store_state && live) {
 #pragma unroll
     for (int n = 0; n < 2 * KT; ++n)
@@ -479,29 +529,39 @@ __global__ void __launch_bounds__(256) delta_norm_kernel(const float* __restrict
   if (h == H - 1)
     for (int64_t c = (int64_t)H * dv + lane; c < ldo; c += 32) out[row * ldo + c] = __float2bfloat16_rn(0.f);
 }
+// the same for heads of 32 N channels and rows that start on four elements: eight lanes per (row, head), everything in registers between the two passes
+template <int N>
 __global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int64_t ldg, const bf16* __restrict__ w, bf16* __restrict__ out, int64_t ldo,
                                                           int64_t rows, int H, int dv, float eps) {
-  const int64_t wid = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (wid >= rows * H) return;
-  const int64_t row = wid / H;
-  const int h = (int)(wid % H);
-  const float4* r = reinterpret_cast<const float4*>(y + wid * dv);
-  const uint2* gr = reinterpret_cast<const uint2*>(gate + row * ldg + (int64_t)h * dv);
-  uint2* orow = reinterpret_cast<uint2*>(out + row * ldo + (int64_t)h * dv);
-  float ss = 0.f;
-  for (int c = lane; c < dv / 4; c += 32) { const float4 o = r[c]; ss = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, fmaf(o.w, o.w, ss)))); }
+  const int64_t id = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int sub = threadIdx.x & 7;
+  const bool on = id < rows * H;
+  const int64_t row = on ? id / H : 0;
+  const int h = on ? (int)(id - row * H) : 0;
+  const float4* r = reinterpret_cast<const float4*>(y + (on ? id : 0) * (32 * N)) + sub;
+  const uint2* gr = reinterpret_cast<const uint2*>(gate + row * ldg + (int64_t)h * (32 * N)) + sub;
+  const uint2* wr = reinterpret_cast<const uint2*>(w) + sub;
+  float4 o[N];
+  uint2 gv[N];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  const float rstd = 1.0f / sqrtf(ss / (float)dv + eps);
-  const auto one = [&](float o, float gv, float wv) { return o * rstd * wv * (gv / (1.f + expf(-gv))); };
-  for (int c = lane; c < dv / 4; c += 32) {
-    const float4 o = r[c];
-    const uint2 gv = gr[c], wv = reinterpret_cast<const uint2*>(w)[c];
-    orow[c] = make_uint2(pack_bf16(one(o.x, bf_lo(gv.x), bf_lo(wv.x)), one(o.y, bf_hi(gv.x), bf_hi(wv.x))), pack_bf16(one(o.z, bf_lo(gv.y), bf_lo(wv.y)), one(o.w, bf_hi(gv.y), bf_hi(wv.y))));
+  for (int i = 0; i < N; ++i) { o[i] = r[8 * i]; gv[i] = gr[8 * i]; }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) ss = fmaf(o[i].x, o[i].x, fmaf(o[i].y, o[i].y, fmaf(o[i].z, o[i].z, fmaf(o[i].w, o[i].w, ss))));
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  const float rstd = 1.0f / sqrtf(ss / (float)(32 * N) + eps);
+  if (!on) return;
+  uint2* orow = reinterpret_cast<uint2*>(out + row * ldo + (int64_t)h * (32 * N)) + sub;
+  const auto one = [&](float v, float g, float wv) { return v * rstd * wv * (g / (1.f + expf(-g))); };
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint2 wv = wr[8 * i];
+    orow[8 * i] = make_uint2(pack_bf16(one(o[i].x, bf_lo(gv[i].x), bf_lo(wv.x)), one(o[i].y, bf_hi(gv[i].x), bf_hi(wv.x))),
+                             pack_bf16(one(o[i].z, bf_lo(gv[i].y), bf_lo(wv.y)), one(o[i].w, bf_hi(gv[i].y), bf_hi(wv.y))));
   }
   if (h == H - 1)
-    for (int64_t c = (int64_t)H * dv + lane; c < ldo; c += 32) out[row * ldo + c] = __float2bfloat16_rn(0.f);
+    for (int64_t c = (int64_t)H * (32 * N) + sub; c < ldo; c += 8) out[row * ldo + c] = __float2bfloat16_rn(0.f);
 }
 
 // Blocks whose T and P are in memory at a time: at most 256 MB of them (a longer call runs slab after slab).
@@ -538,24 +598,30 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   const int64_t warps = (int64_t)p->B * p->H * (p->dv / 16);
   int nw = 2;
   while (nw < 8 && nw * 16 < p->dv && warps > (int64_t)nw * device_sm_count()) nw *= 2;
-  constexpr int PITCH = 2 * DK + 16;
-  const int prep_smem = 2 * BT * PITCH + 2 * BT * (BT + 1) * 4 + 5 * BT * 4, scan_smem = 2 * (2 * BT * PITCH + BT * (nw * 32 + 16) + BLOCK_BYTES);
+  const int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = 1024 + 2 * (2 * BT * DK * 2 + BT * nw * 32 + BLOCK_BYTES);
+  CUtensorMap tmK, tmQ, tmV;
+  const uint64_t kdims[3] = {(uint64_t)p->G * DK, (uint64_t)p->L, (uint64_t)p->B}, vdims[3] = {(uint64_t)p->H * p->dv, (uint64_t)p->L, (uint64_t)p->B};
+  const uint64_t strides[2] = {(uint64_t)p->ld * 2, (uint64_t)p->L * p->ld * 2};
+  const uint32_t kbox[3] = {64, BT, 1}, vbox[3] = {(uint32_t)nw * 16, BT, 1};
+  int rc;
+  if ((rc = make_tmap_nd_bf16(&tmK, p->k, 3, kdims, strides, kbox, true)) || (rc = make_tmap_nd_bf16(&tmQ, p->q, 3, kdims, strides, kbox, true)) ||
+      (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, false))) return rc;
   EVO_CUDA(cudaFuncSetAttribute(delta_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem));
   EVO_CUDA(cudaFuncSetAttribute(delta_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem));
-  int rc;
   for (int64_t first = 0; first < s.blocks; first += s.slab) {
     a.first = first; a.n_blocks = (int)std::min<int64_t>(s.slab, s.blocks - first);
     a.zero_start = first == 0 && (p->zero_start || !p->state);
     a.store_state = p->state || s.state;
     delta_prepare_kernel<DK><<<dim3(a.n_blocks, a.H, a.B), 128, prep_smem, st>>>(a);
     if ((rc = check_launch("evo_gated_delta_fwd(prepare)"))) return rc;
-    delta_scan_kernel<DK><<<dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), nw * 32, scan_smem, st>>>(a);
+    delta_scan_kernel<DK><<<dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), nw * 32, scan_smem, st>>>(tmK, tmQ, tmV, a);
     if ((rc = check_launch("evo_gated_delta_fwd(scan)"))) return rc;
   }
   const int64_t rows = (int64_t)p->B * p->L, w = rows * p->H;
   const bool wide = p->ldz % 4 == 0 && p->ldo % 4 == 0 && (((uintptr_t)p->gate | (uintptr_t)p->out | (uintptr_t)p->norm_w) & 7) == 0;
-  auto norm = wide ? delta_norm4_kernel : delta_norm_kernel;
-  norm<<<(unsigned)((w + 7) / 8), 256, 0, st>>>(a.y, (const bf16*)p->gate, p->ldz, (const bf16*)p->norm_w, (bf16*)p->out, p->ldo, rows, p->H, p->dv, p->eps);
+  auto norm = !wide ? delta_norm_kernel : (p->dv == 128 ? delta_norm4_kernel<4> : (p->dv == 64 ? delta_norm4_kernel<2> : (p->dv == 32 ? delta_norm4_kernel<1> : delta_norm_kernel)));
+  const int per_cta = norm == delta_norm_kernel ? 8 : 32;
+  norm<<<(unsigned)((w + per_cta - 1) / per_cta), 256, 0, st>>>(a.y, (const bf16*)p->gate, p->ldz, (const bf16*)p->norm_w, (bf16*)p->out, p->ldo, rows, p->H, p->dv, p->eps);
   return check_launch("evo_gated_delta_fwd(norm)");
 }
 
