@@ -151,10 +151,130 @@ __global__ void __launch_bounds__(256) sum_norm_kernel(evo_sum_norm_params p) {
   }
 }
 
-// ---- evo_conv_act: a thread owns one channel of one sequence over RT consecutive rows, its last taps inputs in registers
-constexpr int CONV_RT = 32, CONV_MAX_TAPS = 8;
+// The same for rows of up to 1024 NV elements that can be read four at a time: the row stays in registers (NV groups of four per thread), all loads of a
+// pass are issued together, and a sum over the CTA costs one barrier.  One CTA per row, 256 threads.  8190 x 4096, two bf16 branches, two norms: 87 us = 6.2 TB/s (116 through
+// shared memory; 112 with the branches unpacked, whose registers left three rows per SM instead of four).
+__device__ __forceinline__ float cta_sum(float v, float* red) {          // red: 8 floats of this sum's own
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  const float4 a = reinterpret_cast<const float4*>(red)[0], b = reinterpret_cast<const float4*>(red)[1];
+  return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+}
 
-// four channels per thread (8- or 16-byte accesses), taps known at compile time
+// four elements as they lie in memory
+template <typename T> struct Raw4;
+template <> struct Raw4<float> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void get(float* o) const { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+  __device__ __forceinline__ void clear() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+};
+template <> struct Raw4<bf16> {
+  uint2 v;
+  __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void get(float* o) const { o[0] = bf_lo(v.x); o[1] = bf_hi(v.x); o[2] = bf_lo(v.y); o[3] = bf_hi(v.y); }
+  __device__ __forceinline__ void clear() { v = make_uint2(0u, 0u); }
+};
+
+template <typename T, int NV, int NB>
+__global__ void __launch_bounds__(256) sum_norm_row_kernel(const evo_sum_norm_params p) {
+  __shared__ __align__(16) float red[4][8];
+  const int64_t r = blockIdx.x;
+  const int64_t src = p.gather ? p.gather[r] : r;
+  const int D = p.D, c0 = threadIdx.x * 4;
+  float* xr = p.x + src * D;
+  float v[NV][4];
+  Raw4<T> y[NB > 0 ? NB : 1][NV];                         // packed: more rows fit an SM
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = c0 + i * 1024;
+    if (c < D) {
+      Vec4<float>::load(xr + c, v[i]);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) y[b][i].load((const T*)p.y[b] + src * p.ldy[b] + c);
+    } else {
+      v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0.f;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) y[b][i].clear();
+    }
+  }
+  float rstd[NB > 0 ? NB : 1];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    rstd[b] = 1.f;
+    if (p.norm_w[b]) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) { float q[4]; y[b][i].get(q); ss = fmaf(q[0], q[0], fmaf(q[1], q[1], fmaf(q[2], q[2], fmaf(q[3], q[3], ss)))); }
+      rstd[b] = 1.0f / sqrtf(cta_sum(ss, red[b]) / (float)D + p.eps);
+    }
+  }
+  const bf16* cs = (const bf16*)p.col_scale;
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = c0 + i * 1024;
+    if (c < D) {
+      float add[4] = {0.f, 0.f, 0.f, 0.f}, cw[4];
+      if (cs) Vec4<bf16>::load(cs + c, cw);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        float q[4], w[4];
+        y[b][i].get(q);
+        if (p.norm_w[b]) {
+          Vec4<bf16>::load((const bf16*)p.norm_w[b] + c, w);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) q[u] = q[u] * rstd[b] * w[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add[u] = fmaf(p.scale[b], q[u], add[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (NB > 0) v[i][u] = cs ? fmaf(cw[u], add[u], v[i][u]) : v[i][u] + add[u];
+        ss = fmaf(v[i][u], v[i][u], ss);
+      }
+      if (NB > 0 && !p.gather) Vec4<float>::store(xr + c, v[i]);
+    }
+  }
+  if (!p.out[0] && !p.out[1]) return;
+  const float rs = 1.0f / sqrtf(cta_sum(ss, red[3]) / (float)D + p.eps);
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    if (!p.out[n]) continue;
+    T* o = (T*)p.out[n] + r * p.ldo;
+    const bf16* w = (const bf16*)p.w[n];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = c0 + i * 1024;
+      if (c < D) {
+        float wv[4], q[4];
+        Vec4<bf16>::load(w + c, wv);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = v[i][u] * rs * wv[u];
+        Vec4<T>::store(o + c, q);
+      }
+    }
+    for (int64_t c = D + c0; c < p.ldo; c += 1024) { const float z[4] = {0.f, 0.f, 0.f, 0.f}; Vec4<T>::store(o + c, z); }      // D and ldo are multiples of four
+  }
+}
+
+// ---- evo_conv_act: a thread owns one channel of one sequence over RT consecutive rows, its last taps inputs in registers
+constexpr int CONV_RT = 32, CONV_MAX_TAPS = 8, CONV_NB = 4;
+
+// silu for rows stored as bf16: one 2^x and one reciprocal (the special-function pipe's 8 cycles each per warp are what bounds an element; IEEE division and expf
+// took some thirty instructions).  Their errors, below 2^-20 of the result, vanish in its rounding to 8 bits; 1 / (1 + inf) is 0.
+template <typename T> __device__ __forceinline__ float silu_row(float v) { return silu_f(v); }
+template <> __device__ __forceinline__ float silu_row<bf16>(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-v)));
+  return v * r;
+}
+
+// four channels per thread (8- or 16-byte accesses), taps known at compile time.  Bound by memory: 4 x 4096 rows of 6144 bf16 channels, 4 taps, SiLU take 87 us =
+// 4.6 TB/s (168 with one row in flight and IEEE SiLU; 4 + 4 rows in flight beat 8 + 8, whose 118 registers halve the warps per SM: 105)
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) conv_act4_kernel(evo_conv_act_params p, int write_carry) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -164,12 +284,19 @@ __global__ void __launch_bounds__(128) conv_act4_kernel(evo_conv_act_params p, i
   const int64_t t0 = (int64_t)blockIdx.y * CONV_RT, t1 = min(p.L, t0 + CONV_RT);
   const T* in = (const T*)p.in + (int64_t)b * p.L * p.ld + c;
   float* carry = p.carry ? p.carry + (int64_t)b * HALO * p.C + c : nullptr;
-  float w[4][TAPS], win[HALO > 0 ? HALO : 1][4], bias[4] = {0.f, 0.f, 0.f, 0.f};
+  float2 w[2][TAPS];                                      // channel pairs: one packed multiply-add serves two channels
+  float win[HALO > 0 ? HALO : 1][4], bias[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) w[u][j] = __bfloat162float(((const bf16*)p.weight)[(int64_t)(c + u) * TAPS + j]);
+    for (int j = 0; j < TAPS; ++j)
+      w[u][j] = make_float2(__bfloat162float(((const bf16*)p.weight)[(int64_t)(c + 2 * u) * TAPS + j]), __bfloat162float(((const bf16*)p.weight)[(int64_t)(c + 2 * u + 1) * TAPS + j]));
   if (p.bias) Vec4<bf16>::load((const bf16*)p.bias + c, bias);
+  // rows travel packed, as they lie in memory: CONV_NB in work, CONV_NB under way (one row at a time left a single load in flight per thread)
+  Raw4<T> rows[CONV_NB], next[CONV_NB];
+#pragma unroll
+  for (int i = 0; i < CONV_NB; ++i)
+    if (t0 + i < t1) rows[i].load(in + (t0 + i) * p.ld);
 #pragma unroll
   for (int j = 0; j < HALO; ++j) {
     const int64_t s = t0 - HALO + j;
@@ -177,25 +304,38 @@ __global__ void __launch_bounds__(128) conv_act4_kernel(evo_conv_act_params p, i
     if (s >= 0) Vec4<T>::load(in + s * p.ld, win[j]);
     else if (carry && !p.zero_start) Vec4<float>::load(carry + (int64_t)(HALO + s) * p.C, win[j]);
   }
-  for (int64_t t = t0; t < t1; ++t) {
-    float cur[4], acc[4];
-    Vec4<T>::load(in + t * p.ld, cur);
+  T* out = (T*)p.out + (int64_t)b * p.L * p.ldo + c;
+  for (int64_t tb = t0; tb < t1; tb += CONV_NB) {
+    // the next rows are under way while these are worked on
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      float a = fmaf(w[u][HALO], cur[u], bias[u]);
+    for (int i = 0; i < CONV_NB; ++i)
+      if (tb + CONV_NB + i < t1) next[i].load(in + (tb + CONV_NB + i) * p.ld);
 #pragma unroll
-      for (int j = 0; j < HALO; ++j) a = fmaf(w[u][j], win[j][u], a);
-      acc[u] = p.act == 1 ? silu_f(a) : a;
+    for (int i = 0; i < CONV_NB; ++i) {
+      if (tb + i < t1) {
+        float cur[4], acc[4];
+        rows[i].get(cur);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float2 a = __ffma2_rn(w[u][HALO], make_float2(cur[2 * u], cur[2 * u + 1]), make_float2(bias[2 * u], bias[2 * u + 1]));
+#pragma unroll
+          for (int j = 0; j < HALO; ++j) a = __ffma2_rn(w[u][j], make_float2(win[j][2 * u], win[j][2 * u + 1]), a);
+          acc[2 * u] = p.act == 1 ? silu_row<T>(a.x) : a.x;
+          acc[2 * u + 1] = p.act == 1 ? silu_row<T>(a.y) : a.y;
+        }
+        Vec4<T>::store(out + (tb + i) * p.ldo, acc);
+#pragma unroll
+        for (int j = 0; j + 1 < HALO; ++j)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) win[j][u] = win[j + 1][u];
+        if (HALO > 0) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) win[HALO - 1][u] = cur[u];
+        }
+      }
     }
-    Vec4<T>::store((T*)p.out + ((int64_t)b * p.L + t) * p.ldo + c, acc);
 #pragma unroll
-    for (int j = 0; j + 1 < HALO; ++j)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) win[j][u] = win[j + 1][u];
-    if (HALO > 0) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) win[HALO - 1][u] = cur[u];
-    }
+    for (int i = 0; i < CONV_NB; ++i) rows[i] = next[i];
   }
   if (write_carry && carry && t1 == p.L) {
 #pragma unroll
@@ -390,6 +530,20 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
   vec = vec && (!p->col_scale || aligned4<bf16>(p->col_scale));
   for (int n = 0; n < 2; ++n)
     if (p->out[n]) vec = vec && aligned4<bf16>(p->w[n]) && (p->dtype ? aligned4<float>(p->out[n]) : aligned4<bf16>(p->out[n]));
+  if (vec && p->D <= 4096 && p->n_branches <= 3) {
+    // rows in registers: (groups of four per thread) x (branches)
+#define EVO_SUM_NORM(TT, NV) \
+    switch (p->n_branches) { \
+      case 0: sum_norm_row_kernel<TT, NV, 0><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
+      case 1: sum_norm_row_kernel<TT, NV, 1><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
+      case 2: sum_norm_row_kernel<TT, NV, 2><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
+      default: sum_norm_row_kernel<TT, NV, 3><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
+    }
+    if (p->dtype) { if (p->D <= 1024) { EVO_SUM_NORM(float, 1) } else if (p->D <= 2048) { EVO_SUM_NORM(float, 2) } else { EVO_SUM_NORM(float, 4) } }
+    else { if (p->D <= 1024) { EVO_SUM_NORM(bf16, 1) } else if (p->D <= 2048) { EVO_SUM_NORM(bf16, 2) } else { EVO_SUM_NORM(bf16, 4) } }
+#undef EVO_SUM_NORM
+    return check_launch("evo_sum_norm");
+  }
   auto kern = p->dtype ? (vec ? sum_norm_kernel<float, true> : sum_norm_kernel<float, false>) : (vec ? sum_norm_kernel<bf16, true> : sum_norm_kernel<bf16, false>);
   if (smem > 48 * 1024) EVO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<(unsigned)p->rows, 256, smem, st>>>(*p);
@@ -403,8 +557,9 @@ extern "C" int evo_conv_act(const evo_conv_act_params* p, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const unsigned chunks = (unsigned)((p->L + CONV_RT - 1) / CONV_RT);
   const dim3 grid((p->C + 127) / 128, chunks, p->B);
-  // with one thread per (sequence, channel) that thread reads the carried inputs before it replaces them; otherwise a second launch does
-  const int own = chunks == 1;
+  // with one thread per (sequence, channel) that thread reads the carried inputs before it replaces them, and where none are read (zero_start) the thread of the last
+  // rows may replace them; otherwise a second launch does
+  const int own = chunks == 1 || p->zero_start;
   const bool vec = p->C % 4 == 0 && p->ld % 4 == 0 && p->ldo % 4 == 0 && p->taps <= 4 && (!p->carry || ((uintptr_t)p->carry & 15) == 0) &&
                    (!p->bias || aligned4<bf16>(p->bias)) &&
                    (p->dtype ? aligned4<float>(p->in) && aligned4<float>(p->out) : aligned4<bf16>(p->in) && aligned4<bf16>(p->out));
