@@ -18,6 +18,7 @@
 //   of holding the row in registers (0.50-0.57 PFLOP/s: tcgen05.ld bandwidth), a degree-3 FMA-pipe exp2 for half of
 //   the scores (0.82-0.96: issue slots, not MUFU, bind), 64-key tiles with double-buffered S (0.65-0.76).
 #include "common.cuh"
+#include <algorithm>
 #include "../../include/evo_b200.h"
 
 using namespace evo;
@@ -39,6 +40,7 @@ struct Args {
   long long Lq, Lk, q_pos0;
   float scale_log2;
   int n_qblk;
+  int tail;             // the last (head, sequence) pairs, worked through together
 };
 
 __device__ __forceinline__ float ex2(float x) { float y; asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -101,8 +103,10 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pair = (a.n_qblk + 1) / 2 - 1 - (int)blockIdx.x;       // longest pairs first
-  const int h = blockIdx.y, b = blockIdx.z;
+  // (head, sequence) by (head, sequence), its longest query pair first; the last `tail` of them together, the longest pairs of all first (see the launcher)
+  const int pairs = (a.n_qblk + 1) / 2, bulk = (a.B * a.H - a.tail) * pairs, i = (int)blockIdx.x;
+  const int pair = pairs - 1 - (i < bulk ? i % pairs : (i - bulk) / a.tail), hb = i < bulk ? i / pairs : a.B * a.H - a.tail + (i - bulk) % a.tail;
+  const int h = hb % a.H, b = hb / a.H;
   long long q0[2];
   int n_kv[2];
 #pragma unroll
@@ -333,7 +337,12 @@ int evo_attn_pp_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUt
                 "evo_attn_fwd: peer-scattered output needs B == 1, 1..8 peers covering Lq rows, 16-byte aligned strides");
   }
   static unsigned long long done0 = 0, done3 = 0;
-  dim3 grid((unsigned)((a.n_qblk + 1) / 2), p->H, p->B);
+  // Head after head shares keys and values best, but the last head's longest CTAs would start when everything else is done (1 x 8193 tokens x 32 heads: 593 us, with
+  // the last heads taken together 533; 2 x 2325 x 16: 87 / 70; 8 x 8193 x 32 gains nothing).  As many heads as keep their keys and values in half the L2 (64 MB).
+  const long long heads = (long long)p->B * p->H, pairs = (a.n_qblk + 1) / 2;
+  a.tail = (int)std::min(heads, std::max<long long>(1, (64ll << 20) / std::max<long long>(1, p->Lk * 512)));
+  EVO_REQUIRE(heads * pairs < (1ll << 31), "evo_attn_fwd: too many blocks");
+  dim3 grid((unsigned)(heads * pairs));
   if (npoly == 0) {
     { int rc_ = ensure_dyn_smem(attn_pp_kernel<0>, SMEM, done0); if (rc_) return rc_; }
     attn_pp_kernel<0><<<grid, THREADS, SMEM, st>>>(tmQ, tmK, tmV, a);
