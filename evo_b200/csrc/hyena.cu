@@ -319,7 +319,7 @@ struct HyenaPlan { bool tc; int R, nseg; long long seg_len; };
 
 // The tensor-core path does the work of 256 R tokens x 32 channels per tile and item in a time that hardly depends on how many of the tokens exist, and computes its
 // constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 64: scan 14.9, tensor
-// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 46; 4 x 1000: 123 / 78; 8 x 300: 44 / 76; 8 x 8193: 953 / 832.  The smaller estimate decides; both sides are in us.
+// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 44; 4 x 1000: 123 / 76; 8 x 300: 44 / 76; 8 x 8193: 953 / 811.  The smaller estimate decides; both sides are in us.
 // Few items (narrow models, one sequence) are cut into segments: a pass over x1 and v then finds the states between them, at about half the price of the output pass.
 HyenaPlan make_plan(const evo_hyena_params* p) {
   const long long L = p->L;
@@ -330,7 +330,7 @@ HyenaPlan make_plan(const evo_hyena_params* p) {
   const char* env_v = getenv("EVO_B200_HYENA_VARIANT");      // comparisons: 0, 1 = the modal scans, 2 = tensor cores; read per call
   const int variant = env_v ? atoi(env_v) : -1;
   // taps, biases and carried inputs are read four channels at a time
-  const bool can = use_tma_path(p) && (((uintptr_t)p->fir_w | (uintptr_t)p->fir_b | (uintptr_t)p->halo) & 7) == 0;
+  const bool can = use_tma_path(p) && L < (1ll << 30) && (((uintptr_t)p->fir_w | (uintptr_t)p->fir_b | (uintptr_t)p->halo) & 7) == 0;
   if (!can || variant == 0 || variant == 1) return best;
   const long long scan_ctas = (long long)p->D / evo_hy2::CH_PER_CTA * p->B * best.nseg;
   double cost = variant == 2 ? 1e30 : 7.0 + 0.116 * best.seg_len * (best.nseg > 1 ? 1.6 : std::max(1.0, (double)scan_ctas / sms));

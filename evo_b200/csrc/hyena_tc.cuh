@@ -16,9 +16,10 @@
 //                      steps with powers p^{16R}, p^{32R}, p^{64R}); then every block's c, rounded, + D x, back into the place of x
 // The fragment layouts of A operands and sums agree (a lane owns 4 consecutive tokens of rows g and g + 8), so B needs no shuffle besides the fold.
 // z is read once and y written once.
-// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 832 us (modal scan on the CUDA cores 953), 1 x 1999 46 us (138), 4 x 1000 78 us (123), 1 x 301 23 us (42).
+// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 811 us (modal scan on the CUDA cores 953), 1 x 1999 44 us (138), 4 x 1000 76 us (123), 1 x 301 23 us (42).
 // A steady tile of 1024 tokens takes 24.5 k cycles, all of them the tensor-core warps' (tensor pipe 6.7 k, fp32 pipe 9 k, issue 10 k per scheduler): bound by the
-// latencies of its dependent steps with two such warps per scheduler; the element-wise warps are busy for 19 k of them.
+// latencies of its dependent steps with two such warps per scheduler (5.6 cycles per instruction each; issue slots 56 % used).  Register shares of 128 / 88 or 136 / 80
+// are 2 - 3 % slower: the element-wise warps then spill.
 // A channel whose x or state is not finite (or beyond 1e30), or whose poles lie so far outside the unit circle that their powers are not, goes
 // token by token in that tile: a product with a structural zero would otherwise carry an infinity to earlier tokens of its block.
 #pragma once
@@ -181,25 +182,36 @@ template <int R> __device__ __forceinline__ uint32_t cell(int c, int row, int gr
   return (uint32_t)c * (ROWS * BLK * 2 * R) + (uint32_t)(((row * 2 * R + gran) ^ ((c >> 2) & 7) ^ rs) << 4);
 }
 
+__device__ __forceinline__ void lds64(uint32_t& a, uint32_t& b, uint32_t addr) { asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr)); }
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) { asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(addr), "r"(a), "r"(b) : "memory"); }
 __device__ __forceinline__ uint2 ldg64(const bf16* p) { return __ldg(reinterpret_cast<const uint2*>(p)); }
-// three taps of four channels (24 consecutive bytes) as two channel pairs
-struct Taps { float2 w[2][3]; uint2 bias; };
+// three taps of four channels (24 consecutive bytes) as two channel pairs, kept as they are stored: [pair][tap] packed, and the biases
+struct Taps { uint32_t w[2][3]; uint2 bias; };
 __device__ __forceinline__ Taps load_taps(const bf16* fir_w, const bf16* fir_b, int col) {
   const uint2* f = reinterpret_cast<const uint2*>(fir_w + 3LL * col);
   const uint2 q0 = __ldg(f), q1 = __ldg(f + 1), q2 = __ldg(f + 2);
-  const float2 e[6] = {up2(q0.x), up2(q0.y), up2(q1.x), up2(q1.y), up2(q2.x), up2(q2.y)};   // channel 0 taps 0 1 | 2, channel 1 tap 0 | 1 2 | ...
+  const uint32_t e[6] = {q0.x, q0.y, q1.x, q1.y, q2.x, q2.y};           // channel 0 taps 0 1 | tap 2, channel 1 tap 0 | taps 1 2 | ..
   Taps t;
-  t.w[0][0] = make_float2(e[0].x, e[1].y); t.w[0][1] = make_float2(e[0].y, e[2].x); t.w[0][2] = make_float2(e[1].x, e[2].y);
-  t.w[1][0] = make_float2(e[3].x, e[4].y); t.w[1][1] = make_float2(e[3].y, e[5].x); t.w[1][2] = make_float2(e[4].x, e[5].y);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    t.w[u][0] = __byte_perm(e[3 * u], e[3 * u + 1], 0x7610);
+    t.w[u][1] = __byte_perm(e[3 * u], e[3 * u + 2], 0x5432);
+    t.w[u][2] = __byte_perm(e[3 * u + 1], e[3 * u + 2], 0x7610);
+  }
   t.bias = ldg64(fir_b + col);
   return t;
 }
-// short FIR of one channel pair (fp32 accumulate, rounded) + bias (rounded); h = the two inputs before
-__device__ __forceinline__ uint32_t fir(const float2 (&w)[3], float2 (&h)[2], uint32_t zq, uint32_t bias) {
-  const float2 z = up2(zq);
-  const float2 acc = __ffma2_rn(w[2], z, __ffma2_rn(w[1], h[1], __fmul2_rn(w[0], h[0])));
-  h[0] = h[1]; h[1] = z;
-  return addbf(pack_bf16(acc.x, acc.y), bias);
+// short FIR (fp32 accumulate, rounded) + bias (rounded) of one channel pair: eight tokens from ten raw rows; take(e, f) gets each result
+template <typename F> __device__ __forceinline__ void fir8(const uint32_t (&wq)[3], uint32_t bias, const uint32_t (&z)[10], F take) {
+  const float2 w0 = up2(wq[0]), w1 = up2(wq[1]), w2 = up2(wq[2]);
+  float2 h0 = up2(z[0]), h1 = up2(z[1]);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float2 c = up2(z[e + 2]);
+    const float2 acc = __ffma2_rn(w2, c, __ffma2_rn(w1, h1, __fmul2_rn(w0, h0)));
+    h0 = h1; h1 = c;
+    take(e, addbf(pack_bf16(acc.x, acc.y), bias));
+  }
 }
 
 // an mbarrier wait with a limit: a wait that runs out is counted, and the role that gave up ends
@@ -213,13 +225,12 @@ __device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity) 
 
 // position in the sequence of tiles that a CTA walks: its items (channel block, batch row, segment), tile by tile
 struct Walk {
-  int item, k, n_tiles, b, seg, ch0;
-  long long t0, t1;
+  int item, k, n_tiles, b, seg, ch0, t0, t1;                            // (tokens of a sequence are counted in 32 bits: copy coordinates are)
   __device__ __forceinline__ void open(const Args& a, int tile) {
     const int ncb = a.D / CH;
     ch0 = (item % ncb) * CH; b = (item / ncb) % a.B; seg = item / (ncb * a.B);
-    t0 = (long long)seg * a.seg_len; t1 = min(a.L, t0 + a.seg_len);
-    n_tiles = (int)((t1 - t0 + tile - 1) / tile);
+    t0 = seg * (int)a.seg_len; t1 = min((int)a.L, t0 + (int)a.seg_len);
+    n_tiles = (t1 - t0 + tile - 1) / tile;
     k = 0;
   }
   __device__ __forceinline__ bool more(const Args& a) const { return item < a.items; }
@@ -228,8 +239,13 @@ struct Walk {
     item += gridDim.x;
     if (item < a.items) open(a, tile);
   }
-  __device__ __forceinline__ long long first(int tile) const { return t0 + (long long)k * tile; }
-  __device__ __forceinline__ int tokens(int tile) const { return (int)min((long long)tile, t1 - first(tile)); }
+  __device__ __forceinline__ int first(int tile) const { return t0 + k * tile; }
+  __device__ __forceinline__ int tokens(int tile) const { return min(tile, t1 - first(tile)); }
+};
+// what the second phase of a tile has to know of it
+struct Tile {
+  int first, n, b, ch0;
+  __device__ __forceinline__ void of(const Walk& w, int tile) { first = w.first(tile); n = w.tokens(tile); b = w.b; ch0 = w.ch0; }
 };
 
 template <int R, bool STATE_ONLY>
@@ -267,26 +283,26 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
       tma_prefetch_desc(&tmZ);
       uint32_t s = 0;                                                   // running slot number
       bool ok = true;
-      auto put = [&](int col, long long t, int b) {
+      auto put = [&](int col, int t, int b) {
         const uint32_t i = s % SLOTS, round = s / SLOTS;
         if (ok && round > 0) ok = wait_or_give_up(&zempty[i], (round - 1) & 1);
         if (ok) {
           mbar_arrive_expect_tx(&zfull[i], SLOT_BYTES);
-          tma_load_3d(ring + i * SLOT_BYTES, &tmZ, &zfull[i], col, (int)t - 2, b);
+          tma_load_3d(ring + i * SLOT_BYTES, &tmZ, &zfull[i], col, t - 2, b);
           ++s;
         }
       };
-      auto column = [&](const Walk& v, int sig) { return (v.ch0 / HD) * 3 * HD + v.ch0 % HD + sig * HD; };
-      Walk p = w;
+      auto column = [&](int ch0, int sig) { return (ch0 / HD) * 3 * HD + ch0 % HD + sig * HD; };
+      Tile p;
+      p.of(w, TILE);
       bool any = false;
       while (ok && (w.more(a) || any)) {
         if (w.more(a))
-          for (int i = 0; i * STAGE < w.tokens(TILE); ++i) { put(column(w, 1), w.first(TILE) + i * STAGE, w.b); put(column(w, 2), w.first(TILE) + i * STAGE, w.b); }
+          for (int i = 0; i * STAGE < w.tokens(TILE); ++i) { put(column(w.ch0, 1), w.first(TILE) + i * STAGE, w.b); put(column(w.ch0, 2), w.first(TILE) + i * STAGE, w.b); }
         if (!STATE_ONLY && any)
-          for (int i = 0; i * STAGE < p.tokens(TILE); ++i) put(column(p, 0), p.first(TILE) + i * STAGE, p.b);
+          for (int i = 0; i * STAGE < p.n; ++i) put(column(p.ch0, 0), p.first + i * STAGE, p.b);
         any = w.more(a);
-        p = w;
-        if (any) w.next(a, TILE);
+        if (any) { p.of(w, TILE); w.next(a, TILE); }
       }
       // the copies still in flight land before this thread ends
       for (uint32_t q = s > SLOTS ? s - SLOTS : 0; q < s; ++q) wait_or_give_up(&zfull[q % SLOTS], (q / SLOTS) & 1);
@@ -302,56 +318,47 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
     uint32_t s = 0;                                                     // running slot number (both groups count all slots)
     uint32_t q = 0;                                                     // running tile number
     bool ok = true, any = false;
-    Walk p = w;
-    // 10 raw rows of this thread's run from slot s: two before it
-    auto rows = [&](uint32_t slot, uint2 (&z)[10]) {
-      const uint8_t* src = ring + (slot % SLOTS) * SLOT_BYTES + run * 8 * (CH * 2) + quad * 8;
+    Tile p;
+    p.of(w, TILE);
+    // ten raw rows of this thread's run from slot s, the first two in front of it, as two channel pairs; the slot is then free
+    auto rows = [&](uint32_t slot, int t, int b, int col, uint32_t (&z)[2][10]) {
+      const uint32_t i = slot % SLOTS;
+      ok = ok && wait_or_give_up(&zfull[i], (slot / SLOTS) & 1);
+      const uint8_t* src = ring + i * SLOT_BYTES + run * 8 * (CH * 2) + quad * 8;
 #pragma unroll
-      for (int i = 0; i < 10; ++i) z[i] = *reinterpret_cast<const uint2*>(src + i * (CH * 2));
-    };
-    auto release = [&](uint32_t slot) { if (lane == 0) mbar_arrive(&zempty[slot % SLOTS]); };
-    // the rows in front of a sequence's first token: the carried inputs (the copy filled in zeros)
-    auto carried = [&](const Walk& v, long long t, int col, uint2 (&z)[10]) {
+      for (int e = 0; e < 10; ++e) { const uint2 v = *reinterpret_cast<const uint2*>(src + e * (CH * 2)); z[0][e] = v.x; z[1][e] = v.y; }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&zempty[i]);
       if (t < 2 && a.halo) {
-        const bf16* h = a.halo + (long long)v.b * 2 * 3 * a.D + col;
-        z[0] = ldg64(h + t * 3 * a.D);
-        if (t == 0) z[1] = ldg64(h + 3LL * a.D);
+        // in front of a sequence's first token: the carried inputs (the copy filled in zeros)
+        const bf16* h = a.halo + (long long)b * 2 * 3 * a.D + col;
+        const uint2 v = ldg64(h + t * 3LL * a.D);
+        z[0][0] = v.x; z[1][0] = v.y;
+        if (t == 0) { const uint2 u = ldg64(h + 3LL * a.D); z[0][1] = u.x; z[1][1] = u.y; }
       }
     };
     while (ok && (w.more(a) || any)) {
       if (w.more(a)) {
         // ---------------- A: x1 * v of tile q
         const int n = w.tokens(TILE), ns = (n + STAGE - 1) / STAGE, ch = w.ch0 + 4 * quad, zc = (ch / HD) * 3 * HD + ch % HD;
-        const Taps w1 = load_taps(a.fir_w, a.fir_b, zc + HD), wv = load_taps(a.fir_w, a.fir_b, zc + 2 * HD);
         uint8_t* xs = xbuf + (q & 1) * (CH * TILE * 2);
 #pragma unroll 1
         for (int i = group; i < TILE / STAGE; i += 2) {
           const int gran = i * (STAGE / 8) + run, row = gran / (2 * R), gr = gran % (2 * R);
           uint32_t x[2][8];
           if (i < ns) {
-            const uint32_t sl = s + 2 * i;
-            const long long t = w.first(TILE) + gran * 8;
-            uint2 z[10];
-            ok = ok && wait_or_give_up(&zfull[sl % SLOTS], (sl / SLOTS) & 1);
-            rows(sl, z);
-            __syncwarp();
-            release(sl);
-            carried(w, t, zc + HD, z);
+            const int t = w.first(TILE) + gran * 8;
+            uint32_t z[2][10];
             {
-              float2 h[2][2] = {{up2(z[0].x), up2(z[1].x)}, {up2(z[0].y), up2(z[1].y)}};
-#pragma unroll
-              for (int e = 0; e < 8; ++e) { x[0][e] = fir(w1.w[0], h[0], z[e + 2].x, w1.bias.x); x[1][e] = fir(w1.w[1], h[1], z[e + 2].y, w1.bias.y); }
+              const Taps w1 = load_taps(a.fir_w, a.fir_b, zc + HD);       // (from L1; kept over the stages they would not fit the registers)
+              rows(s + 2 * i, t, w.b, zc + HD, z);
+              fir8(w1.w[0], w1.bias.x, z[0], [&](int e, uint32_t f) { x[0][e] = f; });
+              fir8(w1.w[1], w1.bias.y, z[1], [&](int e, uint32_t f) { x[1][e] = f; });
             }
-            ok = ok && wait_or_give_up(&zfull[(sl + 1) % SLOTS], ((sl + 1) / SLOTS) & 1);
-            rows(sl + 1, z);
-            __syncwarp();
-            release(sl + 1);
-            carried(w, t, zc + 2 * HD, z);
-            {
-              float2 h[2][2] = {{up2(z[0].x), up2(z[1].x)}, {up2(z[0].y), up2(z[1].y)}};
-#pragma unroll
-              for (int e = 0; e < 8; ++e) { x[0][e] = mulbf(x[0][e], fir(wv.w[0], h[0], z[e + 2].x, wv.bias.x)); x[1][e] = mulbf(x[1][e], fir(wv.w[1], h[1], z[e + 2].y, wv.bias.y)); }
-            }
+            const Taps wv = load_taps(a.fir_w, a.fir_b, zc + 2 * HD);
+            rows(s + 2 * i + 1, t, w.b, zc + 2 * HD, z);
+            fir8(wv.w[0], wv.bias.x, z[0], [&](int e, uint32_t f) { x[0][e] = mulbf(x[0][e], f); });
+            fir8(wv.w[1], wv.bias.y, z[1], [&](int e, uint32_t f) { x[1][e] = mulbf(x[1][e], f); });
             if (n < TILE) {
 #pragma unroll
               for (int e = 0; e < 8; ++e) if (gran * 8 + e >= n) x[0][e] = x[1][e] = 0u;
@@ -376,51 +383,36 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
         // ---------------- C: tile q - 1, (convolution + D x) * x2.  The cells are this thread's own: A of tile q + 1 may refill them afterwards
         ok = ok && wait_or_give_up(&xdone[(q - 1) & 1], ((q - 1) >> 1) & 1);
         if (!STATE_ONLY) {
-          const int n = p.tokens(TILE), ns = (n + STAGE - 1) / STAGE, ch = p.ch0 + 4 * quad, zc = (ch / HD) * 3 * HD + ch % HD;
-          const Taps w2 = load_taps(a.fir_w, a.fir_b, zc);
+          const int ns = (p.n + STAGE - 1) / STAGE, ch = p.ch0 + 4 * quad, zc = (ch / HD) * 3 * HD + ch % HD;
           const uint8_t* xs = xbuf + ((q - 1) & 1) * (CH * TILE * 2);
 #pragma unroll 1
           for (int i = group; i < ns; i += 2) {
             const int gran = i * (STAGE / 8) + run, row = gran / (2 * R), gr = gran % (2 * R);
-            uint2 z2[10];
-            const uint32_t sl = s + i;
-            ok = ok && wait_or_give_up(&zfull[sl % SLOTS], (sl / SLOTS) & 1);
-            rows(sl, z2);
-            __syncwarp();
-            release(sl);
-            const long long t = p.first(TILE) + gran * 8;
-            carried(p, t, zc, z2);
-            uint32_t u[4][4];
+            const int t = p.first + gran * 8, left = p.n - gran * 8;
+            uint32_t z[2][10], o[2][8];
+            const Taps w2 = load_taps(a.fir_w, a.fir_b, zc);
+            rows(s + i, t, p.b, zc, z);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const uint4 f = *reinterpret_cast<const uint4*>(xs + cell<R>(4 * quad + v, row, gr));
-              u[v][0] = f.x; u[v][1] = f.y; u[v][2] = f.z; u[v][3] = f.w;
+            for (int v = 0; v < 2; ++v) {
+              const uint4 lo = *reinterpret_cast<const uint4*>(xs + cell<R>(4 * quad + 2 * v, row, gr)), hi = *reinterpret_cast<const uint4*>(xs + cell<R>(4 * quad + 2 * v + 1, row, gr));
+              const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, h[4] = {hi.x, hi.y, hi.z, hi.w};
+              fir8(w2.w[v], v ? w2.bias.y : w2.bias.x, z[v], [&](int e, uint32_t f) { o[v][e] = mulbf(__byte_perm(l[e >> 1], h[e >> 1], (e & 1) ? 0x7632 : 0x5410), f); });
             }
             bf16* yr = a.y + ((long long)p.b * a.L + t) * a.D + ch;
-            float2 h2[2][2] = {{up2(z2[0].x), up2(z2[1].x)}, {up2(z2[0].y), up2(z2[1].y)}};
-            const int left = n - gran * 8;
-            uint2 o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const uint32_t sel = (e & 1) ? 0x7632 : 0x5410;
-              o[e] = make_uint2(mulbf(__byte_perm(u[0][e >> 1], u[1][e >> 1], sel), fir(w2.w[0], h2[0], z2[e + 2].x, w2.bias.x)),
-                                mulbf(__byte_perm(u[2][e >> 1], u[3][e >> 1], sel), fir(w2.w[1], h2[1], z2[e + 2].y, w2.bias.y)));
-            }
             if (left >= 8 && a.y_wide) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) *reinterpret_cast<uint2*>(yr + (long long)e * a.D) = o[e];
+              for (int e = 0; e < 8; ++e) *reinterpret_cast<uint2*>(yr + (long long)e * a.D) = make_uint2(o[0][e], o[1][e]);
             } else {
 #pragma unroll
               for (int e = 0; e < 8; ++e)
-                if (e < left) { uint32_t* d = reinterpret_cast<uint32_t*>(yr + (long long)e * a.D); d[0] = o[e].x; d[1] = o[e].y; }
+                if (e < left) { uint32_t* d = reinterpret_cast<uint32_t*>(yr + (long long)e * a.D); d[0] = o[0][e]; d[1] = o[1][e]; }
             }
           }
           s += ns;
         }
       }
       any = w.more(a);
-      p = w;
-      if (any) { w.next(a, TILE); ++q; }
+      if (any) { p.of(w, TILE); w.next(a, TILE); ++q; }
     }
     return;
   }
@@ -458,21 +450,20 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
       carry[c * NS + m] = S;
       __syncwarp();
     }
-    Walk after = w;
-    after.next(a, TILE);
-    const int ch_after = after.more(a) ? after.ch0 : w.ch0;
     uint8_t* xs = xbuf + (q & 1) * (CH * TILE * 2);
     if (!wait_or_give_up(&xfull[q & 1], (q >> 1) & 1)) break;
 #pragma unroll 1
     for (int c = warp; c < CH; c += MMA_WARPS) {
       const int chg = w.ch0 + c;
       float2 E[R][2][2], F[2][2];                                      // [block][rows g | g + 8][mode tq | tq + 4]
+      const uint32_t dsk = STATE_ONLY ? 0u : (uint32_t)__bfloat16_as_ushort(a.Dskip[chg]) * 0x10001u;
       const float2 S0[2] = {carry[c * NS + tq], carry[c * NS + tq + 4]};
       const uint4* tab = reinterpret_cast<const uint4*>(slot) + lane;
       const float2* pw = reinterpret_cast<const float2*>(slot + TAB_WORDS * 128);
       uint32_t T[12], Q[12];
       float2 p16[2];
-      uint8_t* xc = xs + (tq & 1) * 8;
+      // the lane's 8 bytes of block 0 in rows g and g + 8; block j lies at the address with j in bits 5 and 6 exchanged (see cell())
+      const uint32_t x0 = smem_u32(xs) + (tq & 1) * 8 + cell<R>(c, g, tq >> 1), x8 = smem_u32(xs) + (tq & 1) * 8 + cell<R>(c, g + 8, tq >> 1);
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncwarp();
       bool calm = n > 16;                                              // a short rest costs less token by token
@@ -484,8 +475,8 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
           for (int i = 0; i < 3; ++i) { const uint4 t = tab[i * 32]; P[4 * i] = t.x; P[4 * i + 1] = t.y; P[4 * i + 2] = t.z; P[4 * i + 3] = t.w; }
 #pragma unroll
           for (int j = 0; j < R; ++j) {
-            const uint2 xa = *reinterpret_cast<const uint2*>(xc + cell<R>(c, g, 2 * j + (tq >> 1))), xb = *reinterpret_cast<const uint2*>(xc + cell<R>(c, g + 8, 2 * j + (tq >> 1)));
-            const uint32_t x[4] = {xa.x, xb.x, xa.y, xb.y};
+            uint32_t x[4];
+            lds64(x[0], x[2], x0 ^ (j << 5)); lds64(x[1], x[3], x8 ^ (j << 5));
             float e[2][4];
 #pragma unroll
             for (int sp = 2; sp >= 0; --sp)
@@ -502,19 +493,27 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             }
           }
         }
+        if (!STATE_ONLY) {                                             // (under way while the fold waits for its shuffles)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) { const uint4 t = tab[(3 + i) * 32]; T[4 * i] = t.x; T[4 * i + 1] = t.y; T[4 * i + 2] = t.z; T[4 * i + 3] = t.w; }
+#pragma unroll
+          for (int i = 0; i < 3; ++i) { const uint4 t = tab[(6 + i) * 32]; Q[4 * i] = t.x; Q[4 * i + 1] = t.y; Q[4 * i + 2] = t.z; Q[4 * i + 3] = t.w; }
+        }
         // ---- fold the rows: F[hf][.] becomes the state behind row g (+ 8), then the state in front of it
-        float2 S8[2];
+        float2 S8[2], po[3][2];
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1)
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            const float2 po = pw[o * NS + tq + 4 * nt];
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              const float2 u = shfl_up2(F[hf][nt], 4 * o);
-              if (g >= o) F[hf][nt] = cfma(po, u, F[hf][nt]);
-            }
+          for (int nt = 0; nt < 2; ++nt) {                             // a lane without a row that far in front adds nothing
+            po[i][nt] = pw[(1 << i) * NS + tq + 4 * nt];
+            if (g < (1 << i)) po[i][nt] = make_float2(0.f, 0.f);
           }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) F[hf][nt] = cfma(po[i][nt], shfl_up2(F[hf][nt], 4 << i), F[hf][nt]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float2 pg = pw[(g + 1) * NS + tq + 4 * nt];
@@ -533,21 +532,22 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             F[0][nt] = g ? u0 : S0[nt];
             F[1][nt] = g ? u1 : S8[nt];
           }
-          if (!STATE_ONLY) {
-#pragma unroll
-            for (int i = 0; i < 3; ++i) { const uint4 t = tab[(3 + i) * 32]; T[4 * i] = t.x; T[4 * i + 1] = t.y; T[4 * i + 2] = t.z; T[4 * i + 3] = t.w; }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) { const uint4 t = tab[(6 + i) * 32]; Q[4 * i] = t.x; Q[4 * i + 1] = t.y; Q[4 * i + 2] = t.z; Q[4 * i + 3] = t.w; }
-          }
         }
       }
       __syncwarp();
-      fetch(c + MMA_WARPS < CH ? chg + MMA_WARPS : ch_after + warp);   // (behind the warp's last channel: the first one of the next tile)
+      {
+        int nx = chg + MMA_WARPS;                                      // behind the warp's last channel: its first one of the next tile
+        if (c + MMA_WARPS >= CH) {
+          const int it = w.item + (int)gridDim.x;
+          nx = (w.k + 1 < w.n_tiles || it >= a.items ? w.ch0 : it % (a.D / CH) * CH) + warp;
+        }
+        fetch(nx);
+      }
       if (!calm) {
         // token by token: one mode per lane, four copies
         const int m = lane & 7;
         const float2 p = reinterpret_cast<const float2*>(a.poles)[(long long)chg * NS + m], r = reinterpret_cast<const float2*>(a.residues)[(long long)chg * NS + m];
-        const float dsk = __bfloat162float(a.Dskip[chg]);
+        const float skip = __bfloat162float(a.Dskip[chg]);
         float2 S = carry[c * NS + m];
 #pragma unroll 1
         for (int t = 0; t < n; ++t) {
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             float o = fmaf(r.x, S.x, -r.y * S.y);
 #pragma unroll
             for (int d = 1; d < 8; d <<= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
-            if (lane == 0) *xp = __float2bfloat16_rn(rbf(o) + rbf(x * dsk));
+            if (lane == 0) *xp = __float2bfloat16_rn(rbf(o) + rbf(x * skip));
           }
         }
         __syncwarp();
@@ -567,16 +567,13 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
         __syncwarp();
         continue;
       }
-      const uint32_t dsk = STATE_ONLY ? 0u : (uint32_t)__bfloat16_as_ushort(a.Dskip[chg]) * 0x10001u;
       const int fq = last ? n >> 4 : -1;                                // the segment's last block, if it ends within this tile
       if (lane == 0 && last) finm[c] = n & 15;
       if (!STATE_ONLY || last) {
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-          uint2* pa = reinterpret_cast<uint2*>(xc + cell<R>(c, g, 2 * j + (tq >> 1)));
-          uint2* pb = reinterpret_cast<uint2*>(xc + cell<R>(c, g + 8, 2 * j + (tq >> 1)));
-          const uint2 xa = *pa, xb = *pb;
-          const uint32_t x[4] = {xa.x, xb.x, xa.y, xb.y};
+          uint32_t x[4];
+          lds64(x[0], x[2], x0 ^ (j << 5)); lds64(x[1], x[3], x8 ^ (j << 5));
           if (last) {
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf)
@@ -610,8 +607,8 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
               for (int e = 0; e < 4; ++e) o[nt][e] += os[nt][e];
-            *pa = make_uint2(addbf(pack_bf16(o[0][0], o[0][1]), mulbf(x[0], dsk)), addbf(pack_bf16(o[1][0], o[1][1]), mulbf(x[2], dsk)));
-            *pb = make_uint2(addbf(pack_bf16(o[0][2], o[0][3]), mulbf(x[1], dsk)), addbf(pack_bf16(o[1][2], o[1][3]), mulbf(x[3], dsk)));
+            sts64(x0 ^ (j << 5), addbf(pack_bf16(o[0][0], o[0][1]), mulbf(x[0], dsk)), addbf(pack_bf16(o[1][0], o[1][1]), mulbf(x[2], dsk)));
+            sts64(x8 ^ (j << 5), addbf(pack_bf16(o[0][2], o[0][3]), mulbf(x[1], dsk)), addbf(pack_bf16(o[1][2], o[1][3]), mulbf(x[3], dsk)));
           }
           if (j + 1 < R) {
 #pragma unroll
@@ -641,7 +638,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
       }
       __syncwarp();
     }
-    w = after;
+    w.next(a, TILE);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
