@@ -13,7 +13,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libevo_b200.so")
 SOURCES = ["api.cu", "elementwise.cu", "hyena.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "attention.cu", "attention_pp.cu", "decode.cu", "scoring.cu", "sampler.cu", "ingest.cu", "die_map.cu",
-           "rowops.cu", "hgrn2.cu", "window_attention.cu", "window_attention_mma.cu", "gemm_simt.cu",
+           "rowops.cu", "hgrn2.cu", "window_attention.cu", "window_attention_mma.cu", "window_attention_tc.cu", "gemm_simt.cu",
            "mingru.cu", "latent_attention.cu", "moe.cu",
            "branch_ops.cu", "matrix_state.cu", "delta_block.cu", "attention_prep.cu", "post_norm.cu",
            "mixed_attention.cu", "linear_attention.cu"]

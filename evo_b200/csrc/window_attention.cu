@@ -19,6 +19,8 @@
 using namespace evo;
 
 namespace evo {
+bool window_attn_tc_takes(const evo_window_attn_params* p);                 // window_attention_tc.cu
+int window_attn_tc(const evo_window_attn_params* p, cudaStream_t st);
 int window_attn_mma(const evo_window_attn_params* p, cudaStream_t st);      // window_attention_mma.cu; 1 = shape not covered
 }
 
@@ -421,6 +423,7 @@ extern "C" int evo_window_attn_fwd(const evo_window_attn_params* p, void* stream
   cudaStream_t st = (cudaStream_t)stream;
   static const char* env_mma = getenv("EVO_B200_WINDOW_ATTN_MMA");      // "0": always the CUDA-core kernel (comparisons)
   if (!(env_mma && atoi(env_mma) == 0)) {
+    if (window_attn_tc_takes(p)) return window_attn_tc(p, st);
     const int rc = window_attn_mma(p, st);                              // bf16, two maps, >= 16 query rows, heads up to 128
     if (rc <= 0) return rc;
   }
