@@ -13,8 +13,9 @@
 //   place as an MN-major B operand.
 //   Issue order per KV tile j:  PV_A(j) QK_A(j+1) PV_B(j) QK_B(j+1): while softmax A(j+1) runs, the tensor
 //   pipe has PV_B(j) and QK_B(j+1) to do, and vice versa.
-//   Measured on B200 (profiles/): 0.89-1.07 PFLOP/s; tensor pipe 50 % active, softmax warps wait for S a third of
-//   the time (P aliases S, so QK(j+1) queues behind PV(j)).  Tried and rejected: a second TMEM pass over S instead
+//   The MMA warp stays converged and one lane issues: with a branch around the issuing code every product cost 90 to 130 cycles of
+//   operand moves (64 on the tensor pipe), and the softmax waited for them (1 x 8193 tokens x 32 heads 534 -> 491 us, 2 x 4096 294 -> 271).
+//   Measured on B200: 1.01-1.12 PFLOP/s from 4096 tokens on (P aliases S, so QK(j+1) queues behind PV(j)).  Tried and rejected: a second TMEM pass over S instead
 //   of holding the row in registers (0.50-0.57 PFLOP/s: tcgen05.ld bandwidth), a degree-3 FMA-pipe exp2 for half of
 //   the scores (0.82-0.96: issue slots, not MUFU, bind), 64-key tiles with double-buffered S (0.65-0.76).
 #include "common.cuh"
@@ -155,39 +156,44 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
     }
   } else if (warp == 9) {
-    // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------ MMA issuer: the whole warp waits, one lane issues; one copy of each product's loop (the softmax code fills the
+    // instruction cache: unrolled for two tiles and three places, this warp's fetches paced the kernel)
+    {
       constexpr uint32_t idesc_qk = umma_idesc_bf16(BQ, BKV);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(BQ, HD) | (1u << 16);     // B (= V) is MN-major
-      auto last_user = [&](int t, int j) { return t == 1 || j >= n_kv[1]; };  // tile B is the later tile: n_kv[1] >= n_kv[0] when valid
-      auto issue_qk = [&](int t, int j) {
-        const int st = j % KV_STAGES;
-        mbar_wait(&k_full[st], (uint32_t)(j / KV_STAGES) & 1);
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sQ + t * TILE_BYTES), ka = smem_u32(sK + st * TILE_BYTES);
+      const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc = umma_desc_k_sw128(smem_u32(sK)), v_desc = desc_mn_sw128(smem_u32(sV), HALF_BYTES, 1024);
+      const uint32_t lead = elect_one();
+#pragma unroll 1
+      for (int j = -1; j < n_kv_max; ++j) {
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {                                         // tile B is the later tile: n_kv[1] >= n_kv[0] when valid, and the last user of a K or V tile
+          const int n = t ? n_kv[1] : n_kv[0];
+          const uint32_t s_tm = tmem_base + TM_S + t * BKV, o_tm = tmem_base + TM_O + t * HD;
+          if (j >= 0 && j < n) {
+            const int st = j % KV_STAGES;
+            mbar_wait(&v_full[st], (uint32_t)(j / KV_STAGES) & 1);
+            mbar_wait(&p_full[t], (uint32_t)j & 1);
+            tc_fence_after();
+            const uint64_t vd = v_desc + st * (TILE_BYTES >> 4);
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
-          umma_ss<1>(tmem_base + TM_S + t * BKV, umma_desc_k_sw128(qa + off), umma_desc_k_sw128(ka + off), idesc_qk, kk != 0);
-        }
-        if (last_user(t, j)) umma_commit(&k_empty[st]);
-        umma_commit(&s_full[t]);
-      };
-      for (int t = 0; t < 2; ++t) if (n_kv[t] > 0) { mbar_wait(&q_full[t], 0); issue_qk(t, 0); }
-      for (int j = 0; j < n_kv_max; ++j) {
-        const int st = j % KV_STAGES;
-        for (int t = 0; t < 2; ++t) {
-          if (j >= n_kv[t]) continue;
-          mbar_wait(&v_full[st], (uint32_t)(j / KV_STAGES) & 1);
-          mbar_wait(&p_full[t], (uint32_t)j & 1);
-          tc_fence_after();
-          const uint32_t va = smem_u32(sV + st * TILE_BYTES);
+            for (int kk = 0; kk < BKV / 16; ++kk) umma_ts_if(lead, o_tm, s_tm + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv, (j | kk) != 0);
+            if (lead && (t == 1 || j >= n_kv[1])) umma_commit(&v_empty[st]);
+            if (lead && j == n - 1) umma_commit(&o_full[t]);
+          }
+          if (j + 1 < n) {
+            const int st = (j + 1) % KV_STAGES;
+            if (j < 0) mbar_wait(&q_full[t], 0);
+            mbar_wait(&k_full[st], (uint32_t)((j + 1) / KV_STAGES) & 1);
+            tc_fence_after();
+            const uint64_t qd = q_desc + t * (TILE_BYTES >> 4), kd = k_desc + st * (TILE_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk)
-            umma_ts(tmem_base + TM_O + t * HD, tmem_base + TM_S + t * BKV + kk * 8, desc_mn_sw128(va + kk * 16 * 128, HALF_BYTES, 1024), idesc_pv, (j | kk) != 0);
-          if (last_user(t, j)) umma_commit(&v_empty[st]);
-          if (j == n_kv[t] - 1) umma_commit(&o_full[t]);
-          if (j + 1 < n_kv[t]) issue_qk(t, j + 1);
+            for (int kk = 0; kk < HD / 16; ++kk) {
+              const int off = (kk >> 2) * (HALF_BYTES >> 4) + (kk & 3) * 2;
+              umma_ss_if(lead, s_tm, qd + off, kd + off, idesc_qk, kk != 0);
+            }
+            if (lead && (t == 1 || j + 1 >= n_kv[1])) umma_commit(&k_empty[st]);
+            if (lead) umma_commit(&s_full[t]);
+          }
         }
       }
     }
