@@ -334,7 +334,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer (pair leader only)
-    if (lane == 0 && leader) {
+    if (leader) {
+      const uint32_t lead = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(BM * CG, BN);
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
@@ -350,12 +351,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const uint64_t bd = umma_desc_k_sw128(smem_u32(smB + (stage * KSUB + u) * C_::B_BYTES));
 #pragma unroll
             for (int k = 0; k < BK / UK; ++k)   // +32 B per UMMA_K inside the 128B swizzle row
-              umma_ss<CG>(d_tmem, ad + (uint64_t)(k * UK * 2 / 16), bd + (uint64_t)(k * UK * 2 / 16), idesc, (kb | u | k) != 0);
+              umma_ss_if<CG>(lead, d_tmem, ad + (uint64_t)(k * UK * 2 / 16), bd + (uint64_t)(k * UK * 2 / 16), idesc, (kb | u | k) != 0);
           }
-          if constexpr (CG == 1) umma_commit(&empty[stage]); else umma_commit_2sm(&empty[stage], 0b11);
+          if (!lead) {} else if constexpr (CG == 1) umma_commit(&empty[stage]); else umma_commit_2sm(&empty[stage], 0b11);
           if (++stage == NST) { stage = 0; phase ^= 1; }
         }
-        if constexpr (CG == 1) umma_commit(&tfull[acc]); else umma_commit_2sm(&tfull[acc], 0b11);
+        if (!lead) {} else if constexpr (CG == 1) umma_commit(&tfull[acc]); else umma_commit_2sm(&tfull[acc], 0b11);
         acc ^= 1; if (acc == 0) acc_phase ^= 1;
       }
     }
