@@ -4,7 +4,8 @@
 // i.e. U = T diag(beta) (V - diag(G) K S) with T = (1 + A)^-1, A_ij = beta_i Gam_ij (k_i . k_j) below the diagonal; O = diag(G) Q S + P U.
 //
 // delta_prepare_kernel, one CTA per (block, head, sequence), all in parallel: what does not depend on the state.  k . k and q . k as bf16 products (exact) with fp32
-//   sums, norms and gates in fp32, sums of log decays in 64 bits (their differences enter as two floats), T by forward substitution in fp32, one column per thread.
+//   sums, norms and gates in fp32, sums of log decays in 64 bits (their differences enter as two floats), T in fp32 by halves: two triangles of 32 by forward
+//   substitution (one column per thread), the square between them by products.
 //   T diag(beta) and P go to the workspace as three bf16 parts (24 bits), in the order in which the next kernel's lanes read them.
 // delta_scan_kernel, one warp per 16 value channels, blocks one after another.  Everything is held transposed (value channels = rows of the mma tiles): the sums of
 //   one product are then, lane by lane, the first operand of the next, so the 16 x dk piece of the state stays in the warp's registers and warps exchange nothing:

@@ -12,7 +12,7 @@
 // kernel runs.  The tile walk is the CUDA-core kernel's: [0, keep_first), the pooled blocks that the CTA's last query sees, and the
 // union of the CTA's windows.
 // One map without kept tokens, pooled blocks, soft cap, bias and head norm -- what most layers ask for -- has a kernel of its own
-// (window_attn_plain_kernel): with one K and one V tile in shared memory three CTAs fit an SM (two with heads wider than 128), a K tile is replaced as soon as its
+// (window_attn_plain_kernel, for what window_attention_tc.cu does not take): with one K and one V tile in shared memory three CTAs fit an SM (two with heads wider than 128), a K tile is replaced as soon as its
 // scores are taken and a V tile as soon as it is summed, so that each is on its way while the other is in work and other CTAs fill the
 // waits; the exponents' reference follows the running maximum lazily (weights stay below 2^8).
 // In the general kernel a soft cap is applied to the fp32 scores before the softmax (tanh from ex2 and a division), and a

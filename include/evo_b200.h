@@ -133,7 +133,7 @@ int evo_set_pdl(int level);
  *   state_out (B, D, S, 2) fp32: modal state after the last row (== inference_params.
  *        state_dict[layer] of the reference, complex64).
  *   fir_state_out (B, 3D, 2) bf16: last two z rows (== fir_state_dict[layer]).
- * workspace: evo_hyena_fwd_workspace() bytes (segment carries when L is split). */
+ * workspace: evo_hyena_fwd_workspace() bytes (segment carries when L is split; the channels' block constants when the tensor-core form runs). */
 typedef struct {
   const void* z; void* y;
   const void* fir_w; const void* fir_b; const void* Dskip;
@@ -572,7 +572,8 @@ typedef struct {
   void* out; int64_t ldo; int dtype;
   int B; int64_t L; int H, G, dk, dv;
 } evo_gated_delta_params;
-/* workspace: evo_gated_delta_workspace() bytes (0 unless a head's value channels are spread over several CTAs; the head norm then runs in a second kernel) */
+/* workspace: evo_gated_delta_workspace() bytes (0 for a head whose tokens one CTA takes one by one; fp32 read-outs where its value channels are spread over several CTAs;
+ * the blocks' matrices too, at most 256 MB of them at a time, where a prompt runs in 64-token blocks) */
 size_t evo_gated_delta_workspace(const evo_gated_delta_params* p);
 int evo_gated_delta_fwd(const evo_gated_delta_params* p, void* workspace, size_t workspace_bytes, void* stream);
 
