@@ -569,8 +569,9 @@ __global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restric
 constexpr int64_t SLAB_BYTES = 256ll << 20;
 
 // Taken for bf16 heads of 64 or 128 key channels and a multiple of 16 value channels, rows that start on 16 bytes, and calls of 32 tokens or more.
+// (The workspace query comes here with shapes that the call has not looked over: an empty batch has no blocks to count.)
 bool taken(const evo_gated_delta_params* p) {
-  return p->dtype == 0 && (p->dk == 64 || p->dk == 128) && p->dv % 16 == 0 && p->L >= 32 && p->ld % 8 == 0 && p->H <= 65535 && p->B <= 65535 &&
+  return p->B > 0 && p->H > 0 && p->dv > 0 && p->dtype == 0 && (p->dk == 64 || p->dk == 128) && p->dv % 16 == 0 && p->L >= 32 && p->ld % 8 == 0 && p->H <= 65535 && p->B <= 65535 &&
          (((uintptr_t)p->q | (uintptr_t)p->k | (uintptr_t)p->v) & 15) == 0;
 }
 struct Sizes { int64_t blocks, slab; size_t y, tri, state; };

@@ -101,3 +101,20 @@ def test_error_convention_without_a_gpu():
         _lib.check(lib.evo_kv_append(None, None, 1, 10, 2, 128, 10, 16, None), "evo_kv_append")
     rc = lib.evo_rmsnorm(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x2000), ctypes.c_void_p(0x3000), 4, 4096, 1e-6, None)
     assert rc < 0 and b"failed" in lib.evo_last_error()
+
+
+def _workspace_in_a_process(code):
+    """Workspace queries are host arithmetic; one that divides by zero would take this process along."""
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", "import ctypes as C\nfrom evo_b200 import _lib\nfrom evo_b200._lib import *\nlib = _lib.lib()\n" + code],
+                       cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, f"ended with {r.returncode}: {r.stderr[-500:]}"
+    return [int(x) for x in r.stdout.split()]
+
+
+def test_gated_delta_workspace_of_an_empty_call_is_empty():
+    got = _workspace_in_a_process(
+        "for B, H, L in ((0, 4, 64), (0, 4, 16), (0, 4, 5000), (1, 0, 64), (-1, 4, 64), (2, 4, 64)):\n"
+        "    print(lib.evo_gated_delta_workspace(C.byref(GatedDeltaParams(B=B, L=L, H=H, G=1, dk=128, dv=128, ld=384, dtype=0))))\n")
+    assert got[:5] == [0] * 5 and got[5] > 0
