@@ -361,7 +361,7 @@ static size_t segment_bytes(const evo_hyena_params* p, int nseg) {
 }
 
 extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) {
-  if (p->L <= 0) return 0;
+  if (p->L <= 0 || p->B <= 0) return 0;
   const HyenaPlan plan = make_plan(p);
   // the tensor-core path keeps its channels' constants behind the segment states, on the next multiple of 256 bytes
   return segment_bytes(p, plan.nseg) + (plan.tc ? 256 + evo_hytc::table_bytes(p->D) : 0);

@@ -118,3 +118,10 @@ def test_gated_delta_workspace_of_an_empty_call_is_empty():
         "for B, H, L in ((0, 4, 64), (0, 4, 16), (0, 4, 5000), (1, 0, 64), (-1, 4, 64), (2, 4, 64)):\n"
         "    print(lib.evo_gated_delta_workspace(C.byref(GatedDeltaParams(B=B, L=L, H=H, G=1, dk=128, dv=128, ld=384, dtype=0))))\n")
     assert got[:5] == [0] * 5 and got[5] > 0
+
+
+def test_hyena_workspace_of_an_empty_call_is_empty():
+    got = _workspace_in_a_process(
+        "for B, L in ((0, 64), (0, 500), (0, 2000), (-1, 500), (1, 0), (1, 500)):\n"
+        "    print(lib.evo_hyena_fwd_workspace(C.byref(HyenaParams(B=B, L=L, D=512, S=8, nheads=4))))\n")
+    assert got[:5] == [0] * 5 and got[5] > 0
