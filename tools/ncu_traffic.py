@@ -1,7 +1,7 @@
 """Turn `ncu --set full` captures into the small per-launch table bench.py reads for the
 `roofline.traffic` field (dram__bytes_read.sum + dram__bytes_write.sum per launch).
 
-    python tools/ncu_traffic.py profiles/r01_ncu_traffic.json cap1.ncu-rep [cap2.ncu-rep ...]
+    python tools/ncu_traffic.py profiles/ncu_traffic_8k.json cap1.ncu-rep [cap2.ncu-rep ...]
 """
 import csv
 import io
