@@ -270,8 +270,8 @@ def rooflines(by, step_ms, workload, peaks):
                             "peak_source": peaks["source"] + " (sustained cuBLAS bf16)", "share_of_step": by["gemm"][1] / step_ms, "launches_per_step": by["gemm"][2]}
     if "hyena" in by:
         ach = by["hyena"][0] / (by["hyena"][1] / 1e3) / 1e9
-        roof["roofline_hyena"] = {"kernel": "hyena_scan_ms_kernel (fused FIR + gate + modal long conv + gate)", "bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"],
-                                  "unit": "GB/s", "frac": ach / peaks["hbm_gbs"], "traffic": ncu_traffic("hyena_scan", workload),
+        roof["roofline_hyena"] = {"kernel": "hyena_tc_kernel (fused FIR + gate + modal long conv + gate)", "bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"],
+                                  "unit": "GB/s", "frac": ach / peaks["hbm_gbs"], "traffic": ncu_traffic("hyena_tc", workload),
                                   "algorithmic_bytes_per_launch": by["hyena"][0] / by["hyena"][2], "peak_source": peaks["source"],
                                   "share_of_step": by["hyena"][1] / step_ms, "launches_per_step": by["hyena"][2]}
     if "attn" in by:

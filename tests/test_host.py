@@ -537,6 +537,26 @@ def test_bench_helpers_assemble_the_contract_fields():
     assert abs(g["share_of_step"] - 500.0 / 600.0) < 1e-12 and g["launches_per_step"] == 129.0
 
 
+def test_bench_names_the_hyena_kernel_that_its_workload_runs():
+    """The plan puts the scoring shape on the tensor cores (its workspace holds their constants; an unsegmented scan needs none), and the record names that kernel,
+    with the DRAM bytes of a capture of that kernel or none."""
+    import ctypes as C
+    import importlib.util
+    from evo_b200 import _lib
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    spec = importlib.util.spec_from_file_location("bench_mod", os.path.join(root, "bench.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    wl = b.WORKLOADS["8k"]
+    p = _lib.HyenaParams(B=wl["batch"], L=wl["nt"] + 1, D=4096, S=8, nheads=32)
+    on_tensor_cores = _lib.lib().evo_hyena_fwd_workspace(C.byref(p)) > 0
+    peaks = {"hbm_gbs": 6000.0, "bf16_tflops": 1600.0, "bf16_tflops_sustained": 1400.0, "source": "measured"}
+    rec = b.rooflines({"hyena": [1.0e9, 1.0, 29.0]}, 600.0, "8k", peaks)["roofline_hyena"]
+    name = rec["kernel"].split()[0]
+    assert name == ("hyena_tc_kernel" if on_tensor_cores else "hyena_scan_ms_kernel")
+    assert rec["traffic"] == b.ncu_traffic(name, "8k")
+
+
 def test_cli_scripts_keep_the_reference_arguments():
     """scripts/score.py and scripts/generate.py: the reference's argument names and defaults (scripts/score.py:24-30,
     scripts/generate.py:24-37 of evo-design/evo), plus the offline switches; the example FASTA parses to three sequences."""
