@@ -403,8 +403,11 @@ int launch(const evo_window_attn_params* p, cudaStream_t st) {
 
 namespace evo {
 
-// the host knows the position (the maps' extents), and every row of every operand starts on 16 bytes
+// 16 query rows or more, the host knows the position (the maps' extents), and every row of every operand starts on 16 bytes.  Fewer rows -- a step, the rest of a
+// portion -- go to the CUDA-core kernels, which keep their weights and gate in fp32, spread up to four queries' keys over the warps of a CTA, and also serve the captured
+// step: a call's result must not depend on where its position is kept.
 bool window_attn_tc_takes(const evo_window_attn_params* p) {
+  if (p->Lq < 16) return false;
   const auto a16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
   const auto tok = [](int64_t s) { return s > 0 && s % 8 == 0 && s < (1ll << 31); };
   const auto batch = [&](int64_t s) { return p->B == 1 || (s > 0 && s % 8 == 0 && s < (1ll << 38)); };

@@ -41,7 +41,7 @@ def _oracle(q, k, v, pos, window, scale, sink, gate, per_head):
     return out
 
 
-def _run(B, L, H, G, d, pos, window, *, gate=None, sink=False, pad=0, seed=0, spoil=(), cap=0):
+def _run(B, L, H, G, d, pos, window, *, gate=None, sink=False, pad=0, seed=0, spoil=(), cap=0, on_device=False):
     from evo_b200 import _lib
     from evo_b200._lib import WindowAttnParams, check
     lib = _lib.lib()
@@ -61,6 +61,9 @@ def _run(B, L, H, G, d, pos, window, *, gate=None, sink=False, pad=0, seed=0, sp
         p.gate, p.gate_tok_stride, p.gate_per_head = gt.data_ptr(), gt.shape[1], int(gate == "head")
     if sk is not None:
         p.sink = sk.data_ptr()
+    at = torch.tensor([pos], dtype=torch.int64, device="cuda")
+    if on_device:
+        p.pos_dev = at.data_ptr()
     check(lib.evo_window_attn_fwd(C.byref(p), torch.cuda.current_stream().cuda_stream), "evo_window_attn_fwd")
     kk, vv = kv[:, :, :G * d].reshape(B, -1, G, d), kv[:, :, G * d:2 * G * d].reshape(B, -1, G, d)
     gg = None if gt is None else gt[:, :H * d].reshape(B, L, H, d) if gate == "channel" else gt.reshape(B, L, H, 1)
@@ -103,3 +106,16 @@ def test_values_that_are_not_finite_reach_only_the_rows_that_see_them(d, window)
     fin = torch.isfinite(ref)
     assert fin[0, :140].all() and not fin.all()
     _close(out[fin], ref[fin], vmax)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("L", [1, 2, 4, 5, 9, 15])
+@pytest.mark.parametrize("pos,window", [(0, 100), (37, 100), (900, 0), (1000, 256)])
+def test_a_few_queries_run_as_in_a_captured_step(d, L, pos, window):
+    """Up to 15 queries belong to the CUDA-core kernels wherever the position is known: a step called directly gives the bits of its captured twin, whose position
+    is in device memory, with fp32 weights and the exact gate."""
+    opt = dict(gate="channel", sink=True, seed=L, cap=4)
+    out, ref, vmax = _run(2, L, 4, 2, d, pos, window, **opt)
+    twin, _, _ = _run(2, L, 4, 2, d, pos, window, on_device=True, **opt)
+    assert torch.equal(out, twin)
+    _close(out, ref, vmax)
