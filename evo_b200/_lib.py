@@ -244,6 +244,8 @@ SIGNATURES = {
     "evo_gemm_smallm_workspace": (C.c_size_t, [C.c_int64, C.c_int64, C.c_int64, C.c_int]),
     "evo_gemm_smallm": (C.c_int, [C.POINTER(GemmSmallMParams), C.c_void_p]),
     "evo_set_pdl": (C.c_int, [C.c_int]),
+    "evo_lost_waits": (C.c_int, [C.c_int]),
+    "evo_set_wait_polls": (C.c_int, [C.c_int]),
     "evo_hyena_fwd_workspace": (C.c_size_t, [C.POINTER(HyenaParams)]),
     "evo_hyena_fwd": (C.c_int, [C.POINTER(HyenaParams), C.c_void_p, C.c_size_t, C.c_void_p]),
     "evo_hyena_step": (C.c_int, [C.c_void_p] * 9 + [C.c_int] * 4 + [C.c_void_p]),
@@ -342,6 +344,12 @@ def check(rc: int, what: str = ""):
     if rc != 0:
         msg = lib().evo_last_error()
         raise EvoError(f"{what or 'evo_b200'} failed (rc={rc}): {msg.decode() if msg else ''}")
+
+
+def check_lost_waits():
+    """Raises if a wait inside a kernel has run out since the last check (outputs since then are incomplete).  Reads host memory: call it where results have just arrived."""
+    if lib().evo_lost_waits(1):
+        raise EvoError("a wait inside a kernel ran out: results since the last check are incomplete")
 
 
 def ptr(t):

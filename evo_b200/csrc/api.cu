@@ -1,9 +1,10 @@
 // C-ABI plumbing: error string, launch counter, TMA descriptor encode, device query.
-#include "common.cuh"
+#include "waits.cuh"
 #include "../../include/evo_b200.h"
 #include <stdarg.h>
 #include <string.h>
 #include <atomic>
+#include <mutex>
 
 namespace evo {
 
@@ -11,6 +12,28 @@ static thread_local char g_err[512] = "";
 static std::atomic<int64_t> g_launches{0};
 static std::atomic<int> g_pdl{0};
 int pdl_level() { return g_pdl.load(std::memory_order_relaxed); }
+
+// One word of host memory that every device can write and the host reads without a stream; allocated by the first launch that may need it, which may be under capture.
+static std::atomic<unsigned int*> g_lost{nullptr};
+static std::mutex g_lost_mutex;
+static thread_local int g_polls = WAIT_POLLS;
+int wait_limit(WaitLimit* out) {
+  if (!g_lost.load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lock(g_lost_mutex);
+    if (!g_lost.load(std::memory_order_relaxed)) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      EVO_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      void* word = nullptr;
+      const cudaError_t e = cudaHostAlloc(&word, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped);
+      EVO_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      EVO_REQUIRE(e == cudaSuccess, "cudaHostAlloc failed: %s", cudaGetErrorString(e));
+      *(volatile unsigned int*)word = 0u;
+      g_lost.store((unsigned int*)word, std::memory_order_release);
+    }
+  }
+  *out = {g_polls, g_lost.load(std::memory_order_relaxed)};
+  return 0;
+}
 
 void set_error(const char* fmt, ...) {
   va_list ap;
@@ -99,5 +122,16 @@ int evo_abi_version(void) { return 1; }
 int64_t evo_launch_count(void) { return evo::g_launches.load(); }
 void evo_reset_launch_count(void) { evo::g_launches.store(0); }
 void evo_note_graph_replay(int64_t launches) { evo::g_launches.fetch_add(launches); }
+int evo_lost_waits(int clear) {
+  volatile unsigned int* word = evo::g_lost.load();
+  const int lost = word && *word;
+  if (lost && clear) *word = 0u;
+  return lost;
+}
+int evo_set_wait_polls(int polls) {
+  const int before = evo::g_polls;
+  evo::g_polls = polls < 0 ? evo::WAIT_POLLS : polls;
+  return before;
+}
 int evo_set_pdl(int level) { return evo::g_pdl.exchange(level < 0 ? 0 : (level > 4 ? 4 : level)); }
 }

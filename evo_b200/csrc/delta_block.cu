@@ -16,7 +16,7 @@
 // Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 590 us (token by token 2774), of which the scan 395, bound by the tensor pipe (816 mma of 8.7 cycles per block and
 // warp, one warp per scheduler: 7.1 k of 10.4 k cycles) and the splits between its products; 1 x 777 tokens, 32 heads: 110 us (516).
 // A block in which W or U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
-#include "common.cuh"
+#include "waits.cuh"
 #include "mma_sync.cuh"
 #include "../../include/evo_b200.h"
 #include <algorithm>
@@ -50,6 +50,8 @@ struct Args {
   float* y;                                             // (rows, H * dv) fp32 read-outs
   int B; int64_t L; int H, G, dv;
   int64_t first; int n_blocks;                          // the slab: its first block and its length
+  unsigned int* failed;                                 // a wait of this call ran out: later slabs and the states behind them are not computed
+  WaitLimit waits;
 };
 
 __device__ __forceinline__ float2 top2(float x, float y) { return make_float2(__uint_as_float(__float_as_uint(x) & 0xffff0000u), __uint_as_float(__float_as_uint(y) & 0xffff0000u)); }
@@ -69,14 +71,6 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool on) {  
 // global -> shared memory, bytes and both addresses multiples of 16
 __device__ __forceinline__ void bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-// an mbarrier wait with a limit; one that runs out is counted and the kernel ends
-__device__ unsigned int delta_lost_waits;
-__device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 22); ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicAdd(&delta_lost_waits, 1u);
-  return false;
 }
 __device__ __forceinline__ void mma_np(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {       // free to be scheduled
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -104,6 +98,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (p.H / p.G);
   const int64_t t0 = (p.first + blk) * BT, row0 = (int64_t)b * p.L + t0;
   const int nt = (int)min((int64_t)BT, p.L - t0);
+  if (p.first == 0 && (blk | h | b | tid) == 0) *p.failed = 0u;
   for (int e = tid; e < BT * (DK / 8); e += 128) {
     const int r = e / (DK / 8), c = e % (DK / 8);
     const bool on = r < nt;
@@ -311,7 +306,7 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const __grid_constan
     bulk(st + 2 * ROWS_BYTES + BT * vpitch, blocks + (int64_t)blk * BLOCK_BYTES, BLOCK_BYTES, bar);
   };
   if (tid == 0) { mbar_init(&arrived[0], 1); mbar_init(&arrived[1], 1); fence_barrier_init(); }
-  __syncthreads();
+  if (__syncthreads_or(p.first > 0 && tid == 0 && *(volatile unsigned int*)p.failed)) return;
 
   // ---- S^T: rows = value channels cw + gq (+ 8), columns = state rows: S[n][..] covers state rows 8 n + 2 tq, + 1
   float S[2 * KT][4];
@@ -327,8 +322,16 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const __grid_constan
   for (int blk = 0; blk < p.n_blocks; ++blk) {
     if (tid == 0 && blk + 1 < p.n_blocks) fetch(blk + 1);
     const uint8_t* ks = sm + (blk & 1) * stage_bytes;
-    const bool here = wait_or_give_up(&arrived[blk & 1], (blk >> 1) & 1);
-    if (__syncthreads_or(!here)) break;
+    const bool here = wait_or_give_up(&arrived[blk & 1], (blk >> 1) & 1, p.waits);
+    if (__syncthreads_or(!here)) {
+      // no state is kept; the copies under way land before the CTA ends
+      if (tid == 0) {
+        *p.failed = 1u;
+        wait_to_end(&arrived[blk & 1], (blk >> 1) & 1, p.waits);
+        if (blk + 1 < p.n_blocks) wait_to_end(&arrived[(blk + 1) & 1], ((blk + 1) >> 1) & 1, p.waits);
+      }
+      return;
+    }
     const uint8_t* qs = ks + ROWS_BYTES;
     const uint8_t* vs = qs + ROWS_BYTES;
     const uint8_t* tri = vs + BT * vpitch;
@@ -574,7 +577,10 @@ bool taken(const evo_gated_delta_params* p) {
   return p->B > 0 && p->H > 0 && p->dv > 0 && p->dtype == 0 && (p->dk == 64 || p->dk == 128) && p->dv % 16 == 0 && p->L >= 32 && p->ld % 8 == 0 && p->H <= 65535 && p->B <= 65535 &&
          (((uintptr_t)p->q | (uintptr_t)p->k | (uintptr_t)p->v) & 15) == 0;
 }
-struct Sizes { int64_t blocks, slab; size_t y, tri, state; };
+struct Sizes {
+  int64_t blocks, slab; size_t y, tri, state;
+  size_t total() const { return y + tri + state + 2 * 256; }         // with the call's `failed` word, and the start moved up to a multiple of 256
+};
 Sizes sizes(const evo_gated_delta_params* p) {
   Sizes s;
   s.blocks = (p->L + BT - 1) / BT;
@@ -589,6 +595,8 @@ Sizes sizes(const evo_gated_delta_params* p) {
 template <int DK>
 int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream_t st) {
   Args a = {};
+  if (const int rc = wait_limit(&a.waits)) return rc;
+  a.failed = (unsigned int*)(ws + s.y + s.tri + s.state);
   a.k = (const bf16*)p->k; a.q = (const bf16*)p->q; a.v = (const bf16*)p->v; a.ld = p->ld;
   a.b = (const bf16*)p->b; a.a = (const bf16*)p->a; a.ldz = p->ldz;
   a.A_log = (const bf16*)p->A_log; a.dt_bias = (const bf16*)p->dt_bias;
@@ -632,12 +640,12 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
 size_t evo::delta_block_workspace(const evo_gated_delta_params* p) {
   if (!taken(p)) return 0;
   const Sizes s = sizes(p);
-  return s.y + s.tri + s.state + 256;
+  return s.total();
 }
 
 int evo::delta_block_fwd(const evo_gated_delta_params* p, void* ws, size_t bytes, cudaStream_t st) {
   const Sizes s = sizes(p);
-  EVO_REQUIRE(ws && bytes >= s.y + s.tri + s.state + 256, "evo_gated_delta_fwd: workspace too small (%zu < %zu)", bytes, s.y + s.tri + s.state + 256);
+  EVO_REQUIRE(ws && bytes >= s.total(), "evo_gated_delta_fwd: workspace too small (%zu < %zu)", bytes, s.total());
   uint8_t* base = (uint8_t*)(((uintptr_t)ws + 255) & ~(uintptr_t)255);
   return p->dk == 64 ? run<64>(p, s, base, st) : run<128>(p, s, base, st);
 }

@@ -382,6 +382,7 @@ static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, voi
   a.consts = consts; a.seg_pow = seg_pow;
   a.B = p->B; a.D = p->D; a.nseg = nseg; a.L = p->L; a.seg_len = seg_len;
   a.y_wide = ((uintptr_t)p->y & 7) == 0;
+  if ((rc = wait_limit(&a.waits))) return rc;
   CUtensorMap tmZ;
   uint64_t dims[3] = {(uint64_t)3 * p->D, (uint64_t)p->L, (uint64_t)p->B};
   uint64_t str[2] = {(uint64_t)3 * p->D * 2, (uint64_t)p->L * 3 * p->D * 2};

@@ -23,7 +23,7 @@
 // A channel whose x or state is not finite (or beyond 1e30), or whose poles lie so far outside the unit circle that their powers are not, goes
 // token by token in that tile: a product with a structural zero would otherwise carry an infinity to earlier tokens of its block.
 #pragma once
-#include "common.cuh"
+#include "waits.cuh"
 
 namespace evo_hytc {
 
@@ -57,6 +57,7 @@ struct Args {
   const float2* seg_pow;                     // (D, 8) p^seg_len
   int B, D, nseg, items, y_wide;
   long long L, seg_len;
+  WaitLimit waits;
 };
 
 constexpr size_t table_bytes(int D) { return (size_t)D * (CONST_BYTES + NS * 8); }
@@ -214,14 +215,8 @@ template <typename F> __device__ __forceinline__ void fir8(const uint32_t (&wq)[
   }
 }
 
-// an mbarrier wait with a limit: a wait that runs out is counted, and the role that gave up ends
-__device__ unsigned int lost_waits;
-__device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 22); ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicAdd(&lost_waits, 1u);
-  return false;
-}
+// a warp's wait: what one lane lost all have lost
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const WaitLimit& w) { return __all_sync(0xffffffffu, wait_or_give_up(bar, parity, w)); }
 
 // position in the sequence of tiles that a CTA walks: its items (channel block, batch row, segment), tile by tile
 struct Walk {
@@ -285,7 +280,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
       bool ok = true;
       auto put = [&](int col, int t, int b) {
         const uint32_t i = s % SLOTS, round = s / SLOTS;
-        if (ok && round > 0) ok = wait_or_give_up(&zempty[i], (round - 1) & 1);
+        if (ok && round > 0) ok = wait_or_give_up(&zempty[i], (round - 1) & 1, a.waits);
         if (ok) {
           mbar_arrive_expect_tx(&zfull[i], SLOT_BYTES);
           tma_load_3d(ring + i * SLOT_BYTES, &tmZ, &zfull[i], col, t - 2, b);
@@ -305,7 +300,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
         if (any) { p.of(w, TILE); w.next(a, TILE); }
       }
       // the copies still in flight land before this thread ends
-      for (uint32_t q = s > SLOTS ? s - SLOTS : 0; q < s; ++q) wait_or_give_up(&zfull[q % SLOTS], (q / SLOTS) & 1);
+      for (uint32_t q = s > SLOTS ? s - SLOTS : 0; q < s; ++q) wait_to_end(&zfull[q % SLOTS], (q / SLOTS) & 1, a.waits);
     }
     return;
   }
@@ -320,10 +315,11 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
     bool ok = true, any = false;
     Tile p;
     p.of(w, TILE);
-    // ten raw rows of this thread's run from slot s, the first two in front of it, as two channel pairs; the slot is then free
+    // ten raw rows of this thread's run from slot s, the first two in front of it, as two channel pairs; the slot is then free (and not ok: none)
     auto rows = [&](uint32_t slot, int t, int b, int col, uint32_t (&z)[2][10]) {
       const uint32_t i = slot % SLOTS;
-      ok = ok && wait_or_give_up(&zfull[i], (slot / SLOTS) & 1);
+      ok = warp_wait(&zfull[i], (slot / SLOTS) & 1, a.waits);
+      if (!ok) return;
       const uint8_t* src = ring + i * SLOT_BYTES + run * 8 * (CH * 2) + quad * 8;
 #pragma unroll
       for (int e = 0; e < 10; ++e) { const uint2 v = *reinterpret_cast<const uint2*>(src + e * (CH * 2)); z[0][e] = v.x; z[1][e] = v.y; }
@@ -352,11 +348,13 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             {
               const Taps w1 = load_taps(a.fir_w, a.fir_b, zc + HD);       // (from L1; kept over the stages they would not fit the registers)
               rows(s + 2 * i, t, w.b, zc + HD, z);
+              if (!ok) break;
               fir8(w1.w[0], w1.bias.x, z[0], [&](int e, uint32_t f) { x[0][e] = f; });
               fir8(w1.w[1], w1.bias.y, z[1], [&](int e, uint32_t f) { x[1][e] = f; });
             }
             const Taps wv = load_taps(a.fir_w, a.fir_b, zc + 2 * HD);
             rows(s + 2 * i + 1, t, w.b, zc + 2 * HD, z);
+            if (!ok) break;
             fir8(wv.w[0], wv.bias.x, z[0], [&](int e, uint32_t f) { x[0][e] = mulbf(x[0][e], f); });
             fir8(wv.w[1], wv.bias.y, z[1], [&](int e, uint32_t f) { x[1][e] = mulbf(x[1][e], f); });
             if (n < TILE) {
@@ -375,13 +373,15 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
                 make_uint4(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), __byte_perm(v[4], v[5], sel), __byte_perm(v[6], v[7], sel));
           }
         }
+        if (!ok) break;                                                 // the tensor-core warps wait in vain and end, too
         s += 2 * ns;
         __syncwarp();
         if (lane == 0) mbar_arrive(&xfull[q & 1]);
       }
       if (any) {
         // ---------------- C: tile q - 1, (convolution + D x) * x2.  The cells are this thread's own: A of tile q + 1 may refill them afterwards
-        ok = ok && wait_or_give_up(&xdone[(q - 1) & 1], ((q - 1) >> 1) & 1);
+        ok = warp_wait(&xdone[(q - 1) & 1], ((q - 1) >> 1) & 1, a.waits);
+        if (!ok) break;
         if (!STATE_ONLY) {
           const int ns = (p.n + STAGE - 1) / STAGE, ch = p.ch0 + 4 * quad, zc = (ch / HD) * 3 * HD + ch % HD;
           const uint8_t* xs = xbuf + ((q - 1) & 1) * (CH * TILE * 2);
@@ -392,6 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
             uint32_t z[2][10], o[2][8];
             const Taps w2 = load_taps(a.fir_w, a.fir_b, zc);
             rows(s + i, t, p.b, zc, z);
+            if (!ok) break;
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
               const uint4 lo = *reinterpret_cast<const uint4*>(xs + cell<R>(4 * quad + 2 * v, row, gr)), hi = *reinterpret_cast<const uint4*>(xs + cell<R>(4 * quad + 2 * v + 1, row, gr));
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
       __syncwarp();
     }
     uint8_t* xs = xbuf + (q & 1) * (CH * TILE * 2);
-    if (!wait_or_give_up(&xfull[q & 1], (q >> 1) & 1)) break;
+    if (!warp_wait(&xfull[q & 1], (q >> 1) & 1, a.waits)) break;
 #pragma unroll 1
     for (int c = warp; c < CH; c += MMA_WARPS) {
       const int chg = w.ch0 + c;

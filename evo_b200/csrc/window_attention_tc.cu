@@ -17,7 +17,7 @@
 // although its denominator is, is therefore summed again over the keys that it sees alone, on the CUDA cores.
 //
 // Every wait has a limit; a role that gives up ends, and the CTA ends when its copies and products have.
-#include "common.cuh"
+#include "waits.cuh"
 #include <algorithm>
 #include "../../include/evo_b200.h"
 
@@ -35,25 +35,17 @@ template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setma
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr uint32_t TM_S = 0, TM_O = 256;         // + 128 * tile
 
-__device__ unsigned int lost_waits;
-
 struct Args {
   const bf16 *q, *k, *v, *gate, *sink;
   bf16* out;
   long long q_tok, k_tok, v_tok, k_batch, v_batch, gate_tok, ldo, Lq, pos;
   int B, H, G, n_qblk, window, gate_per_head, tail;
   float scale2;
+  WaitLimit waits;
 };
 
 __device__ __forceinline__ float ex2(float x) { float y; asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-
-__device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 22); ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicAdd(&lost_waits, 1u);
-  return false;
-}
 
 // values as the second operand: rows are keys, 64-channel halves HALF_BYTES apart
 __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
@@ -126,18 +118,18 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int j = 0; j < n_kv; ++j) {
           const int st = j % KV_STAGES;
           const uint32_t ph = (uint32_t)(j / KV_STAGES) & 1;
-          if (!wait_or_give_up(&k_empty[st], ph ^ 1)) break;
+          if (!wait_or_give_up(&k_empty[st], ph ^ 1, a.waits)) break;
           load(sK + st * TILE_BYTES, &tmK, &k_full[st], g, key0 + (long long)j * BKV);
           ++kn;
-          if (!wait_or_give_up(&v_empty[st], ph ^ 1)) break;
+          if (!wait_or_give_up(&v_empty[st], ph ^ 1, a.waits)) break;
           load(sV + st * TILE_BYTES, &tmV, &v_full[st], g, key0 + (long long)j * BKV);
           ++vn;
         }
         // every copy has landed before this thread ends
-        wait_or_give_up(&q_full[0], 0);
-        if (j1[1] > 0) wait_or_give_up(&q_full[1], 0);
-        for (int j = max(0, kn - KV_STAGES); j < kn; ++j) wait_or_give_up(&k_full[j % KV_STAGES], (uint32_t)(j / KV_STAGES) & 1);
-        for (int j = max(0, vn - KV_STAGES); j < vn; ++j) wait_or_give_up(&v_full[j % KV_STAGES], (uint32_t)(j / KV_STAGES) & 1);
+        wait_to_end(&q_full[0], 0, a.waits);
+        if (j1[1] > 0) wait_to_end(&q_full[1], 0, a.waits);
+        for (int j = max(0, kn - KV_STAGES); j < kn; ++j) wait_to_end(&k_full[j % KV_STAGES], (uint32_t)(j / KV_STAGES) & 1, a.waits);
+        for (int j = max(0, vn - KV_STAGES); j < vn; ++j) wait_to_end(&v_full[j % KV_STAGES], (uint32_t)(j / KV_STAGES) & 1, a.waits);
       }
     } else if (warp == WARPS + 1) {
       // One copy of each product in a small loop: this warp shares the SM's instruction cache with the long softmax code (see above)
@@ -154,7 +146,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           const uint32_t s_tm = tmem_base + TM_S + t * BKV, o_tm = tmem_base + TM_O + t * 128;
           if (j >= first && j < last) {
             const int st = j % KV_STAGES;
-            ok = wait_or_give_up(&v_full[st], (uint32_t)(j / KV_STAGES) & 1) && wait_or_give_up(&p_full[t], (uint32_t)(j - first) & 1);
+            ok = wait_or_give_up(&v_full[st], (uint32_t)(j / KV_STAGES) & 1, a.waits) && wait_or_give_up(&p_full[t], (uint32_t)(j - first) & 1, a.waits);
             if (!ok) break;
             tc_fence_after();
             const uint64_t vd = v_desc + st * (TILE_BYTES >> 4);
@@ -168,7 +160,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           if (j + 1 >= first && j + 1 < last) {
             const int st = (j + 1) % KV_STAGES;
-            ok = (j + 1 != first || wait_or_give_up(&q_full[t], 0)) && wait_or_give_up(&k_full[st], (uint32_t)((j + 1) / KV_STAGES) & 1);
+            ok = (j + 1 != first || wait_or_give_up(&q_full[t], 0, a.waits)) && wait_or_give_up(&k_full[st], (uint32_t)((j + 1) / KV_STAGES) & 1, a.waits);
             if (!ok) break;
             tc_fence_after();
             const uint64_t qd = q_desc + t * (TILE_BYTES >> 4), kd = k_desc + st * (TILE_BYTES >> 4);
@@ -183,7 +175,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       }
       if (lead) umma_commit(&ended);                 // every product has been summed before TMEM is given back
-      wait_or_give_up(&ended, 0);
+      wait_to_end(&ended, 0, a.waits);
     }
   } else {
     regs_up<SOFTMAX_REGS>();
@@ -197,7 +189,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       bool ok = true;
       for (int j = j0[t]; j < j1[t]; ++j) {
         // a wait that runs out ends both halves: the maximum's place says so
-        ok = __all_sync(0xffffffffu, wait_or_give_up(&s_full[t], (uint32_t)(j - j0[t]) & 1));
+        ok = __all_sync(0xffffffffu, wait_or_give_up(&s_full[t], (uint32_t)(j - j0[t]) & 1, a.waits));
         tc_fence_after();
         const int key = j * BKV + half * HK, top_row = row0 + t * BQ + w * 32 + 31;
         const bool some = ok && key <= top_row && top_row - 31 - (key + HK - 1) < win;      // does any row of the warp see any key of the half
@@ -280,7 +272,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         side[par][half][mine] = l;
         meet();
         l = side[par][0][mine] + side[par][1][mine];
-        ok = __all_sync(0xffffffffu, wait_or_give_up(&o_full[t], 0));
+        ok = __all_sync(0xffffffffu, wait_or_give_up(&o_full[t], 0, a.waits));
       }
       if (ok) {
         tc_fence_after();
@@ -374,6 +366,7 @@ int launch(const evo_window_attn_params* p, cudaStream_t st) {
   a.B = p->B; a.H = p->H; a.G = p->G; a.n_qblk = (int)((p->Lq + BQ - 1) / BQ); a.gate_per_head = p->gate_per_head;
   a.window = p->window > 0 ? (int)std::min<int64_t>(p->window, 1 << 30) : 0;
   a.scale2 = p->scale * 1.4426950408889634f;
+  if (const int rc_ = wait_limit(&a.waits)) return rc_;
   const int64_t heads = (int64_t)p->B * p->H, pairs = (a.n_qblk + 1) / 2, Lk = p->q_pos0 + p->Lq;
   // without a window the last heads' longest blocks would start when everything else is done: as many heads as keep their keys and values in half the L2 go together
   a.tail = p->window > 0 ? 1 : (int)std::min<int64_t>(heads, std::max<int64_t>(1, (64ll << 20) / (Lk * 4 * HD)));

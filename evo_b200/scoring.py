@@ -80,6 +80,8 @@ def score_sequences(seqs: List[str], model, tokenizer: CharLevelTokenizer, reduc
         else:
             logprobs = logits_to_logprobs(logits, input_ids, trim_bos=True).float()
     logprobs = logprobs.cpu().numpy()
+    if input_ids.is_cuda:
+        _lib.check_lost_waits()
     reduce = np.mean if reduce_method == "mean" else np.sum
     return [reduce(logprobs[i][:n]) for i, n in enumerate(lengths)]
 
@@ -93,6 +95,8 @@ def positional_entropies(seqs: List[str], model, tokenizer: CharLevelTokenizer, 
             logits, _ = model(input_ids)
         lp = torch.log_softmax(logits.float(), dim=-1)[:, :-1]
         ent = -(lp.exp() * lp).sum(dim=-1).cpu().numpy()
+    if input_ids.is_cuda:
+        _lib.check_lost_waits()
     out = [ent[i][:n] for i, n in enumerate(lengths)]
     if any(len(s) != len(e) for s, e in zip(seqs, out)):
         raise AssertionError("entropy length mismatch")

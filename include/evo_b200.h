@@ -120,6 +120,12 @@ int evo_gemm_smallm(const evo_gemm_smallm_params* p, void* stream);
  * evo_hyena_step (which fetches its filter parameters and states ahead of the wait).  Every decode-step kernel begins with griddepcontrol.launch_dependents and waits
  * (griddepcontrol.wait) before it first touches dependent data.  Process-wide switch; returns the previous value. */
 int evo_set_pdl(int level);
+/* Waits inside the kernels of evo_hyena_fwd, evo_gated_delta_fwd and evo_window_attn_fwd have a limit: one that runs out ends its CTA without writing a state, and the
+ * call's outputs are incomplete although it returned 0 (launches are asynchronous).  evo_lost_waits returns 1 if that has happened, on any device of the process, since the
+ * word was last cleared (clear != 0 does); it reads host memory, so ask after the work has been waited for. */
+int evo_lost_waits(int clear);
+/* Tries of such a wait in the launches of the CALLING THREAD (for tests: 0 lets every wait run out); negative restores the default.  Returns the previous value. */
+int evo_set_wait_polls(int polls);
 
 /* ---- fused Hyena operator: HyenaInferenceEngine.parallel_fir + ParallelHyenaFilter.
  * compute_filter + parallel_iir (+ prefill_via_modal_fft) of stripedhyena 0.2.2, as one

@@ -125,3 +125,17 @@ def test_hyena_workspace_of_an_empty_call_is_empty():
         "for B, L in ((0, 64), (0, 500), (0, 2000), (-1, 500), (1, 0), (1, 500)):\n"
         "    print(lib.evo_hyena_fwd_workspace(C.byref(HyenaParams(B=B, L=L, D=512, S=8, nheads=4))))\n")
     assert got[:5] == [0] * 5 and got[5] > 0
+
+
+def test_lost_waits_are_none_and_their_limit_belongs_to_the_thread():
+    import threading
+    lib = _lib.lib()
+    assert lib.evo_lost_waits(1) == 0
+    _lib.check_lost_waits()
+    default = lib.evo_set_wait_polls(5)
+    seen = []
+    t = threading.Thread(target=lambda: seen.append(lib.evo_set_wait_polls(7)))
+    t.start()
+    t.join()
+    assert seen == [default] and default > 1 << 16
+    assert lib.evo_set_wait_polls(-1) == 5 and lib.evo_set_wait_polls(default) == default
