@@ -592,6 +592,9 @@ Sizes sizes(const evo_gated_delta_params* p) {
   return s;
 }
 
+constexpr int scan_smem_bytes(int dk, int warps) { return 1024 + 2 * (2 * BT * dk * 2 + BT * warps * 32 + BLOCK_BYTES); }
+static_assert(scan_smem_bytes(128, 8) <= 227 * 1024, "two stages of eight warps");
+
 template <int DK>
 int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream_t st) {
   Args a = {};
@@ -608,7 +611,7 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   const int64_t warps = (int64_t)p->B * p->H * (p->dv / 16);
   int nw = 2;
   while (nw < 8 && nw * 16 < p->dv && warps > (int64_t)nw * device_sm_count()) nw *= 2;
-  const int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = 1024 + 2 * (2 * BT * DK * 2 + BT * nw * 32 + BLOCK_BYTES);
+  const int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = scan_smem_bytes(DK, nw);
   CUtensorMap tmK, tmQ, tmV;
   const uint64_t kdims[3] = {(uint64_t)p->G * DK, (uint64_t)p->L, (uint64_t)p->B}, vdims[3] = {(uint64_t)p->H * p->dv, (uint64_t)p->L, (uint64_t)p->B};
   const uint64_t strides[2] = {(uint64_t)p->ld * 2, (uint64_t)p->L * p->ld * 2};
@@ -616,8 +619,8 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   int rc;
   if ((rc = make_tmap_nd_bf16(&tmK, p->k, 3, kdims, strides, kbox, true)) || (rc = make_tmap_nd_bf16(&tmQ, p->q, 3, kdims, strides, kbox, true)) ||
       (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, false))) return rc;
-  EVO_CUDA(cudaFuncSetAttribute(delta_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem));
-  EVO_CUDA(cudaFuncSetAttribute(delta_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem));
+  static unsigned long long done_prep = 0, done_scan = 0;
+  if ((rc = ensure_dyn_smem(delta_prepare_kernel<DK>, prep_smem, done_prep)) || (rc = ensure_dyn_smem(delta_scan_kernel<DK>, scan_smem_bytes(DK, 8), done_scan))) return rc;
   for (int64_t first = 0; first < s.blocks; first += s.slab) {
     a.first = first; a.n_blocks = (int)std::min<int64_t>(s.slab, s.blocks - first);
     a.zero_start = first == 0 && (p->zero_start || !p->state);

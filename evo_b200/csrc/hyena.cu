@@ -315,7 +315,7 @@ int pick_segments(const evo_hyena_params* p) {
 }  // namespace
 
 // Which kernel, how many blocks per row (tensor-core path) and how many segments.
-struct HyenaPlan { bool tc; int R, nseg; long long seg_len; };
+struct HyenaPlan { bool tc; int R, nseg; long long seg_len; int scan_variant; };
 
 // The tensor-core path does the work of 256 R tokens x 32 channels per tile and item in a time that hardly depends on how many of the tokens exist, and computes its
 // constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 64: scan 14.9, tensor
@@ -324,18 +324,20 @@ struct HyenaPlan { bool tc; int R, nseg; long long seg_len; };
 HyenaPlan make_plan(const evo_hyena_params* p) {
   const long long L = p->L;
   const int sms = device_sm_count();
-  HyenaPlan best = {false, 0, pick_segments(p), 0};
+  HyenaPlan best = {false, 0, pick_segments(p), 0, 1};
   best.seg_len = (L + best.nseg - 1) / best.nseg;
   best.nseg = (int)((L + best.seg_len - 1) / best.seg_len);
   const char* env_v = getenv("EVO_B200_HYENA_VARIANT");      // comparisons: 0, 1 = the modal scans, 2 = tensor cores; read per call
   const int variant = env_v ? atoi(env_v) : -1;
+  best.scan_variant = variant == 0 ? 0 : 1;
   // taps, biases and carried inputs are read four channels at a time
   const bool can = use_tma_path(p) && L < (1ll << 30) && (((uintptr_t)p->fir_w | (uintptr_t)p->fir_b | (uintptr_t)p->halo) & 7) == 0;
   if (!can || variant == 0 || variant == 1) return best;
   const long long scan_ctas = (long long)p->D / evo_hy2::CH_PER_CTA * p->B * best.nseg;
   double cost = variant == 2 ? 1e30 : 7.0 + 0.116 * best.seg_len * (best.nseg > 1 ? 1.6 : std::max(1.0, (double)scan_ctas / sms));
-  const char* env_r = getenv("EVO_B200_HYENA_R");
   const double per_tile[3] = {5.7, 8.0, 14.4}, fill[3] = {6.0, 9.0, 9.0};
+  if (cost <= 8.0 + fill[0] + per_tile[0]) return best;      // a single tile costs more: short calls need no trial plans
+  const char* env_r = variant == 2 ? getenv("EVO_B200_HYENA_R") : nullptr;
   const long long items = (long long)p->D / evo_hytc::CH * p->B;
   for (int r = 0; r < 3; ++r) {
     const int R = 1 << r;
@@ -350,7 +352,7 @@ HyenaPlan make_plan(const evo_hyena_params* p) {
       const long long tiles = (std::min(len, L) + tile - 1) / tile, rounds = (items * nseg + sms - 1) / sms;
       double c = 8.0 + fill[r] + rounds * tiles * per_tile[r];
       if (nseg > 1) c += 4.0 + 0.5 * ((items * (nseg - 1) + sms - 1) / sms) * tiles * per_tile[r];
-      if (c < cost) { cost = c; best = {true, R, (int)nseg, len}; }
+      if (c < cost) { cost = c; best = {true, R, (int)nseg, len, 1}; }
     }
   }
   return best;
@@ -360,12 +362,12 @@ static size_t segment_bytes(const evo_hyena_params* p, int nseg) {
   return nseg <= 1 && !p->state_only ? 0 : (size_t)p->B * nseg * p->D * NS * 2 * sizeof(float);
 }
 
-extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) {
-  if (p->L <= 0 || p->B <= 0) return 0;
-  const HyenaPlan plan = make_plan(p);
-  // the tensor-core path keeps its channels' constants behind the segment states, on the next multiple of 256 bytes
+// the tensor-core path keeps its channels' constants behind the segment states, on the next multiple of 256 bytes
+static size_t workspace_bytes_of(const evo_hyena_params* p, const HyenaPlan& plan) {
   return segment_bytes(p, plan.nseg) + (plan.tc ? 256 + evo_hytc::table_bytes(p->D) : 0);
 }
+
+extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) { return p->L <= 0 || p->B <= 0 ? 0 : workspace_bytes_of(p, make_plan(p)); }
 
 // evo_hytc: constants, then (more than one segment) the segments' end states, then the output
 template <int R>
@@ -415,7 +417,7 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
   const HyenaPlan plan = make_plan(p);
   const int nseg = plan.nseg;
   const long long seg_len = plan.seg_len;
-  size_t need = evo_hyena_fwd_workspace(p);
+  const size_t need = workspace_bytes_of(p, plan);
   EVO_REQUIRE(workspace_bytes >= need && (need == 0 || workspace), "evo_hyena_fwd: workspace too small (%zu < %zu)", workspace_bytes, need);
   if (p->state_only) EVO_REQUIRE(p->state_out != nullptr, "evo_hyena_fwd: state_only needs state_out");
   else EVO_REQUIRE(p->y != nullptr, "evo_hyena_fwd: y is NULL");
@@ -438,16 +440,15 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     static unsigned long long done_s = 0, done_o = 0;
     if ((rc = ensure_dyn_smem(hyena_scan_tma_kernel<true>, smem_bytes(STAGES), done_s))) return rc;
     if ((rc = ensure_dyn_smem(hyena_scan_tma_kernel<false>, smem_bytes(STAGES), done_o))) return rc;
-    // 1 (default) = mode-split kernel (hyena_ms.cuh: 8 compute warps, 4 modal states per thread); 0 = round-1 kernel
-    // (4 compute warps, 8 states per thread), kept for A/B timing and as a second implementation in the parity tests
-    const char* env_v = getenv("EVO_B200_HYENA_VARIANT");
-    const int variant = env_v ? atoi(env_v) : 1;
+    // mode-split kernel (hyena_ms.cuh: 8 compute warps, 4 modal states per thread) or, for comparisons and as a second implementation in the parity tests,
+    // its predecessor (hyena_tma.cuh: 4 compute warps, 8 states per thread)
+    const bool split = plan.scan_variant != 0;
     static unsigned long long done_ms = 0, done_mo = 0;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<true>, smem_bytes(STAGES), done_ms))) return rc;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<false>, smem_bytes(STAGES), done_mo))) return rc;
-    dim3 grid(p->D / CH_PER_CTA, p->B, nseg), block(variant != 0 ? evo_hy3::THREADS : evo_hy2::THREADS);
-    auto k_state = variant != 0 ? evo_hy3::hyena_scan_ms_kernel<true> : hyena_scan_tma_kernel<true>;
-    auto k_out = variant != 0 ? evo_hy3::hyena_scan_ms_kernel<false> : hyena_scan_tma_kernel<false>;
+    dim3 grid(p->D / CH_PER_CTA, p->B, nseg), block(split ? evo_hy3::THREADS : evo_hy2::THREADS);
+    auto k_state = split ? evo_hy3::hyena_scan_ms_kernel<true> : hyena_scan_tma_kernel<true>;
+    auto k_out = split ? evo_hy3::hyena_scan_ms_kernel<false> : hyena_scan_tma_kernel<false>;
     // ring depth 4 (96 KB): two CTAs can co-reside and hide each other's latency when the grid exceeds the SM count.
     // An 8-deep ring for single-CTA-per-SM grids was measured and did not help (1.21 vs 1.06-1.13 ms at B=8, L=8193).
     a.nst = 4;

@@ -385,10 +385,10 @@ int launch(const evo_window_attn_params* p, cudaStream_t st) {
   if ((rc = make_tmap_nd_bf16(&tmK, p->k, 4, kd, s, box, true))) return rc;
   strides(s, p->v_tok_stride, p->v_batch_stride, Lk);
   if ((rc = make_tmap_nd_bf16(&tmV, p->v, 4, kd, s, box, true))) return rc;
-  const size_t smem = (size_t)BQ * HD * 2 * (2 + 2 * KV_STAGES) + 1024;
-  auto kern = window_attn_tc_kernel<HD>;
-  EVO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<(unsigned)(heads * pairs), THREADS, smem, st>>>(tmQ, tmK, tmV, a);
+  constexpr int smem = BQ * HD * 2 * (2 + 2 * KV_STAGES) + 1024;
+  static unsigned long long done = 0;
+  if ((rc = ensure_dyn_smem(window_attn_tc_kernel<HD>, smem, done))) return rc;
+  window_attn_tc_kernel<HD><<<(unsigned)(heads * pairs), THREADS, smem, st>>>(tmQ, tmK, tmV, a);
   return check_launch("evo_window_attn_fwd");
 }
 
