@@ -568,7 +568,8 @@ __global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restric
     for (int64_t c = (int64_t)H * (32 * N) + sub; c < ldo; c += 8) out[row * ldo + c] = __float2bfloat16_rn(0.f);
 }
 
-// Blocks whose T and P are in memory at a time: at most 256 MB of them (a longer call runs slab after slab).
+// Blocks whose T and P are in memory at a time: at most 256 MB of them, or one block of every (head, sequence) pair where that is more (32 KB each, above 8192 pairs).
+// A longer call runs slab after slab, the state carried in between.
 constexpr int64_t SLAB_BYTES = 256ll << 20;
 
 // Taken for bf16 heads of 64 or 128 key channels and a multiple of 16 value channels, rows that start on 16 bytes, and calls of 32 tokens or more.

@@ -579,7 +579,7 @@ typedef struct {
   int B; int64_t L; int H, G, dk, dv;
 } evo_gated_delta_params;
 /* workspace: evo_gated_delta_workspace() bytes (0 for a head whose tokens one CTA takes one by one; fp32 read-outs where its value channels are spread over several CTAs;
- * the blocks' matrices too, at most 256 MB of them at a time, where a prompt runs in 64-token blocks) */
+ * the blocks' matrices too where a prompt runs in 64-token blocks: at most 256 MB of them at a time, or 32 KB per head and sequence where that is more) */
 size_t evo_gated_delta_workspace(const evo_gated_delta_params* p);
 int evo_gated_delta_fwd(const evo_gated_delta_params* p, void* workspace, size_t workspace_bytes, void* stream);
 

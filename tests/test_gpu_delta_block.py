@@ -117,3 +117,27 @@ def test_decays_that_reach_zero_and_come_back():
     out, S, _ = _run(t, B, L, H, H, dk, dv)
     want, state = _oracle(t, B, L, H, H, dk, dv, 0)
     assert (out.double() - want).norm() <= 2.2e-3 * want.norm() and (S.double() - state).norm() <= 1e-6 * state.norm()
+
+
+@pytest.mark.parametrize("B,H,L", [(64, 32, 589), (300, 32, 130)])
+def test_slabs_hand_the_state_on(B, H, L):
+    """A call whose blocks' matrices pass 256 MB runs slab after slab: 4 + 4 + 2 blocks (the last one ragged), and one block at a time where a single one of every
+    (head, sequence) pair is more than that.  Bit for bit the sequences one by one (a single slab each), with a state carried, from zero, and with none given."""
+    G, dk, dv = 2, 64, 16
+    t = _inputs(B, L, H, G, dk, dv, seed=B)
+    one = lambda b: {k: (v[b * L:(b + 1) * L] if k in "xz" else v[b:b + 1] if k == "S" else v) for k, v in t.items()}  # noqa: E731
+    out, S, nb = _run(t, B, L, H, G, dk, dv)
+    block = 32768 * B * H                                                       # T, P and vectors of one block of every pair
+    assert nb - 4 * B * L * H * dv < max(256 << 20, block) + 1024 < (L + 63) // 64 * block
+    zero, S0, _ = _run(t, B, L, H, G, dk, dv, 1)
+    none, _, nb_none = _run(t, B, L, H, G, dk, dv, 1, state=False)
+    assert torch.equal(none, zero) and nb_none >= nb + 4 * B * H * dk * dv      # the state between the slabs is the workspace's
+    for b in (0, B // 2, B - 1):
+        o, s, _ = _run(one(b), 1, L, H, G, dk, dv)
+        assert torch.equal(out[b * L:(b + 1) * L], o) and torch.equal(S[b], s[0])
+        o, s, _ = _run(one(b), 1, L, H, G, dk, dv, 1)
+        assert torch.equal(zero[b * L:(b + 1) * L], o) and torch.equal(S0[b], s[0])
+    b = B // 3
+    want, state = _oracle(one(b), 1, L, H, G, dk, dv, 0)
+    assert (out[b * L:(b + 1) * L].double() - want).norm() <= 2.2e-3 * want.norm()
+    assert (S[b].double() - state[0]).norm() <= 1e-6 * state.norm()
