@@ -1,8 +1,8 @@
-"""bench.py — nucleotides/sec of the Evo-1 7B forward on B200 (BASELINE.json metric).
+"""bench.py — nucleotides/sec of the Evo-1 7B forward on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload 8k|131k|1k|32k|gen|zaverax|movalorn|nelovik|gakupel|gagotar|nilatar] [--impl ours|reference]
 
-Workload "8k" (default, BASELINE.json configs[1]): evo-1-8k-base scoring forward, batch 8 x
+Workload "8k" (default): evo-1-8k-base scoring forward, batch 8 x
 8192 nt of synthetic uniform ACGT (+BOS => L = 8193), bf16, random-init weights of the 7B
 architecture (no network for checkpoints).  One "step" = one forward over one batch.
   value : whole-job nt/s with the token ids already resident in HBM (model(input_ids)).
@@ -40,7 +40,7 @@ WORKLOADS = {
     "1k": dict(model="evo-1-8k-base", batch=64, nt=1024, desc="evo-1-8k-base 7B scoring forward, batch 64 x 1024 nt (+BOS), bf16"),
     "32k": dict(model="evo-1-131k-base", batch=2, nt=32768, desc="evo-1-131k-base 7B forward, batch 2 x 32768 nt (+BOS), bf16"),
     "131k": dict(model="evo-1-131k-base", batch=1, nt=131072, desc="evo-1-131k-base 7B forward, batch 1 x 131072 nt, bf16"),
-    # BASELINE configs[3] (secondary line, not the headline): cached generation, one step = one new nucleotide per sequence
+    # secondary line, not the headline: cached generation, one step = one new nucleotide per sequence
     "gen": dict(model="evo-1.5-8k-base", batch=16, nt=4096, desc="evo-1.5-8k-base 7B cached generation, batch 16, prompt 4096 nt, greedy decode steps, bf16"),
 }
 
@@ -299,7 +299,7 @@ def variant_of(model, model_name):
 
 
 def sp131k_record(model8k, world, rank, dev, steps, warmup, peaks):
-    """BASELINE.json configs[2]: evo-1-131k-base, batch 1 x 131072 nt, the sequence sharded over the `world` GPUs of the
+    """evo-1-131k-base, batch 1 x 131072 nt, the sequence sharded over the `world` GPUs of the
     box (strong scaling; world == 1: the plain single-GPU forward).  Timed like the main line; afterwards, outside the
     timed region, one instrumented step names where the time went (kernels and every communication piece) and every
     rank compares its shard of the logits with the UNSHARDED single-GPU forward of the same ids."""
@@ -356,7 +356,7 @@ def sp131k_record(model8k, world, rank, dev, steps, warmup, peaks):
 
 
 def sweep_record(model8k, dev, steps=3, warmup=1):
-    """BASELINE.json configs[4] at one GPU: the same 65 536-token budget as 1k and 32k sequences (8k is the headline `value`,
+    """One GPU: the same 65 536-token budget as 1k and 32k sequences (8k is the headline `value`,
     131k the `sp131k` record).  nt/s with ids resident in HBM, CUDA events around `steps` forwards."""
     import torch
     from evo_b200 import CharLevelTokenizer, prepare_batch
@@ -438,7 +438,7 @@ def bench_ours(args, wl):
     peaks = measured_peaks()
     sub = {}
     if args.workload == "8k" and not args.no_sub:
-        # BASELINE.json configs[2] next to the headline, at every N
+        # the 131k sequence next to the headline, at every N
         try:
             sub["sp131k"] = sp131k_record(model, world, rank, dev, steps=args.sub_steps, warmup=1, peaks=peaks)
         except Exception as ex:  # noqa  (a failed sub-record must not cost the headline line)
@@ -479,7 +479,7 @@ def bench_ours(args, wl):
 
 
 def generate_record(model, dev, peaks, steps=64, warmup=4, n_new=None, world=1, rank=0):
-    """cached generation, batch 16, prompt 4096 nt, greedy.  One step = one new nucleotide per
+    """Cached generation, batch 16, prompt 4096 nt, greedy.  One step = one new nucleotide per
     sequence through the L == 1 path (recurrent Hyena state + KV cache).
     value = generated nt/s with the state resident on the GPU; e2e = evo_b200.generate() from prompt strings to generated
     strings, the 4096-nt prefill and `n_new` decode steps included."""
@@ -489,7 +489,7 @@ def generate_record(model, dev, peaks, steps=64, warmup=4, n_new=None, world=1, 
     wl = WORKLOADS["gen"]
     tok = CharLevelTokenizer(512)
     B, P = wl["batch"], wl["nt"]
-    n_new = n_new if n_new is not None else P          # configs[3]: prefill 4096 + decode 4096
+    n_new = n_new if n_new is not None else P          # prefill 4096 + decode 4096
     seqs = synthetic_seqs(B, P, seed=rank)
     ids = torch.tensor([tok.tokenize(s) for s in seqs], dtype=torch.long, device=dev)
     d = model.initialize_inference_params()
@@ -832,7 +832,7 @@ def main():
     ap.add_argument("--no-sub", action="store_true", help="default workload only: skip the sp131k / gen sub-records")
     ap.add_argument("--no-gen", action="store_true", help="skip the cached-generation sub-record")
     ap.add_argument("--sub-steps", type=int, default=3, help="timed steps of the 131k sub-record")
-    ap.add_argument("--gen-tokens", type=int, default=None, help="new tokens of the end-to-end generate() run (default: 4096 = BASELINE configs[3])")
+    ap.add_argument("--gen-tokens", type=int, default=None, help="new tokens of the end-to-end generate() run (default: 4096)")
     args = ap.parse_args()
     if args.workload in ("zaverax", "movalorn", "nelovik", "gakupel", "gagotar", "nilatar"):
         return bench_arch(args)

@@ -13,9 +13,10 @@
 //   place as an MN-major B operand.
 //   Issue order per KV tile j:  PV_A(j) QK_A(j+1) PV_B(j) QK_B(j+1): while softmax A(j+1) runs, the tensor
 //   pipe has PV_B(j) and QK_B(j+1) to do, and vice versa.
-//   The MMA warp stays converged and one lane issues: with a branch around the issuing code every product cost 90 to 130 cycles of
-//   operand moves (64 on the tensor pipe), and the softmax waited for them (1 x 8193 tokens x 32 heads 534 -> 491 us, 2 x 4096 294 -> 271).
-//   Measured on B200: 1.01-1.12 PFLOP/s from 4096 tokens on (P aliases S, so QK(j+1) queues behind PV(j)).  Tried and rejected: a second TMEM pass over S instead
+//   The MMA warp stays converged and one lane issues: with a branch around the issuing code every product took that lane 90 to 130 cycles by clock
+//   stamps (64 on the tensor pipe), and the softmax waited for them (warm loop: 1 x 8193 tokens x 32 heads 534 -> 491 us, 2 x 4096 294 -> 271).
+//   Measured on B200: 1.01-1.12 PFLOP/s from 4096 tokens on in a warm loop, 0.95 for 1 x 8193 x 32 with cold L2 (576 us; P aliases S, so QK(j+1)
+//   queues behind PV(j)).  Tried and rejected: a second TMEM pass over S instead
 //   of holding the row in registers (0.50-0.57 PFLOP/s: tcgen05.ld bandwidth), a degree-3 FMA-pipe exp2 for half of
 //   the scores (0.82-0.96: issue slots, not MUFU, bind), 64-key tiles with double-buffered S (0.65-0.76).
 #include "common.cuh"
@@ -82,7 +83,7 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
 }
 
 // NPOLY: of every 8 score pairs, how many take exp2_poly2 instead of MUFU.EX2 (0 = variant 2; 3 = variant 3: MUFU and the FMA
-// pipe finish a tile's exponentials at about the same time, DESIGN 3.3)
+// pipe finish a tile's exponentials at about the same time)
 template <int NPOLY>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -156,8 +157,7 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
     }
   } else if (warp == 9) {
-    // ------------------------------------------------ MMA issuer: the whole warp waits, one lane issues; one copy of each product's loop (the softmax code fills the
-    // instruction cache: unrolled for two tiles and three places, this warp's fetches paced the kernel)
+    // ------------------------------------------------ MMA issuer: the whole warp waits, one lane issues (the same loop behind `if (lane == 0)`: 543 us for 491)
     {
       constexpr uint32_t idesc_qk = umma_idesc_bf16(BQ, BKV);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(BQ, HD) | (1u << 16);     // B (= V) is MN-major
@@ -343,8 +343,8 @@ int evo_attn_pp_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUt
                 "evo_attn_fwd: peer-scattered output needs B == 1, 1..8 peers covering Lq rows, 16-byte aligned strides");
   }
   static unsigned long long done0 = 0, done3 = 0;
-  // Head after head shares keys and values best, but the last head's longest CTAs would start when everything else is done (1 x 8193 tokens x 32 heads: 593 us, with
-  // the last heads taken together 533; 2 x 2325 x 16: 87 / 70; 8 x 8193 x 32 gains nothing).  As many heads as keep their keys and values in half the L2 (64 MB).
+  // Head after head shares keys and values best, but the last head's longest CTAs would start when everything else is done (warm loop, 1 x 8193 tokens x 32 heads: 593 us,
+  // with the last heads taken together 533; 2 x 2325 x 16: 87 / 70; 8 x 8193 x 32 gains nothing).  As many heads as keep their keys and values in half the L2 (64 MB).
   const long long heads = (long long)p->B * p->H, pairs = (a.n_qblk + 1) / 2;
   a.tail = (int)std::min(heads, std::max<long long>(1, (64ll << 20) / std::max<long long>(1, p->Lk * 512)));
   EVO_REQUIRE(heads * pairs < (1ll << 31), "evo_attn_fwd: too many blocks");

@@ -1,7 +1,7 @@
 // Decode-step kernels (one new token per sequence): everything a CUDA-graph replay of the
 // step needs, with the sequence position read from DEVICE memory so the same captured graph
 // serves every step (the reference re-launches ~20 tiny kernels per layer per token from
-// Python, SURVEY.md 8a row a9/a12).
+// Python).
 #include "common.cuh"
 #include "../../include/evo_b200.h"
 #include <cstdlib>

@@ -287,7 +287,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       int stage = 0; uint32_t phase = 0;
       const uint32_t full_leader_mask = 0xFEFFFFFFu;   // shared::cluster address of the pair leader's copy
       // L2 eviction priorities (experiment, EVO_B200_GEMM_L2_HINTS; default 0 = plain loads).  1: resident slab evict_last, streaming
-      // operand evict_first -- measured WORSE on B200 (profiles/r02_gemm_l2_hints_call11.txt: DRAM bytes 5.5 -> 10.6 GB for the
+      // operand evict_first -- measured WORSE on B200 (DRAM bytes 5.5 -> 10.6 GB for the
       // projection, 89.2 -> 84.0 k nt/s): an evict_first tile is dropped before the other CTAs of the wave have fetched it.
       // 2: only the slab is marked (evict_last), the stream keeps the default policy.
       const uint64_t keep = l2_policy_evict_last(), first = g.l2_hints == 1 ? l2_policy_evict_first() : l2_policy_evict_normal();
@@ -475,8 +475,7 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
     const double a_blk = (double)BM * CG * p->K * 2, w_blk = (double)BN * p->K * 2;
     const double a_tot = (double)p->M * p->K * 2, w_tot = (double)p->N * p->K * 2, budget = 40e6;
     // a short last group (16 column-blocks in groups of 7 leave 2) sweeps the other operand almost unshared: use one group
-    // fewer when that stretches the slab by <= 20 %, else spread the blocks evenly (profiles/r02_gemm_raster_sweep_call25.txt:
-    // K = 11008, groups 7+7+2 -> 8+8: DRAM reads 12.2 -> 10.2 GB, 2.4 % faster under ncu)
+    // fewer when that stretches the slab by <= 20 %, else spread the blocks evenly (K = 11008, groups 7+7+2 -> 8+8: DRAM reads 12.2 -> 10.2 GB, 2.4 % faster under ncu)
     static const char* env_b = getenv("EVO_B200_GEMM_REBALANCE");     // experiments only: 0 restores the plain budget rule
     auto balanced = [](int blocks, int gmax) {
       if (env_b && atoi(env_b) == 0) return gmax;
@@ -495,7 +494,7 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
     g.l2_hints = (BN == BN_BIG && env_h) ? atoi(env_h) : 0;
     const char* env_s = getenv("EVO_B200_GEMM_SKEW");               // experiments only (read per launch)
     g.skew = (BN == BN_BIG && env_s) ? atoi(env_s) : 0;
-    const char* env_g = getenv("EVO_B200_GEMM_GROUP");      // experiments only (read per launch: tools/gemm_raster_sweep.py changes them)
+    const char* env_g = getenv("EVO_B200_GEMM_GROUP");      // experiments only (read per launch: a sweep changes them)
     const char* env_r = getenv("EVO_B200_GEMM_RASTER_N");
     if (env_r) g.raster_n = atoi(env_r);
     if (env_g) g.group_m = std::max(1, atoi(env_g));
@@ -515,8 +514,8 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
     int pairs = min(n_tiles, sms / 2);
     // Die-aware rasterisation (see the kernel's tile walk; EVO_B200_GEMM_DIE_RASTER=0 turns it off, 2 is a test hook): a full
     // grid of pairs, enough row-blocks for both dies, and a self-consistent SM -> die map of this device.  m_split balances the two
-    // dies' wave counts.  In-step +2.0 / +2.7 % on the 8k workload (profiles/r02_gemm_die_raster_call28.txt).
-    const char* env_d = getenv("EVO_B200_GEMM_DIE_RASTER");          // read per launch (tools/gemm_raster_sweep.py toggles it)
+    // dies' wave counts.  In-step +2.0 / +2.7 % on the 8k workload.
+    const char* env_d = getenv("EVO_B200_GEMM_DIE_RASTER");          // read per launch
     const int die_mode = env_d ? atoi(env_d) : 1;
     if (BN == BN_BIG && die_mode != 0 && pairs == sms / 2 && g.m_blocks >= 32) {
       const DieMap* dm = die_map(st);
@@ -597,7 +596,7 @@ extern "C" int evo_gemm(const evo_gemm_params* p, void* stream) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fused scoring head (SURVEY 8f-1): unembed GEMM + log-softmax + gather (+ entropy); the (M, V) logits never reach HBM.
+// Fused scoring head: unembed GEMM + log-softmax + gather (+ entropy); the (M, V) logits never reach HBM.
 // The GEMM's epilogue leaves one float4 of statistics per (row, 256-column half); the finish kernel folds the halves:
 //   lse = M + log(sum_j s_j e^(m_j - M)),  logprob = x_target - lse,  entropy = lse - (sum_j w_j e^(m_j - M)) / S.
 // ---------------------------------------------------------------------------------------------

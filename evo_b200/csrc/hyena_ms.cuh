@@ -1,9 +1,9 @@
-// Hyena scan, mode-split variant (round 2): the production path for head_dim 128 / D % 256 == 0.
+// Hyena scan, mode-split variant: short sequences with head_dim 128 and D % 256 == 0 (longer ones: hyena_tc.cuh).
 //
 // Same operator, same rounding points and the same TMA ring as hyena_scan_tma_kernel (hyena_tma.cuh); what changes
 // is the work assignment, because that kernel was latency-starved, not bandwidth- or pipe-bound: 128 CTAs x 4
-// compute warps = ONE warp per SM sub-partition, 214 registers per thread, fma pipe 55 % busy, issue slots 47 %
-// (profiles/r01_ncu_full_hyena_call5.csv).  Here
+// compute warps = ONE warp per SM sub-partition, 214 registers per thread, fma pipe 55 % busy, issue slots 47 %.
+// Here
 //   * a thread still carries a channel PAIR (so every fp32 op stays a packed FFMA2 -- the only way to the FP32
 //     pipe's 128 lanes/SM/clk), but only FOUR of the eight modal states: lanes l and l^16 of a warp share a pair.
 //     Registers per thread drop to ~half and a 256-channel CTA has 8 compute warps = two per sub-partition, so a

@@ -1,4 +1,4 @@
-// Batch front-end on the device (SURVEY 8f-4): raw sequence bytes -> padded token-id matrix.
+// Batch front-end on the device: raw sequence bytes -> padded token-id matrix.
 //
 // The reference's prepare_batch (evo/scoring.py:9-33) tokenises on the host into Python lists, builds one int64 tensor per
 // sequence and copies each to the GPU separately.  Here the host ships the concatenated bytes once (1 byte per

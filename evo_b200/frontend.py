@@ -1,4 +1,4 @@
-"""Batch front-end (SURVEY.md 8f-4): sequences on disk -> padded id matrices on the GPU, in length buckets.
+"""Batch front-end: sequences on disk -> padded id matrices on the GPU, in length buckets.
 
 What it replaces in the reference:
   * scripts/score.py:40-55       Bio.SeqIO FASTA parse + fixed-size batches in file order (one pad-to-longest per batch)

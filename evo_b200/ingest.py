@@ -1,4 +1,4 @@
-"""Streaming checkpoint ingest (SURVEY.md 8f-3): safetensors shards -> the model's device tensors, tensor by tensor.
+"""Streaming checkpoint ingest: safetensors shards -> the model's device tensors, tensor by tensor.
 
 The reference (evo/models.py:96-150) materialises the whole checkpoint as a host state dict (`load_file` per shard),
 builds the model on the CPU, `load_state_dict`s (a second full copy), casts to bf16 on the CPU and only then moves

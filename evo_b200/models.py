@@ -85,7 +85,7 @@ def load_checkpoint(model_name: str = "evo-1-8k-base", config_path: Optional[str
         model.load_state_dict(state, strict=True)
         model.to_bfloat16_except_poles_residues()
         return model if device is None else model.to(device)
-    # streaming ingest (SURVEY 8f-3): parameters are allocated once, on the target device, in their final dtype and layout;
+    # streaming ingest: parameters are allocated once, on the target device, in their final dtype and layout;
     # each checkpoint tensor goes mmap -> pinned staging -> device and is cast / packed there (evo_b200/ingest.py)
     from .ingest import load_streaming
     dev = torch.device(device) if device is not None else torch.device("cpu")

@@ -1,7 +1,7 @@
 """Sequence-parallel StripedHyena forward for contexts that do not fit / are too slow on one
-GPU (BASELINE.json configs[2]: evo-1-131k-base, batch 1 x 131072 nt over 8 B200).
+GPU (evo-1-131k-base, batch 1 x 131072 nt over 8 B200).
 
-The reference has no multi-GPU code at all (SURVEY.md section 5); this is new.  One process per
+The reference has no multi-GPU code at all; this is new.  One process per
 GPU, weights replicated, every rank holds a contiguous slice of the sequence.  Token-local
 work (embedding, RMSNorm, every GEMM, the gated MLP, unembed) needs no communication.
 
@@ -30,8 +30,7 @@ from ._lib import EPI_BIAS, EPI_BIAS_RESID, EPI_BIAS_ROPE, EPI_NONE, EPI_RESID, 
 
 
 # attention re-shard through our own NVLink peer stores (PeerUlysses) instead of NCCL all-to-alls; "0" = NCCL Ulysses.
-# Validated on 2 and 8 GPUs (profiles/r02_seqpar_check_{2gpu_peer_ulysses_call10,8gpu_call13}.json: identical to the NCCL path on
-# every rank; r02_sp{2,8}_peer_ulysses_ab_*.txt: 0.3-1.4 % faster on one box).
+# Validated on 2 and 8 GPUs: identical to the NCCL path on every rank, 0.3-1.4 % faster on one machine.
 PEER_ULYSSES = os.environ.get("EVO_B200_PEER_ULYSSES", "1") != "0"
 
 

@@ -7,7 +7,7 @@ copy of 1 byte per nucleotide and the id matrix is built on the GPU (the referen
 copy per sequence, :22-30); score_sequences / positional_entropies read log-likelihood and entropy
 from the fused scoring head (model.score_tokens: unembed GEMM + log-softmax + gather in one kernel,
 the (B, L, 512) logits are never written; fp32 statistics instead of the reference's bf16
-log_softmax, quirk Q4 in SURVEY.md 8c)."""
+log_softmax, quirk Q4)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -70,7 +70,7 @@ def score_sequences(seqs: List[str], model, tokenizer: CharLevelTokenizer, reduc
         raise ValueError(f"Invalid reduce_method {reduce_method}")
     input_ids, lengths = prepare_batch(seqs, tokenizer, device=device, prepend_bos=True)
     if hasattr(model, "score_tokens") and input_ids.is_cuda:
-        # fused head: unembed + log-softmax + gather in the GEMM epilogue, logits never written (SURVEY 8f-1)
+        # fused head: unembed + log-softmax + gather in the GEMM epilogue, logits never written
         logprobs = model.score_tokens(input_ids, want_logprobs=True)[0][:, :-1]
     else:
         with torch.inference_mode():

@@ -1,6 +1,6 @@
 """`StripedHyena` with the object protocol evo-design/evo relies on, executed by libevo_b200.so.
 
-Boundary obligations (SURVEY.md section 8b), each pinned by a reference call site:
+Boundary obligations, each pinned by a reference call site:
   StripedHyena(cfg)                                  evo/models.py:146
   .load_state_dict(sd, strict=True) with HF names    evo/models.py:124-147
   .to_bfloat16_except_poles_residues(); .to(device)  evo/models.py:148-150
@@ -29,9 +29,9 @@ from ..engine import KernelOps
 from .cache import InferenceParams, RecurrentInferenceParams
 
 # kernel variants (see include/evo_b200.h); overridable for experiments
-# measured on B200, same box, interleaved A/B inside the power-capped 0.7 s step (profiles/r01_gemm_variant_ab_call32.txt):
+# measured on B200, same box, interleaved A/B inside the power-capped 0.7 s step:
 # the 2-CTA 256x256 tile (variant 0) gives 93.1-93.2 k nt/s against 88.3-88.5 k for the 1-CTA 128x256 tile -- each CTA
-# stages 32 KB instead of 48 KB per k-block, so the same FLOPs cost less operand traffic and power.  (An early-round
+# stages 32 KB instead of 48 KB per k-block, so the same FLOPs cost less operand traffic and power.  (An early
 # comparison had the 1-CTA tile ahead by 2 %; that was before the traffic-aware rasterisation and with a
 # release.cluster arrive in the pair's epilogue.)
 GEMM_VARIANT = int(os.environ.get("EVO_B200_GEMM_VARIANT", "0"))
@@ -75,7 +75,7 @@ def unpack_w12(w12: torch.Tensor, inner: int):
 
 
 class _GatedMLP(nn.Module):
-    """ParallelGatedMLP parameters, held ONLY in the layouts the GEMMs read (SURVEY 8f-3: no second copy):
+    """ParallelGatedMLP parameters, held ONLY in the layouts the GEMMs read (no second copy):
       w12 (2*ipad, D)  l1 / l2 interleaved per 128 rows, zero-padded 10928 -> 11008 (pack_w12)
       w3  (D, ipad)    l3 zero-padded along K
     The checkpoint's key names (mlp.l1.weight, mlp.l2.weight, mlp.l3.weight; evo/models.py:124-147) are what state_dict()
@@ -142,8 +142,8 @@ class _HyenaFilter(nn.Module):
 
 class _Rotary(nn.Module):
     """Carrier of `inv_freq`.  flash_attn registers it as a NON-persistent buffer (layers/rotary.py:366); stripedhyena re-registers it
-    as a persistent one, so its checkpoints carry `...rotary_emb.inv_freq`.  That second fact is recalled, not verified here (SURVEY.md
-    A.7), so loading accepts both: a checkpoint value is used when present, the constructor's analytic value when absent -- what the
+    as a persistent one, so its checkpoints carry `...rotary_emb.inv_freq`.  That second fact is recalled, not verified here,
+    so loading accepts both: a checkpoint value is used when present, the constructor's analytic value when absent -- what the
     reference ends up with in either world."""
 
     def __init__(self, head_dim, base):
@@ -226,7 +226,7 @@ class StripedHyena(KernelOps, nn.Module):
         # programmatic dependent launch inside a decode step (evo_set_pdl): 0 off, 1 every kernel, 2 weight-streaming GEMMs only
         self.decode_pdl = int(os.environ.get("EVO_B200_DECODE_PDL", "4"))
         # the Hyena decode step inside the in-projection GEMM's epilogue (EVO_EPI_HYENA_STEP).  Bit-identical to the separate
-        # evo_hyena_step launch but SLOWER on B200 (5.12 vs 4.30 ms/step at batch 16, profiles/r02_decode_fused_step_call8.txt): the
+        # evo_hyena_step launch but SLOWER on B200 (5.12 vs 4.30 ms/step at batch 16): the
         # step of a tile runs on the 128 epilogue threads of its last contributor -- 16 batch rows x 8 states of dependent
         # load -> update -> store per thread in the GEMM's serial tail -- where the stand-alone kernel spreads the same 8 MB of state
         # traffic over 524 288 threads.  Off by default; kept as a tested option.
@@ -471,7 +471,7 @@ class StripedHyena(KernelOps, nn.Module):
         return u
 
     def score_tokens(self, input_ids, want_logprobs=True, want_entropy=False):
-        """Fused scoring head (SURVEY 8f-1): what evo/scoring.py computes from `model(input_ids)` -- log_softmax of the
+        """Fused scoring head: what evo/scoring.py computes from `model(input_ids)` -- log_softmax of the
         logits gathered at the NEXT token (logits_to_logprobs, :36-59) and the per-position entropy (:119-121) -- without
         the (B, L, 512) logits ever reaching HBM: the unembed GEMM's epilogue keeps max / sum-exp / sum-exp*logit / target
         logit per row (evo_unembed_score).  Returns (logprobs (B, L) fp32 or None, entropy (B, L) fp32 or None);
@@ -618,7 +618,7 @@ class StripedHyena(KernelOps, nn.Module):
         lin(u, tiled["unembed"] if tiled is not None else self.unembed.weight, logits, V, d, EPI_NONE)
         return logits
 
-    # ---- on-device generation loop (SURVEY 8f-2): token pick + bookkeeping + feedback inside the captured step ------
+    # ---- on-device generation loop: token pick + bookkeeping + feedback inside the captured step ------
     def decode_loop(self, first_token, ipd, n_steps, start_pos, *, top_k=1, top_p=0.0, temperature=1.0, forced=None, n_out=None, seed=None):
         """Run `n_steps` single-token steps without returning to the host in between.
 

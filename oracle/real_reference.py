@@ -1,8 +1,8 @@
 """Bridge to the REAL `stripedhyena` package, for the day it is importable next to this repo.
 
 TEST INFRASTRUCTURE ONLY (same rule as stripedhyena_oracle.py: only tests/, __graft_entry__.smoke() and bench.py's CPU legs may
-import this).  stripedhyena==0.2.2 (/root/reference/requirements.txt:1) holds the arithmetic of the reference path and could be
-obtained neither in the build container nor on the GPU boxes (profiles/r02_pin_attempt_call1.log), so NOTHING in this file has run
+import this).  stripedhyena==0.2.2 (requirements.txt:1) holds the arithmetic of the reference path and could
+not be obtained here, so NOTHING in this file has run
 against the real package: it is written from the package's published interface -- `stripedhyena.model.StripedHyena(config)`,
 `.load_state_dict(sd, strict=True)`, `.to_bfloat16_except_poles_residues()`, `model(ids, inference_params_dict=...)`,
 `.initialize_inference_params()`, `stripedhyena.utils.dotdict` (the call sites evo/models.py:141-150, evo/scoring.py:81,
@@ -11,8 +11,8 @@ What it is for:
   * `available()`      is the package importable?
   * `build(...)`       the real model on CPU: flash kernels off (use_flash_attn / use_flash_rmsnorm / use_flash_depthwise /
                        use_flashfft False -- the torch branches), and the one statement of flash_attn's rotary that is a Triton
-                       kernel replaced by flash_attn's own torch statement of it (SURVEY.md 8c names both patches);
-  * `compare(...)`     SURVEY.md A.9's verify-first checklist: same weights into the real model and into the oracle, logits of the
+                       kernel replaced by flash_attn's own torch statement of it;
+  * `compare(...)`     the verify-first checklist: same weights into the real model and into the oracle, logits of the
                        stateless forward, of a prefill and of single-token steps, and the recurrent states, side by side;
                        tests/test_oracle.py::test_oracle_against_the_real_stripedhyena_package asserts on it whenever the
                        package is present (and is skipped, saying so, when it is not) -- that test passing is what would remove

@@ -4,13 +4,11 @@ TEST INFRASTRUCTURE ONLY.  Nothing under ``evo_b200/`` may import this module;
 only ``tests/``, ``__graft_entry__.smoke()`` and ``bench.py``'s CPU-baseline /
 ``--impl reference`` legs do, and there only as the checker / the CPU arm.
 
-PARITY UNPINNED (stated as the task requires): the arithmetic of the reference
+PARITY UNPINNED: the arithmetic of the reference
 path lives in the third-party package ``stripedhyena==0.2.2`` (pinned at
-/root/reference/requirements.txt:1 and environment.yml:10), which is neither
-vendored in /root/reference nor installed in the build container -- nor obtainable on the
-GPU box (round 2: no package index, no wheel in /opt/wheelhouse, no HF cache; log in
-profiles/r02_pin_attempt_call1.log) -- and the reference repository has no tests, golden
-vectors or fixtures for this path (SURVEY.md section 4, section 8c).  This file therefore RESTATES the published
+requirements.txt:1 and environment.yml:10), which is neither
+vendored in the reference nor installed or obtainable here -- and the reference repository has no tests, golden
+vectors or fixtures for this path.  This file therefore RESTATES the published
 algorithm of stripedhyena 0.2.2 (model.py / engine.py / layers.py / cache.py /
 sample.py / positional_embeddings.py of github.com/togethercomputer/stripedhyena
 at the 0.2.x tag) in plain PyTorch, anchored on the reference's call sites:
@@ -23,7 +21,7 @@ at the 0.2.x tag) in plain PyTorch, anchored on the reference's call sites:
   evo/generation.py:162   stripedhyena.sample.sample(...)
 
 What IS run from the reference itself: the host code around the model call.  tests/golden/
-make_reference_host_golden.py imports /root/reference/evo/{tokenizer,scoring,generation,models}.py,
+make_reference_host_golden.py imports evo/{tokenizer,scoring,generation,models}.py,
 scripts/{score,generate}.py and semantic_design/semantic_design.py unmodified (a stand-in satisfies
 their `import stripedhyena`) and drives them with THIS model; tests/golden/reference_host.{json,npz}
 hold what they returned.  That pins evo_b200's host layer, not this file's arithmetic.
@@ -53,7 +51,7 @@ import torch
 import torch.nn.functional as F
 
 # --------------------------------------------------------------------------
-# Config (keys: /root/reference/evo/configs/evo-1-8k-base_inference.yml:1-38,
+# Config (keys: evo/configs/evo-1-8k-base_inference.yml:1-38,
 #         evo-1-131k-base_inference.yml:39-40)
 # --------------------------------------------------------------------------
 
@@ -104,7 +102,7 @@ def mlp_inner_size(cfg) -> int:
 
 # --------------------------------------------------------------------------
 # State dict (key names = HF checkpoint after the 'backbone.' strip,
-# /root/reference/evo/models.py:124-137)
+# evo/models.py:124-137)
 # --------------------------------------------------------------------------
 
 def state_dict_spec(cfg) -> Dict[str, tuple]:
@@ -140,7 +138,7 @@ def state_dict_spec(cfg) -> Dict[str, tuple]:
 
 def random_state_dict(cfg, seed: int = 0, dtype=torch.bfloat16, share_blocks: bool = False) -> Dict[str, torch.Tensor]:
     """Random-init weights with sane activation scales.  Poles are drawn inside the
-    unit disc (|p| in [0.5, 0.999], random phase) as SURVEY.md section 8d prescribes.
+    unit disc (|p| in [0.5, 0.999], random phase) as the workloads prescribe.
     Everything is `dtype` except poles/residues (fp32), mirroring
     to_bfloat16_except_poles_residues (evo/models.py:148).  share_blocks=True makes
     every block of a kind alias block 0's tensors (CPU-baseline timing with a
@@ -193,7 +191,7 @@ def random_state_dict(cfg, seed: int = 0, dtype=torch.bfloat16, share_blocks: bo
 
 # --------------------------------------------------------------------------
 # Inference-state holders (stripedhyena cache.py; attribute names pinned by
-# /root/reference/evo/generation.py:109-119,140-148)
+# evo/generation.py:109-119,140-148)
 # --------------------------------------------------------------------------
 
 @dataclass

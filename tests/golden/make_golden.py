@@ -5,8 +5,8 @@
    382-416), apply_rotary_emb_torch (layers/rotary.py:23-35) and SelfAttention (modules/
    mha.py:230-279).  These pin the oracle's rotary/attention restatement to the real thing.
 2. tiny_model_oracle.npz -- ids + fp64 logits + prefill states of the oracle on a 3-layer
-   model (Hyena, attention, Hyena).  stripedhyena itself is not importable here (SURVEY.md
-   section 0.1), so this fixture guards the oracle against regressions; it does not pin it.
+   model (Hyena, attention, Hyena).  stripedhyena itself is not importable here,
+   so this fixture guards the oracle against regressions; it does not pin it.
 
 3. kvcache_sampling_flash_attn.npz -- flash_attn's _update_kv_cache, CrossAttention(causal=True) and utils.generation.sample
    run on CPU (see kvcache_and_sampling_fixture).
@@ -122,7 +122,7 @@ def mha_block_fixture():
     AttentionBlock configures it (causal, qkv and out-proj bias, rotary over the full head_dim 128, use_flash_attn=False -- the
     torch SelfAttention / CrossAttention branch): stateless over 8 tokens; then with flash_attn's InferenceParams a 6-token
     prefill and two single-token steps (rotary at seqlen_offset with the table built to max_seqlen, _update_kv_cache,
-    cache-form attention).  ONE patch, the one SURVEY.md 8c names: RotaryEmbedding.forward ends in a Triton kernel that cannot run
+    cache-form attention).  ONE patch: RotaryEmbedding.forward ends in a Triton kernel that cannot run
     on CPU, so `apply_rotary_emb_qkv_` is replaced by flash_attn's own torch statement of it (apply_rotary_emb_torch on q and k at
     cos/sin[offset : offset + L]); everything else -- Wqkv, the `(three h d)` split, the cos/sin cache, the cache write, the masks,
     out_proj -- is flash_attn's code as installed."""

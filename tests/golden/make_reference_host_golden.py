@@ -1,11 +1,11 @@
 """Generates tests/golden/reference_host.{json,npz}: outputs of the REFERENCE'S OWN host code, run in the build container.
 
-What is pinned.  /root/reference/evo/{tokenizer,scoring,generation,models}.py are the reference for everything on either
-side of the model call (SURVEY.md 8b, 8f-1..4): tokenisation, batch preparation, the logits -> log-likelihood / entropy
+What is pinned.  evo/{tokenizer,scoring,generation,models}.py are the reference for everything on either
+side of the model call: tokenisation, batch preparation, the logits -> log-likelihood / entropy
 reductions, the generation loop's state protocol (which slices of the prompt the model sees and which `seqlen_offset` it is
 handed at every call, quirks Q1-Q4 included) and checkpoint ingest (HF repo / revision, 'backbone.' strip, tied unembed,
 YAML config, strict load, dtype policy call order).  Those files import `stripedhyena`, which does not exist here
- -- so this script registers a stand-in `stripedhyena` package whose `StripedHyena` is a recorder, whose
+-- so this script registers a stand-in `stripedhyena` package whose `StripedHyena` is a recorder, whose
 `sample` is flash_attn.utils.generation.sample (installed here; the function stripedhyena/sample.py copies) and whose `dotdict`
 is a plain attribute dict, imports the reference's modules UNMODIFIED from /root/reference, and drives them on CPU with the
 oracle model (oracle/stripedhyena_oracle.py) standing where the real model would.
@@ -14,7 +14,7 @@ What is NOT pinned by this: the model arithmetic (the oracle stays a restatement
 The fixtures pin the host layer: tests/test_reference_host_golden.py runs evo_b200's host code over the SAME oracle model and
 must reproduce every id, call, string and score; the GPU tests compare the CUDA path's scores with the fp64 numbers.
 
-    python tests/golden/make_reference_host_golden.py        (build container only: needs /root/reference)
+    python tests/golden/make_reference_host_golden.py        (needs the reference's files at REFERENCE below)
 """
 import hashlib
 import json
@@ -266,7 +266,7 @@ def checkpoint_cases(RM):
 
 
 def _load_reference_script(name):
-    """A file under /root/reference/scripts as a module of its own (the repo has a `scripts` package of the same name)."""
+    """A file of the reference's scripts folder as a module of its own (the repo has a `scripts` package of the same name)."""
     import importlib.util
     spec = importlib.util.spec_from_file_location("reference_scripts_" + name, os.path.join(REFERENCE, "scripts", name + ".py"))
     mod = importlib.util.module_from_spec(spec)
@@ -375,7 +375,7 @@ def bucketing_cases():
 
 def main():
     if not os.path.isdir(os.path.join(REFERENCE, "evo")):
-        raise SystemExit("needs /root/reference (build container only)")
+        raise SystemExit("needs the reference's files")
     install_stand_in()
     sys.path.insert(0, REFERENCE)
     import evo.generation as RG

@@ -1,10 +1,10 @@
-"""GPU bring-up / diagnostics harness (development tool, run under gpurun).
+"""GPU bring-up / diagnostics harness (development tool; needs a GPU).
 
     python tests/harness/gpu_bringup.py                 # all stages, each in its own subprocess + timeout
     python tests/harness/gpu_bringup.py --stage gemm1   # one stage inline
 
 Every stage compares the CUDA kernels with the CPU oracle (and with torch-on-GPU where that
-is a useful second opinion) and appends JSON lines to gpurun_out/bringup.jsonl, so a hang
+is a useful second opinion) and appends JSON lines to bringup.jsonl in $EVO_BRINGUP_OUT (default: the working folder), so a hang
 or crash in one stage cannot hide the results of the others."""
 from __future__ import annotations
 
@@ -19,7 +19,7 @@ import time
 
 ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 sys.path.insert(0, ROOT)
-OUT = os.path.join(ROOT, "gpurun_out")
+OUT = os.environ.get("EVO_BRINGUP_OUT", ".")
 os.makedirs(OUT, exist_ok=True)
 
 STAGES = ["elementwise", "hyena", "gemm1", "gemm2", "attn0", "attn1", "attn2", "model", "perf_gemm", "perf_hyena", "perf_attn"]
@@ -388,7 +388,7 @@ def stage_perf_attn():
 
 
 def stage_perf_decode():
-    """BASELINE configs[3]: evo-1.5-8k-base generate, batch 16, prompt 4096 + decode (recurrent state path)."""
+    """evo-1.5-8k-base generate, batch 16, prompt 4096 + decode (recurrent state path)."""
     from evo_b200.models import load_checkpoint
     dev = "cuda:0"
     m = load_checkpoint("evo-1.5-8k-base", device=dev, random_init=True, seed=0)

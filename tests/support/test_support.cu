@@ -1,6 +1,6 @@
 // Test-support library (tests/support/libevo_b200_test.so) -- NOT part of the product.
 // Comparators the GPU tests check the product kernels against, kept out of libevo_b200.so and out
-// of include/evo_b200.h (VERDICT r1 weak #12): a cuBLASLt GEMM, a one-warp-per-row CUDA-core
+// of include/evo_b200.h: a cuBLASLt GEMM, a one-warp-per-row CUDA-core
 // attention and a bf16 add.  Built by evo_b200/build.py:build_test_support(); links cuBLASLt
 // (the product library does not).
 #include <cuda_runtime.h>

@@ -1,4 +1,4 @@
-"""GPU side of the batch front-end and of the streaming checkpoint ingest (SURVEY 8f-3, 8f-4): integer / byte work, so
+"""GPU side of the batch front-end and of the streaming checkpoint ingest: integer / byte work, so
 everything here is BIT-EXACT against the host implementations that mirror the reference (evo/scoring.py:9-33
 prepare_batch; evo/models.py:96-150 load sequence)."""
 import json

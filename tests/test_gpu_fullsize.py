@@ -1,4 +1,4 @@
-"""Parity at BASELINE.json's sizes with the kernel variants the product ships:
+"""Parity at the full sizes with the kernel variants the product ships:
 the default GEMM (variant 0, 2-CTA 256x256 tiles), the default attention (variant 2, ping-pong), the default Hyena
 scan (mode-split) -- each against the CPU oracle on the same seeded inputs, at the 7B width and the 8k / 16k / 131k
 lengths; plus the fused scoring head and an end-to-end bound on the quantity evo/scoring.py returns.
@@ -118,7 +118,7 @@ def test_hyena_7b_width_8193_vs_oracle():
 
 @pytest.mark.parametrize("nseg", [0, 1])
 def test_hyena_131072_tokens_poles_near_the_unit_circle(nseg):
-    """L = 131 072 (BASELINE configs[2]) on a 256-channel slice with pole magnitudes up to 0.9999 -- filter memories of
+    """L = 131 072 on a 256-channel slice with pole magnitudes up to 0.9999 -- filter memories of
     ~10^5 tokens, the regime where an fp32 recurrence and an fp32 FFT could part ways.  nseg = 0: the launcher's own
     segmentation (16 CTAs x segments + carry pass), 1: one sequential scan."""
     D, H, B, L = 256, 2, 1, 131072
@@ -193,7 +193,7 @@ def test_rotary_scaled_16_plus_attention_variant2_16384_vs_oracle():
     assert meanerr(out, truth) <= 1.25 * meanerr(ref, truth) + 1e-5
 
 
-# ------------------------------------------------------------------ GEMM, shipped variant, BASELINE shapes
+# ------------------------------------------------------------------ GEMM, shipped variant, full shapes
 def _row_subset(M):
     """First block, an interior 256-row pair block, and the ragged tail (65544 = 256 * 256 + 8)."""
     idx = list(range(0, 256)) + list(range(M // 2 - 128, M // 2 + 128)) + list(range(M - 264, M))
@@ -285,9 +285,9 @@ def test_fused_unembed_score_vs_fp64(M):
 
 # ------------------------------------------------------------------ 7B-width model at 8193 tokens; end-to-end scoring bound
 def test_two_layer_7b_width_8193_tokens_logits_and_score_vs_oracle():
-    """1 Hyena + 1 attention block at D = 4096 / 32 heads, batch 1 x 8192 nt + BOS (the per-sequence shape of BASELINE
-    configs[1]): logits vs both oracle modes, and the number evo/scoring.py returns -- the mean log-likelihood through
-    evo_b200.score_sequences (fused head) -- against the bf16-faithful oracle within BASELINE.md section 4's 2e-3."""
+    """1 Hyena + 1 attention block at D = 4096 / 32 heads, batch 1 x 8192 nt + BOS (the per-sequence shape of the
+    scoring workload): logits vs both oracle modes, and the number evo/scoring.py returns -- the mean log-likelihood through
+    evo_b200.score_sequences (fused head) -- against the bf16-faithful oracle within 2e-3."""
     import evo_b200
     cfg = O.evo_config("evo-1-8k-base")
     cfg.update(num_layers=2, attn_layer_idxs=[1], hyena_layer_idxs=[0])

@@ -1,4 +1,4 @@
-"""Device-side sampler and on-device generation loop (SURVEY 8f-2) against the host implementations that
+"""Device-side sampler and on-device generation loop against the host implementations that
 mirror stripedhyena.sample.sample and the reference's per-token loop (evo/generation.py:131-189).
 
 Bars: greedy picks and everything the loop records (tokens, logits, final positions) BIT-EXACT against the

@@ -1,5 +1,5 @@
 """Parity tests proper: every sm_100a kernel, called through the C ABI, against the CPU oracle
-on the same seeded inputs; plus size-independent properties at BASELINE.json's full sizes.
+on the same seeded inputs; plus size-independent properties at the full sizes.
 
 Tolerances.  Integer/index work (embedding gather, KV append, FIR state) and every op whose
 bf16 rounding points are reproduced one-for-one (RMSNorm, rotary tables, the decode step) must
@@ -293,7 +293,7 @@ def test_hyena_step_bit_exact():
 
 
 def test_hyena_full_size_properties():
-    """BASELINE configs[1] shape (B=8, L=8193, D=4096): segment-count invariance and
+    """The scoring shape (B=8, L=8193, D=4096): segment-count invariance and
     state-pass == output-pass end state (size-independent properties, no oracle needed)."""
     D, H, B, L = 4096, 32, 8, 8193
     _, _, f = _filter(D, H)
@@ -488,7 +488,7 @@ def test_gemm_rejects_bad_shapes():
 
 
 def test_gemm_full_size_against_cublaslt():
-    """BASELINE-size projection GEMM (65544 x 12288 x 4096): tcgen05 kernel vs the cuBLASLt comparator."""
+    """Full-size projection GEMM (65544 x 12288 x 4096): tcgen05 kernel vs the cuBLASLt comparator."""
     M, N, K = 65544, 12288, 4096
     torch.manual_seed(0)
     a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
@@ -756,7 +756,7 @@ def test_public_api_scoring_and_generation():
 
 
 def test_baseline_config0_two_layer_7b_width_L1024():
-    """random-init 2-layer StripedHyena (1 Hyena + 1 attn) at the 7B
+    """Random-init 2-layer StripedHyena (1 Hyena + 1 attn) at the 7B
     width (D=4096, 32 heads), batch 1 x 1024: GPU forward vs the CPU oracle."""
     cfg = O.evo_config("evo-1-8k-base")
     cfg.update(num_layers=2, attn_layer_idxs=[1], hyena_layer_idxs=[0])

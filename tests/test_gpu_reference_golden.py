@@ -1,5 +1,5 @@
 """The CUDA path against numbers produced by the REFERENCE'S OWN scoring code (tests/golden/reference_host.json / .npz, made
-by tests/golden/make_reference_host_golden.py: /root/reference/evo/scoring.py run unmodified over the oracle model).
+by tests/golden/make_reference_host_golden.py: evo/scoring.py run unmodified over the oracle model).
 
 `score_sequences` / `positional_entropies` of evo_b200 on the GPU -- device tokenise + pad, the sm_100a forward, the fused
 unembed + log-softmax + gather / entropy head -- must land on what evo/scoring.py:62-131 returned for the same sequences and

@@ -405,7 +405,7 @@ def test_untied_model_without_unembed_in_the_checkpoint_is_filled_from_the_embed
 
 def test_checkpoint_without_inv_freq_keys_loads_with_the_analytic_buffer(tmp_path):
     """flash_attn registers rotary_emb.inv_freq as a non-persistent buffer; that stripedhyena re-registers it persistently (so that
-    the HF checkpoints carry it) is recalled, not verified (SURVEY.md A.7).  Both ingest paths therefore accept a checkpoint with
+    the HF checkpoints carry it) is recalled, not verified.  Both ingest paths therefore accept a checkpoint with
     or without those keys: present -> the checkpoint's values (see test_streaming_ingest...), absent -> the analytic table."""
     from safetensors.torch import save_file
     cfg = O.tiny_config(num_layers=2, attn_layer_idxs=(1,), hidden_size=256, num_heads=2)
@@ -516,7 +516,7 @@ def test_bench_cpu_leg_switches_to_the_reference_package_when_it_is_importable(m
 
 def test_bench_helpers_assemble_the_contract_fields():
     """bench.py's pure helpers: synthetic inputs are reproducible per seed, the roofline records carry the contract's keys and
-    consistent arithmetic (achieved = work / time, frac = achieved / peak), and the workloads are the BASELINE.json configs."""
+    consistent arithmetic (achieved = work / time, frac = achieved / peak), and the workloads are the reference's configurations."""
     import importlib.util
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     spec = importlib.util.spec_from_file_location("bench_mod", os.path.join(root, "bench.py"))

@@ -71,7 +71,7 @@ def test_filter_is_sum_of_pole_powers():
 
 
 def test_column_split_mapping():
-    """x2 <- z[(c//hd)*3hd + c%hd], x1 <- +hd, v <- +2hd (SURVEY.md A.3)."""
+    """x2 <- z[(c//hd)*3hd + c%hd], x1 <- +hd, v <- +2hd."""
     H, hd = 3, 4
     z = torch.arange(3 * H * hd, dtype=torch.float32)[None, :, None].repeat(1, 1, 2)
     x2, x1, v = O.column_split(z, H, hd)
@@ -127,7 +127,7 @@ def test_evo_7b_shapes():
     assert spec["blocks.0.filter.poles"] == (4096, 8, 1, 2)
     assert spec["blocks.8.inner_mha_cls.Wqkv.weight"] == (12288, 4096)
     n = sum(int(np.prod(s)) for k, s in spec.items() if k != "unembed.weight" and "inv_freq" not in k)
-    assert abs(n - 6.45e9) < 0.03e9       # "7B" = 6.45 B parameters (SURVEY.md 8d)
+    assert abs(n - 6.45e9) < 0.03e9       # "7B" = 6.45 B parameters
     assert cfg["rotary_emb_scaling_factor"] == 16
 
 
@@ -277,7 +277,7 @@ def test_real_reference_bridge_runs_against_a_stand_in_package(monkeypatch):
 
 
 def test_oracle_against_the_real_stripedhyena_package():
-    """SURVEY.md A.9's verify-first checklist.  Skipped wherever `import stripedhyena` fails -- which is everywhere this repo has been
+    """The verify-first checklist against the published package.  Skipped wherever `import stripedhyena` fails -- which is everywhere this repo has been
     built or run so far; the oracle's "parity unpinned" label stands until this test has passed somewhere."""
     from oracle import real_reference as RR
     ver = RR.available()

@@ -1,10 +1,10 @@
 """evo_b200's host layer against outputs of the REFERENCE'S OWN host code (tests/golden/reference_host.{json,npz}).
 
-The fixtures were produced by tests/golden/make_reference_host_golden.py: /root/reference/evo/{tokenizer,scoring,generation,
+The fixtures were produced by tests/golden/make_reference_host_golden.py: evo/{tokenizer,scoring,generation,
 models}.py imported unmodified (with a stand-in for the absent `stripedhyena` package) and driven on CPU with the oracle model.
 Here the same oracle model is put behind evo_b200's tokenizer / scoring / generation / checkpoint code: every id, every model
 call (prompt slice and seqlen_offset), every generated string and every score must come out as the reference's did.
-This pins the host side of the path (SURVEY.md 8b, 8f).  It does not pin the model arithmetic: the oracle is a restatement."""
+This pins the host side of the path.  It does not pin the model arithmetic: the oracle is a restatement."""
 import json
 import math
 import os
