@@ -144,7 +144,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
-          umma_ss<1>(tmem_base + TM_S0 + sb * BKV, umma_desc_k_sw128(qa + off), umma_desc_k_sw128(ka + off), idesc_qk, kk != 0);
+          umma_ss(tmem_base + TM_S0 + sb * BKV, umma_desc_k_sw128(qa + off), umma_desc_k_sw128(ka + off), idesc_qk, kk != 0);
         }
         umma_commit(&k_empty[st]);
         umma_commit(&s_full[sb]);
@@ -164,7 +164,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           uint64_t bd;
           if constexpr (V_MN) bd = umma_desc_mn_sw128(va + kk * 16 * 128, HALF_BYTES, 1024);
           else                bd = umma_desc_k_sw128(va + aoff);
-          umma_ss<1>(tmem_base + TM_O, umma_desc_k_sw128(pa + aoff), bd, idesc_pv, (j | kk) != 0);
+          umma_ss(tmem_base + TM_O, umma_desc_k_sw128(pa + aoff), bd, idesc_pv, (j | kk) != 0);
         }
         umma_commit(&v_empty[st]);
         umma_commit(&pv_done[pb]);

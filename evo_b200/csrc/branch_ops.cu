@@ -530,7 +530,8 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
   vec = vec && (!p->col_scale || aligned4<bf16>(p->col_scale));
   for (int n = 0; n < 2; ++n)
     if (p->out[n]) vec = vec && aligned4<bf16>(p->w[n]) && (p->dtype ? aligned4<float>(p->out[n]) : aligned4<bf16>(p->out[n]));
-  if (vec && p->D <= 4096 && p->n_branches <= 3) {
+  if (vec && p->D <= 4096) {
+    static_assert(EVO_SUM_NORM_BRANCHES == 3, "the switch below");
     // rows in registers: (groups of four per thread) x (branches)
 #define EVO_SUM_NORM(TT, NV) \
     switch (p->n_branches) { \

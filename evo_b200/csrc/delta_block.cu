@@ -54,17 +54,6 @@ struct Args {
   WaitLimit waits;
 };
 
-__device__ __forceinline__ float2 top2(float x, float y) { return make_float2(__uint_as_float(__float_as_uint(x) & 0xffff0000u), __uint_as_float(__float_as_uint(y) & 0xffff0000u)); }
-__device__ __forceinline__ uint32_t tops(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
-// two fp32 numbers as three packed bf16 parts, cut off: 8 + 8 + 8 bits are the whole mantissa
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = tops(x, y);
-  float2 t = top2(x, y);
-  x -= t.x; y -= t.y;
-  mid = tops(x, y);
-  t = top2(x, y);
-  lo = tops(x - t.x, y - t.y);
-}
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool on) {       // zero-filled when off
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
 }

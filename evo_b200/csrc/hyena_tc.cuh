@@ -38,8 +38,6 @@ constexpr int THREADS = (MMA_WARPS + EW_WARPS + 4) * 32;      // the last warpgr
 // registers: 640 threads are launched with 96 each; the warpgroups then share them out
 constexpr int MMA_REGS = 120, EW_REGS = 96, PRODUCER_REGS = 40;
 static_assert(MMA_WARPS * 32 * MMA_REGS + EW_WARPS * 32 * EW_REGS + 128 * PRODUCER_REGS <= THREADS * 96, "register shares exceed the launch");
-template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr int STAGE = 128;                   // tokens of a ring slot (one signal), with two rows in front
 constexpr int SLOTS = 6;
 constexpr int SLOT_BYTES = (STAGE + 2) * CH * 2;
@@ -79,7 +77,7 @@ __device__ __forceinline__ void mma0(float (&d)[4], const uint32_t (&a)[4], uint
 struct D2 { double r, i; };
 __device__ __forceinline__ D2 mul(D2 a, D2 b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
 // the fp32 value of a constant as three bf16 parts, cut off: 8 + 8 + 8 bits
-__device__ __forceinline__ void split3(double v, uint32_t (&out)[3]) {
+__device__ __forceinline__ void parts3(double v, uint32_t (&out)[3]) {
   float f = (float)v;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -149,7 +147,7 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) hyena_tc_constants_kernel(con
 #pragma unroll
       for (int kind = 0; kind < 3; ++kind) {
         uint32_t a3[3], b3[3];
-        split3(vals[kind][0], a3); split3(vals[kind][1], b3);
+        parts3(vals[kind][0], a3); parts3(vals[kind][1], b3);
 #pragma unroll
         for (int k = 0; k < 3; ++k) word[kind * 12 + (nt * 2 + reg) * 3 + k] = a3[k] | (b3[k] << 16);
       }
@@ -164,18 +162,6 @@ __device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {        //
 }
 __device__ __forceinline__ float2 shfl_up2(float2 v, int d) { return make_float2(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d)); }
 __device__ __forceinline__ float2 shfl2(float2 v, int src) { return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)); }
-// (re, im) as three packed bf16 parts, cut off rather than rounded: 8 + 8 + 8 bits are the whole fp32 mantissa
-__device__ __forceinline__ float2 top2(float2 v) { return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u)); }
-__device__ __forceinline__ uint32_t tops(float2 v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
-__device__ __forceinline__ void split3_pack(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = tops(v);
-  float2 t = top2(v);
-  v = make_float2(v.x - t.x, v.y - t.y);
-  mid = tops(v);
-  t = top2(v);
-  lo = tops(make_float2(v.x - t.x, v.y - t.y));
-}
-
 // byte offset of granule `gran` (8 tokens) of row `row` of channel c in the tile: the low three bits of the granule index are mixed with the channel
 // quad (phases A and C: 8 lanes = 8 quads) and with the row (phase B: 4 rows x 2 granules), so that both access patterns touch every bank once
 template <int R> __device__ __forceinline__ uint32_t cell(int c, int row, int gran) {
@@ -588,7 +574,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-              for (int hf = 0; hf < 2; ++hf) split3_pack(F[hf][nt], sh[nt * 2 + hf], smd[nt * 2 + hf], sl[nt * 2 + hf]);
+              for (int hf = 0; hf < 2; ++hf) split3(F[hf][nt].x, F[hf][nt].y, sh[nt * 2 + hf], smd[nt * 2 + hf], sl[nt * 2 + hf]);
             // two sums per column group, small products first: what the block itself gives, and what the state gives
             float o[2][4], os[2][4];
 #pragma unroll

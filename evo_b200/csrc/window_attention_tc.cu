@@ -31,8 +31,6 @@ constexpr int WARPS = 16, HK = BKV / 2;         // softmax warps; keys of a tile
 // registers per thread: the launch's 96 shared out again, the softmax warps' from the other four's
 constexpr int SOFTMAX_REGS = 112, OTHER_REGS = 32;
 static_assert(WARPS * 32 * SOFTMAX_REGS + 128 * OTHER_REGS <= THREADS * 96, "register shares exceed the launch");
-template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr uint32_t TM_S = 0, TM_O = 256;         // + 128 * tile
 
 struct Args {
@@ -45,7 +43,6 @@ struct Args {
 };
 
 __device__ __forceinline__ float ex2(float x) { float y; asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // values as the second operand: rows are keys, 64-channel halves HALF_BYTES apart
 __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {

@@ -119,3 +119,10 @@ def test_a_few_queries_run_as_in_a_captured_step(d, L, pos, window):
     twin, _, _ = _run(2, L, 4, 2, d, pos, window, on_device=True, **opt)
     assert torch.equal(out, twin)
     _close(out, ref, vmax)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("L,pos,window", [(16, 0, 0), (200, 5, 0), (300, 77, 100)])
+def test_rows_that_do_not_start_on_16_bytes(d, L, pos, window):
+    """What the tensor maps cannot read goes to the mma.sync form, whose heads of 64 and 128 nothing else reaches."""
+    _close(*_run(2, L, 4, 2, d, pos, window, gate="channel", sink=True, pad=4, seed=L))
