@@ -561,10 +561,22 @@ __global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restric
 // A longer call runs slab after slab, the state carried in between.
 constexpr int64_t SLAB_BYTES = 256ll << 20;
 
-// Taken for bf16 heads of 64 or 128 key channels and a multiple of 16 value channels, rows that start on 16 bytes, and calls of 32 tokens or more.
+// From how many tokens on the blocks are faster.  Three launches and a 64-token block take 25 us (8 pairs of head and sequence) to 300 (2048 pairs of 128 x 128) whether the block is
+// full or not; token by token a call takes 0.5 to 1 us per token while the pairs fit the SMs, in proportion to their number beyond.  Measured (us, token by token / blocks):
+//   heads of 64 x 64, 32 pairs: 32 tokens 23 / 26, 40 tokens 27 / 26, 48 tokens 31 / 26;  128 x 128, 128 pairs: 32 / 36, 39 / 37, 45 / 37;  64 x 128, 128 pairs: 25 / 32, 31 / 33, 33 / 33
+//   512 pairs, where token by token has more than a wave: 64 x 64: 32 tokens 52 / 51;  128 x 128: 125 / 86
+//   few value channels, whose token-by-token CTAs are nearly empty: 128 x 16, 32 pairs: 32 tokens 50 / 29;  but 1024 pairs: 48 tokens 97 / 120
+int64_t block_tokens(const evo_gated_delta_params* p) {
+  const int64_t pairs = (int64_t)p->B * p->H;
+  if (p->dv >= 48) return pairs >= 512 ? 32 : 48;
+  if (pairs <= 128) return 32;
+  return p->dv < 32 && pairs > 512 ? 128 : 48;
+}
+
+// Taken for bf16 heads of 64 or 128 key channels and a multiple of 16 value channels, rows that start on 16 bytes, and enough tokens.
 // (The workspace query comes here with shapes that the call has not looked over: an empty batch has no blocks to count.)
 bool taken(const evo_gated_delta_params* p) {
-  return p->B > 0 && p->H > 0 && p->dv > 0 && p->dtype == 0 && (p->dk == 64 || p->dk == 128) && p->dv % 16 == 0 && p->L >= 32 && p->ld % 8 == 0 && p->H <= 65535 && p->B <= 65535 &&
+  return p->B > 0 && p->H > 0 && p->dv > 0 && p->dtype == 0 && (p->dk == 64 || p->dk == 128) && p->dv % 16 == 0 && p->L >= block_tokens(p) && p->ld % 8 == 0 && p->H <= 65535 && p->B <= 65535 &&
          (((uintptr_t)p->q | (uintptr_t)p->k | (uintptr_t)p->v) & 15) == 0;
 }
 struct Sizes {

@@ -29,7 +29,7 @@
 // The per-channel decay is the state-space loop with one decay per state row, staged beside the (key, query) pairs, and the delta rule's
 // epilogue; evo_low_rank_decay computes the decays sigmoid(A2 u + b)^(1/tau) of all rows and channels beforehand, in fp32.
 // The single-token step is the same kernel with L == 1.
-// The delta rule's prompts in bf16 (heads of 64 or 128 key channels, 32 tokens or more) go by blocks on the tensor cores instead: delta_block.cu.
+// The delta rule's prompts in bf16 (heads of 64 or 128 key channels, from 32, 48 or 128 tokens on) go by blocks on the tensor cores instead: delta_block.cu.
 #include "common.cuh"
 #include <stdlib.h>
 #include "../../include/evo_b200.h"

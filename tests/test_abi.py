@@ -139,3 +139,15 @@ def test_lost_waits_are_none_and_their_limit_belongs_to_the_thread():
     t.join()
     assert seen == [default] and default > 1 << 16
     assert lib.evo_set_wait_polls(-1) == 5 and lib.evo_set_wait_polls(default) == default
+
+
+def test_short_gated_delta_calls_go_token_by_token_where_that_is_faster():
+    """The line between the token-by-token kernel (no workspace, or fp32 read-outs) and the 64-token blocks (their matrices, 32 KB each, as well)."""
+    lib = _lib.lib()
+
+    def blocks(pairs, dk, dv, L):
+        p = _lib.GatedDeltaParams(B=pairs // 8, L=L, H=8, G=8, dk=dk, dv=dv, ld=8 * (2 * dk + dv), dtype=0)
+        return lib.evo_gated_delta_workspace(ctypes.byref(p)) > 4 * pairs * L * dv + 32768 * pairs
+    for pairs, dk, dv, first in ((8, 64, 64, 48), (32, 128, 128, 48), (128, 64, 128, 48), (256, 128, 64, 48), (512, 64, 64, 32), (2048, 128, 128, 32), (8, 128, 16, 32), (128, 64, 32, 32),
+                                 (512, 128, 16, 48), (1024, 128, 16, 128), (1024, 64, 32, 48)):
+        assert not blocks(pairs, dk, dv, first - 1) and blocks(pairs, dk, dv, first), (pairs, dk, dv, first)
