@@ -42,7 +42,7 @@ extern "C" int evo_embed(const void* ids, int ids_are_i64, const void* table, vo
 // significands, so x/n is either exactly representable or at least 2^-17 (relative) away from every bf16 rounding
 // midpoint (a 9-bit significand m with x = n*m would need x to have >= 9 significant bits), while x * rcp_rn(n)
 // is within 2^-23 of x/n: both round to the same bf16.
-template <int MAXV>
+constexpr int MAXV = 16;              // vectors of eight per lane: rows of up to 4096
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* __restrict__ x, const uint4* __restrict__ scale,
                                                       uint4* __restrict__ out, int64_t rows, int nvec_per_lane,
                                                       float inv_sqrt_d, float eps) {
@@ -149,9 +149,10 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
                         D / 8, (float)(1.0 / sqrt((double)D)), eps));
     return check_launch("evo_rmsnorm");
   }
-  // one CTA per row while the rows do not fill the chip with eight of them per CTA: 903 x 4096: 7.9 us against 9.1, 8192 x 4096: 28.8 against 31.8;
-  // 2048-wide rows have too few bytes per CTA for that from 4096 rows on (12.4 us against 10.9)
-  if (rows <= (D >= 4096 ? 8192 : 2048)) {
+  // one CTA per row, or one warp per row (eight to a CTA).  Us, CTA / warp: 4096 wide: 903 rows 7.8 / 10.4, 8193 rows 29.1 / 32.4, 12288 rows 41.1 / 42.6, 16384 rows 53.3 / 52.1;
+  // 2048 wide: 1024 rows 7.9 / 8.0, 2048 rows 8.4 / 8.0, 8192 rows 22.7 / 18.6 (too few bytes per CTA), narrower the same; 8192 wide: 903 rows 8.4 / 15.1, 32768 rows 156 / 268
+  // (a warp would hold 32 vectors per lane)
+  if (D > 4096 || rows <= (D >= 4096 ? 12288 : 1024)) {
     EVO_CUDA(launch_pdl(rmsnorm_row_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
                         D / 8, (float)(1.0 / sqrt((double)D)), eps));
     return check_launch("evo_rmsnorm");
@@ -159,10 +160,7 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
   int nvec = D / 256;
   dim3 grid((unsigned)((rows + 7) / 8)), block(256);
   float isd = (float)(1.0 / sqrt((double)D));
-  if (nvec <= 16)
-    EVO_CUDA(launch_pdl(rmsnorm_kernel<16>, grid, block, 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out, rows, nvec, isd, eps));
-  else
-    EVO_CUDA(launch_pdl(rmsnorm_kernel<32>, grid, block, 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out, rows, nvec, isd, eps));
+  EVO_CUDA(launch_pdl(rmsnorm_kernel, grid, block, 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out, rows, nvec, isd, eps));
   return check_launch("evo_rmsnorm");
 }
 

@@ -95,7 +95,7 @@ def test_conv_act_limits():
     assert torch.equal(out.float()[torch.isinf(want)], want[torch.isinf(want)])
 
 
-@pytest.mark.parametrize("rows,D", [(65, 256), (2048, 2048), (2049, 2048), (8192, 4096), (8193, 4096)])
+@pytest.mark.parametrize("rows,D", [(65, 256), (2048, 2048), (2049, 2048), (8192, 4096), (8193, 4096), (1024, 1024), (1025, 1024), (12288, 4096), (12289, 4096), (300, 8192), (12300, 8192), (70, 4352)])
 def test_rmsnorm_forms(rows, D):
     g = torch.Generator(device=DEV).manual_seed(rows)
     x, s = torch.randn(rows, D, generator=g, device=DEV).bfloat16(), (1 + 0.1 * torch.randn(D, generator=g, device=DEV)).bfloat16()
