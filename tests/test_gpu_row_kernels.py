@@ -95,6 +95,25 @@ def test_conv_act_limits():
     assert torch.equal(out.float()[torch.isinf(want)], want[torch.isinf(want)])
 
 
+def test_conv_act_silu_of_every_bf16_number():
+    """The activation of every finite bf16 argument within half a step of bf16 plus 2^-20 of the result in 64 bits, also where e^-v is beyond fp32's 1 / x (from -87.3 down)."""
+    bits = torch.arange(1 << 16, dtype=torch.int32, device=DEV).to(torch.int16)
+    v = bits.view(torch.bfloat16)
+    v = torch.where(torch.isfinite(v.float()), v, torch.zeros_like(v)).view(1024, 64)
+    for lo in range(0, 1024, 32):
+        x = v[lo:lo + 32].contiguous()
+        w, out = torch.ones(64, 1, device=DEV).bfloat16(), torch.empty(32, 64, device=DEV, dtype=torch.bfloat16)
+        p = ConvActParams(inp=x.data_ptr(), ld=64, weight=w.data_ptr(), out=out.data_ptr(), ldo=64, zero_start=1, B=1, L=32, C=64, taps=1, act=1, dtype=0)
+        check(_lib.lib().evo_conv_act(C.byref(p), _stream()), "evo_conv_act")
+        d = x.double()
+        want = d * torch.exp(torch.minimum(d, torch.zeros_like(d))) / (1 + torch.exp(-d.abs()))
+        # the step of bf16 at `want`: 2^-7 of its power of two; 2^-133 below its smallest normal number.  silu_f ends at zero from -88.73 (e^-v overflows) on
+        step = torch.exp2(torch.floor(torch.log2(want.abs().clamp(min=2.0 ** -126))) - 7)
+        err = (out.double() - want).abs()
+        ok = (err <= 0.5 * step + 2.0 ** -20 * want.abs() + 2.0 ** -134) | ((d < -88.7) & (out == 0))
+        assert ok.all(), (x[~ok][:4], out[~ok][:4], want[~ok][:4])
+
+
 @pytest.mark.parametrize("rows,D", [(65, 256), (2048, 2048), (2049, 2048), (8192, 4096), (8193, 4096), (1024, 1024), (1025, 1024), (12288, 4096), (12289, 4096), (300, 8192), (12300, 8192), (70, 4352)])
 def test_rmsnorm_forms(rows, D):
     g = torch.Generator(device=DEV).manual_seed(rows)
