@@ -306,7 +306,7 @@ int pick_segments(const evo_hyena_params* p) {
   int sms = device_sm_count();
   if (blocks * 5 >= sms * 3 || L < 1024) return 1;
   // ONE wave: the largest segment count whose grid still fits the SMs (16 channel blocks x 9 segments = 144 CTAs on 148 SMs;
-  // rounding up to 10 gave 160 CTAs = two waves: 0.52 ms against 0.36 ms at B = 1, L = 16384, profiles/r02_hyena_micro_call2.jsonl)
+  // rounding up to 10 gave 160 CTAs = two waves: 0.52 ms against 0.36 ms at B = 1, L = 16384)
   long long want = std::max<long long>(1, sms / blocks);
   long long max_by_len = std::max<long long>(1, L / 512);
   return (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, max_by_len), 64));
@@ -319,7 +319,10 @@ struct HyenaPlan { bool tc; int R, nseg; long long seg_len; int scan_variant; };
 
 // The tensor-core path does the work of 256 R tokens x 32 channels per tile and item in a time that hardly depends on how many of the tokens exist, and computes its
 // constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 64: scan 14.9, tensor
-// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 44; 4 x 1000: 123 / 76; 8 x 300: 44 / 76; 8 x 8193: 953 / 811.  The smaller estimate decides; both sides are in us.
+// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 44; 4 x 1000: 123 / 76; 8 x 300: 44 / 76; 8 x 8193: 953 / 811.  D = 2048: 1 x 300: 42 / 21; 8 x 300: 42 / 48; 8 x 500: 64 / 51;
+// 2 x 4096: 117 / 70; 1 x 8193, both in segments: 126 / 134; 8 x 8193: 774 / 463.  D = 256, from 1000 tokens on in segments: 1 x 300: 42 / 21; 1 x 1999: 136 / 23; 8 x 8193: 126 / 133.
+// The smaller estimate decides; both sides are in us.  Over 1 to 8 sequences of 20 to 8193 tokens at the three widths it picks the faster side, or one within 5 % of it, with one
+// exception: narrow models' constants take less than estimated (a single tile 14.5 us at D = 256, 17 at 2048, 19 at 4096), so between about 75 and 110 tokens the scan's 16 to 19 are kept.
 // Few items (narrow models, one sequence) are cut into segments: a pass over x1 and v then finds the states between them, at about half the price of the output pass.
 HyenaPlan make_plan(const evo_hyena_params* p) {
   const long long L = p->L;

@@ -18,8 +18,8 @@
 // z is read once and y written once.
 // Measured (B200, D = 4096, constants included): 8 x 8193 tokens 811 us (modal scan on the CUDA cores 953), 1 x 1999 44 us (138), 4 x 1000 76 us (123), 1 x 301 23 us (42).
 // A steady tile of 1024 tokens takes 24.5 k cycles, all of them the tensor-core warps' (tensor pipe 6.7 k, fp32 pipe 9 k, issue 10 k per scheduler): bound by the
-// latencies of its dependent steps with two such warps per scheduler (5.6 cycles per instruction each; issue slots 56 % used).  Register shares of 128 / 88 or 136 / 80
-// are 2 - 3 % slower: the element-wise warps then spill.
+// latencies of its dependent steps with two such warps per scheduler (5.6 cycles per instruction each, by clock stamps; ncu on 1 x 8193: issue slots 59 % used, tensor pipe 23 %).  Register shares of 128 / 88 or 136 / 80
+// are 2 - 3 % slower: the element-wise warps then spill more (the output kernels spill 16 to 112 bytes as it is, -Xptxas -v).
 // A channel whose x or state is not finite (or beyond 1e30), or whose poles lie so far outside the unit circle that their powers are not, goes
 // token by token in that tile: a product with a structural zero would otherwise carry an infinity to earlier tokens of its block.
 #pragma once

@@ -5,9 +5,9 @@
 //   warps 0-7, 8-15  softmax and epilogue of the tiles: query r <-> TMEM lane r, its keys' two halves with two threads that exchange their maxima through shared memory
 //   warp  16         copies: both query tiles once, keys and values through two-deep rings that both tiles read
 //   warp  17         the products, TMEM (the warps of its warpgroup give their registers to the softmax)
-// A tile pair of 128 queries and 128 keys costs the tensor pipe 1536 cycles; 4 x 4096 queries, 16 heads of 128, window 1024: 727 us in the mma.sync form, 335 with one thread per
-// query and a single issuing thread (its instruction fetches and operand moves paced the kernel: the softmax waited for scores more than half of the time), 260 with a
-// converged issuing warp, 237 with two threads per query (without a window 1518 / 535 / 393 / 362; 16 heads, 300 tokens 31 / 23 / 22 / 20).
+// A tile pair of 128 queries and 128 keys costs the tensor pipe 1536 cycles; 4 x 4096 queries, 16 heads of 128, window 1024, in a warm loop: 727 us in the mma.sync form, 335 with
+// one thread per query and a single issuing thread (by clock stamps the softmax then waited for scores more than half of the time; its products in a loop of eight: 288), 260 with
+// a converged issuing warp, 237 with two threads per query (without a window 1518 / 535 / 393 / 362; 16 heads, 300 tokens 31 / 23 / 22 / 20).  With cold L2 257 us.
 // The scores (fp32, 128 columns of TMEM) are read once into registers; each probability goes back as a bf16 high part (columns 0-63 of its scores) plus a bf16 low part
 // (64-127), and two products with the values add them up in fp32: relative error 2^-17 per weight, as in the mma.sync form.  The exponents' reference follows the
 // running maximum lazily (weights stay below 2^8).  A key tile is counted from the first key that the first query tile sees, so the second tile's first key is a tile
@@ -129,7 +129,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int j = max(0, vn - KV_STAGES); j < vn; ++j) wait_to_end(&v_full[j % KV_STAGES], (uint32_t)(j / KV_STAGES) & 1, a.waits);
       }
     } else if (warp == WARPS + 1) {
-      // One copy of each product in a small loop: this warp shares the SM's instruction cache with the long softmax code (see above)
+      // one copy of each product, in a small loop (see above)
       constexpr uint32_t idesc_qk = umma_idesc_bf16(BQ, BKV);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(BQ, HD) | (1u << 16);     // the values are MN-major
       const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc = umma_desc_k_sw128(smem_u32(sK)), v_desc = desc_mn_sw128(smem_u32(sV));
@@ -395,7 +395,8 @@ namespace evo {
 
 // 16 query rows or more, the host knows the position (the maps' extents), and every row of every operand starts on 16 bytes.  Fewer rows -- a step, the rest of a
 // portion -- go to the CUDA-core kernels, which keep their weights and gate in fp32, spread up to four queries' keys over the warps of a CTA, and also serve the captured
-// step: a call's result must not depend on where its position is kept.
+// step: a call's result must not depend on where its position is kept.  One query behind 1000 keys, window 256, 16 heads of 128: 10.6 us there, 14.6 here; behind 4000 without
+// a window 65.7 / 74.  (5 to 15 queries behind 1000 keys take 195 us there and 26 here, with 2e-3 of the bf16 results rounded to the other side instead of 3e-4.)
 bool window_attn_tc_takes(const evo_window_attn_params* p) {
   if (p->Lq < 16) return false;
   const auto a16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
