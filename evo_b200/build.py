@@ -1,5 +1,5 @@
 """Builds evo_b200/libevo_b200.so (sm_100a) in-tree with nvcc.  No JIT cache: the .so
-travels with the repo snapshot to the GPU box."""
+travels with the tree."""
 from __future__ import annotations
 
 import hashlib

@@ -7,7 +7,7 @@ handed at every call, quirks Q1-Q4 included) and checkpoint ingest (HF repo / re
 YAML config, strict load, dtype policy call order).  Those files import `stripedhyena`, which does not exist here
 -- so this script registers a stand-in `stripedhyena` package whose `StripedHyena` is a recorder, whose
 `sample` is flash_attn.utils.generation.sample (installed here; the function stripedhyena/sample.py copies) and whose `dotdict`
-is a plain attribute dict, imports the reference's modules UNMODIFIED from /root/reference, and drives them on CPU with the
+is a plain attribute dict, imports the reference's modules UNMODIFIED from REFERENCE, and drives them on CPU with the
 oracle model (oracle/stripedhyena_oracle.py) standing where the real model would.
 
 What is NOT pinned by this: the model arithmetic (the oracle stays a restatement; "parity unpinned" in its header stands).

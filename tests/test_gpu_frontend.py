@@ -126,7 +126,7 @@ def test_public_scoring_entry_points_take_the_device_front_end_and_the_fused_hea
 
 
 def test_cli_scripts_run_end_to_end_on_random_weights(tmp_path, capsys):
-    """python -m scripts.score / scripts.generate / scripts.example_inference with --random-init (no network on the GPU box): the
+    """python -m scripts.score / scripts.generate / scripts.example_inference with --random-init (no network): the
     7B architecture is built on the device, the example FASTA is scored through the bucketed front-end, a short sample is generated."""
     import scripts.example_inference as ex
     import scripts.generate as gen

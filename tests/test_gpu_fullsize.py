@@ -4,7 +4,7 @@ scan (mode-split) -- each against the CPU oracle on the same seeded inputs, at t
 lengths; plus the fused scoring head and an end-to-end bound on the quantity evo/scoring.py returns.
 
 Collected before tests/test_gpu_parity.py (alphabetical order) so that a time-out late in the suite cannot skip them.
-The CPU oracle runs on the GPU box's host cores: the sizes are chosen so that each test's oracle side takes seconds
+The CPU oracle runs on the host cores: the sizes are chosen so that each test's oracle side takes seconds
 (row / head subsets where the full problem would take minutes; the subset always covers the first, an interior and
 the ragged last tile)."""
 import ctypes as C
