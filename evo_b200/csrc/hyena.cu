@@ -298,12 +298,11 @@ bool use_tma_path(const evo_hyena_params* p) {
 
 // Sequential-in-L is the efficient form (one HBM pass, no carry pass); split L only when the
 // (channel block x batch) grid cannot occupy the chip.
-int pick_segments(const evo_hyena_params* p) {
+int pick_segments(const evo_hyena_params* p, int sms) {
   const long long L = p->L;
   if (p->force_segments > 0) return (int)std::min<long long>(p->force_segments, std::max<long long>(1, L));
   const int per_cta = use_tma_path(p) ? evo_hy2::CH_PER_CTA : THREADS;
   long long blocks = (long long)((p->D + per_cta - 1) / per_cta) * p->B;
-  int sms = device_sm_count();
   if (blocks * 5 >= sms * 3 || L < 1024) return 1;
   // ONE wave: the largest segment count whose grid still fits the SMs (16 channel blocks x 9 segments = 144 CTAs on 148 SMs;
   // rounding up to 10 gave 160 CTAs = two waves: 0.52 ms against 0.36 ms at B = 1, L = 16384)
@@ -327,7 +326,7 @@ struct HyenaPlan { bool tc; int R, nseg; long long seg_len; int scan_variant; };
 HyenaPlan make_plan(const evo_hyena_params* p) {
   const long long L = p->L;
   const int sms = device_sm_count();
-  HyenaPlan best = {false, 0, pick_segments(p), 0, 1};
+  HyenaPlan best = {false, 0, pick_segments(p, sms), 0, 1};
   best.seg_len = (L + best.nseg - 1) / best.nseg;
   best.nseg = (int)((L + best.seg_len - 1) / best.seg_len);
   const char* env_v = getenv("EVO_B200_HYENA_VARIANT");      // comparisons: 0, 1 = the modal scans, 2 = tensor cores; read per call
