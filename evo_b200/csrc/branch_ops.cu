@@ -264,24 +264,9 @@ __global__ void __launch_bounds__(256) sum_norm_row_kernel(const evo_sum_norm_pa
 // ---- evo_conv_act: a thread owns one channel of one sequence over RT consecutive rows, its last taps inputs in registers
 constexpr int CONV_RT = 32, CONV_MAX_TAPS = 8, CONV_NB = 4;
 
-// silu of two values.  For rows stored as bf16: v / (1 + e^-v) with the bare 2^x and reciprocal instructions and packed multiply-adds, about half of what expf and the IEEE
-// division take.  t = -v log2 e is rounded; its remainder `lo` (exact product, and the constant's own remainder) corrects 2^t to first order, so that the exponential keeps the
-// 2^-22 of the instruction at every argument.  Everything is a quarter of its size: 1 + e^-v stays below 2^126 wherever e^-v is finite, and its reciprocal is not flushed.
-// The argument of the exponential ends at 100 (e^-v is nothing beside 1 from 17 on; an infinity would make the remainder a NaN).  Result within 2^-21 of itself, as silu_f's.
+// silu of two values
 template <typename T> __device__ __forceinline__ float2 silu2(float2 v) { return make_float2(silu_f(v.x), silu_f(v.y)); }
-template <> __device__ __forceinline__ float2 silu2<bf16>(float2 v) {
-  constexpr float LOG2E = 1.44269502f, LOG2E_REST = 1.92596303e-8f, QUARTER_LN2 = 0.25f * 0.693147182f;
-  const float2 x = make_float2(fminf(v.x, 100.f), fminf(v.y, 100.f)), up = make_float2(-LOG2E, -LOG2E), quarter = make_float2(0.25f, 0.25f);
-  const float2 t = __fmul2_rn(x, up);
-  const float2 lo = __ffma2_rn(x, make_float2(-LOG2E_REST, -LOG2E_REST), __ffma2_rn(x, up, make_float2(-t.x, -t.y)));
-  float2 e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
-  const float2 d = __ffma2_rn(e, __ffma2_rn(lo, make_float2(QUARTER_LN2, QUARTER_LN2), quarter), quarter);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
-  return __fmul2_rn(__fmul2_rn(v, quarter), r);
-}
+template <> __device__ __forceinline__ float2 silu2<bf16>(float2 v) { return silu2_bf16(v); }
 
 // four channels per thread (8- or 16-byte accesses), taps known at compile time.  Bound by instructions per element: 4 x 4096 rows of 6144 bf16 channels, 4 taps, SiLU take
 // 86 us (92 with cold L2 and carried inputs), 76 without the activation, where a plain copy of the same bytes takes 64; issue slots 74 % used, special functions 53 %, DRAM 50 %.

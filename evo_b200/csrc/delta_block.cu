@@ -7,15 +7,16 @@
 //   sums, norms and gates in fp32, sums of log decays in 64 bits (their differences enter as two floats), T in fp32 by halves: two triangles of 32 by forward
 //   substitution (one column per thread), the square between them by products.
 //   T diag(beta) and P go to the workspace as three bf16 parts (24 bits), in the order in which the next kernel's lanes read them.
-// delta_scan_kernel, one warp per 16 value channels, blocks one after another.  Everything is held transposed (value channels = rows of the mma tiles): the sums of
-//   one product are then, lane by lane, the first operand of the next, so the 16 x dk piece of the state stays in the warp's registers and warps exchange nothing:
+// delta_scan_kernel, blocks one after another on the fifth-generation tensor cores, everything transposed (value channels = rows): the sums of one product, split by the warps that
+//   read them from TMEM, are the first operand of the next, in TMEM too:
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
 //   S, W, U are fp32 and enter as three bf16 parts; K and Q are bf16 as they stand (their norms scale the sums); T, P have three parts and meet W, U in the six products
-//   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work.
-// delta_norm_kernel: head norm, weight and SiLU gate of the fp32 read-outs.
-// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 590 us (token by token 2774), of which the scan 395, bound by the tensor pipe (816 mma of 8.7 cycles per block and
-// warp, one warp per scheduler: 7.1 k of 10.4 k cycles) and the splits between its products; 1 x 777 tokens, 32 heads: 110 us (516).
-// A block in which W or U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
+//   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work; the read-outs are normed, weighted and gated by warps of their own.
+// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 360 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
+// which the scan 224 (395 + 51) and delta_prepare_kernel 135; 1 x 777 tokens, 32 heads: 70 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
+// cycles, by clock stamps); what is left of the chain  state's parts - K S - W's parts - T W - U's parts - K U - state  is the splitting, bound by instructions (11 k warp instructions a
+// block and CTA, four per element of W, U and S; three byte permutations of the half-rate integer pipe and four mixed multiply-adds of two numbers).
+// A block in which U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
 #include "waits.cuh"
 #include "mma_sync.cuh"
 #include "../../include/evo_b200.h"
@@ -33,9 +34,9 @@ namespace {
 
 constexpr int BT = 64;                                  // tokens of a block
 constexpr int TILES = 20;                               // 16 x 8 tiles of a lower triangle: k-tile kt with n-tiles 2 kt .. 7
-constexpr int PART_BYTES = 256;                         // one part of one tile: 32 lanes x 2 words
+constexpr int PART_BYTES = 256;                         // one part of one tile: two 8 x 8 matrices, rows of 16 bytes
 constexpr int TRI_BYTES = TILES * 3 * PART_BYTES;       // T or P of a block
-enum { V_GK = 0, V_GQ, V_CK, V_RK, V_RQ, V_BETA, V_G, V_ROWS };       // G rk | G rq | Gam_64 rk | rk | rq | beta | g
+enum { V_GK = 0, V_GQ, V_CK, V_RK, V_RQ, V_BETA, V_G, V_ROWS };       // -G rk | G rq | Gam_64 rk | rk | rq | beta | g
 constexpr int VEC_BYTES = V_ROWS * BT * 4 + 256;        // + the block's decay G_64
 constexpr int BLOCK_BYTES = 2 * TRI_BYTES + VEC_BYTES;  // of one (block, head, sequence)
 __host__ __device__ constexpr int tile_index(int kt, int nt) { return kt * (9 - kt) + nt - 2 * kt; }
@@ -47,7 +48,9 @@ struct Args {
   float unit_eps, q_scale;
   uint8_t* blocks;                                      // (sequence, head, block of the slab)
   float* state; int zero_start, store_state;
-  float* y;                                             // (rows, H * dv) fp32 read-outs
+  float* y;                                             // (rows, H * dv) fp32 read-outs, where more than one CTA has a head's channels
+  int norm, pair, wide;                                 // head norm, weight and gate here; with a second CTA; their rows start on four elements
+  const bf16* gate; const bf16* norm_w; bf16* out; int64_t ldo; float eps;
   int B; int64_t L; int H, G, dv;
   int64_t first; int n_blocks;                          // the slab: its first block and its length
   unsigned int* failed;                                 // a wait of this call ran out: later slabs and the states behind them are not computed
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   } else {
     const int t = tid - BT;
     const float G = expf(lh[t] + ll[t]);
-    vec[V_GK * BT + t] = G * rk[t];
+    vec[V_GK * BT + t] = -G * rk[t];
     vec[V_GQ * BT + t] = G * rq[t];
     vec[V_CK * BT + t] = expf((lh[BT - 1] - lh[t]) + (ll[BT - 1] - ll[t])) * rk[t];
     vec[V_RK * BT + t] = rk[t]; vec[V_RQ * BT + t] = rq[t]; vec[V_BETA * BT + t] = beta[t];
@@ -260,238 +263,532 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
       const float f0 = e < TILES ? beta[jj] : 1.f, f1 = e < TILES ? beta[jj + 1] : 1.f;
       split3(jj <= i ? x.x * f0 : 0.f, jj + 1 <= i ? x.y * f1 : 0.f, w[u][0], w[u][1], w[u][2]);
     }
-    uint2* dst = reinterpret_cast<uint2*>(out + (e < TILES ? 0 : TRI_BYTES) + (e % TILES) * 3 * PART_BYTES) + lane;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(out + (e < TILES ? 0 : TRI_BYTES) + (e % TILES) * PART_BYTES) + lane;
 #pragma unroll
-    for (int s = 0; s < 3; ++s) dst[s * 32] = make_uint2(w[0][s], w[1][s]);
+    for (int s = 0; s < 3; ++s)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) dst[(s * TILES * PART_BYTES + u * 128) / 4] = w[u][s];
   }
 }
 
 // ------------------------------------------------------------------------------------------------ the recurrence
+// A CTA has 64 value channels of a (head, sequence): 16 lanes of each quarter of TMEM (the layout of products with M = 64).  TMEM's lanes belong to
+// the schedulers, so a warp instruction on a quarter's 16 lanes (shapes 16x256b and 16x128b, whose fragments are those of mma.sync) does half the work of one on 32, and 128 channels go
+// to two CTAs, a cluster (one CTA for 128 channels, 32 lanes an instruction: 13.4 k cycles a block, bound by the issue of 27 k instructions; two: 6.3 k).
+// Eight warps split what one product leaves as fp32 sums into the three parts that the next one multiplies; the two warps of a channel hold half of its state each (HC columns, in
+// registers) and 32 of the block's tokens of W and U.
+// TMEM columns: the state's parts, which the state's update overwrites once they are multiplied (DK = 128; DK = 64 has columns to spare), W (then U) and O as they are summed, the
+// parts of W (then U), the parts of U Gam rk
+template <int DK> struct Columns {
+  static constexpr int HC = DK / 2, S = 0, S_HALF = 3 * HC / 2, DS = DK == 128 ? 0 : 96, DS_HALF = DK == 128 ? S_HALF : HC, W = 192, O = 256, WP = 320, UP = 416;
+};
+static_assert(Columns<64>::DS + 64 <= Columns<64>::W && Columns<128>::S_HALF * 2 <= Columns<128>::W, "TMEM columns overlap");
+constexpr int MMA_M = 64;
+constexpr int CH = 64;                                                     // value channels of a CTA
+constexpr int SPLIT_WARPS = 8, EPI_WARPS = 4, SCAN_THREADS = 640;         // two groups of read-out warps, which take the blocks in turn; a warp each for the copies and the products
+constexpr int COPY_WARP = SPLIT_WARPS + 2 * EPI_WARPS, MMA_WARP = COPY_WARP + 1;
+constexpr int SPLIT_REGS = 112, EPI_REGS = 104, OTHER_REGS = 40;          // shares of the launch's 96 a thread
+static_assert(SPLIT_WARPS * 32 * SPLIT_REGS + 2 * EPI_WARPS * 32 * EPI_REGS + 128 * OTHER_REGS <= SCAN_THREADS * 96, "register shares exceed the launch");
+constexpr int OUT_PITCH = CH + 4;                       // floats of a token's row on its way from lanes to rows
+constexpr int OUT_BYTES = BT * OUT_PITCH * 4;           // of a block
+constexpr int V_BYTES = BT * CH * 2;
+
+// 16 lanes; a thread has row lane / 4 (and + 8), columns 2 (lane & 3) and the next of every eight: [8 columns][row, row + 8][2]
+template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float2 (&x)[N]) {
+  static_assert(N == 4 || N == 8, "");
+  uint32_t r[2 * N];
+  if constexpr (N == 4)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+  else
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+  tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+// packed pairs of the same thread and columns: four columns of words for every eight
+template <int N> __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[N]) {
+  static_assert(N == 2 || N == 4 || N == 8, "");
+  if constexpr (N == 2) asm volatile("tcgen05.st.sync.aligned.16x128b.x1.b32 [%2], {%0, %1};" ::"r"(r[0]), "r"(r[1]), "r"(taddr) : "memory");
+  else if constexpr (N == 4) asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%4], {%0, %1, %2, %3};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(taddr) : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
+}
+// x and y without what is cut off in w (exact): the mixed multiply-add leaves the half-rate integer pipe, which bounds the splitting, to the byte permutations
+__device__ __forceinline__ float2 take_away(float2 x, uint32_t w) {
+  float2 r;
+  asm("{\n\t.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %4;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, lo, m, %2;\n\tfma.rn.f32.bf16 %1, hi, m, %3;\n\t}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "r"(w));
+  return r;
+}
+// the three parts (split3) of a thread's fragment, `apart` columns from one to the next
+template <int N> __device__ __forceinline__ void put_parts(uint32_t at, uint32_t apart, const float2* given) {
+  float2 x[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = given[i];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    uint32_t w[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      w[i] = tops(x[i].x, x[i].y);
+      if (s < 2) x[i] = take_away(x[i], w[i]);
+    }
+    tmem_st(at + s * apart, w);
+  }
+}
+// a triangle's tiles as delta_prepare_kernel lays them down: 8 x 8 matrices of 128 bytes, two of them a step of 16 tokens j, 256 bytes from eight tokens i to the next
+__device__ __forceinline__ uint64_t desc_tri(uint32_t addr) { return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46; }
+// one product, the second operand's descriptor in two words
+template <bool ADD> __device__ __forceinline__ void product(uint32_t lead, uint32_t d, uint32_t a, uint32_t lo, uint32_t hi, uint32_t idesc) {
+  asm volatile("{\n\t.reg .pred e;\n\t.reg .b64 b;\n\tsetp.ne.b32 e, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, %6;\n\t}\n"
+               ::"r"(d), "r"(a), "r"(lo), "r"(hi), "r"(idesc), "r"(lead), "n"(ADD ? 1 : 0) : "memory");
+}
+
+__host__ __device__ constexpr int stage_bytes(int dk) { return 2 * BT * dk * 2 + V_BYTES + BLOCK_BYTES; }          // a multiple of 1024
+__host__ __device__ constexpr int scan_smem_bytes(int dk) { return 1024 + 2 * stage_bytes(dk) + 2 * OUT_BYTES; }
+
 template <int DK>
-__global__ void __launch_bounds__(256, 1) delta_scan_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmV, const Args p) {
-  constexpr int KT = DK / 16, BOX = BT * 128, ROWS_BYTES = DK / 64 * BOX;      // keys and queries: boxes of 64 columns, 16-byte pieces of a row swizzled by row & 7
+__global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmV, const Args p) {
+  using T = Columns<DK>;
+  constexpr int BOX = BT * 128, ROWS_BYTES = DK / 64 * BOX, HC = T::HC, STAGE = stage_bytes(DK);      // boxes of 64 columns, 16-byte pieces of a row swizzled by row & 7
+  static_assert(STAGE % 1024 == 0, "");
   extern __shared__ __align__(16) uint8_t sm_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t arrived[2];
-  const int nw = blockDim.x >> 5, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-  const int vpitch = nw * 32, stage_bytes = 2 * ROWS_BYTES + BT * vpitch + BLOCK_BYTES;
-  const int h = blockIdx.x, b = blockIdx.y, g = h / (p.H / p.G), dv = p.dv;
-  const int c0 = blockIdx.z * nw * 16, cw = c0 + warp * 16;            // the CTA's and the warp's first value channel
+  __shared__ uint64_t full[2], empty[2], s_ready, w_done, wp_ready, u_done, up_ready, pu_ready, ds_done[2], qs_done[2], o_done[2], o_free, fixed[2], half_met[4], rows_met[2], norm_met[2], ended;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int odd[2];                                // W or U of block (parity) holds something that is not finite
+  __shared__ float part_sum[2][3][2][CH];               // of a token (parity): S^T k, S^T q, k . q over half the key channels
+  __shared__ float norm_sum[2][BT];                     // of a block (parity): the other CTA's sums of squares
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+  const int h = blockIdx.x, b = blockIdx.y, g = h / (p.H / p.G), dv = p.dv, c0 = blockIdx.z * CH;
   const int64_t rowb = (int64_t)b * p.L + p.first * BT, left = p.L - p.first * BT;       // the slab's first row; tokens from there
   const uint8_t* blocks = p.blocks + ((int64_t)b * p.H + h) * p.n_blocks * (int64_t)BLOCK_BYTES;
 
-  // a block's rows of K, Q, V (rows behind the last token arrive as zeros) and its T, P and vectors: one lane
-  auto fetch = [&](int blk) {
-    uint8_t* st = sm + (blk & 1) * stage_bytes;
-    uint64_t* bar = &arrived[blk & 1];
-    const int t0 = (int)(p.first + blk) * BT;
-    mbar_arrive_expect_tx(bar, stage_bytes);
-#pragma unroll
-    for (int i = 0; i < DK / 64; ++i) {
-      tma_load_3d(st + i * BOX, &tmK, bar, g * DK + i * 64, t0, b);
-      tma_load_3d(st + ROWS_BYTES + i * BOX, &tmQ, bar, g * DK + i * 64, t0, b);
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1 + SPLIT_WARPS + EPI_WARPS); mbar_init(&ds_done[i], 1); odd[i] = 0;
+      mbar_init(&qs_done[i], 1); mbar_init(&o_done[i], 1); mbar_init(&fixed[i], 4); mbar_init(&rows_met[i], EPI_WARPS); mbar_init(&norm_met[i], 1);
     }
-    tma_load_3d(st + 2 * ROWS_BYTES, &tmV, bar, h * dv + c0, t0, b);
-    bulk(st + 2 * ROWS_BYTES + BT * vpitch, blocks + (int64_t)blk * BLOCK_BYTES, BLOCK_BYTES, bar);
-  };
-  if (tid == 0) { mbar_init(&arrived[0], 1); mbar_init(&arrived[1], 1); fence_barrier_init(); }
-  if (__syncthreads_or(p.first > 0 && tid == 0 && *(volatile unsigned int*)p.failed)) return;
+    mbar_init(&s_ready, SPLIT_WARPS); mbar_init(&w_done, 1); mbar_init(&wp_ready, SPLIT_WARPS); mbar_init(&u_done, 1); mbar_init(&up_ready, SPLIT_WARPS);
+    mbar_init(&pu_ready, SPLIT_WARPS + EPI_WARPS);               // the parts of U, and Q S read
+    mbar_init(&o_free, EPI_WARPS); mbar_init(&ended, 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&half_met[i], 2);
+    fence_barrier_init();
+  }
+  if (warp == MMA_WARP) { tmem_alloc<1>(&tmem_slot, 512); tmem_relinquish<1>(); }
+  const bool given_up = p.first > 0 && *(volatile unsigned int*)p.failed;
+  tc_fence_before();
+  const bool skip = __syncthreads_or(given_up);
+  tc_fence_after();
+  if (p.pair) cluster_sync_all();                        // the other CTA's barriers are there
+  const uint32_t tmem = tmem_slot;
+  const int n_blocks = skip ? 0 : p.n_blocks;
+  const auto wait = [&](uint64_t* bar, uint32_t parity) { return warp_wait_or_give_up(bar, parity, p.waits); };
+  // a warp's report behind its reads (or, after their completion, writes) of TMEM
+  const auto report = [&](uint64_t* bar) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(bar); __syncwarp(); };
+  bool ok = true;
 
-  // ---- S^T: rows = value channels cw + gq (+ 8), columns = state rows: S[n][..] covers state rows 8 n + 2 tq, + 1
-  float S[2 * KT][4];
-  float* Sg = p.state + ((int64_t)b * p.H + h) * DK * (int64_t)dv;
-  const bool live = cw < dv;                                            // (dv is a multiple of 16)
+  if (warp < SPLIT_WARPS) {
+    regs_up<SPLIT_REGS>();
+    const int q = warp & 3, hf = warp >> 2, c = q * 16 + gq;                       // the thread's channels: c and c + 8
+    const bool works = c0 + q * 16 < dv;                                   // (dv is a multiple of 16)  a warp without a channel only reports: its lanes' products are read by nobody
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+    float* Sg = p.state + (((int64_t)b * p.H + h) * DK + hf * HC + 2 * tq) * (int64_t)dv + c0 + c;
+    float2 S[HC / 4];                                                      // [8 columns][row]
+    const auto state_at = [&](int i, int e) -> float& { return Sg[(int64_t)(i / 2 * 8 + e) * dv + (i & 1) * 8]; };
 #pragma unroll
-  for (int n = 0; n < 2 * KT; ++n)
+    for (int i = 0; i < HC / 4; ++i) S[i] = (p.zero_start || !works || skip) ? make_float2(0.f, 0.f) : make_float2(state_at(i, 0), state_at(i, 1));
+    const auto publish = [&] {
+      if (works) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      S[n][e] = (p.zero_start || !live) ? 0.f : Sg[(int64_t)(8 * n + 2 * tq + (e & 1)) * dv + cw + gq + (e >> 1) * 8];
-
-  if (tid == 0) fetch(0);
-  for (int blk = 0; blk < p.n_blocks; ++blk) {
-    if (tid == 0 && blk + 1 < p.n_blocks) fetch(blk + 1);
-    const uint8_t* ks = sm + (blk & 1) * stage_bytes;
-    const bool here = wait_or_give_up(&arrived[blk & 1], (blk >> 1) & 1, p.waits);
-    if (__syncthreads_or(!here)) {
-      // no state is kept; the copies under way land before the CTA ends
-      if (tid == 0) {
-        *p.failed = 1u;
-        wait_to_end(&arrived[blk & 1], (blk >> 1) & 1, p.waits);
-        if (blk + 1 < p.n_blocks) wait_to_end(&arrived[(blk + 1) & 1], ((blk + 1) >> 1) & 1, p.waits);
+        for (int i = 0; i < HC / 32; ++i) put_parts<8>(lanes + T::S + hf * T::S_HALF + 16 * i, HC / 2, S + 8 * i);
+        tmem_st_wait();
       }
-      return;
-    }
-    const uint8_t* qs = ks + ROWS_BYTES;
-    const uint8_t* vs = qs + ROWS_BYTES;
-    const uint8_t* tri = vs + BT * vpitch;
-    const float* vec = reinterpret_cast<const float*>(tri + 2 * TRI_BYTES);
-    const int nt = (int)min((int64_t)BT, left - (int64_t)blk * BT);
-    float* yr = p.y + (rowb + (int64_t)blk * BT) * p.H * dv + (int64_t)h * dv + cw + gq;
-    if (live) {
-      float W[8][4], O[8][4];                                           // columns = tokens 8 n + 2 tq, + 1
+      report(&s_ready);
+    };
+    // (with the state's parts a warp reports that it has seen the block's copies land: the products wait for nothing else)
+    if (n_blocks) { ok = wait(&full[0], 0); if (ok) publish(); }
+#pragma unroll 1
+    for (int blk = 0; blk < n_blocks && ok; ++blk) {
+      const uint32_t ph = blk & 1;
+      const uint8_t* ks = sm + ph * STAGE;
+      const uint8_t* vs = ks + 2 * ROWS_BYTES;
+      const float* vec = reinterpret_cast<const float*>(vs + V_BYTES + 2 * TRI_BYTES);
+      const float* vec2 = vec + 32 * hf + 2 * tq;        // of the thread's tokens 32 hf + 8 n + 2 tq, + 1
+      // ---- W = V - G rk (K S)
+      ok = wait(&w_done, ph);
+      if (!ok) break;
+      tc_fence_after();
+      if (works) {
+        float2 x[8];
+        tmem_ld(lanes + T::W + 32 * hf, x);
 #pragma unroll
-      for (int n = 0; n < 8; ++n)
+        for (int m = 0; m < 2; ++m) {
+          uint32_t v[4];                                 // (tokens 0-7, channels 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15), turned
+          ldmatrix_x4_trans_at(v, smem_u32(vs) + (32 * hf + 16 * m + (lane & 7) + ((lane >> 4) << 3)) * 128 + (((2 * q + (lane >> 3 & 1)) ^ (lane & 7)) << 4));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) W[n][e] = O[n][e] = 0.f;
-      const uint32_t brow = ((lane & 7) + ((lane >> 4) << 3)) * 128, piece = (lane >> 3) & 1, turn = lane & 7;
-#pragma unroll
-      for (int kt = 0; kt < KT; ++kt) {
-        const uint32_t at = (kt >> 2) * BOX + brow + (((2 * (kt & 3) + piece) ^ turn) << 4), kb = smem_u32(ks) + at, qb = smem_u32(qs) + at;
-        uint32_t a[3][4];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          split3(S[2 * kt + u][0], S[2 * kt + u][1], a[0][2 * u], a[1][2 * u], a[2][2 * u]);
-          split3(S[2 * kt + u][2], S[2 * kt + u][3], a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
+          for (int i = 0; i < 4; ++i)
+            x[4 * m + i] = __ffma2_rn(*reinterpret_cast<const float2*>(vec2 + V_GK * BT + 16 * m + i / 2 * 8), x[4 * m + i], make_float2(bf_lo(v[i]), bf_hi(v[i])));
         }
-#pragma unroll
-        for (int n2 = 0; n2 < 4; ++n2) {
-          uint32_t bk[4], bq[4];
-          ldmatrix_x4_at(bk, kb + n2 * 16 * 128);
-          ldmatrix_x4_at(bq, qb + n2 * 16 * 128);
-#pragma unroll
-          for (int s = 2; s >= 0; --s) {
-            mma_np(W[2 * n2], a[s], bk[0], bk[1]); mma_np(W[2 * n2 + 1], a[s], bk[2], bk[3]);
-            mma_np(O[2 * n2], a[s], bq[0], bq[1]); mma_np(O[2 * n2 + 1], a[s], bq[2], bq[3]);
-          }
-        }
+        put_parts<8>(lanes + T::WP + 16 * hf, 32, x);
+        tmem_st_wait();
       }
-      // ---- W = V - G rk (K S); O = G rq (Q S)
-      float wrong = 0.f;
-      {
-        const uint32_t vb = smem_u32(vs) + ((lane & 7) + ((lane >> 4) << 3)) * vpitch + warp * 32 + ((lane >> 3) & 1) * 16;
+      report(&wp_ready);
+      // ---- U, first weighted for the state, then as it is for the read-outs
+      ok = wait(&u_done, ph);
+      if (!ok) break;
+      tc_fence_after();
+      if (works) {
+        float2 u[8], x[8], wrong = make_float2(0.f, 0.f);
+        tmem_ld(lanes + T::W + 32 * hf, u);
 #pragma unroll
-        for (int n2 = 0; n2 < 4; ++n2) {
-          uint32_t v[4];                                                // (tokens 0-7, channels 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15), turned
-          ldmatrix_x4_trans_at(v, vb + n2 * 16 * vpitch);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int n = 2 * n2 + u;
-            const float2 gk = *reinterpret_cast<const float2*>(vec + V_GK * BT + 8 * n + 2 * tq), gqv = *reinterpret_cast<const float2*>(vec + V_GQ * BT + 8 * n + 2 * tq);
-            W[n][0] = fmaf(-gk.x, W[n][0], bf_lo(v[2 * u])); W[n][1] = fmaf(-gk.y, W[n][1], bf_hi(v[2 * u]));
-            W[n][2] = fmaf(-gk.x, W[n][2], bf_lo(v[2 * u + 1])); W[n][3] = fmaf(-gk.y, W[n][3], bf_hi(v[2 * u + 1]));
-            O[n][0] *= gqv.x; O[n][1] *= gqv.y; O[n][2] *= gqv.x; O[n][3] *= gqv.y;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) wrong = fmaf(0.f, W[n][e], wrong);
-          }
+        for (int n = 0; n < 8; ++n) {
+          x[n] = __fmul2_rn(u[n], *reinterpret_cast<const float2*>(vec2 + V_CK * BT + n / 2 * 8));
+          wrong = __ffma2_rn(make_float2(0.f, 0.f), u[n], wrong);          // (a W that is not finite leaves no U that is: T's diagonal times a NaN among its parts)
         }
-      }
-      // second operands of a triangle: the three parts of tile (kt, n)
-      auto tri_mul = [&](const uint8_t* base, const float (&X)[8][4], float (&Y)[8][4]) {
+        if (wrong.x + wrong.y != 0.f) odd[ph] = 1;
+        __syncwarp();
+        put_parts<8>(lanes + T::UP + 16 * hf, 32, x);
+        tmem_st_wait();
+        report(&up_ready);
+        put_parts<8>(lanes + T::WP + 16 * hf, 32, u);
+        tmem_st_wait();
+      } else report(&up_ready);
+      report(&pu_ready);
+      // ---- S = G_64 S + (U Gam rk)^T K
+      const float G = vec[V_ROWS * BT];
+      ok = wait(&ds_done[hf], ph);
+      if (!ok) break;
+      tc_fence_after();
+      if (*(volatile int*)&odd[ph] == 0) {
+        if (works) {
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          uint32_t a[3][4];
+          for (int n = 0; n < HC / 4; n += 8) {
+            float2 x[8];
+            tmem_ld(lanes + T::DS + hf * T::DS_HALF + 4 * n, x);
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            split3(X[2 * kt + u][0], X[2 * kt + u][1], a[0][2 * u], a[1][2 * u], a[2][2 * u]);
-            split3(X[2 * kt + u][2], X[2 * kt + u][3], a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
-          }
-#pragma unroll
-          for (int n0 = 2 * kt; n0 < 8; n0 += 4) {                       // four sums at a time: a sum's next mma is four later (23 cycles of latency, 8.7 of issue)
-            uint2 t[4][3];
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (n0 + c < 8)
-#pragma unroll
-                for (int s = 0; s < 3; ++s) t[c][s] = (reinterpret_cast<const uint2*>(base + tile_index(kt, n0 + c) * 3 * PART_BYTES) + lane)[s * 32];
-            const int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};       // small products first
-#pragma unroll
-            for (int m = 0; m < 6; ++m)
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-                if (n0 + c < 8) mma_np(Y[n0 + c], a[pa[m]], t[c][pb[m]].x, t[c][pb[m]].y);
-          }
-        }
-      };
-      float U[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) U[n][e] = 0.f;
-      tri_mul(tri, W, U);
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wrong = fmaf(0.f, U[n][e], wrong);
-      if (__all_sync(0xffffffffu, wrong == 0.f)) {
-        tri_mul(tri + TRI_BYTES, U, O);
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = 8 * n + 2 * tq + (e & 1);
-            if (t < nt) yr[(int64_t)t * p.H * dv + (e >> 1) * 8] = O[n][e];
-          }
-        // ---- S = G_64 S + (Gam rk U)^T K
-        const float G = vec[V_ROWS * BT];
-#pragma unroll
-        for (int n = 0; n < 2 * KT; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) S[n][e] *= G;
-        const uint32_t kt_b = smem_u32(ks) + ((lane & 7) + (((lane >> 3) & 1) << 3)) * 128;
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          uint32_t a[3][4];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int n = 2 * kt + u;
-            const float2 ck = *reinterpret_cast<const float2*>(vec + V_CK * BT + 8 * n + 2 * tq);
-            split3(U[n][0] * ck.x, U[n][1] * ck.y, a[0][2 * u], a[1][2 * u], a[2][2 * u]);
-            split3(U[n][2] * ck.x, U[n][3] * ck.y, a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
-          }
-#pragma unroll
-          for (int n2 = 0; n2 < KT; n2 += 2) {
-            uint32_t bk[8];
-            ldmatrix_x4_trans_at(bk, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + (lane >> 4)) ^ turn) << 4));
-            ldmatrix_x4_trans_at(bk + 4, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + 2 + (lane >> 4)) ^ turn) << 4));
-#pragma unroll
-            for (int s = 2; s >= 0; --s)
-#pragma unroll
-              for (int c = 0; c < 4; ++c) mma_np(S[2 * n2 + c], a[s], bk[2 * c], bk[2 * c + 1]);
+            for (int i = 0; i < 8; ++i) S[n + i] = __ffma2_rn(make_float2(G, G), S[n + i], x[i]);
           }
         }
       } else {
-        // token by token, as the recurrence is defined; lanes of a quad share the rows of the state
-        for (int t = 0; t < nt; ++t) {
-          const float dec = vec[V_G * BT + t], be = vec[V_BETA * BT + t], nk = vec[V_RK * BT + t], nq = vec[V_RQ * BT + t];
+        // token by token, as the recurrence is defined; a channel's quads and halves exchange their sums.  The read-outs go to the columns of O once the products there are through.
+        ok = wait(&o_done[ph], (blk >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const int nt = (int)min((int64_t)BT, left - (int64_t)blk * BT);
+        float kept[2] = {0.f, 0.f};
+#pragma unroll 1
+        for (int t = 0; t < BT; ++t) {
+          const float dec = t < nt ? vec[V_G * BT + t] : 1.f, be = vec[V_BETA * BT + t], nk = vec[V_RK * BT + t], nq = vec[V_RQ * BT + t];
+          const auto two = [&](int side, int n, float norm) {            // keys (side 0) or queries hf HC + 8 n + 2 tq and the next
+            const int d = hf * HC + 8 * n;
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(ks + side * ROWS_BYTES + (d >> 6) * BOX + t * 128 + ((((d >> 3) & 7) ^ (t & 7)) << 4) + 4 * tq);
+            return make_float2(bf_lo(w) * norm, bf_hi(w) * norm);
+          };
           float pk[2] = {0.f, 0.f}, po[2] = {0.f, 0.f}, kq = 0.f;
 #pragma unroll
-          for (int n = 0; n < 2 * KT; ++n) {
-            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq), qw = *reinterpret_cast<const uint32_t*>(qs + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
-            const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk, q0 = bf_lo(qw) * nq, q1 = bf_hi(qw) * nq;
-            kq = fmaf(k1, q1, fmaf(k0, q0, kq));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) S[n][e] *= dec;
+          for (int n = 0; n < HC / 8; ++n) {
+            const float2 kv = two(0, n, nk), qv = two(1, n, nq);
+            kq = fmaf(kv.y, qv.y, fmaf(kv.x, qv.x, kq));
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-              pk[u] = fmaf(S[n][2 * u + 1], k1, fmaf(S[n][2 * u], k0, pk[u]));
-              po[u] = fmaf(S[n][2 * u + 1], q1, fmaf(S[n][2 * u], q0, po[u]));
+              float2& s = S[2 * n + u];
+              s.x *= dec; s.y *= dec;
+              pk[u] = fmaf(s.y, kv.y, fmaf(s.x, kv.x, pk[u]));
+              po[u] = fmaf(s.y, qv.y, fmaf(s.x, qv.x, po[u]));
             }
           }
           kq = quad_sum(kq);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            pk[u] = be * (__bfloat162float(*reinterpret_cast<const bf16*>(vs + t * vpitch + (warp * 16 + gq + 8 * u) * 2)) - quad_sum(pk[u]));
-            po[u] = fmaf(pk[u], kq, quad_sum(po[u]));
-            if (tq == 0) yr[(int64_t)t * p.H * dv + 8 * u] = po[u];
+            pk[u] = quad_sum(pk[u]); po[u] = quad_sum(po[u]);
+            if (tq == 0) { part_sum[t & 1][0][hf][c + 8 * u] = pk[u]; part_sum[t & 1][1][hf][c + 8 * u] = po[u]; part_sum[t & 1][2][hf][c + 8 * u] = kq; }
           }
+          report(&half_met[q]);
+          ok = wait(&half_met[q], t & 1);                                // (64 meetings a block: the parity starts anew)
+          if (!ok) break;
 #pragma unroll
-          for (int n = 0; n < 2 * KT; ++n) {
-            const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
-            const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk;
+          for (int u = 0; u < 2; ++u) {
+            const auto sum = [&](int k) { return part_sum[t & 1][k][0][c + 8 * u] + part_sum[t & 1][k][1][c + 8 * u]; };
+            const int col = c + 8 * u;
+            const float x = be * (__bfloat162float(*reinterpret_cast<const bf16*>(vs + t * 128 + (((col >> 3) ^ (t & 7)) << 4) + (col & 7) * 2)) - sum(0));
+            if ((t & 3) == tq) kept[u] = fmaf(x, sum(2), sum(1));
+            if (t < nt) {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) { S[n][2 * u] = fmaf(k0, pk[u], S[n][2 * u]); S[n][2 * u + 1] = fmaf(k1, pk[u], S[n][2 * u + 1]); }
+              for (int n = 0; n < HC / 8; ++n) { const float2 kv = two(0, n, nk); float2& s = S[2 * n + u]; s.x = fmaf(kv.x, x, s.x); s.y = fmaf(kv.y, x, s.y); }
+            }
+          }
+          __syncwarp();
+          if (hf == 0 && (t & 3) == 3) { const uint32_t w[2] = {__float_as_uint(kept[0]), __float_as_uint(kept[1])}; tmem_st(lanes + T::O + (t & ~3), w); }
+        }
+        if (!ok) break;
+        if (hf == 0) { tmem_st_wait(); report(&fixed[ph]); }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[ph]);
+      if (tid == 0 && blk) odd[ph ^ 1] = 0;              // the last block's: everyone has read it (the read-outs' warps before this block's Q S could be asked for)
+      __syncwarp();
+      if (blk + 1 < n_blocks) { ok = wait(&full[ph ^ 1], ((blk + 1) >> 1) & 1); if (ok) publish(); }
+    }
+    const bool lost = __syncthreads_or(!ok);
+    if (lost) { if (tid == 0) *p.failed = 1u; }
+    else if (p.store_state && works && !skip) {
+      asm volatile("" : "+l"(Sg));                       // (or the compiler keeps the addresses of the loads above, two registers each, over the whole recurrence)
+#pragma unroll
+      for (int i = 0; i < HC / 4; ++i) { state_at(i, 0) = S[i].x; state_at(i, 1) = S[i].y; }
+    }
+  } else if (warp < COPY_WARP) {
+    // ================================================ read-outs: O = G rq (Q S) + P U, turned from lanes to rows, normed and gated
+    regs_up<EPI_REGS>();
+    const int q = warp & 3, c = q * 16 + gq, group = (warp - SPLIT_WARPS) >> 2;          // the group's blocks: those of its parity
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+    float* rows_out = reinterpret_cast<float*>(sm + 2 * STAGE + group * OUT_BYTES);
+    int repaired = 0, met = 0;
+    const auto meet = [&] { __syncwarp(); if (lane == 0) mbar_arrive(&rows_met[group]); __syncwarp(); const bool all = wait(&rows_met[group], met & 1); ++met; return all; };
+    // rows: half a warp per token, four channels per lane; tokens 16 q + 2 u + side, u = 0..7
+    const int side = lane >> 4, e0 = c0 + 4 * (lane & 15);
+    const bool mine = e0 < dv;
+    float2 w01 = make_float2(0.f, 0.f), w23 = w01;
+    if (p.norm && mine) {
+      const bf16* w = p.norm_w + e0;
+      w01 = make_float2(__bfloat162float(w[0]), __bfloat162float(w[1])); w23 = make_float2(__bfloat162float(w[2]), __bfloat162float(w[3]));
+    }
+#pragma unroll 1
+    for (int blk = group; blk < n_blocks; blk += 2) {
+      const uint32_t ph = group, turn = (blk >> 1) & 1;
+      const float* vec = reinterpret_cast<const float*>(sm + ph * STAGE + 2 * ROWS_BYTES + V_BYTES + 2 * TRI_BYTES);
+      const int nt = (int)min((int64_t)BT, left - (int64_t)blk * BT), mine_nt = mine ? nt - q * 16 - side : 0;      // (the thread's tokens 2 u < mine_nt)
+      const int64_t row0 = rowb + (int64_t)blk * BT + q * 16 + side;
+      uint2 gates[8];
+      if (p.norm) {
+        const bf16* gr = p.gate + row0 * p.ldz + (int64_t)h * dv + e0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          gates[u] = make_uint2(0u, 0u);
+          const bf16* r = gr + 2 * u * p.ldz;
+          if (2 * u < mine_nt) {
+            if (p.wide) gates[u] = __ldg(reinterpret_cast<const uint2*>(r));
+            else gates[u] = make_uint2((uint32_t)__bfloat16_as_ushort(r[0]) | (uint32_t)__bfloat16_as_ushort(r[1]) << 16, (uint32_t)__bfloat16_as_ushort(r[2]) | (uint32_t)__bfloat16_as_ushort(r[3]) << 16);
           }
         }
       }
+      ok = wait(&full[ph], turn) && wait(&qs_done[ph], turn);
+      if (!ok) break;
+      tc_fence_after();
+      float2 o[16];                                      // [8 tokens][channel c, c + 8]
+#pragma unroll
+      for (int i = 0; i < 16; i += 8) {
+        float2 x[8];
+        tmem_ld(lanes + T::O + 4 * i, x);
+#pragma unroll
+        for (int n = 0; n < 8; ++n) o[i + n] = __fmul2_rn(x[n], *reinterpret_cast<const float2*>(vec + V_GQ * BT + 4 * i + n / 2 * 8 + 2 * tq));
+      }
+      report(&pu_ready);
+      if (lane == 0) mbar_arrive(&empty[ph]);
+      __syncwarp();
+      if (blk >= 2 && p.norm) { ok = meet(); if (!ok) break; }           // the rows of the group's last block are read
+      if (p.pair && q == 0 && lane == 0) mbar_arrive_expect_tx(&norm_met[ph], BT * 4);      // (now: every warp here has seen the last block's)
+      __syncwarp();
+      ok = wait(&o_done[ph], turn);
+      if (!ok) break;
+      const bool anew = *(volatile int*)&odd[ph] != 0;   // the split warps computed this block's token by token
+      if (anew) {
+        ok = wait(&fixed[ph], repaired & 1);
+        if (!ok) break;
+        ++repaired;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = make_float2(0.f, 0.f);
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < 16; i += 8) {
+        float2 x[8];
+        tmem_ld(lanes + T::O + 4 * i, x);
+#pragma unroll
+        for (int n = 0; n < 8; ++n) o[i + n] = __fadd2_rn(o[i + n], x[n]);
+      }
+      report(&o_free);
+      if (!p.norm) {
+        if (c0 + q * 16 < dv) {
+          float* yr = p.y + (rowb + (int64_t)blk * BT) * p.H * dv + (int64_t)h * dv + c0 + c;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const int t = i / 4 * 8 + 2 * tq + (i & 1);
+            if (t < nt) yr[(int64_t)t * p.H * dv + (i >> 1 & 1) * 8] = (i & 1) ? o[i / 2].y : o[i / 2].x;
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) rows_out[(i / 4 * 8 + 2 * tq + (i & 1)) * OUT_PITCH + c + (i >> 1 & 1) * 8] = (i & 1) ? o[i / 2].y : o[i / 2].x;
+      ok = meet();
+      if (!ok) break;
+      float4 x[8];
+      float ss[8];
+      const float* src = rows_out + (q * 16 + side) * OUT_PITCH + 4 * (lane & 15);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        x[u] = mine ? *reinterpret_cast<const float4*>(src + 2 * u * OUT_PITCH) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float2 a = make_float2(x[u].x, x[u].y), c2 = make_float2(x[u].z, x[u].w), sq = __ffma2_rn(a, a, __fmul2_rn(c2, c2));
+        ss[u] = sq.x + sq.y;
+      }
+      // eight sums over 16 lanes: a lane keeps half of them at each of three steps and ends with that of u = (lane >> 1) & 7
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int n = 4 >> k, d = 8 >> k;
+        const bool up = lane & d;
+#pragma unroll
+        for (int u = 0; u < n; ++u) {
+          const float keep = up ? ss[u + n] : ss[u], give = up ? ss[u] : ss[u + n];
+          ss[u] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+        }
+      }
+      ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+      if (p.pair) {
+        // the head's other channels are the other CTA's
+        const uint32_t other = cluster_ctarank() ^ 1;
+        const int t = q * 16 + (lane & 14) + side;
+        if (!(lane & 1))
+          asm volatile("{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\tmapa.shared::cluster.u32 rb, %1, %2;\n\t"
+                       "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [ra], %3, [rb];\n\t}\n"
+                       ::"r"(smem_u32(&norm_sum[ph][t])), "r"(smem_u32(&norm_met[ph])), "r"(other), "r"(__float_as_uint(ss[0])) : "memory");
+        __syncwarp();
+        ok = wait(&norm_met[ph], turn);
+        if (!ok) break;
+        ss[0] += norm_sum[ph][t];
+      }
+      const float rstd = 1.0f / sqrtf(ss[0] / (float)dv + p.eps);
+      bf16* orow = p.out + row0 * p.ldo + (int64_t)h * dv + e0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u, orow += 2 * p.ldo) {
+        const float r1 = __shfl_sync(0xffffffffu, rstd, (lane & 16) + 2 * u);
+        const float2 r2 = make_float2(r1, r1);
+        const float2 a01 = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(x[u].x, x[u].y), r2), w01), silu2_bf16(make_float2(bf_lo(gates[u].x), bf_hi(gates[u].x))));
+        const float2 a23 = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(x[u].z, x[u].w), r2), w23), silu2_bf16(make_float2(bf_lo(gates[u].y), bf_hi(gates[u].y))));
+        const uint2 r = make_uint2(pack_bf16(a01.x, a01.y), pack_bf16(a23.x, a23.y));
+        if (2 * u < mine_nt) {
+          if (p.wide) *reinterpret_cast<uint2*>(orow) = r;
+          else {
+            orow[0] = __ushort_as_bfloat16((unsigned short)(r.x & 0xffffu)); orow[1] = __ushort_as_bfloat16((unsigned short)(r.x >> 16));
+            orow[2] = __ushort_as_bfloat16((unsigned short)(r.y & 0xffffu)); orow[3] = __ushort_as_bfloat16((unsigned short)(r.y >> 16));
+          }
+        }
+      }
+      if (h == p.H - 1 && c0 == 0 && p.ldo > (int64_t)p.H * dv)
+        for (int t = q * 16; t < min(nt, q * 16 + 16); ++t)
+          for (int64_t e = (int64_t)p.H * dv + lane; e < p.ldo; e += 32) p.out[(rowb + (int64_t)blk * BT + t) * p.ldo + e] = __float2bfloat16_rn(0.f);
     }
-    __syncthreads();                                                    // the stage may be filled again
-  }
-  if (p.store_state && live) {
+    __syncthreads_or(!ok);
+  } else {
+    regs_down<OTHER_REGS>();
+    if (warp == COPY_WARP) {
+      // ================================================ copies: a block's rows of K, Q, V (rows behind the last token arrive as zeros) and its T, P and vectors
+      if (lane == 0 && n_blocks) {
+        tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmV);
+        int blk = 0;
+        for (; blk < n_blocks; ++blk) {
+          const int s = blk & 1;
+          if (blk >= 2 && !wait_or_give_up(&empty[s], ((blk >> 1) - 1) & 1, p.waits)) { ok = false; break; }
+          uint8_t* st = sm + s * STAGE;
+          const int t0 = (int)(p.first + blk) * BT;
+          mbar_arrive_expect_tx(&full[s], STAGE);
 #pragma unroll
-    for (int n = 0; n < 2 * KT; ++n)
+          for (int i = 0; i < DK / 64; ++i) {
+            tma_load_3d(st + i * BOX, &tmK, &full[s], g * DK + i * 64, t0, b);
+            tma_load_3d(st + ROWS_BYTES + i * BOX, &tmQ, &full[s], g * DK + i * 64, t0, b);
+          }
+          tma_load_3d(st + 2 * ROWS_BYTES, &tmV, &full[s], h * dv + c0, t0, b);            // (columns behind the head's own are multiplied and not read)
+          bulk(st + 2 * ROWS_BYTES + V_BYTES, blocks + (int64_t)blk * BLOCK_BYTES, BLOCK_BYTES, &full[s]);
+        }
+        // every copy has landed before this thread ends
+        for (int i = max(0, blk - 2); i < blk; ++i) wait_to_end(&full[i & 1], (i >> 1) & 1, p.waits);
+      }
+    } else if (warp == MMA_WARP) {
+      // ================================================ products, issued by one lane of a converged warp, in small loops
+      const uint32_t lead = elect_one();
+      constexpr uint32_t id64 = umma_idesc_bf16(MMA_M, BT), id_mn = umma_idesc_bf16(MMA_M, 64) | (1u << 16);
+#pragma unroll 1
+      for (int blk = 0; blk < n_blocks && ok; ++blk) {
+        const uint32_t ph = blk & 1, base = smem_u32(sm + ph * STAGE);
+        // (descriptors' low words; the high ones do not change)
+        const uint32_t kd = (uint32_t)umma_desc_k_sw128(base), qd = (uint32_t)umma_desc_k_sw128(base + ROWS_BYTES), td = (uint32_t)desc_tri(base + 2 * ROWS_BYTES + V_BYTES);
+        constexpr uint32_t ROWS_HI = (uint32_t)(1024 >> 4) | 1u << 14 | 2u << 29, TRI_HI = (uint32_t)(256 >> 4) | 1u << 14;
+        // half of K S or Q S, the small parts first
+        const auto state_times = [&](uint32_t d, uint32_t rows, int hf, bool add) {
+          const uint32_t at = tmem + T::S + hf * T::S_HALF, from = rows + hf * (DK == 128 ? BOX >> 4 : 4);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) Sg[(int64_t)(8 * n + 2 * tq + (e & 1)) * dv + cw + gq + (e >> 1) * 8] = S[n][e];
+          for (int s = 2; s >= 0; --s)
+#pragma unroll
+            for (int i = 0; i < DK / 32; ++i) {
+              const int col = s * (HC / 2) + i * 8;
+              if (s < 2 || i > 0) product<true>(lead, d, at + col, from + i * 2, ROWS_HI, id64);
+              else if (add) product<true>(lead, d, at + col, from + i * 2, ROWS_HI, id64);
+              else product<false>(lead, d, at + col, from + i * 2, ROWS_HI, id64);
+            }
+        };
+        // sums over a triangle: parts (0, 2) (2, 0) (1, 1) (0, 1) (1, 0) (0, 0), the small products first
+        const auto tri_times = [&](uint32_t d, uint32_t tri) {
+          constexpr int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+          for (int m = 0; m < 6; ++m)
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) {
+              const uint32_t a = tmem + T::WP + pa[m] * 32 + kt * 8, from = tri + (pb[m] * TILES * PART_BYTES + tile_index(kt, 2 * kt) * PART_BYTES) / 16;
+              if (m || kt) product<true>(lead, d + 16 * kt, a, from, TRI_HI, umma_idesc_bf16(MMA_M, BT - 16 * kt));
+              else product<false>(lead, d, a, from, TRI_HI, umma_idesc_bf16(MMA_M, BT));
+            }
+        };
+        ok = wait(&s_ready, ph);
+        if (!ok) break;
+        tc_fence_after();
+        state_times(tmem + T::W, kd, 0, false);
+        state_times(tmem + T::W, kd, 1, true);
+        if (lead) umma_commit(&w_done);
+        ok = wait(&wp_ready, ph);
+        if (!ok) break;
+        tc_fence_after();
+        tri_times(tmem + T::W, td);
+        if (lead) umma_commit(&u_done);
+        // Q S fills the time in which U is split, P U that of the state
+        if (blk) { ok = wait(&o_free, (blk - 1) & 1); if (!ok) break; tc_fence_after(); }
+        state_times(tmem + T::O, qd, 0, false);
+        state_times(tmem + T::O, qd, 1, true);
+        if (lead) umma_commit(&qs_done[ph]);
+        ok = wait(&up_ready, ph);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int hf = 0; hf < DK / 64; ++hf) {
+#pragma unroll
+          for (int s = 2; s >= 0; --s)
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) {
+              const uint32_t d = tmem + T::DS + hf * T::DS_HALF, a = tmem + T::UP + s * 32 + kt * 8, from = kd + hf * (BOX >> 4) + kt * (16 * 128 >> 4);
+              if (s < 2 || kt) product<true>(lead, d, a, from, ROWS_HI, id_mn);
+              else product<false>(lead, d, a, from, ROWS_HI, id_mn);
+            }
+          if (lead) umma_commit(&ds_done[hf]);
+        }
+        if (DK == 64 && lead) umma_commit(&ds_done[1]);
+        // (the next block's copies are looked for here, off the chain from the state's parts to the next products)
+        ok = wait(&pu_ready, ph);
+        if (!ok) break;
+        tc_fence_after();
+        tri_times(tmem + T::O, td + TRI_BYTES / 16);
+        if (lead) { umma_commit(&o_done[ph]); umma_commit(&empty[ph]); }
+      }
+      if (lead) umma_commit(&ended);                     // every product has been summed before TMEM is given back
+      wait_to_end(&ended, 0, p.waits);
+    }
+    __syncwarp();
+    __syncthreads_or(!ok);
   }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == MMA_WARP) tmem_dealloc<1>(tmem, 512);
+  if (p.pair) { __syncwarp(); cluster_sync_all(); }      // the other CTA may still write its sums here
 }
 
 // head norm, weight and SiLU gate of the read-outs of (row, head): one warp, four channels per lane and step
@@ -521,40 +818,6 @@ __global__ void __launch_bounds__(256) delta_norm_kernel(const float* __restrict
   }
   if (h == H - 1)
     for (int64_t c = (int64_t)H * dv + lane; c < ldo; c += 32) out[row * ldo + c] = __float2bfloat16_rn(0.f);
-}
-// the same for heads of 32 N channels and rows that start on four elements: eight lanes per (row, head), everything in registers between the two passes
-template <int N>
-__global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int64_t ldg, const bf16* __restrict__ w, bf16* __restrict__ out, int64_t ldo,
-                                                          int64_t rows, int H, int dv, float eps) {
-  const int64_t id = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
-  const int sub = threadIdx.x & 7;
-  const bool on = id < rows * H;
-  const int64_t row = on ? id / H : 0;
-  const int h = on ? (int)(id - row * H) : 0;
-  const float4* r = reinterpret_cast<const float4*>(y + (on ? id : 0) * (32 * N)) + sub;
-  const uint2* gr = reinterpret_cast<const uint2*>(gate + row * ldg + (int64_t)h * (32 * N)) + sub;
-  const uint2* wr = reinterpret_cast<const uint2*>(w) + sub;
-  float4 o[N];
-  uint2 gv[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) { o[i] = r[8 * i]; gv[i] = gr[8 * i]; }
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < N; ++i) ss = fmaf(o[i].x, o[i].x, fmaf(o[i].y, o[i].y, fmaf(o[i].z, o[i].z, fmaf(o[i].w, o[i].w, ss))));
-#pragma unroll
-  for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-  const float rstd = 1.0f / sqrtf(ss / (float)(32 * N) + eps);
-  if (!on) return;
-  uint2* orow = reinterpret_cast<uint2*>(out + row * ldo + (int64_t)h * (32 * N)) + sub;
-  const auto one = [&](float v, float g, float wv) { return v * rstd * wv * (g / (1.f + expf(-g))); };
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const uint2 wv = wr[8 * i];
-    orow[8 * i] = make_uint2(pack_bf16(one(o[i].x, bf_lo(gv[i].x), bf_lo(wv.x)), one(o[i].y, bf_hi(gv[i].x), bf_hi(wv.x))),
-                             pack_bf16(one(o[i].z, bf_lo(gv[i].y), bf_lo(wv.y)), one(o[i].w, bf_hi(gv[i].y), bf_hi(wv.y))));
-  }
-  if (h == H - 1)
-    for (int64_t c = (int64_t)H * (32 * N) + sub; c < ldo; c += 8) out[row * ldo + c] = __float2bfloat16_rn(0.f);
 }
 
 // Blocks whose T and P are in memory at a time: at most 256 MB of them, or one block of every (head, sequence) pair where that is more (32 KB each, above 8192 pairs).
@@ -588,14 +851,11 @@ Sizes sizes(const evo_gated_delta_params* p) {
   s.blocks = (p->L + BT - 1) / BT;
   s.slab = std::max<int64_t>(1, std::min<int64_t>(s.blocks, SLAB_BYTES / ((int64_t)BLOCK_BYTES * p->B * p->H)));
   const auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-  s.y = up(sizeof(float) * (size_t)p->B * p->L * p->H * p->dv);
+  s.y = p->dv <= 2 * CH ? 0 : up(sizeof(float) * (size_t)p->B * p->L * p->H * p->dv);
   s.tri = up((size_t)BLOCK_BYTES * s.slab * p->B * p->H);
   s.state = p->state || s.slab == s.blocks ? 0 : up(sizeof(float) * (size_t)p->B * p->H * p->dk * p->dv);
   return s;
 }
-
-constexpr int scan_smem_bytes(int dk, int warps) { return 1024 + 2 * (2 * BT * dk * 2 + BT * warps * 32 + BLOCK_BYTES); }
-static_assert(scan_smem_bytes(128, 8) <= 227 * 1024, "two stages of eight warps");
 
 template <int DK>
 int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream_t st) {
@@ -609,34 +869,36 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   a.y = (float*)ws; a.blocks = ws + s.y;
   a.state = p->state ? p->state : (s.state ? (float*)(ws + s.y + s.tri) : (float*)ws);      // (never read nor written in the last case)
   a.B = p->B; a.L = p->L; a.H = p->H; a.G = p->G; a.dv = p->dv;
-  // warps spread over the schedulers: two (32 channels) to eight per CTA, as few as fill the chip (592 schedulers)
-  const int64_t warps = (int64_t)p->B * p->H * (p->dv / 16);
-  int nw = 2;
-  while (nw < 8 && nw * 16 < p->dv && warps > (int64_t)nw * device_sm_count()) nw *= 2;
-  const int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = scan_smem_bytes(DK, nw);
+  a.gate = (const bf16*)p->gate; a.norm_w = (const bf16*)p->norm_w; a.out = (bf16*)p->out; a.ldo = p->ldo; a.eps = p->eps;
+  a.norm = p->dv <= 2 * CH; a.pair = a.norm && p->dv > CH;
+  a.wide = p->ldz % 4 == 0 && p->ldo % 4 == 0 && (((uintptr_t)p->gate | (uintptr_t)p->out) & 7) == 0;
+  constexpr int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = scan_smem_bytes(DK);
   CUtensorMap tmK, tmQ, tmV;
   const uint64_t kdims[3] = {(uint64_t)p->G * DK, (uint64_t)p->L, (uint64_t)p->B}, vdims[3] = {(uint64_t)p->H * p->dv, (uint64_t)p->L, (uint64_t)p->B};
   const uint64_t strides[2] = {(uint64_t)p->ld * 2, (uint64_t)p->L * p->ld * 2};
-  const uint32_t kbox[3] = {64, BT, 1}, vbox[3] = {(uint32_t)nw * 16, BT, 1};
+  const uint32_t kbox[3] = {64, BT, 1}, vbox[3] = {CH, BT, 1};
   int rc;
   if ((rc = make_tmap_nd_bf16(&tmK, p->k, 3, kdims, strides, kbox, true)) || (rc = make_tmap_nd_bf16(&tmQ, p->q, 3, kdims, strides, kbox, true)) ||
-      (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, false))) return rc;
+      (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, true))) return rc;
   static unsigned long long done_prep = 0, done_scan = 0;
-  if ((rc = ensure_dyn_smem(delta_prepare_kernel<DK>, prep_smem, done_prep)) || (rc = ensure_dyn_smem(delta_scan_kernel<DK>, scan_smem_bytes(DK, 8), done_scan))) return rc;
+  if ((rc = ensure_dyn_smem(delta_prepare_kernel<DK>, prep_smem, done_prep)) || (rc = ensure_dyn_smem(delta_scan_kernel<DK>, scan_smem, done_scan))) return rc;
   for (int64_t first = 0; first < s.blocks; first += s.slab) {
     a.first = first; a.n_blocks = (int)std::min<int64_t>(s.slab, s.blocks - first);
     a.zero_start = first == 0 && (p->zero_start || !p->state);
     a.store_state = p->state || s.state;
     delta_prepare_kernel<DK><<<dim3(a.n_blocks, a.H, a.B), 128, prep_smem, st>>>(a);
     if ((rc = check_launch("evo_gated_delta_fwd(prepare)"))) return rc;
-    delta_scan_kernel<DK><<<dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), nw * 32, scan_smem, st>>>(tmK, tmQ, tmV, a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.H, a.B, (a.dv + CH - 1) / CH); cfg.blockDim = dim3(SCAN_THREADS); cfg.dynamicSmemBytes = scan_smem; cfg.stream = st;
+    cudaLaunchAttribute two = {};
+    two.id = cudaLaunchAttributeClusterDimension; two.val.clusterDim = {1, 1, 2};
+    if (a.pair) { cfg.attrs = &two; cfg.numAttrs = 1; }
+    EVO_CUDA(cudaLaunchKernelEx(&cfg, delta_scan_kernel<DK>, tmK, tmQ, tmV, a));
     if ((rc = check_launch("evo_gated_delta_fwd(scan)"))) return rc;
   }
+  if (a.norm) return 0;
   const int64_t rows = (int64_t)p->B * p->L, w = rows * p->H;
-  const bool wide = p->ldz % 4 == 0 && p->ldo % 4 == 0 && (((uintptr_t)p->gate | (uintptr_t)p->out | (uintptr_t)p->norm_w) & 7) == 0;
-  auto norm = !wide ? delta_norm_kernel : (p->dv == 128 ? delta_norm4_kernel<4> : (p->dv == 64 ? delta_norm4_kernel<2> : (p->dv == 32 ? delta_norm4_kernel<1> : delta_norm_kernel)));
-  const int per_cta = norm == delta_norm_kernel ? 8 : 32;
-  norm<<<(unsigned)((w + per_cta - 1) / per_cta), 256, 0, st>>>(a.y, (const bf16*)p->gate, p->ldz, (const bf16*)p->norm_w, (bf16*)p->out, p->ldo, rows, p->H, p->dv, p->eps);
+  delta_norm_kernel<<<(unsigned)((w + 7) / 8), 256, 0, st>>>(a.y, a.gate, p->ldz, a.norm_w, a.out, p->ldo, rows, p->H, p->dv, p->eps);
   return check_launch("evo_gated_delta_fwd(norm)");
 }
 

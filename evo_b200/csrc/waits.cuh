@@ -18,6 +18,14 @@ __device__ __forceinline__ bool wait_polls(uint64_t* bar, uint32_t parity, int p
   return false;
 }
 __device__ __forceinline__ bool wait_or_give_up(uint64_t* bar, uint32_t parity, const WaitLimit& w) { return wait_polls(bar, parity, w.polls, w.lost); }
+// of a whole warp, which stays together: what one lane has lost all have
+__device__ __forceinline__ bool warp_wait_or_give_up(uint64_t* bar, uint32_t parity, const WaitLimit& w) {
+  for (int i = 0; i < w.polls; ++i)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  *(volatile unsigned int*)w.lost = 1u;
+  __threadfence_system();
+  return false;
+}
 // for what the CTA itself has under way (copies into its shared memory, products): the full limit, whatever the caller's
 __device__ __forceinline__ void wait_to_end(uint64_t* bar, uint32_t parity, const WaitLimit& w) { wait_polls(bar, parity, WAIT_POLLS, w.lost); }
 
