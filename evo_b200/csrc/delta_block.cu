@@ -5,15 +5,17 @@
 //
 // delta_prepare_kernel, one CTA per (block, head, sequence), all in parallel: what does not depend on the state.  k . k and q . k as bf16 products (exact) with fp32
 //   sums, norms and gates in fp32, sums of log decays in 64 bits (their differences enter as two floats), T in fp32 by halves: two triangles of 32 by forward
-//   substitution (one column per thread), the square between them by products.
+//   substitution (one column per thread), the square between them by products of three-part splits.
 //   T diag(beta) and P go to the workspace as three bf16 parts (24 bits), in the order in which the next kernel's lanes read them.
 // delta_scan_kernel, blocks one after another on the fifth-generation tensor cores, everything transposed (value channels = rows): the sums of one product, split by the warps that
 //   read them from TMEM, are the first operand of the next, in TMEM too:
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
 //   S, W, U are fp32 and enter as three bf16 parts; K and Q are bf16 as they stand (their norms scale the sums); T, P have three parts and meet W, U in the six products
 //   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work; the read-outs are normed, weighted and gated by warps of their own.
-// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 360 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
-// which the scan 224 (395 + 51) and delta_prepare_kernel 135; 1 x 777 tokens, 32 heads: 70 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
+// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 316 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
+// which the scan 224 (395 + 51) and delta_prepare_kernel 92 (135 with the norms summed apart, both matrices stored and read again, and the square of T by
+// multiply-adds from shared memory: 15.7 k instructions and 5.5 k shared-memory wavefronts an item then, 10.5 k and 2.3 k now; its four warps wait for one another at barriers; six CTAs per
+// SM, which spill: 135); 1 x 777 tokens, 32 heads: 65 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
 // cycles, by clock stamps); what is left of the chain  state's parts - K S - W's parts - T W - U's parts - K U - state  is the splitting, bound by instructions (11 k warp instructions a
 // block and CTA, four per element of W, U and S; three byte permutations of the half-rate integer pipe and four mixed multiply-adds of two numbers).
 // A block in which U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
@@ -72,16 +74,32 @@ __device__ __forceinline__ void mma_np(float* d, const uint32_t* a, uint32_t b0,
 __device__ __forceinline__ float softplus_f(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // ------------------------------------------------------------------------------------------------ what does not depend on the state
-__host__ __device__ constexpr int prepare_rows_bytes(int dk) { return 2 * BT * (2 * dk + 16) > 2 * BT * (BT + 4) * 4 ? 2 * BT * (2 * dk + 16) : 2 * BT * (BT + 4) * 4; }
+// x without what is cut off in w (exact): the mixed multiply-add leaves the half-rate integer pipe, which bounds the splitting, to the byte permutations
+__device__ __forceinline__ float2 take_away(float2 x, uint32_t w) {
+  float2 r;
+  asm("{\n\t.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %4;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, lo, m, %2;\n\tfma.rn.f32.bf16 %1, hi, m, %3;\n\t}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "r"(w));
+  return r;
+}
+// the three parts (split3) of two neighbours of a row, to a lane's place in the tiles of each part
+__device__ __forceinline__ void store_parts(uint8_t* dst, float2 x) {
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const uint32_t w = tops(x.x, x.y);
+    *reinterpret_cast<uint32_t*>(dst + s * TILES * PART_BYTES) = w;
+    if (s < 2) x = take_away(x, w);
+  }
+}
+
+constexpr int AP = BT + 4;                                   // floats of a row of A (16-byte pieces)
+__host__ __device__ constexpr int prepare_smem_bytes(int dk) { return 2 * BT * (2 * dk + 16) + 5 * BT * 4; }
 template <int DK>
 __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
-  constexpr int PITCH = 2 * DK + 16, AP = BT + 4;            // bytes of a key row; floats of a row of A (16-byte pieces)
+  constexpr int PITCH = 2 * DK + 16;                         // bytes of a key row
+  static_assert(BT * AP * 4 <= 2 * BT * PITCH, "A fits where the keys and queries were");
   extern __shared__ __align__(16) uint8_t sm[];
-  uint8_t* ks = sm;
-  uint8_t* qs = ks + BT * PITCH;
+  uint8_t* ks = sm;                                          // [BT] keys, [BT] queries
   float* As = reinterpret_cast<float*>(sm);                  // [BT][AP] A, then T, in the place of the keys and queries once they are multiplied
-  float* Ps = As + BT * AP;                                  // [BT][AP]
-  float* rk = reinterpret_cast<float*>(sm + prepare_rows_bytes(DK));
+  float* rk = reinterpret_cast<float*>(sm + 2 * BT * PITCH);
   float* rq = rk + BT;
   float* beta = rq + BT;
   float* lh = beta + BT;                                     // running log decay, high and low float
@@ -90,13 +108,22 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (p.H / p.G);
   const int64_t t0 = (p.first + blk) * BT, row0 = (int64_t)b * p.L + t0;
   const int nt = (int)min((int64_t)BT, p.L - t0);
+  uint8_t* out = p.blocks + (((int64_t)b * p.H + h) * p.n_blocks + blk) * BLOCK_BYTES;
+  float* vec = reinterpret_cast<float*>(out + 2 * TRI_BYTES);
   if (p.first == 0 && (blk | h | b | tid) == 0) *p.failed = 0u;
-  for (int e = tid; e < BT * (DK / 8); e += 128) {
-    const int r = e / (DK / 8), c = e % (DK / 8);
-    const bool on = r < nt;
-    const int64_t off = (row0 + (on ? r : 0)) * p.ld + (int64_t)g * DK + c * 8;
-    cp16(smem_u32(ks + r * PITCH + c * 16), p.k + off, on);
-    cp16(smem_u32(qs + r * PITCH + c * 16), p.q + off, on);
+  {
+    constexpr int STEP = 128 / (DK / 8);                     // rows that the CTA copies at a time
+    const int c = tid % (DK / 8), r0 = tid / (DK / 8);
+    const int64_t col = (int64_t)g * DK + c * 8;
+    const bf16 *kp = p.k + (row0 + r0) * p.ld + col, *qp = p.q + (row0 + r0) * p.ld + col;
+    const uint32_t dst = smem_u32(ks) + r0 * PITCH + c * 16;
+#pragma unroll
+    for (int i = 0; i < BT / STEP; ++i) {
+      const bool on = r0 + i * STEP < nt;
+      cp16(dst + i * STEP * PITCH, on ? kp : p.k, on);
+      cp16(dst + (BT + i * STEP) * PITCH, on ? qp : p.q, on);
+      kp += STEP * p.ld; qp += STEP * p.ld;
+    }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (warp == 0) {
@@ -124,77 +151,75 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
       const float hi = (float)v;
       lh[2 * lane + u] = hi; ll[2 * lane + u] = (float)(v - (double)hi);
     }
-    float* vec = reinterpret_cast<float*>(p.blocks + (((int64_t)b * p.H + h) * p.n_blocks + blk) * BLOCK_BYTES + 2 * TRI_BYTES);
 #pragma unroll
     for (int u = 0; u < 2; ++u) vec[V_G * BT + 2 * lane + u] = expf(gl[u]);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // ---- norms: one warp per 16 tokens, two lanes per token
   {
-    const int t = warp * 16 + (lane >> 1);
-    const uint8_t* kr = ks + t * PITCH + (lane & 1) * DK;
-    const uint8_t* qr = qs + t * PITCH + (lane & 1) * DK;
-    float sk = 0.f, sq = 0.f;
-#pragma unroll 4
-    for (int c = 0; c < DK / 16; ++c) {
-      const uint4 x = *reinterpret_cast<const uint4*>(kr + c * 16), y = *reinterpret_cast<const uint4*>(qr + c * 16);
-      const uint32_t xw[4] = {x.x, x.y, x.z, x.w}, yw[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        sk = fmaf(bf_lo(xw[i]), bf_lo(xw[i]), fmaf(bf_hi(xw[i]), bf_hi(xw[i]), sk));
-        sq = fmaf(bf_lo(yw[i]), bf_lo(yw[i]), fmaf(bf_hi(yw[i]), bf_hi(yw[i]), sq));
-      }
-    }
-    sk += __shfl_xor_sync(0xffffffffu, sk, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-    if (!(lane & 1)) { rk[t] = 1.0f / sqrtf(sk + p.unit_eps); rq[t] = p.q_scale / sqrtf(sq + p.unit_eps); }
-  }
-  __syncthreads();
-  // ---- k . k and q . k: warp = 16 rows i, tiles of 8 columns j up to the diagonal
-  {
+    // ---- k . k and q . k: warp = 16 rows i, the 16 columns of [d] d warps further to the left; and q . q of the rows themselves for their norms (k . k has them on its diagonal)
     const int gq = lane >> 2, tq = lane & 3, i0 = warp * 16;
-    float kk[8][4], qk[8][4];
+    float kk[4][2][4], qk[4][2][4], qq[2][4];
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int d = 0; d < 4; ++d)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) kk[n][e] = qk[n][e] = 0.f;
-    const int arow = i0 + (lane & 15), acol = (lane >> 4) * 16;
-    const int brow = (lane & 7) + ((lane >> 4) << 3), bcol = ((lane >> 3) & 1) * 16;
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { kk[d][u][e] = qk[d][u][e] = 0.f; if (d == 0) qq[u][e] = 0.f; }
+    const uint32_t arow = smem_u32(ks) + (i0 + (lane & 15)) * PITCH + (lane >> 4) * 16;
+    const uint32_t brow = smem_u32(ks) + (i0 + (lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 16;
 #pragma unroll 2
     for (int kt = 0; kt < DK / 16; ++kt) {
-      uint32_t ak[4], aq[4];
-      ldmatrix_x4(ak, ks + arow * PITCH + kt * 32 + acol);
-      ldmatrix_x4(aq, qs + arow * PITCH + kt * 32 + acol);
+      uint32_t ak[4], aq[4], bk[4];
+      ldmatrix_x4_at(ak, arow + kt * 32);
+      ldmatrix_x4_at(aq, arow + BT * PITCH + kt * 32);
+      ldmatrix_x4_at(bk, brow + BT * PITCH + kt * 32);
+      mma_np(qq[0], aq, bk[0], bk[1]); mma_np(qq[1], aq, bk[2], bk[3]);
 #pragma unroll
-      for (int n2 = 0; n2 < 4; ++n2) {
-        if (n2 <= warp) {
-          uint32_t bk[4];
-          ldmatrix_x4(bk, ks + (n2 * 16 + brow) * PITCH + kt * 32 + bcol);
-          mma_np(kk[2 * n2], ak, bk[0], bk[1]); mma_np(kk[2 * n2 + 1], ak, bk[2], bk[3]);
-          mma_np(qk[2 * n2], aq, bk[0], bk[1]); mma_np(qk[2 * n2 + 1], aq, bk[2], bk[3]);
+      for (int d = 0; d < 4; ++d) {
+        if (d <= warp) {
+          ldmatrix_x4_at(bk, brow - d * 16 * PITCH + kt * 32);
+          mma_np(kk[d][0], ak, bk[0], bk[1]); mma_np(kk[d][1], ak, bk[2], bk[3]);
+          mma_np(qk[d][0], aq, bk[0], bk[1]); mma_np(qk[d][1], aq, bk[2], bk[3]);
         }
       }
     }
+    if (tq == gq >> 1) {
+      const bool odd = gq & 1;
+      rk[i0 + gq] = 1.0f / sqrtf((odd ? kk[0][0][1] : kk[0][0][0]) + p.unit_eps);
+      rk[i0 + gq + 8] = 1.0f / sqrtf((odd ? kk[0][1][3] : kk[0][1][2]) + p.unit_eps);
+      rq[i0 + gq] = p.q_scale / sqrtf((odd ? qq[0][1] : qq[0][0]) + p.unit_eps);
+      rq[i0 + gq + 8] = p.q_scale / sqrtf((odd ? qq[1][3] : qq[1][2]) + p.unit_eps);
+    }
     __syncthreads();
+    // ---- A to shared memory; P goes to the workspace from here, as a second operand: column n = token i, k = token j; lane (gq, tq) of tile (kt, nt): i = 8 nt + gq,
+    // j = 16 kt + 8 u + 2 tq + {0, 1}
+    float lhi[2], lli[2], rqi[2], bri[2];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      if (n / 2 > warp) continue;
+    for (int r = 0; r < 2; ++r) { const int i = i0 + gq + 8 * r; lhi[r] = lh[i]; lli[r] = ll[i]; rqi[r] = rq[i]; bri[r] = beta[i] * rk[i]; }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = i0 + gq + (e >> 1) * 8, j = n * 8 + 2 * tq + (e & 1);
-        if (j <= i) {
-          const float gam = expf((lh[i] - lh[j]) + (ll[i] - ll[j])) * rk[j];
-          Ps[i * AP + j] = gam * rq[i] * qk[n][e];
-          if (j < i) As[i * AP + j] = beta[i] * (gam * rk[i] * kk[n][e]);
+    for (int d = 0; d < 4; ++d) {
+      if (d > warp) continue;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int kt = warp - d, j = kt * 16 + 8 * u + 2 * tq;
+        const float2 lhj = *reinterpret_cast<const float2*>(lh + j), llj = *reinterpret_cast<const float2*>(ll + j), rkj = *reinterpret_cast<const float2*>(rk + j);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int i = i0 + gq + 8 * r;
+          const float g0 = expf((lhi[r] - lhj.x) + (lli[r] - llj.x)) * rkj.x, g1 = expf((lhi[r] - lhj.y) + (lli[r] - llj.y)) * rkj.y;
+          float2 P = make_float2(g0 * rqi[r] * qk[d][u][2 * r], g1 * rqi[r] * qk[d][u][2 * r + 1]);
+          if (d == 0) { if (j > i) P.x = 0.f; if (j + 1 > i) P.y = 0.f; }
+          store_parts(out + TRI_BYTES + (kt * (9 - kt) + 2 * (warp - kt) + r) * PART_BYTES + u * 128 + lane * 4, P);
+          // (what lies on and above the diagonal of A is not used)
+          *reinterpret_cast<float2*>(As + i * AP + j) = make_float2(bri[r] * (g0 * kk[d][u][2 * r]), bri[r] * (g1 * kk[d][u][2 * r + 1]));
         }
       }
     }
   }
   __syncthreads();
-  // ---- T = (1 + A)^-1 in fp32: the two diagonal blocks of 32 by forward substitution, one column per thread; then T21 = -T22 (A21 T11), with the
-  // inner product in the unused upper right block (one block of 64 would be 2016 multiply-adds in a row, an instruction stream no cache holds)
-  uint8_t* out = p.blocks + (((int64_t)b * p.H + h) * p.n_blocks + blk) * BLOCK_BYTES;
-  float* vec = reinterpret_cast<float*>(out + 2 * TRI_BYTES);
+  // ---- T = (1 + A)^-1 in fp32: the two diagonal blocks of 32 by forward substitution, one column per thread (one block of 64 would be 2016 multiply-adds in a row, an instruction
+  // stream no cache holds); then the square below them
   if (tid < BT) {
     const int d = tid & 32, c = tid & 31;
     const float* Ad = As + d * AP + d;
@@ -225,49 +250,71 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   }
   __syncthreads();
   {
-    const int r = tid >> 2, c = (tid & 3) * 8;
-    // acc[0..7] = sum_k left[k] * right[k][c ..]
-    auto row_times = [&](const float* left, const float* right, float (&acc)[8]) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = 0.f;
-#pragma unroll 4
-      for (int k = 0; k < 32; ++k) {
-        const float l = left[k];
-        const float4 x = *reinterpret_cast<const float4*>(right + k * AP + c), y = *reinterpret_cast<const float4*>(right + k * AP + c + 4);
-        acc[0] = fmaf(l, x.x, acc[0]); acc[1] = fmaf(l, x.y, acc[1]); acc[2] = fmaf(l, x.z, acc[2]); acc[3] = fmaf(l, x.w, acc[3]);
-        acc[4] = fmaf(l, y.x, acc[4]); acc[5] = fmaf(l, y.y, acc[5]); acc[6] = fmaf(l, y.z, acc[6]); acc[7] = fmaf(l, y.w, acc[7]);
-      }
+    // T21^T = -(T11^T A21^T) T22^T: the sums of the first product are, lane by lane, the first operand of the second.  A warp has 16 columns c of T11 and 16 rows i of T22
+    const int gq = lane >> 2, tq = lane & 3, c = (warp & 1) * 16 + gq, ih = warp >> 1;
+    const float* A21 = As + 32 * AP;
+    const float* T22 = A21 + 32;
+    constexpr int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};       // small products first
+    const auto second = [&](const float* at, uint32_t (&w)[3][2]) {             // a column of the second operand: two neighbours, and those eight further on
+      const float2 x = *reinterpret_cast<const float2*>(at), y = *reinterpret_cast<const float2*>(at + 8);
+      split3(x.x, x.y, w[0][0], w[1][0], w[2][0]);
+      split3(y.x, y.y, w[0][1], w[1][1], w[2][1]);
     };
-    float acc[8];
-    row_times(As + (32 + r) * AP, As, acc);
+    float X[4][4], Y[2][4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) As[r * AP + 32 + c + u] = acc[u];
-    __syncthreads();
-    row_times(As + (32 + r) * AP + 32, As + 32, acc);
-    // (A21 was read before the barrier)
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) As[(32 + r) * AP + c + u] = -acc[u];
+      for (int e = 0; e < 4; ++e) { X[n][e] = 0.f; if (n < 2) Y[n][e] = 0.f; }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k < (warp & 1)) continue;                                             // (T11 is zero there)
+      uint32_t a[3][4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const float* at = As + (16 * k + 8 * (v >> 1) + 2 * tq) * AP + c + 8 * (v & 1);
+        split3(at[0], at[AP], a[0][v], a[1][v], a[2][v]);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        if (n >= 2 && !ih) continue;                                            // (nor does T22 have what would meet these)
+        uint32_t w[3][2];
+        second(A21 + (8 * n + gq) * AP + 16 * k + 2 * tq, w);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) mma_np(X[n], a[pa[m]], w[pb[m]][0], w[pb[m]][1]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k > ih) continue;
+      uint32_t a[3][4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) split3(X[2 * k + (v >> 1)][2 * (v & 1)], X[2 * k + (v >> 1)][2 * (v & 1) + 1], a[0][v], a[1][v], a[2][v]);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        uint32_t w[3][2];
+        second(T22 + (16 * ih + 8 * n + gq) * AP + 16 * k + 2 * tq, w);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) mma_np(Y[n], a[pa[m]], w[pb[m]][0], w[pb[m]][1]);
+      }
+    }
+    __syncthreads();                                                            // A21 has been read
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) As[(32 + 16 * ih + 8 * n + 2 * tq + (e & 1)) * AP + c + 8 * (e >> 1)] = -Y[n][e];
   }
   __syncthreads();
-  // ---- as second operands: column n = token i, k = token j; lane (g, tq) of tile (kt, nt): i = 8 nt + g, j = 16 kt + 2 tq + {0, 1} | + 8
-  for (int e = warp; e < 2 * TILES; e += 4) {
-    const float* src = e < TILES ? As : Ps;
-    int kt = 0, x = e % TILES;
+  // ---- T diag(beta), laid down like P
+  for (int e = warp; e < TILES; e += 4) {
+    int kt = 0, x = e;
     while (x >= 8 - 2 * kt) { x -= 8 - 2 * kt; ++kt; }
     const int i = 8 * (x + 2 * kt) + (lane >> 2), j = 16 * kt + 2 * (lane & 3);
-    uint32_t w[2][3];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int jj = j + 8 * u;
-      const float2 x = *reinterpret_cast<const float2*>(src + i * AP + jj);
-      const float f0 = e < TILES ? beta[jj] : 1.f, f1 = e < TILES ? beta[jj + 1] : 1.f;
-      split3(jj <= i ? x.x * f0 : 0.f, jj + 1 <= i ? x.y * f1 : 0.f, w[u][0], w[u][1], w[u][2]);
+      const float2 t = *reinterpret_cast<const float2*>(As + i * AP + jj), bt = *reinterpret_cast<const float2*>(beta + jj);
+      store_parts(out + e * PART_BYTES + u * 128 + lane * 4, make_float2(jj <= i ? t.x * bt.x : 0.f, jj + 1 <= i ? t.y * bt.y : 0.f));
     }
-    uint32_t* dst = reinterpret_cast<uint32_t*>(out + (e < TILES ? 0 : TRI_BYTES) + (e % TILES) * PART_BYTES) + lane;
-#pragma unroll
-    for (int s = 0; s < 3; ++s)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) dst[(s * TILES * PART_BYTES + u * 128) / 4] = w[u][s];
   }
 }
 
@@ -316,12 +363,6 @@ template <int N> __device__ __forceinline__ void tmem_st(uint32_t taddr, const u
   else
     asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
                  ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
-}
-// x and y without what is cut off in w (exact): the mixed multiply-add leaves the half-rate integer pipe, which bounds the splitting, to the byte permutations
-__device__ __forceinline__ float2 take_away(float2 x, uint32_t w) {
-  float2 r;
-  asm("{\n\t.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %4;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, lo, m, %2;\n\tfma.rn.f32.bf16 %1, hi, m, %3;\n\t}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "r"(w));
-  return r;
 }
 // the three parts (split3) of a thread's fragment, `apart` columns from one to the next
 template <int N> __device__ __forceinline__ void put_parts(uint32_t at, uint32_t apart, const float2* given) {
@@ -872,7 +913,7 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   a.gate = (const bf16*)p->gate; a.norm_w = (const bf16*)p->norm_w; a.out = (bf16*)p->out; a.ldo = p->ldo; a.eps = p->eps;
   a.norm = p->dv <= 2 * CH; a.pair = a.norm && p->dv > CH;
   a.wide = p->ldz % 4 == 0 && p->ldo % 4 == 0 && (((uintptr_t)p->gate | (uintptr_t)p->out) & 7) == 0;
-  constexpr int prep_smem = prepare_rows_bytes(DK) + 5 * BT * 4, scan_smem = scan_smem_bytes(DK);
+  constexpr int prep_smem = prepare_smem_bytes(DK), scan_smem = scan_smem_bytes(DK);
   CUtensorMap tmK, tmQ, tmV;
   const uint64_t kdims[3] = {(uint64_t)p->G * DK, (uint64_t)p->L, (uint64_t)p->B}, vdims[3] = {(uint64_t)p->H * p->dv, (uint64_t)p->L, (uint64_t)p->B};
   const uint64_t strides[2] = {(uint64_t)p->ld * 2, (uint64_t)p->L * p->ld * 2};
