@@ -95,27 +95,29 @@ __device__ __forceinline__ void load_resid16(const SmArgs& g, long long n, int b
   }
 }
 
-// epilogue of 16 batch rows [b0, b0+16) of output column n; v0 (and v1 for the gate) are fp32 sums
+// epilogue of one element: fp32 sums v0 (and v1 for the gate), residual value rv
+template <int EPI>
+__device__ __forceinline__ float finish(const SmArgs& g, long long n, float bias, float rv, float v0, float v1) {
+  if constexpr (EPI == EVO_EPI_GELU_GATE) {
+    return rbf(gelu_erf(rbf(v0))) * rbf(v1);
+  } else if constexpr (EPI == EVO_EPI_GELU_TANH_GATE) {
+    return gelu_tanh(v0) * v1;
+  } else if constexpr (EPI == EVO_EPI_SILU_COLS) {
+    return n < g.act_cols ? silu(v0) : v0;
+  } else {
+    float o = v0;
+    if constexpr (EPI == EVO_EPI_BIAS || EPI == EVO_EPI_BIAS_RESID) o += bias;
+    if constexpr (EPI == EVO_EPI_BIAS_RESID || EPI == EVO_EPI_RESID) o = rbf(o) + rv;
+    return o;
+  }
+}
+// 16 batch rows [b0, b0+16) of output column n
 template <int EPI>
 __device__ __forceinline__ void finalize16(const SmArgs& g, long long n, int b0, float bias, const float (&rv)[16],
                                            const float (&v0)[16], const float (&v1)[16]) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int b = b0 + j;
-    float o;
-    if constexpr (EPI == EVO_EPI_GELU_GATE) {
-      o = rbf(gelu_erf(rbf(v0[j]))) * rbf(v1[j]);
-    } else if constexpr (EPI == EVO_EPI_GELU_TANH_GATE) {
-      o = gelu_tanh(v0[j]) * v1[j];
-    } else if constexpr (EPI == EVO_EPI_SILU_COLS) {
-      o = n < g.act_cols ? silu(v0[j]) : v0[j];
-    } else {
-      o = v0[j];
-      if constexpr (EPI == EVO_EPI_BIAS || EPI == EVO_EPI_BIAS_RESID) o += bias;
-      if constexpr (EPI == EVO_EPI_BIAS_RESID || EPI == EVO_EPI_RESID) o = rbf(o) + rv[j];
-    }
-    if (b < g.M) g.C[(long long)b * g.ldc + n] = __float2bfloat16_rn(o);
-  }
+  for (int j = 0; j < 16; ++j)
+    if (b0 + j < g.M) g.C[(long long)(b0 + j) * g.ldc + n] = __float2bfloat16_rn(finish<EPI>(g, n, bias, rv[j], v0[j], v1[j]));
 }
 
 constexpr int EPI_HYENA_STEP = 7;   // EVO_EPI_HYENA_STEP
@@ -183,6 +185,63 @@ __device__ __forceinline__ void hyena_step16(const SmArgs& g, int tile, int row,
   }
 }
 
+// The slots of a tile are summed by its last contributor, in contributor order (deterministic), and the epilogue applied.  This runs once per launch at the end of its serial chain, with
+// cold instruction caches: four columns per lane and a warp per batch row (two in flight) are a quarter of the loads, and a quarter of the code, of a thread per column.  One step of
+// one request 446 -> 394 us, of 16 664 -> 623; (only fewer rows for a thread per column: 400 / 680).
+template <int EPI>
+__device__ __forceinline__ void fix_up(const SmArgs& g, int tile, int c_first, int c_last, bool first_begins_before, int slot_floats) {
+  constexpr int R = RowGroups<EPI>::R, FX = 8 / R;
+  const int col = (threadIdx.x & 31) * 4;
+  const long long n = (long long)tile * WROWS + col;
+  const float* base = g.slots + col;
+#pragma unroll 1
+  for (int b0 = (threadIdx.x >> 5) - EPI_WARP0; b0 < g.M; b0 += 8) {
+    const int b[2] = {b0, min(b0 + 4, g.M - 1)};                      // (the last row twice rather than none)
+    float4 v[2][R];
+    float bias[4], rv[2][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      bias[e] = rv[0][e] = rv[1][e] = 0.f;
+      if constexpr (EPI == EVO_EPI_BIAS || EPI == EVO_EPI_BIAS_RESID) bias[e] = __bfloat162float(g.bias[n + e]);
+      if constexpr (EPI == EVO_EPI_BIAS_RESID || EPI == EVO_EPI_RESID) { rv[0][e] = __bfloat162float(g.resid[b[0] * g.ldr + n + e]); rv[1][e] = __bfloat162float(g.resid[b[1] * g.ldr + n + e]); }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int cb = c_first; cb <= c_last; cb += FX) {
+      float4 t[FX][2][R];
+#pragma unroll
+      for (int u = 0; u < FX; ++u) {                                  // all in flight together
+        const int cc = min(cb + u, c_last);
+        // a contributor's second slot is that of a range which begins in an earlier tile: only the first one's can
+        const float* s = base + (size_t)(2 * cc + (cc == c_first && first_begins_before ? 1 : 0)) * slot_floats;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int q = 0; q < R; ++q) t[u][i][q] = __ldcg(reinterpret_cast<const float4*>(s + (q * g.Mb + b[i]) * WROWS));
+      }
+#pragma unroll
+      for (int u = 0; u < FX; ++u)
+        if (cb + u <= c_last) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int q = 0; q < R; ++q) { v[i][q].x += t[u][i][q].x; v[i][q].y += t[u][i][q].y; v[i][q].z += t[u][i][q].z; v[i][q].w += t[u][i][q].w; }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (i && b0 + 4 >= g.M) continue;
+      const float v0[4] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w}, v1[4] = {v[i][R - 1].x, v[i][R - 1].y, v[i][R - 1].z, v[i][R - 1].w};
+      bf16* out = g.C + b[i] * g.ldc + n;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[e] = __float2bfloat16_rn(finish<EPI>(g, n + e, bias[e], rv[i][e], v0[e], v1[e]));
+    }
+  }
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const SmArgs g) {
@@ -207,11 +266,21 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if ((smem_u32(smem) & 1023u) != 0) __trap();
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 0] = gtimer(); g.trace[blockIdx.x * 16 + 1] = clock64(); }
 
-  if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmA); }
-  if (warp == 1 && lane == 0) {
-    for (int i = 0; i < MAXST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+  const uint32_t total = (uint32_t)g.n_tiles * KB, parts = gridDim.x;
+  const int it_begin = (int)range_start(blockIdx.x, total, parts), it_end = (int)range_start(blockIdx.x + 1, total, parts);
+  const int n_it = it_end - it_begin;
+  const uint32_t STAGE_TX = (uint32_t)(W_STAGE + A_STAGE);
+  const auto load_w = [&](int stage, int tile, int kb) {
+#pragma unroll
+    for (int bx = 0; bx < NBOX; ++bx) tma_load_2d(smW + stage * W_STAGE + bx * (WBOX * BK * 2), &tmW, &full[stage], kb * BK, tile * (R * WROWS) + bx * WBOX);
+  };
+  const int pre = min(NST, n_it);
+  if (warp == 0 && lane == 0) {
+    for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 4); }
     fence_barrier_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmA);
   }
   const int acc_cols = R * Mb;                                // fp32 columns of one accumulator
   uint32_t tmem_cols = 32; while ((int)tmem_cols < 2 * acc_cols) tmem_cols *= 2;
@@ -222,25 +291,17 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) stamp(g, 2);                          // setup done
 
-  const uint32_t total = (uint32_t)g.n_tiles * KB, parts = gridDim.x;
-  const int it_begin = (int)range_start(blockIdx.x, total, parts), it_end = (int)range_start(blockIdx.x + 1, total, parts);
-  const int n_it = it_end - it_begin;
-  const uint32_t STAGE_TX = (uint32_t)(W_STAGE + A_STAGE);
-
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
     if (lane == 0) {
-      const int tile_b = it_begin / KB, kb_b = it_begin - tile_b * KB;
-      const int pre = min(NST, n_it);
-      int tile = tile_b, kb = kb_b;
+      int tile = it_begin / KB, kb = it_begin - tile * KB;
       for (int i = 0; i < pre; ++i) {                         // weights first: they do not depend on the previous kernel
         mbar_arrive_expect_tx(&full[i], STAGE_TX);
-#pragma unroll
-        for (int bx = 0; bx < NBOX; ++bx) tma_load_2d(smW + i * W_STAGE + bx * (WBOX * BK * 2), &tmW, &full[i], kb * BK, tile * (R * WROWS) + bx * WBOX);
+        load_w(i, tile, kb);
         if (++kb == KB) { kb = 0; ++tile; }
       }
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      tile = tile_b; kb = kb_b;
+      tile = it_begin / KB; kb = it_begin - tile * KB;
       for (int i = 0; i < pre; ++i) {
         tma_load_2d(smA + i * A_STAGE, &tmA, &full[i], kb * BK, 0);
         if (++kb == KB) { kb = 0; ++tile; }
@@ -249,8 +310,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       for (int i = pre; i < n_it; ++i) {
         mbar_wait(&empty[stage], phase ^ 1);
         mbar_arrive_expect_tx(&full[stage], STAGE_TX);
-#pragma unroll
-        for (int bx = 0; bx < NBOX; ++bx) tma_load_2d(smW + stage * W_STAGE + bx * (WBOX * BK * 2), &tmW, &full[stage], kb * BK, tile * (R * WROWS) + bx * WBOX);
+        load_w(stage, tile, kb);
         tma_load_2d(smA + stage * A_STAGE, &tmA, &full[stage], kb * BK, 0);
         if (++kb == KB) { kb = 0; ++tile; }
         if (++stage == NST) { stage = 0; phase ^= 1; }
@@ -307,6 +367,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const long long n = (long long)tile * WROWS + row;      // output column (gate: of the N/2-wide output)
       float bias = 0.f;
       if constexpr (EPI == EVO_EPI_BIAS || EPI == EVO_EPI_BIAS_RESID) bias = __bfloat162float(g.bias[n]);
+      // (the tile's contributors, found while its products are under way)
+      const int c_first = whole ? 0 : cta_of((uint32_t)tile * KB, total, parts), c_last = whole ? 0 : cta_of((uint32_t)(tile + 1) * KB - 1, total, parts);
       mbar_wait(&tfull[acc], acc_phase);
       if (threadIdx.x == EPI_WARP0 * 32) stamp(g, it + (k1 - k0) >= it_end ? 5 : 9);   // (last) accumulator complete
       tc_fence_after();
@@ -335,9 +397,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         for (int c = 0; c < acc_cols; c += 16) {
           uint32_t r0[16];
           tmem_ld_32x16(t0 + c, r0);
+          const int live = g.M - c % Mb;                      // rows behind A's last one are neither stored nor read
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) slot[(c + j) * WROWS + row] = __uint_as_float(r0[j]);
+          for (int j = 0; j < 16; ++j) if (j < live) slot[(c + j) * WROWS + row] = __uint_as_float(r0[j]);
         }
       }
       tc_fence_before();
@@ -347,7 +410,6 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (!whole) {
         // publication: the CTA barrier orders every thread's partial stores before thread 0's acq_rel atomic (release
         // is cumulative), whose acquire half orders the finisher's slot reads after the other contributors' releases
-        const int c_first = cta_of((uint32_t)tile * KB, total, parts), c_last = cta_of((uint32_t)(tile + 1) * KB - 1, total, parts);
         named_bar(1, 128);
         if (threadIdx.x == EPI_WARP0 * 32) {
           int old;
@@ -358,38 +420,22 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const bool last = *flag == c_last - c_first;
         if (threadIdx.x == EPI_WARP0 * 32) stamp(g, 6);       // partial published
         if (last) {
-          for (int c = 0; c < Mb; c += 16) {
-            float v0[16], v1[16], v2[16], rv[16];
-            load_resid16<EPI>(g, n, c, rv);
+          const bool first_begins_before = range_start((uint32_t)c_first, total, parts) < (uint32_t)tile * KB;
+          if constexpr (EPI == EPI_HYENA_STEP) {
+            for (int c = 0; c < Mb; c += 16) {
+              float v[3][16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) { v0[j] = 0.f; v1[j] = 0.f; v2[j] = 0.f; }
-            // slots are summed in contributor order (deterministic); the loads of FX contributors are in flight together
-            constexpr int FX = R == 3 ? 2 : (R == 2 ? 4 : 8);
-            for (int cb = c_first; cb <= c_last; cb += FX) {
-              float t0v[FX][16], t1v[FX][16], t2v[FX][16];
+              for (int j = 0; j < 16; ++j) v[0][j] = v[1][j] = v[2][j] = 0.f;
+              for (int cc = c_first; cc <= c_last; ++cc) {
+                const float* s = g.slots + (size_t)(2 * cc + (cc == c_first && first_begins_before ? 1 : 0)) * slot_floats;
 #pragma unroll
-              for (int u = 0; u < FX; ++u) {
-                const int cc = min(cb + u, c_last);
-                const int first_tile_cc = (int)(range_start((uint32_t)cc, total, parts) / (uint32_t)KB);
-                const float* s = g.slots + (size_t)(2 * cc + (first_tile_cc == tile ? 0 : 1)) * slot_floats;
+                for (int q = 0; q < 3; ++q)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  t0v[u][j] = __ldcg(s + (c + j) * WROWS + row);
-                  if constexpr (R >= 2) t1v[u][j] = __ldcg(s + (Mb + c + j) * WROWS + row);
-                  if constexpr (R == 3) t2v[u][j] = __ldcg(s + (2 * Mb + c + j) * WROWS + row);
-                }
+                  for (int j = 0; j < 16; ++j) if (c + j < g.M) v[q][j] += __ldcg(s + (q * Mb + c + j) * WROWS + row);
               }
-#pragma unroll
-              for (int u = 0; u < FX; ++u) {
-                if (cb + u <= c_last) {
-#pragma unroll
-                  for (int j = 0; j < 16; ++j) { v0[j] += t0v[u][j]; if constexpr (R >= 2) v1[j] += t1v[u][j]; if constexpr (R == 3) v2[j] += t2v[u][j]; }
-                }
-              }
+              hyena_step16(g, tile, row, c, v[0], v[1], v[2]);
             }
-            if constexpr (EPI == EPI_HYENA_STEP) hyena_step16(g, tile, row, c, v0, v1, v2);
-            else finalize16<EPI>(g, n, c, bias, rv, v0, v1);
-          }
+          } else fix_up<EPI>(g, tile, c_first, c_last, first_begins_before, slot_floats);
           if (threadIdx.x == EPI_WARP0 * 32) g.counters[tile] = 0;   // self-cleaning for the next launch
         }
       }
@@ -405,9 +451,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 8] = clock64(); g.trace[blockIdx.x * 16 + 15] = gtimer(); }
 }
 
+// Shared memory of the ring.  Two CTAs of neighbouring layers do not fit an SM together (168 registers a thread), so a CTA starts when that of the layer in front has ended there: in
+// the tail in which memory idles, and what its ring holds by the time the sums are published is ahead of the stream.  One step of one request / of 16 (us): 104 KB 399 / 625,
+// 150 KB 389 / 616, 180 KB 385 / 614, 216 KB 388 / 615.  (Two to an SM, 128 registers and 104 KB: 410 / 642; the ring is then filled during the layer in front, which it slows.)
 int smem_budget_bytes() {
   static int kb = 0;
-  if (!kb) { const char* e = getenv("EVO_B200_SMALLM_SMEM_KB"); kb = e ? atoi(e) : 104; kb = std::max(40, std::min(kb, 224)); }
+  if (!kb) { const char* e = getenv("EVO_B200_SMALLM_SMEM_KB"); kb = e ? atoi(e) : 180; kb = std::max(40, std::min(kb, 224)); }
   return kb * 1024;
 }
 
