@@ -27,15 +27,19 @@ __device__ __forceinline__ float rbf(float x) { return __bfloat162float(__float2
 __device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 // two fp32 numbers as three packed bf16 parts, cut off rather than rounded: 8 + 8 + 8 bits are the whole mantissa
-__device__ __forceinline__ float2 top2(float x, float y) { return make_float2(__uint_as_float(__float_as_uint(x) & 0xffff0000u), __uint_as_float(__float_as_uint(y) & 0xffff0000u)); }
 __device__ __forceinline__ uint32_t tops(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+// x minus the packed bf16 pair w, exact where w is x cut off (or rounded): the mixed multiply-add takes the halves as they are, and leaves the half-rate integer pipe to the permutations
+__device__ __forceinline__ float2 take_away(float2 x, uint32_t w) {
+  float2 r;
+  asm("{\n\t.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %4;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, lo, m, %2;\n\tfma.rn.f32.bf16 %1, hi, m, %3;\n\t}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "r"(w));
+  return r;
+}
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = tops(x, y);
-  float2 t = top2(x, y);
-  x -= t.x; y -= t.y;
-  mid = tops(x, y);
-  t = top2(x, y);
-  lo = tops(x - t.x, y - t.y);
+  float2 r = take_away(make_float2(x, y), hi);
+  mid = tops(r.x, r.y);
+  r = take_away(r, mid);
+  lo = tops(r.x, r.y);
 }
 // silu of two values for rows stored as bf16: v / (1 + e^-v) with the bare 2^x and reciprocal instructions and packed multiply-adds, about half of what expf and the IEEE
 // division take.  t = -v log2 e is rounded; its remainder `lo` (exact product, and the constant's own remainder) corrects 2^t to first order, so that the exponential keeps the

@@ -74,12 +74,6 @@ __device__ __forceinline__ void mma_np(float* d, const uint32_t* a, uint32_t b0,
 __device__ __forceinline__ float softplus_f(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // ------------------------------------------------------------------------------------------------ what does not depend on the state
-// x without what is cut off in w (exact): the mixed multiply-add leaves the half-rate integer pipe, which bounds the splitting, to the byte permutations
-__device__ __forceinline__ float2 take_away(float2 x, uint32_t w) {
-  float2 r;
-  asm("{\n\t.reg .b16 lo, hi, m;\n\tmov.b32 {lo, hi}, %4;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, lo, m, %2;\n\tfma.rn.f32.bf16 %1, hi, m, %3;\n\t}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "r"(w));
-  return r;
-}
 // the three parts (split3) of two neighbours of a row, to a lane's place in the tiles of each part
 __device__ __forceinline__ void store_parts(uint8_t* dst, float2 x) {
 #pragma unroll
