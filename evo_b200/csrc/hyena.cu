@@ -215,19 +215,10 @@ __global__ void hyena_fold_states_kernel(const float* __restrict__ seg_states, c
   reinterpret_cast<float2*>(out)[idx] = make_float2(acc.r, acc.i);
 }
 
-__global__ void fir_state_kernel(const bf16* __restrict__ z, const bf16* __restrict__ halo, bf16* __restrict__ out,
-                                 int B, long long L, long long C3) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // (b, c)
-  if (idx >= (long long)B * C3) return;
-  long long b = idx / C3, c = idx % C3;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    long long t = L - 2 + k;
-    bf16 v = __float2bfloat16_rn(0.f);
-    if (t >= 0) v = z[(b * L + t) * C3 + c];
-    else if (halo) v = halo[(b * 2 + (t + 2)) * C3 + c];
-    out[idx * 2 + k] = v;
-  }
+__global__ void fir_state_kernel(const bf16* __restrict__ z, const bf16* __restrict__ halo, bf16* __restrict__ out, int B, long long L, long long C3) {
+  pdl_launch_dependents();
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // (b, c)
+  if (idx < (long long)B * C3) evo_hytc::fir_state(z, halo, out, idx, L, C3);
 }
 
 // decode step (engine.step_fir + step_iir): 8 lanes per (b, channel).  Lane s owns modal state s (its pole, residue
@@ -371,6 +362,24 @@ static size_t workspace_bytes_of(const evo_hyena_params* p, const HyenaPlan& pla
 
 extern "C" size_t evo_hyena_fwd_workspace(const evo_hyena_params* p) { return p->L <= 0 || p->B <= 0 ? 0 : workspace_bytes_of(p, make_plan(p)); }
 
+// a launch that may begin while the kernel in front is still running (dependent: that kernel lets it), or an ordinary one
+template <typename... KArgs, typename... A>
+static cudaError_t launch_after(bool dependent, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization; attr.val.programmaticStreamSerializationAllowed = 1;
+  if (dependent) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
+// Are the inputs that the call leaves for the next one written over those that it begins with?  Then they are copied last.
+static bool fir_state_over_halo(const evo_hyena_params* p) {
+  if (!p->fir_state_out || !p->halo) return false;
+  const uintptr_t n = (uintptr_t)p->B * 3 * p->D * 2 * sizeof(bf16), o = (uintptr_t)p->fir_state_out, h = (uintptr_t)p->halo;
+  return o < h + n && h < o + n;
+}
+
 // evo_hytc: constants, then (more than one segment) the segments' end states, then the output
 template <int R>
 static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, void* workspace, cudaStream_t st) {
@@ -396,18 +405,32 @@ static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, voi
   static unsigned long long done_s = 0, done_o = 0;
   if ((rc = ensure_dyn_smem(hyena_tc_kernel<R, true>, smem, done_s))) return rc;
   if ((rc = ensure_dyn_smem(hyena_tc_kernel<R, false>, smem, done_o))) return rc;
-  hyena_tc_constants_kernel<<<p->D / PREP_WARPS, PREP_WARPS * 32, 0, st>>>(p->poles, p->residues, consts, seg_pow, p->D, R, nseg > 1 ? seg_len : 0);
+  bf16* fir_out = fir_state_over_halo(p) ? nullptr : (bf16*)p->fir_state_out;
+  const int copies = fir_out ? (int)(((long long)p->B * 3 * p->D + PREP_WARPS * 32 - 1) / (PREP_WARPS * 32)) : 0;
+  hyena_tc_constants_kernel<<<p->D / PREP_WARPS + copies, PREP_WARPS * 32, 0, st>>>(p->poles, p->residues, consts, seg_pow, p->D, R, nseg > 1 ? seg_len : 0, a.z, a.halo, fir_out, p->B, p->L);
   if ((rc = check_launch("hyena_tc_constants"))) return rc;
   const int per_seg = p->D / CH * p->B, sms = device_sm_count();
-  if (p->state_only || (nseg > 1 && !p->reuse_segment_states)) {
+  const bool states = p->state_only || (nseg > 1 && !p->reuse_segment_states);
+  // A dependent launch takes about 4 us off a call, but its CTAs do not start together, and long calls lose more by that: neighbouring channels' CTAs then no longer read a token's row at
+  // the same time.  Normal / dependent (us, D = 4096): 1 x 500: 23.8 / 20.6, 1 x 1999: 45.1 / 41.5, 2 x 4096 127 / 124, 4 x 4096 236 / 233, 4 x 8193 464 / 464, 8 x 4096 412 / 416,
+  // 8 x 8193 850 / 867.  The line: 16 k tokens that a CTA walks.
+  const long long walked = (long long)((per_seg * nseg + sms - 1) / sms) * std::min<long long>(seg_len, p->L);
+  const bool soon = walked <= (16 << 10) + 1024;
+  if (states) {
     a.items = per_seg * (p->state_only ? nseg : nseg - 1);
-    hyena_tc_kernel<R, true><<<std::min(a.items, sms), evo_hytc::THREADS, smem, st>>>(tmZ, a);
+    EVO_CUDA(launch_after(soon, hyena_tc_kernel<R, true>, dim3(std::min(a.items, sms)), dim3(evo_hytc::THREADS), smem, st, tmZ, a));
     if ((rc = check_launch("hyena_tc<state>"))) return rc;
   }
   if (p->state_only) return 0;
   a.items = per_seg * nseg;
-  hyena_tc_kernel<R, false><<<std::min(a.items, sms), evo_hytc::THREADS, smem, st>>>(tmZ, a);
+  EVO_CUDA(launch_after(soon && !states, hyena_tc_kernel<R, false>, dim3(std::min(a.items, sms)), dim3(evo_hytc::THREADS), smem, st, tmZ, a));
   return check_launch("hyena_tc<out>");
+}
+
+static int copy_fir_state(const evo_hyena_params* p, cudaStream_t st) {
+  const long long n = (long long)p->B * 3 * p->D;
+  fir_state_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const bf16*)p->z, (const bf16*)p->halo, (bf16*)p->fir_state_out, p->B, p->L, 3LL * p->D);
+  return check_launch("fir_state");
 }
 
 extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -424,11 +447,15 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
   if (p->state_only) EVO_REQUIRE(p->state_out != nullptr, "evo_hyena_fwd: state_only needs state_out");
   else EVO_REQUIRE(p->y != nullptr, "evo_hyena_fwd: y is NULL");
   int rc;
+  bool fir_done = false;
   if (plan.tc) {
     const int R = plan.R;
+    fir_done = !fir_state_over_halo(p);
     if ((rc = R == 4 ? launch_tc<4>(p, nseg, seg_len, workspace, st) : (R == 2 ? launch_tc<2>(p, nseg, seg_len, workspace, st) : launch_tc<1>(p, nseg, seg_len, workspace, st)))) return rc;
   } else if (use_tma_path(p)) {
     using namespace evo_hy2;
+    // the copy of the inputs that a state keeps goes first, and the (split) scan begins beside it
+    const bool split = plan.scan_variant != 0, copied = split && p->fir_state_out && !fir_state_over_halo(p);
     CUtensorMap tmZ;
     uint64_t dims[3] = {(uint64_t)3 * p->D, (uint64_t)p->L, (uint64_t)p->B};
     uint64_t str[2] = {(uint64_t)3 * p->D * 2, (uint64_t)p->L * 3 * p->D * 2};
@@ -444,7 +471,6 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     if ((rc = ensure_dyn_smem(hyena_scan_tma_kernel<false>, smem_bytes(STAGES), done_o))) return rc;
     // mode-split kernel (hyena_ms.cuh: 8 compute warps, 4 modal states per thread) or, for comparisons and as a second implementation in the parity tests,
     // its predecessor (hyena_tma.cuh: 4 compute warps, 8 states per thread)
-    const bool split = plan.scan_variant != 0;
     static unsigned long long done_ms = 0, done_mo = 0;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<true>, smem_bytes(STAGES), done_ms))) return rc;
     if ((rc = ensure_dyn_smem(evo_hy3::hyena_scan_ms_kernel<false>, smem_bytes(STAGES), done_mo))) return rc;
@@ -455,18 +481,21 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     // An 8-deep ring for single-CTA-per-SM grids was measured and did not help (1.21 vs 1.06-1.13 ms at B=8, L=8193).
     a.nst = 4;
     const int SMEM_BYTES = smem_bytes(a.nst);
+    if (copied) { if ((rc = copy_fir_state(p, st))) return rc; }
     if (p->state_only) {
-      k_state<<<grid, block, SMEM_BYTES, st>>>(tmZ, a);
+      EVO_CUDA(launch_after(copied, k_state, grid, block, SMEM_BYTES, st, tmZ, a));
       if ((rc = check_launch("hyena_scan<state>"))) return rc;
     } else {
-      if (nseg > 1 && !p->reuse_segment_states) {
+      const bool states = nseg > 1 && !p->reuse_segment_states;
+      if (states) {
         dim3 g2(grid.x, grid.y, nseg - 1);
-        k_state<<<g2, block, SMEM_BYTES, st>>>(tmZ, a);
+        EVO_CUDA(launch_after(copied, k_state, g2, block, SMEM_BYTES, st, tmZ, a));
         if ((rc = check_launch("hyena_scan<state>"))) return rc;
       }
-      k_out<<<grid, block, SMEM_BYTES, st>>>(tmZ, a);
+      EVO_CUDA(launch_after(copied && !states, k_out, grid, block, SMEM_BYTES, st, tmZ, a));
       if ((rc = check_launch("hyena_scan<out>"))) return rc;
     }
+    if (copied) fir_done = true;
   } else {
     Args a;
     a.z = (const bf16*)p->z; a.y = (bf16*)p->y;
@@ -495,12 +524,7 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     hyena_fold_states_kernel<<<(n + 255) / 256, 256, 0, st>>>((const float*)workspace, p->state_in, p->poles, p->state_out, p->B, p->D, nseg, seg_len, p->L);
     if ((rc = check_launch("hyena_fold_states"))) return rc;
   }
-  if (p->fir_state_out) {
-    long long n = (long long)p->B * 3 * p->D;
-    fir_state_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const bf16*)p->z, (const bf16*)p->halo, (bf16*)p->fir_state_out, p->B, p->L, 3LL * p->D);
-    if ((rc = check_launch("fir_state"))) return rc;
-  }
-  return 0;
+  return p->fir_state_out && !fir_done ? copy_fir_state(p, st) : 0;
 }
 
 extern "C" int evo_hyena_step(const void* u, void* y, void* fir_state, float* state,

@@ -254,6 +254,7 @@ hyena_scan_ms_kernel(const __grid_constant__ CUtensorMap tmZ, const Args2 a) {
     if (lane == 0) mbar_arrive(&empty[st]);
   }
 
+  pdl_wait();                                  // launched behind the copy of the inputs that a state keeps, whose results nothing here reads: it is through before this kernel is
   float* dst = nullptr;
   if (STATE_ONLY) dst = a.seg_states + ((((long long)b * a.nseg + seg) * a.D + ch) * NS) * 2;
   else if (a.state_out && seg == a.nseg - 1) dst = a.state_out + (((long long)b * a.D + ch) * NS) * 2;

@@ -16,7 +16,7 @@
 //                      steps with powers p^{16R}, p^{32R}, p^{64R}); then every block's c, rounded, + D x, back into the place of x
 // The fragment layouts of A operands and sums agree (a lane owns 4 consecutive tokens of rows g and g + 8), so B needs no shuffle besides the fold.
 // z is read once and y written once.
-// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 811 us (modal scan on the CUDA cores 953), 1 x 1999 44 us (138), 4 x 1000 76 us (123), 1 x 301 23 us (42).
+// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 850 us sustained (modal scan on the CUDA cores 953), 1 x 1999 41.5 us (138), 4 x 1000 76 us (123), 1 x 301 20 us (42).
 // A steady tile of 1024 tokens takes 24.5 k cycles, all of them the tensor-core warps' (tensor pipe 6.7 k, fp32 pipe 9 k, issue 10 k per scheduler): bound by the
 // latencies of its dependent steps with two such warps per scheduler (5.6 cycles per instruction each, by clock stamps; ncu on 1 x 8193: issue slots 59 % used, tensor pipe 23 %).  Register shares of 128 / 88 or 136 / 80
 // are 2 - 3 % slower: the element-wise warps then spill more (the output kernels spill 16 to 112 bytes as it is, -Xptxas -v).
@@ -87,9 +87,31 @@ __device__ __forceinline__ void parts3(double v, uint32_t (&out)[3]) {
   }
 }
 
+// the last two inputs of a sequence, for what continues it: element idx = (b, column) of (B, 3D, 2)
+__device__ __forceinline__ void fir_state(const bf16* __restrict__ z, const bf16* __restrict__ halo, bf16* __restrict__ out, long long idx, long long L, long long C3) {
+  const long long b = idx / C3, c = idx % C3;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const long long t = L - 2 + k;
+    bf16 v = __float2bfloat16_rn(0.f);
+    if (t >= 0) v = z[(b * L + t) * C3 + c];
+    else if (halo) v = halo[(b * 2 + (t + 2)) * C3 + c];
+    out[idx * 2 + k] = v;
+  }
+}
+
+// The operator's kernel is launched dependent where a call is short: its CTAs start where this one's have ended, and filter their first inputs while the rest of the constants is computed.  The blocks behind
+// the channels' copy the inputs that a state keeps, which had a launch of their own (B, L, C3 are theirs; fir_out NULL: none).
 constexpr int PREP_WARPS = 4;
 __global__ void __launch_bounds__(PREP_WARPS * 32) hyena_tc_constants_kernel(const float* __restrict__ poles, const float* __restrict__ residues, uint8_t* __restrict__ consts,
-                                                                             float2* __restrict__ seg_pow, int D, int R, long long seg_len) {
+                                                                             float2* __restrict__ seg_pow, int D, int R, long long seg_len, const bf16* __restrict__ z,
+                                                                             const bf16* __restrict__ halo, bf16* __restrict__ fir_out, int B, long long L) {
+  pdl_launch_dependents();
+  if ((int)blockIdx.x >= D / PREP_WARPS) {
+    const long long idx = (long long)(blockIdx.x - D / PREP_WARPS) * (PREP_WARPS * 32) + threadIdx.x;
+    if (idx < (long long)B * 3 * D) fir_state(z, halo, fir_out, idx, L, 3ll * D);
+    return;
+  }
   __shared__ D2 pw[PREP_WARPS][NS][BLK + 1];
   __shared__ D2 rq[PREP_WARPS][NS][BLK + 1];                // R_s p_s^k
   __shared__ double h[PREP_WARPS][BLK];
@@ -418,6 +440,7 @@ __global__ void __launch_bounds__(THREADS, 1) hyena_tc_kernel(const __grid_const
     if (lane < REST) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + CONST_BYTES / 512 * 512), "l"(src + CONST_BYTES / 512 * 512) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  pdl_wait();                                                           // the constants
   fetch(w.ch0 + warp);
   for (uint32_t q = 0; w.more(a); ++q) {
     const int n = w.tokens(TILE);
