@@ -12,10 +12,10 @@
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
 //   S, W, U are fp32 and enter as three bf16 parts; K and Q are bf16 as they stand (their norms scale the sums); T, P have three parts and meet W, U in the six products
 //   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work; the read-outs are normed, weighted and gated by warps of their own.
-// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 316 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
+// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 313 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
 // which the scan 224 (395 + 51) and delta_prepare_kernel 92 (135 with the norms summed apart, both matrices stored and read again, and the square of T by
 // multiply-adds from shared memory: 15.7 k instructions and 5.5 k shared-memory wavefronts an item then, 10.5 k and 2.3 k now; its four warps wait for one another at barriers; six CTAs per
-// SM, which spill: 135); 1 x 777 tokens, 32 heads: 65 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
+// SM, which spill: 135); 1 x 777 tokens, 32 heads: 60 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
 // cycles, by clock stamps); what is left of the chain  state's parts - K S - W's parts - T W - U's parts - K U - state  is the splitting, bound by instructions (11 k warp instructions a
 // block and CTA, four per element of W, U and S; three byte permutations of the half-rate integer pipe and four mixed multiply-adds of two numbers).
 // A block in which U is not finite goes token by token: a product with a structural zero would carry a NaN to earlier tokens.
@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   float* beta = rq + BT;
   float* lh = beta + BT;                                     // running log decay, high and low float
   float* ll = lh + BT;
+  pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (p.H / p.G);
   const int64_t t0 = (p.first + blk) * BT, row0 = (int64_t)b * p.L + t0;
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
     fence_barrier_init();
   }
   if (warp == MMA_WARP) { tmem_alloc<1>(&tmem_slot, 512); tmem_relinquish<1>(); }
-  const bool given_up = p.first > 0 && *(volatile unsigned int*)p.failed;
+  const bool given_up = p.first > 0 && *(volatile unsigned int*)p.failed;      // (of the slab in front, which was through before this one's delta_prepare_kernel began)
   tc_fence_before();
   const bool skip = __syncthreads_or(given_up);
   tc_fence_after();
@@ -723,6 +724,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
       if (lane == 0 && n_blocks) {
         tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmV);
         int blk = 0;
+        pdl_wait();                                      // T, P and vectors; nothing else of this kernel, which may be launched dependent, comes from delta_prepare_kernel
         for (; blk < n_blocks; ++blk) {
           const int s = blk & 1;
           if (blk >= 2 && !wait_or_give_up(&empty[s], ((blk >> 1) - 1) & 1, p.waits)) { ok = false; break; }
@@ -925,9 +927,14 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
     if ((rc = check_launch("evo_gated_delta_fwd(prepare)"))) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.H, a.B, (a.dv + CH - 1) / CH); cfg.blockDim = dim3(SCAN_THREADS); cfg.dynamicSmemBytes = scan_smem; cfg.stream = st;
-    cudaLaunchAttribute two = {};
-    two.id = cudaLaunchAttributeClusterDimension; two.val.clusterDim = {1, 1, 2};
-    if (a.pair) { cfg.attrs = &two; cfg.numAttrs = 1; }
+    cudaLaunchAttribute attrs[2] = {};
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension; attrs[1].val.clusterDim = {1, 1, 2};
+    // Launched dependent, the scan's CTAs are set up while the last of delta_prepare_kernel's run, which is worth 2 to 4 us: normal / dependent (us) 1 x 300 tokens, 8 heads of 64 x 64
+    // 28.8 / 26.7, 1 x 777, 32 heads of 128 x 128 62.9 / 60.4, 1 x 4096 253 / 249.  But CTAs that come to most of the SMs one by one are placed worse: 64 pairs, 128 CTAs, 4 x 4096 tokens
+    // 313 / 340, 4 x 1024 95 / 99; 128 pairs of 128 x 64 67.0 / 67.6.
+    const bool dependent = (int64_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z * 2 <= device_sm_count();
+    cfg.attrs = dependent ? attrs : attrs + 1; cfg.numAttrs = (dependent ? 1 : 0) + (a.pair ? 1 : 0);
     EVO_CUDA(cudaLaunchKernelEx(&cfg, delta_scan_kernel<DK>, tmK, tmQ, tmV, a));
     if ((rc = check_launch("evo_gated_delta_fwd(scan)"))) return rc;
   }
