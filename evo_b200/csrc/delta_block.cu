@@ -888,7 +888,8 @@ Sizes sizes(const evo_gated_delta_params* p) {
   s.blocks = (p->L + BT - 1) / BT;
   s.slab = std::max<int64_t>(1, std::min<int64_t>(s.blocks, SLAB_BYTES / ((int64_t)BLOCK_BYTES * p->B * p->H)));
   const auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-  s.y = p->dv <= 2 * CH ? 0 : up(sizeof(float) * (size_t)p->B * p->L * p->H * p->dv);
+  // the read-outs' place is asked for in any case, so that a call takes the workspace it always took (up to 128 channels the scan norms them itself and leaves it alone)
+  s.y = up(sizeof(float) * (size_t)p->B * p->L * p->H * p->dv);
   s.tri = up((size_t)BLOCK_BYTES * s.slab * p->B * p->H);
   s.state = p->state || s.slab == s.blocks ? 0 : up(sizeof(float) * (size_t)p->B * p->H * p->dk * p->dv);
   return s;
