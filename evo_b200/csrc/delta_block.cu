@@ -863,6 +863,7 @@ constexpr int64_t SLAB_BYTES = 256ll << 20;
 
 // From how many tokens on the blocks are faster.  Three launches and a 64-token block take 25 us (8 pairs of head and sequence) to 300 (2048 pairs of 128 x 128) whether the block is
 // full or not; token by token a call takes 0.5 to 1 us per token while the pairs fit the SMs, in proportion to their number beyond.  Measured (us, token by token / blocks):
+// (the block figures are those of the mma.sync scan with a launch for the norm; the present one takes less, and the lines have been left where they were)
 //   heads of 64 x 64, 32 pairs: 32 tokens 23 / 26, 40 tokens 27 / 26, 48 tokens 31 / 26;  128 x 128, 128 pairs: 32 / 36, 39 / 37, 45 / 37;  64 x 128, 128 pairs: 25 / 32, 31 / 33, 33 / 33
 //   512 pairs, where token by token has more than a wave: 64 x 64: 32 tokens 52 / 51;  128 x 128: 125 / 86
 //   few value channels, whose token-by-token CTAs are nearly empty: 128 x 16, 32 pairs: 32 tokens 50 / 29;  but 1024 pairs: 48 tokens 97 / 120
