@@ -128,11 +128,9 @@ __global__ void __launch_bounds__(DT) decode_attn_kernel(const bf16* __restrict_
   if (tid == 0) { part_ml[pidx * 2] = M; part_ml[pidx * 2 + 1] = L; }
 }
 
-// ---- decode attention, TMA-fed (default; rows of the tensor map are counted in 32 bits) ----
-// A sequence's last tile may reach behind its keys, into rows not written yet, the next sequence or past the cache (zeros): their scores are masked and their values not read.
-// Caches of other lengths than multiples of 64 keep their weights in fp32: the kernel above, to which they went, rounds them against a maximum per thread, and a thread with one key has
-// the weight 1.  ( one step of one request behind 999 keys,
-// four blocks of which one has attention, takes 373 us instead of 384, of four requests behind 500 keys 395 instead of 421, the three kernels' dependent launch included.)
+// ---- decode attention, TMA-fed (default where the cache is whole tiles; rows of the tensor map are counted in 32 bits) ----
+// Caches of other lengths go to the kernel above, whose order of sums and of rounding their callers' results are in.  Through this one (its last tile masked, with fp32 weights) a step of
+// one request behind 999 keys, four blocks of which one has attention, took 374 us instead of 383, but its logits moved by 5.5e-3 of their norm: taken back.
 // The per-thread-row kernel above issues 16-byte loads whose 32 lanes touch 32 different 128-byte lines (K rows of
 // one head are 16 KB apart): the L1 tag stage caps it near 3 TB/s.  Here a producer warp streams 64-key K and V tiles
 // of one (b, h) into a 3-stage shared-memory ring with TMA (box {128, 1, 64} of the cache viewed as
@@ -143,7 +141,6 @@ constexpr int TK = 64;                 // keys per tile
 constexpr int AST = 3;                 // ring stages
 constexpr int TILE_BYTES = TK * HD * 2;          // 16 KB (K) + 16 KB (V) per stage
 constexpr int ATT2_SMEM = AST * 2 * TILE_BYTES + 1024;
-template <bool ROUND>
 __global__ void __launch_bounds__(160, 2) decode_attn_tma_kernel(const __grid_constant__ CUtensorMap tm, const bf16* __restrict__ qkv,
                                                                  float* __restrict__ part_o, float* __restrict__ part_ml,
                                                                  const long long* __restrict__ pos_ptr, int H, long long S, int nsplit, float scale) {
@@ -207,7 +204,7 @@ __global__ void __launch_bounds__(160, 2) decode_attn_tma_kernel(const __grid_co
       if (mn != -INFINITY) {                                           // warp-uniform
         const float alpha = __expf(m - mn), pe = __expf(sd - mn);
         l = l * alpha + (half == 0 ? pe : 0.f);
-        const float pb = ROUND ? rbf(pe) : pe;                         // P rounded to bf16 before the PV product, like the prefill kernel
+        const float pb = rbf(pe);                                      // P rounded to bf16 before the PV product, like the prefill kernel
         o0 *= alpha; o1 *= alpha; o2 *= alpha; o3 *= alpha;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -299,7 +296,7 @@ extern "C" int evo_decode_attn(const void* qkv, const void* cache, void* out, co
   float* part_o = (float*)workspace;
   float* part_ml = part_o + (size_t)B * H * nsplit * HD;
   static const bool force_v1 = getenv("EVO_B200_DECODE_ATTN_V1") != nullptr;
-  if (!force_v1 && (long long)B * max_seqlen < (1LL << 31)) {
+  if (max_seqlen % TK == 0 && !force_v1 && (long long)B * max_seqlen < (1LL << 31)) {
     CUtensorMap tm;
     const uint64_t dims[3] = {(uint64_t)HD, (uint64_t)(2 * H), (uint64_t)B * (uint64_t)max_seqlen};
     const uint64_t str[2] = {(uint64_t)HD * 2, (uint64_t)2 * H * HD * 2};
@@ -307,11 +304,8 @@ extern "C" int evo_decode_attn(const void* qkv, const void* cache, void* out, co
     int rc = make_tmap_nd_bf16(&tm, cache, 3, dims, str, box, false);
     if (rc) return rc;
     static unsigned long long attr_done = 0;
-    static unsigned long long attr_done_exact = 0;
-    const bool round = max_seqlen % TK == 0;
-    const auto kern = round ? decode_attn_tma_kernel<true> : decode_attn_tma_kernel<false>;
-    if ((rc = ensure_dyn_smem(kern, ATT2_SMEM, round ? attr_done : attr_done_exact))) return rc;
-    EVO_CUDA(launch_pdl_light(kern, dim3(H, B, nsplit), dim3(160), (size_t)ATT2_SMEM, (cudaStream_t)stream, tm, (const bf16*)qkv, part_o, part_ml,
+    if ((rc = ensure_dyn_smem(decode_attn_tma_kernel, ATT2_SMEM, attr_done))) return rc;
+    EVO_CUDA(launch_pdl_light(decode_attn_tma_kernel, dim3(H, B, nsplit), dim3(160), (size_t)ATT2_SMEM, (cudaStream_t)stream, tm, (const bf16*)qkv, part_o, part_ml,
                         (const long long*)pos, H, (long long)max_seqlen, nsplit, softmax_scale));
     rc = check_launch("evo_decode_attn");
     if (rc) return rc;
