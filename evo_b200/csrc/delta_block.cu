@@ -334,6 +334,7 @@ static_assert(SPLIT_WARPS * 32 * SPLIT_REGS + 2 * EPI_WARPS * 32 * EPI_REGS + 12
 constexpr int OUT_PITCH = CH + 4;                       // floats of a token's row on its way from lanes to rows
 constexpr int OUT_BYTES = BT * OUT_PITCH * 4;           // of a block
 constexpr int V_BYTES = BT * CH * 2;
+constexpr int NORM_TURNS = 2;                           // places for the other CTA's sums of squares, for the blocks of a parity in turn
 
 // 16 lanes; a thread has row lane / 4 (and + 8), columns 2 (lane & 3) and the next of every eight: [8 columns][row, row + 8][2]
 template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float2 (&x)[N]) {
@@ -393,11 +394,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
   static_assert(STAGE % 1024 == 0, "");
   extern __shared__ __align__(16) uint8_t sm_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[2], empty[2], s_ready, w_done, wp_ready, u_done, up_ready, pu_ready, ds_done[2], qs_done[2], o_done[2], o_free, fixed[2], half_met[4], rows_met[2], norm_met[2], ended;
+  __shared__ uint64_t full[2], empty[2], s_ready, w_done, wp_ready, u_done, up_ready, pu_ready, ds_done[2], qs_done[2], o_done[2], o_free, fixed[2], half_met[4], rows_met[2], norm_met[2][NORM_TURNS], ended;
   __shared__ uint32_t tmem_slot;
   __shared__ int odd[2];                                // W or U of block (parity) holds something that is not finite
   __shared__ float part_sum[2][3][2][CH];               // of a token (parity): S^T k, S^T q, k . q over half the key channels
-  __shared__ float norm_sum[2][BT];                     // of a block (parity): the other CTA's sums of squares
+  __shared__ float norm_sum[2][NORM_TURNS][BT];         // of a block (parity, and its turn among those of that parity): the other CTA's sums of squares
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int h = blockIdx.x, b = blockIdx.y, g = h / (p.H / p.G), dv = p.dv, c0 = blockIdx.z * CH;
   const int64_t rowb = (int64_t)b * p.L + p.first * BT, left = p.L - p.first * BT;       // the slab's first row; tokens from there
@@ -405,7 +406,8 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1 + SPLIT_WARPS + EPI_WARPS); mbar_init(&ds_done[i], 1); odd[i] = 0;
-      mbar_init(&qs_done[i], 1); mbar_init(&o_done[i], 1); mbar_init(&fixed[i], 4); mbar_init(&rows_met[i], EPI_WARPS); mbar_init(&norm_met[i], 1);
+      mbar_init(&qs_done[i], 1); mbar_init(&o_done[i], 1); mbar_init(&fixed[i], 4); mbar_init(&rows_met[i], EPI_WARPS);
+      for (int k = 0; k < NORM_TURNS; ++k) mbar_init(&norm_met[i][k], 1);
     }
     mbar_init(&s_ready, SPLIT_WARPS); mbar_init(&w_done, 1); mbar_init(&wp_ready, SPLIT_WARPS); mbar_init(&u_done, 1); mbar_init(&up_ready, SPLIT_WARPS);
     mbar_init(&pu_ready, SPLIT_WARPS + EPI_WARPS);               // the parts of U, and Q S read
@@ -625,7 +627,12 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
       if (lane == 0) mbar_arrive(&empty[ph]);
       __syncwarp();
       if (blk >= 2 && p.norm) { ok = meet(); if (!ok) break; }           // the rows of the group's last block are read
-      if (p.pair && q == 0 && lane == 0) mbar_arrive_expect_tx(&norm_met[ph], BT * 4);      // (now: every warp here has seen the last block's)
+      // The exchange of the sums of squares: each CTA writes a block's into the other, where they are read behind the barrier of their place.  The blocks of a parity take two places in turn,
+      // so that no sum is written over one that is still to be read, and no two blocks' bytes meet at a barrier: the other CTA sends block n + 4's, the next into block n's place, when its
+      // warps have met at block n + 4, each with every sum of block n + 2 from here; and a warp here sends those of n + 2 when all have met there, with block n's read.  (With one place the
+      // other CTA goes on to block n + 2 once block n's sums have left here, read or not.)
+      const int place = (blk >> 1) % NORM_TURNS;
+      if (p.pair && q == 0 && lane == 0) mbar_arrive_expect_tx(&norm_met[ph][place], BT * 4);
       __syncwarp();
       ok = wait(&o_done[ph], turn);
       if (!ok) break;
@@ -689,11 +696,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
         if (!(lane & 1))
           asm volatile("{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\tmapa.shared::cluster.u32 rb, %1, %2;\n\t"
                        "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [ra], %3, [rb];\n\t}\n"
-                       ::"r"(smem_u32(&norm_sum[ph][t])), "r"(smem_u32(&norm_met[ph])), "r"(other), "r"(__float_as_uint(ss[0])) : "memory");
+                       ::"r"(smem_u32(&norm_sum[ph][place][t])), "r"(smem_u32(&norm_met[ph][place])), "r"(other), "r"(__float_as_uint(ss[0])) : "memory");
         __syncwarp();
-        ok = wait(&norm_met[ph], turn);
+        ok = wait(&norm_met[ph][place], ((blk >> 1) / NORM_TURNS) & 1);
         if (!ok) break;
-        ss[0] += norm_sum[ph][t];
+        ss[0] += norm_sum[ph][place][t];
       }
       const float rstd = 1.0f / sqrtf(ss[0] / (float)dv + p.eps);
       bf16* orow = p.out + row0 * p.ldo + (int64_t)h * dv + e0;

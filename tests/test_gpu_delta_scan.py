@@ -69,3 +69,19 @@ def test_pairs_around_the_number_of_sms(H, B):
         one = {k: (v[b * L:(b + 1) * L] if k in "xz" else v[b:b + 1] if k == "S" else v) for k, v in t.items()}
         o, s, _ = D._run(one, 1, L, H, H, dk, dv)
         assert torch.equal(out[b * L:(b + 1) * L], o) and torch.equal(S[b], s[0])
+
+
+@pytest.mark.parametrize("dv", [80, 128])
+def test_heads_over_two_ctas_for_many_blocks(dv):
+    """The two CTAs of a head exchange a sum per token for every block: each row of each head is scaled by its own (a result is rounded to bf16, 2^-9 of it, against fp32), and a
+    sequence's results do not depend on what runs beside it."""
+    B, L, H, dk = 3, 64 * 66 + 5, 4, 64
+    t = D._inputs(B, L, H, H, dk, dv, seed=dv)
+    out, S, _ = D._run(t, B, L, H, H, dk, dv)
+    want, _, _ = D._run(dict(t, x=t["x"].float(), z=t["z"].float()), B, L, H, H, dk, dv)
+    off = (out.float() - want).view(B * L, H, dv).norm(dim=-1) / want.view(B * L, H, dv).norm(dim=-1)
+    assert off.max() <= 2.0 ** -8
+    for b in range(B):
+        one = {k: (v[b * L:(b + 1) * L] if k in "xz" else v[b:b + 1] if k == "S" else v) for k, v in t.items()}
+        o, s, _ = D._run(one, 1, L, H, H, dk, dv)
+        assert torch.equal(out[b * L:(b + 1) * L], o) and torch.equal(S[b], s[0])
