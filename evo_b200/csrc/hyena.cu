@@ -454,8 +454,10 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
     if ((rc = R == 4 ? launch_tc<4>(p, nseg, seg_len, workspace, st) : (R == 2 ? launch_tc<2>(p, nseg, seg_len, workspace, st) : launch_tc<1>(p, nseg, seg_len, workspace, st)))) return rc;
   } else if (use_tma_path(p)) {
     using namespace evo_hy2;
-    // the copy of the inputs that a state keeps goes first, and the (split) scan begins beside it
-    const bool split = plan.scan_variant != 0, copied = split && p->fir_state_out && !fir_state_over_halo(p);
+    // The copy of the inputs that a state keeps goes first, and the (split) scan begins beside it: 1 x 20 tokens of 4096 channels 17.4 -> 13.3 us, 1 x 100 25.6 -> 23.5, 8 x 300 50 -> 48,
+    // 128 x 100 243 -> 239, 8 x 8193 959 -> 957.  Not with segments: the CTAs of the pass that finds the states between them are then placed two to an SM while others are idle
+    // (with states kept, normal / dependent: 1 x 8193 198 / 253, 4 x 4096 402 / 527; 8 x 8193 of 2048 channels 781 / 1038).
+    const bool split = plan.scan_variant != 0, copied = split && p->fir_state_out && nseg == 1 && !fir_state_over_halo(p);
     CUtensorMap tmZ;
     uint64_t dims[3] = {(uint64_t)3 * p->D, (uint64_t)p->L, (uint64_t)p->B};
     uint64_t str[2] = {(uint64_t)3 * p->D * 2, (uint64_t)p->L * 3 * p->D * 2};
@@ -486,13 +488,12 @@ extern "C" int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t 
       EVO_CUDA(launch_after(copied, k_state, grid, block, SMEM_BYTES, st, tmZ, a));
       if ((rc = check_launch("hyena_scan<state>"))) return rc;
     } else {
-      const bool states = nseg > 1 && !p->reuse_segment_states;
-      if (states) {
+      if (nseg > 1 && !p->reuse_segment_states) {
         dim3 g2(grid.x, grid.y, nseg - 1);
-        EVO_CUDA(launch_after(copied, k_state, g2, block, SMEM_BYTES, st, tmZ, a));
+        k_state<<<g2, block, SMEM_BYTES, st>>>(tmZ, a);
         if ((rc = check_launch("hyena_scan<state>"))) return rc;
       }
-      EVO_CUDA(launch_after(copied && !states, k_out, grid, block, SMEM_BYTES, st, tmZ, a));
+      EVO_CUDA(launch_after(copied, k_out, grid, block, SMEM_BYTES, st, tmZ, a));
       if ((rc = check_launch("hyena_scan<out>"))) return rc;
     }
     if (copied) fir_done = true;
