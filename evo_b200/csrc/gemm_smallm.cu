@@ -111,13 +111,16 @@ __device__ __forceinline__ float finish(const SmArgs& g, long long n, float bias
     return o;
   }
 }
-// 16 batch rows [b0, b0+16) of output column n
-template <int EPI>
+// 16 batch rows [b0, b0+16) of output column n; for many rows all of them are computed, interleaved, and only the stores are skipped (for few, what is not needed is not computed)
+template <int EPI, bool MANY>
 __device__ __forceinline__ void finalize16(const SmArgs& g, long long n, int b0, float bias, const float (&rv)[16],
                                            const float (&v0)[16], const float (&v1)[16]) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
-    if (b0 + j < g.M) g.C[(long long)(b0 + j) * g.ldc + n] = __float2bfloat16_rn(finish<EPI>(g, n, bias, rv[j], v0[j], v1[j]));
+  for (int j = 0; j < 16; ++j) {
+    if (!MANY && b0 + j >= g.M) continue;
+    const bf16 o = __float2bfloat16_rn(finish<EPI>(g, n, bias, rv[j], v0[j], v1[j]));
+    if (b0 + j < g.M) g.C[(long long)(b0 + j) * g.ldc + n] = o;
+  }
 }
 
 constexpr int EPI_HYENA_STEP = 7;   // EVO_EPI_HYENA_STEP
@@ -188,37 +191,47 @@ __device__ __forceinline__ void hyena_step16(const SmArgs& g, int tile, int row,
 // The slots of a tile are summed by its last contributor, in contributor order (deterministic), and the epilogue applied.  This runs once per launch at the end of its serial chain, with
 // cold instruction caches: four columns per lane and a warp per batch row (two in flight) are a quarter of the loads, and a quarter of the code, of a thread per column.  One step of
 // one request 446 -> 394 us, of 16 664 -> 623; (only fewer rows for a thread per column: 400 / 680).
-template <int EPI>
-__device__ __forceinline__ void fix_up(const SmArgs& g, int tile, int c_first, int c_last, bool first_begins_before, int slot_floats) {
-  constexpr int R = RowGroups<EPI>::R, FX = 8 / R;
+// For more rows (MANY, see launch()) what counts is how often a warp waits for sums.  Four rows are then in flight, but for residual layers, which are square or deep and have five and more
+// contributors to a tile: two rows with all of these at once are better there.  Gated epilogues, whose tiles have few, keep a thread per column with 128 loads in flight.  (us, launched one
+// behind the other; a thread per column throughout / two rows / as it is)  8192 x 2048: 16 rows 15.3 / 15.7 / 14.8, 32 rows 17.4 / 18.6 / 16.9, 64 rows 21.4 / 23.0 / 21.1;  gated,
+// 11264 x 2048, 64 rows 28.9 / 32.9 / 26.8;  22016 x 4096 54.0 / 56.7 / 51.1;  4096 x 11008 with residual, 64 rows 46.9 / 33.4 / 33.4 (four rows 35.2).
+template <int EPI, bool MANY>
+__device__ __forceinline__ void sum_rows(const SmArgs& g, int tile, int c_first, int c_last, bool first_begins_before, int slot_floats) {
+  constexpr int R = RowGroups<EPI>::R, NB = MANY && EPI != EVO_EPI_RESID && EPI != EVO_EPI_BIAS_RESID ? 4 : 2, FX = 16 / (R * NB);
   const int col = (threadIdx.x & 31) * 4;
   const long long n = (long long)tile * WROWS + col;
   const float* base = g.slots + col;
 #pragma unroll 1
-  for (int b0 = (threadIdx.x >> 5) - EPI_WARP0; b0 < g.M; b0 += 8) {
-    const int b[2] = {b0, min(b0 + 4, g.M - 1)};                      // (the last row twice rather than none)
-    float4 v[2][R];
-    float bias[4], rv[2][4];
+  for (int b0 = (threadIdx.x >> 5) - EPI_WARP0; b0 < g.M; b0 += 4 * NB) {
+    int b[NB];                                                         // (the last row again rather than none)
+#pragma unroll
+    for (int i = 0; i < NB; ++i) b[i] = min(b0 + 4 * i, g.M - 1);
+    float4 v[NB][R];
+    float bias[4], rv[NB][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      bias[e] = rv[0][e] = rv[1][e] = 0.f;
+      bias[e] = 0.f;
       if constexpr (EPI == EVO_EPI_BIAS || EPI == EVO_EPI_BIAS_RESID) bias[e] = __bfloat162float(g.bias[n + e]);
-      if constexpr (EPI == EVO_EPI_BIAS_RESID || EPI == EVO_EPI_RESID) { rv[0][e] = __bfloat162float(g.resid[b[0] * g.ldr + n + e]); rv[1][e] = __bfloat162float(g.resid[b[1] * g.ldr + n + e]); }
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        rv[i][e] = 0.f;
+        if constexpr (EPI == EVO_EPI_BIAS_RESID || EPI == EVO_EPI_RESID) rv[i][e] = __bfloat162float(g.resid[b[i] * g.ldr + n + e]);
+      }
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < NB; ++i)
 #pragma unroll
       for (int q = 0; q < R; ++q) v[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
     for (int cb = c_first; cb <= c_last; cb += FX) {
-      float4 t[FX][2][R];
+      float4 t[FX][NB][R];
 #pragma unroll
       for (int u = 0; u < FX; ++u) {                                  // all in flight together
         const int cc = min(cb + u, c_last);
         // a contributor's second slot is that of a range which begins in an earlier tile: only the first one's can
         const float* s = base + (size_t)(2 * cc + (cc == c_first && first_begins_before ? 1 : 0)) * slot_floats;
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < NB; ++i)
 #pragma unroll
           for (int q = 0; q < R; ++q) t[u][i][q] = __ldcg(reinterpret_cast<const float4*>(s + (q * g.Mb + b[i]) * WROWS));
       }
@@ -226,14 +239,14 @@ __device__ __forceinline__ void fix_up(const SmArgs& g, int tile, int c_first, i
       for (int u = 0; u < FX; ++u)
         if (cb + u <= c_last) {
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+          for (int i = 0; i < NB; ++i)
 #pragma unroll
             for (int q = 0; q < R; ++q) { v[i][q].x += t[u][i][q].x; v[i][q].y += t[u][i][q].y; v[i][q].z += t[u][i][q].z; v[i][q].w += t[u][i][q].w; }
         }
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (i && b0 + 4 >= g.M) continue;
+    for (int i = 0; i < NB; ++i) {
+      if (i && b0 + 4 * i >= g.M) continue;
       const float v0[4] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w}, v1[4] = {v[i][R - 1].x, v[i][R - 1].y, v[i][R - 1].z, v[i][R - 1].w};
       bf16* out = g.C + b[i] * g.ldc + n;
 #pragma unroll
@@ -241,11 +254,50 @@ __device__ __forceinline__ void fix_up(const SmArgs& g, int tile, int c_first, i
     }
   }
 }
-
+// the same with a thread per column, sixteen rows and the sums of FX contributors at a time: the gated epilogues for many rows, and the Hyena step, whose threads own a channel
+// (one contributor at a time: 40 us instead of 38 for a row, 78 instead of 62 for 16, 222 instead of 149 for 64)
 template <int EPI>
+__device__ __forceinline__ void sum_columns(const SmArgs& g, int Mb, int tile, int row, int c_first, int c_last, bool first_begins_before, int slot_floats) {
+  constexpr int R = RowGroups<EPI>::R, FX = R == 3 ? 2 : 4;
+  for (int c = 0; c < Mb; c += 16) {
+    float v[R][16];
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[q][j] = 0.f;
+    for (int cb = c_first; cb <= c_last; cb += FX) {
+      float t[FX][R][16];
+#pragma unroll
+      for (int u = 0; u < FX; ++u) {
+        const int cc = min(cb + u, c_last);
+        const float* s = g.slots + (size_t)(2 * cc + (cc == c_first && first_begins_before ? 1 : 0)) * slot_floats + row;
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) t[u][q][j] = __ldcg(s + (q * Mb + c + j) * WROWS);
+      }
+#pragma unroll
+      for (int u = 0; u < FX; ++u)
+        if (cb + u <= c_last) {
+#pragma unroll
+          for (int q = 0; q < R; ++q)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[q][j] += t[u][q][j];
+        }
+    }
+    if constexpr (EPI == EPI_HYENA_STEP) hyena_step16(g, tile, row, c, v[0], v[1], v[2]);
+    else {
+      const float none[16] = {};
+      finalize16<EPI, true>(g, (long long)tile * WROWS + row, c, 0.f, none, v[0], v[R - 1]);
+    }
+  }
+}
+
+template <int EPI, bool MANY>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const SmArgs g) {
   constexpr int R = RowGroups<EPI>::R;                         // MMA row groups per tile
+  constexpr bool COLUMNS = EPI == EPI_HYENA_STEP || (MANY && R == 2);
   constexpr int WBOX = R == 2 ? 2 * WROWS : WROWS;             // W rows per TMA box (a box dimension is at most 256)
   constexpr int NBOX = R * WROWS / WBOX;
   constexpr int W_STAGE = R * WROWS * BK * 2;
@@ -390,14 +442,14 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 16; ++j) v2[j] = __uint_as_float(r2[j]);
             hyena_step16(g, tile, row, c, v0, v1, v2);
-          } else finalize16<EPI>(g, n, c, bias, rv, v0, v1);
+          } else finalize16<EPI, MANY>(g, n, c, bias, rv, v0, v1);
         }
       } else {
         float* slot = g.slots + (size_t)(2 * blockIdx.x + (tile == my_first_tile ? 0 : 1)) * slot_floats;
         for (int c = 0; c < acc_cols; c += 16) {
           uint32_t r0[16];
           tmem_ld_32x16(t0 + c, r0);
-          const int live = EPI == EPI_HYENA_STEP ? 16 : g.M - c % Mb;   // rows behind A's last one are neither stored nor read (but by the Hyena step's tail)
+          const int live = COLUMNS ? 16 : g.M - c % Mb;       // a warp per row: rows behind A's last one are neither stored nor read
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j) if (j < live) slot[(c + j) * WROWS + row] = __uint_as_float(r0[j]);
@@ -421,35 +473,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (threadIdx.x == EPI_WARP0 * 32) stamp(g, 6);       // partial published
         if (last) {
           const bool first_begins_before = range_start((uint32_t)c_first, total, parts) < (uint32_t)tile * KB;
-          if constexpr (EPI == EPI_HYENA_STEP) {
-            // a thread per channel, the loads of two contributors in flight (one at a time: 40 us instead of 38 for a row, 78 instead of 62 for 16, 222 instead of 149 for 64)
-            for (int c = 0; c < Mb; c += 16) {
-              float v[3][16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j) v[0][j] = v[1][j] = v[2][j] = 0.f;
-              for (int cb = c_first; cb <= c_last; cb += 2) {
-                float t[2][3][16];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                  const int cc = min(cb + u, c_last);
-                  const float* s = g.slots + (size_t)(2 * cc + (cc == c_first && first_begins_before ? 1 : 0)) * slot_floats + row;
-#pragma unroll
-                  for (int q = 0; q < 3; ++q)
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) t[u][q][j] = __ldcg(s + (q * Mb + c + j) * WROWS);
-                }
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-                  if (cb + u <= c_last) {
-#pragma unroll
-                    for (int q = 0; q < 3; ++q)
-#pragma unroll
-                      for (int j = 0; j < 16; ++j) v[q][j] += t[u][q][j];
-                  }
-              }
-              hyena_step16(g, tile, row, c, v[0], v[1], v[2]);
-            }
-          } else fix_up<EPI>(g, tile, c_first, c_last, first_begins_before, slot_floats);
+          if constexpr (COLUMNS) sum_columns<EPI>(g, Mb, tile, row, c_first, c_last, first_begins_before, slot_floats);
+          else sum_rows<EPI, MANY>(g, tile, c_first, c_last, first_begins_before, slot_floats);
           if (threadIdx.x == EPI_WARP0 * 32) g.counters[tile] = 0;   // self-cleaning for the next launch
         }
       }
@@ -474,8 +499,8 @@ int smem_budget_bytes() {
   return kb * 1024;
 }
 
-template <int EPI>
-int launch(const evo_gemm_smallm_params* p, cudaStream_t st) {
+template <int EPI, bool MANY>
+int launch_as(const evo_gemm_smallm_params* p, cudaStream_t st) {
   constexpr int R = RowGroups<EPI>::R;
   const int Mb = (int)((p->M + 15) / 16 * 16);
   CUtensorMap tmW, tmA;
@@ -506,7 +531,7 @@ int launch(const evo_gemm_smallm_params* p, cudaStream_t st) {
   g.counters = (int*)p->workspace;
   g.slots = (float*)((uint8_t*)p->workspace + 16384);
   static unsigned long long attr_done = 0;
-  auto kern = gemm_smallm_kernel<EPI>;
+  auto kern = gemm_smallm_kernel<EPI, MANY>;
   { int rc_ = ensure_dyn_smem(kern, 224 * 1024, attr_done); if (rc_) return rc_; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
@@ -521,6 +546,14 @@ int launch(const evo_gemm_smallm_params* p, cudaStream_t st) {
   }
   EVO_CUDA(cudaLaunchKernelEx(&cfg, kern, tmW, tmA, g));
   return check_launch("evo_gemm_smallm");
+}
+
+// MANY: where a pass of four rows per warp halves the passes (9 to 16 rows: one instead of two), and from 25 rows on; 17 to 24 rows are two passes instead of three, each with fewer
+// contributors at once: a block's four layers 251 us by a thread per column, 210 with two rows, 212 with four.
+template <int EPI>
+int launch(const evo_gemm_smallm_params* p, cudaStream_t st) {
+  if constexpr (EPI == EPI_HYENA_STEP) return launch_as<EPI, false>(p, st);
+  else return (p->M > 8 && p->M <= 16) || p->M > 24 ? launch_as<EPI, true>(p, st) : launch_as<EPI, false>(p, st);
 }
 
 }  // namespace

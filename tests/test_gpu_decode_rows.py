@@ -44,3 +44,16 @@ def test_few_rows_are_the_first_rows_of_more(N, K, epi):
         full = _linear(a, w, widest, getattr(_lib, epi), bias, resid)
         for M in rows:
             assert torch.equal(_linear(a, w, M, getattr(_lib, epi), bias, resid), full[:M]), M
+
+
+@pytest.mark.parametrize("epi", ["EPI_NONE", "EPI_BIAS_RESID", "EPI_GELU_GATE", "EPI_GELU_TANH_GATE"])
+@pytest.mark.parametrize("N,K", [(768, 256), (8192, 2048), (2048, 5632)])
+def test_many_rows_are_the_first_rows_of_more(N, K, epi):
+    """The same around the number of rows from which on their sums are added up four rows at a time (or, gated, by column), and for each wider tile."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    n = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    a, w, bias, resid = n(64, K).to(BF), (n(N, K) / math.sqrt(K)).to(BF), n(N).to(BF), n(65, N).to(BF)
+    for widest, rows in ((32, (17, 24, 25, 26, 29)), (48, (33, 40, 47)), (64, (49, 50, 63))):
+        full = _linear(a, w, widest, getattr(_lib, epi), bias, resid)
+        for M in rows:
+            assert torch.equal(_linear(a, w, M, getattr(_lib, epi), bias, resid), full[:M]), M
