@@ -7,6 +7,7 @@
 //   sums, norms and gates in fp32, sums of log decays in 64 bits (their differences enter as two floats), T in fp32 by halves: two triangles of 32 by forward
 //   substitution (one column per thread), the square between them by products of three-part splits.
 //   T diag(beta) and P go to the workspace as three bf16 parts (24 bits), in the order in which the next kernel's lanes read them.
+// delta_single_kernel, the recurrence of a call of one block where there are many (head, sequence) pairs.
 // delta_scan_kernel, blocks one after another on the fifth-generation tensor cores, everything transposed (value channels = rows): the sums of one product, split by the warps that
 //   read them from TMEM, are the first operand of the next, in TMEM too:
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
@@ -835,6 +836,219 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
   if (p.pair) { __syncwarp(); cluster_sync_all(); }      // the other CTA may still write its sums here
 }
 
+// ------------------------------------------------------------------------------------------------ a call of one block, on more CTAs than the chip takes at once
+// delta_scan_kernel is alone on its SM, so that nothing covers what surrounds a block there: its copies, the state's way in and out, the start of the next CTA, 5 of 8 us.  Here a warp has 16
+// value channels (again the rows of the products, on mma.sync: the sums of one are, lane by lane, the first operand of the next, and warps exchange nothing) and two to eight warps make a CTA,
+// several of which share an SM; the state is in registers, the read-outs are left to a norm of their own.  single() says where it is taken.
+template <int DK>
+__global__ void __launch_bounds__(256, 1) delta_single_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmV, const Args p) {
+  constexpr int KT = DK / 16, BOX = BT * 128, ROWS_BYTES = DK / 64 * BOX;      // keys and queries: boxes of 64 columns, 16-byte pieces of a row swizzled by row & 7
+  extern __shared__ __align__(16) uint8_t sm_raw[];
+  uint8_t* ks = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t arrived;
+  const int nw = blockDim.x >> 5, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+  const int vpitch = nw * 32, h = blockIdx.x, b = blockIdx.y, dv = p.dv, nt = (int)p.L;
+  const int c0 = blockIdx.z * nw * 16, cw = c0 + warp * 16;            // the CTA's and the warp's first value channel
+  const uint8_t* qs = ks + ROWS_BYTES;
+  const uint8_t* vs = qs + ROWS_BYTES;
+  const uint8_t* tri = vs + BT * vpitch;
+  const float* vec = reinterpret_cast<const float*>(tri + 2 * TRI_BYTES);
+  if (tid == 0) {
+    mbar_init(&arrived, 1);
+    fence_barrier_init();
+    const int g = h / (p.H / p.G);
+    mbar_arrive_expect_tx(&arrived, 2 * ROWS_BYTES + BT * vpitch + BLOCK_BYTES);       // (rows behind the last token arrive as zeros)
+#pragma unroll
+    for (int i = 0; i < DK / 64; ++i) {
+      tma_load_3d(ks + i * BOX, &tmK, &arrived, g * DK + i * 64, 0, b);
+      tma_load_3d(ks + ROWS_BYTES + i * BOX, &tmQ, &arrived, g * DK + i * 64, 0, b);
+    }
+    tma_load_3d(ks + 2 * ROWS_BYTES, &tmV, &arrived, h * dv + c0, 0, b);
+    bulk(ks + 2 * ROWS_BYTES + BT * vpitch, p.blocks + ((int64_t)b * p.H + h) * (int64_t)BLOCK_BYTES, BLOCK_BYTES, &arrived);
+  }
+  // ---- S^T: rows = value channels cw + gq (+ 8), columns = state rows: S[n][..] covers state rows 8 n + 2 tq, + 1
+  float S[2 * KT][4];
+  float* Sg = p.state + ((int64_t)b * p.H + h) * DK * (int64_t)dv;
+  const bool live = cw < dv;                                            // (dv is a multiple of 16)
+#pragma unroll
+  for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      S[n][e] = (p.zero_start || !live) ? 0.f : Sg[(int64_t)(8 * n + 2 * tq + (e & 1)) * dv + cw + gq + (e >> 1) * 8];
+  __syncthreads();
+  if (__syncthreads_or(!wait_or_give_up(&arrived, 0, p.waits))) {
+    if (tid == 0) wait_to_end(&arrived, 0, p.waits);                    // no state is kept; the copies under way land before the CTA ends
+    return;
+  }
+  if (!live) return;
+  float* yr = p.y + (int64_t)b * p.L * p.H * dv + (int64_t)h * dv + cw + gq;
+  float W[8][4], O[8][4];                                           // columns = tokens 8 n + 2 tq, + 1
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) W[n][e] = O[n][e] = 0.f;
+  const uint32_t brow = ((lane & 7) + ((lane >> 4) << 3)) * 128, piece = (lane >> 3) & 1, turn = lane & 7;
+#pragma unroll
+  for (int kt = 0; kt < KT; ++kt) {
+    const uint32_t at = (kt >> 2) * BOX + brow + (((2 * (kt & 3) + piece) ^ turn) << 4), kb = smem_u32(ks) + at, qb = smem_u32(qs) + at;
+    uint32_t a[3][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      split3(S[2 * kt + u][0], S[2 * kt + u][1], a[0][2 * u], a[1][2 * u], a[2][2 * u]);
+      split3(S[2 * kt + u][2], S[2 * kt + u][3], a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
+    }
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+      uint32_t bk[4], bq[4];
+      ldmatrix_x4_at(bk, kb + n2 * 16 * 128);
+      ldmatrix_x4_at(bq, qb + n2 * 16 * 128);
+#pragma unroll
+      for (int s = 2; s >= 0; --s) {
+        mma_np(W[2 * n2], a[s], bk[0], bk[1]); mma_np(W[2 * n2 + 1], a[s], bk[2], bk[3]);
+        mma_np(O[2 * n2], a[s], bq[0], bq[1]); mma_np(O[2 * n2 + 1], a[s], bq[2], bq[3]);
+      }
+    }
+  }
+  // ---- W = V - G rk (K S); O = G rq (Q S)
+  float wrong = 0.f;
+  {
+    const uint32_t vb = smem_u32(vs) + ((lane & 7) + ((lane >> 4) << 3)) * vpitch + warp * 32 + ((lane >> 3) & 1) * 16;
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+      uint32_t v[4];                                                // (tokens 0-7, channels 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15), turned
+      ldmatrix_x4_trans_at(v, vb + n2 * 16 * vpitch);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int n = 2 * n2 + u;
+        const float2 gk = *reinterpret_cast<const float2*>(vec + V_GK * BT + 8 * n + 2 * tq), gqv = *reinterpret_cast<const float2*>(vec + V_GQ * BT + 8 * n + 2 * tq);
+        W[n][0] = fmaf(gk.x, W[n][0], bf_lo(v[2 * u])); W[n][1] = fmaf(gk.y, W[n][1], bf_hi(v[2 * u]));
+        W[n][2] = fmaf(gk.x, W[n][2], bf_lo(v[2 * u + 1])); W[n][3] = fmaf(gk.y, W[n][3], bf_hi(v[2 * u + 1]));
+        O[n][0] *= gqv.x; O[n][1] *= gqv.y; O[n][2] *= gqv.x; O[n][3] *= gqv.y;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) wrong = fmaf(0.f, W[n][e], wrong);
+      }
+    }
+  }
+  // second operands of a triangle: the three parts of tile (kt, n)
+  auto tri_mul = [&](const uint8_t* base, const float (&X)[8][4], float (&Y)[8][4]) {
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+      uint32_t a[3][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        split3(X[2 * kt + u][0], X[2 * kt + u][1], a[0][2 * u], a[1][2 * u], a[2][2 * u]);
+        split3(X[2 * kt + u][2], X[2 * kt + u][3], a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
+      }
+#pragma unroll
+      for (int n0 = 2 * kt; n0 < 8; n0 += 4) {                       // four sums at a time: a sum's next mma is four later (23 cycles of latency, 8.7 of issue)
+        uint2 t[4][3];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (n0 + c < 8)
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+              const uint32_t* part = reinterpret_cast<const uint32_t*>(base + (s * TILES + tile_index(kt, n0 + c)) * PART_BYTES) + lane;
+              t[c][s] = make_uint2(part[0], part[32]);
+            }
+        const int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};       // small products first
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (n0 + c < 8) mma_np(Y[n0 + c], a[pa[m]], t[c][pb[m]].x, t[c][pb[m]].y);
+      }
+    }
+  };
+  float U[8][4];
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) U[n][e] = 0.f;
+  tri_mul(tri, W, U);
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) wrong = fmaf(0.f, U[n][e], wrong);
+  if (__all_sync(0xffffffffu, wrong == 0.f)) {
+    tri_mul(tri + TRI_BYTES, U, O);
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = 8 * n + 2 * tq + (e & 1);
+        if (t < nt) yr[(int64_t)t * p.H * dv + (e >> 1) * 8] = O[n][e];
+      }
+    // ---- S = G_64 S + (Gam rk U)^T K
+    const float G = vec[V_ROWS * BT];
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[n][e] *= G;
+    const uint32_t kt_b = smem_u32(ks) + ((lane & 7) + (((lane >> 3) & 1) << 3)) * 128;
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+      uint32_t a[3][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int n = 2 * kt + u;
+        const float2 ck = *reinterpret_cast<const float2*>(vec + V_CK * BT + 8 * n + 2 * tq);
+        split3(U[n][0] * ck.x, U[n][1] * ck.y, a[0][2 * u], a[1][2 * u], a[2][2 * u]);
+        split3(U[n][2] * ck.x, U[n][3] * ck.y, a[0][2 * u + 1], a[1][2 * u + 1], a[2][2 * u + 1]);
+      }
+#pragma unroll
+      for (int n2 = 0; n2 < KT; n2 += 2) {
+        uint32_t bk[8];
+        ldmatrix_x4_trans_at(bk, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + (lane >> 4)) ^ turn) << 4));
+        ldmatrix_x4_trans_at(bk + 4, kt_b + kt * 16 * 128 + (n2 >> 2) * BOX + (((2 * (n2 & 3) + 2 + (lane >> 4)) ^ turn) << 4));
+#pragma unroll
+        for (int s = 2; s >= 0; --s)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mma_np(S[2 * n2 + c], a[s], bk[2 * c], bk[2 * c + 1]);
+      }
+    }
+  } else {
+    // token by token, as the recurrence is defined; lanes of a quad share the rows of the state
+    for (int t = 0; t < nt; ++t) {
+      const float dec = vec[V_G * BT + t], be = vec[V_BETA * BT + t], nk = vec[V_RK * BT + t], nq = vec[V_RQ * BT + t];
+      float pk[2] = {0.f, 0.f}, po[2] = {0.f, 0.f}, kq = 0.f;
+#pragma unroll
+      for (int n = 0; n < 2 * KT; ++n) {
+        const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq), qw = *reinterpret_cast<const uint32_t*>(qs + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
+        const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk, q0 = bf_lo(qw) * nq, q1 = bf_hi(qw) * nq;
+        kq = fmaf(k1, q1, fmaf(k0, q0, kq));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[n][e] *= dec;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          pk[u] = fmaf(S[n][2 * u + 1], k1, fmaf(S[n][2 * u], k0, pk[u]));
+          po[u] = fmaf(S[n][2 * u + 1], q1, fmaf(S[n][2 * u], q0, po[u]));
+        }
+      }
+      kq = quad_sum(kq);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        pk[u] = be * (__bfloat162float(*reinterpret_cast<const bf16*>(vs + t * vpitch + (warp * 16 + gq + 8 * u) * 2)) - quad_sum(pk[u]));
+        po[u] = fmaf(pk[u], kq, quad_sum(po[u]));
+        if (tq == 0) yr[(int64_t)t * p.H * dv + 8 * u] = po[u];
+      }
+#pragma unroll
+      for (int n = 0; n < 2 * KT; ++n) {
+        const uint32_t kw = *reinterpret_cast<const uint32_t*>(ks + (n >> 3) * BOX + t * 128 + (((n & 7) ^ (t & 7)) << 4) + 4 * tq);
+        const float k0 = bf_lo(kw) * nk, k1 = bf_hi(kw) * nk;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) { S[n][2 * u] = fmaf(k0, pk[u], S[n][2 * u]); S[n][2 * u + 1] = fmaf(k1, pk[u], S[n][2 * u + 1]); }
+      }
+    }
+  }
+  if (p.store_state) {
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) Sg[(int64_t)(8 * n + 2 * tq + (e & 1)) * dv + cw + gq + (e >> 1) * 8] = S[n][e];
+  }
+}
+constexpr int single_smem_bytes(int dk, int warps) { return 1024 + 2 * BT * dk * 2 + BT * warps * 32 + BLOCK_BYTES; }
+
 // head norm, weight and SiLU gate of the read-outs of (row, head): one warp, four channels per lane and step
 __global__ void __launch_bounds__(256) delta_norm_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int64_t ldg, const bf16* __restrict__ w, bf16* __restrict__ out, int64_t ldo,
                                                          int64_t rows, int H, int dv, float eps) {
@@ -862,6 +1076,41 @@ __global__ void __launch_bounds__(256) delta_norm_kernel(const float* __restrict
   }
   if (h == H - 1)
     for (int64_t c = (int64_t)H * dv + lane; c < ldo; c += 32) out[row * ldo + c] = __float2bfloat16_rn(0.f);
+}
+
+// the same for heads of 32 N channels and rows that start on four elements: eight lanes per (row, head), everything in registers between the two passes
+template <int N>
+__global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restrict__ y, const bf16* __restrict__ gate, int64_t ldg, const bf16* __restrict__ w, bf16* __restrict__ out, int64_t ldo,
+                                                          int64_t rows, int H, int dv, float eps) {
+  const int64_t id = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int sub = threadIdx.x & 7;
+  const bool on = id < rows * H;
+  const int64_t row = on ? id / H : 0;
+  const int h = on ? (int)(id - row * H) : 0;
+  const float4* r = reinterpret_cast<const float4*>(y + (on ? id : 0) * (32 * N)) + sub;
+  const uint2* gr = reinterpret_cast<const uint2*>(gate + row * ldg + (int64_t)h * (32 * N)) + sub;
+  const uint2* wr = reinterpret_cast<const uint2*>(w) + sub;
+  float4 o[N];
+  uint2 gv[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) { o[i] = r[8 * i]; gv[i] = gr[8 * i]; }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) ss = fmaf(o[i].x, o[i].x, fmaf(o[i].y, o[i].y, fmaf(o[i].z, o[i].z, fmaf(o[i].w, o[i].w, ss))));
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  const float rstd = 1.0f / sqrtf(ss / (float)(32 * N) + eps);
+  if (!on) return;
+  uint2* orow = reinterpret_cast<uint2*>(out + row * ldo + (int64_t)h * (32 * N)) + sub;
+  const auto one = [&](float v, float g, float wv) { return v * rstd * wv * (g / (1.f + expf(-g))); };
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint2 wv = wr[8 * i];
+    orow[8 * i] = make_uint2(pack_bf16(one(o[i].x, bf_lo(gv[i].x), bf_lo(wv.x)), one(o[i].y, bf_hi(gv[i].x), bf_hi(wv.x))),
+                             pack_bf16(one(o[i].z, bf_lo(gv[i].y), bf_lo(wv.y)), one(o[i].w, bf_hi(gv[i].y), bf_hi(wv.y))));
+  }
+  if (h == H - 1)
+    for (int64_t c = (int64_t)H * (32 * N) + sub; c < ldo; c += 8) out[row * ldo + c] = __float2bfloat16_rn(0.f);
 }
 
 // Blocks whose T and P are in memory at a time: at most 256 MB of them, or one block of every (head, sequence) pair where that is more (32 KB each, above 8192 pairs).
@@ -903,6 +1152,16 @@ Sizes sizes(const evo_gated_delta_params* p) {
   return s;
 }
 
+// One block, and so many CTAs of the scan (64 channels) that they take more than a wave: delta_single_kernel.  Measured, 64 tokens with a state (us, scan launched dependent / single):
+//   64 x 32, 160 pairs: 31.6 / 27.6, 1024: 85 / 62;  128 x 32, 160: 35.9 / 33.8, 1024: 101 / 77;  (read-outs of more than 128 channels need a norm of their own in any case) 64 x 192, 64: 37.9 /
+//   33.8, 512: 124 / 101;  128 x 192, 64: 44 / 40;  else only from more waves on: 64 x 128, 128: 33.8 / 33.9, 256: 52 / 46, 1024: 159 / 124;  128 x 128, 160: 48 / 54, 256: 60 / 54, 1024: 185 /
+//   159;  64 x 16, 160: 29.7 / 31.8, 512: 49 / 48.  Heads of 48 and 64 channels fill the scan's lanes and stay there (64 x 64, 512: 50 / 58, 2048: 161 / 163).
+bool single(const evo_gated_delta_params* p, const Sizes& s) {
+  const int64_t ctas = (int64_t)p->B * p->H * ((p->dv + CH - 1) / CH), sms = device_sm_count();
+  if (s.blocks > 1 || (p->dv > 32 && p->dv <= 64)) return false;
+  return 2 * ctas > (p->dv > 128 || p->dv == 32 ? 2 * sms : 5 * sms);
+}
+
 template <int DK>
 int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream_t st) {
   Args a = {};
@@ -916,24 +1175,34 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
   a.state = p->state ? p->state : (s.state ? (float*)(ws + s.y + s.tri) : (float*)ws);      // (never read nor written in the last case)
   a.B = p->B; a.L = p->L; a.H = p->H; a.G = p->G; a.dv = p->dv;
   a.gate = (const bf16*)p->gate; a.norm_w = (const bf16*)p->norm_w; a.out = (bf16*)p->out; a.ldo = p->ldo; a.eps = p->eps;
-  a.norm = p->dv <= 2 * CH; a.pair = a.norm && p->dv > CH;
+  const bool one = single(p, s);
+  a.norm = !one && p->dv <= 2 * CH; a.pair = a.norm && p->dv > CH;
   a.wide = p->ldz % 4 == 0 && p->ldo % 4 == 0 && (((uintptr_t)p->gate | (uintptr_t)p->out) & 7) == 0;
   constexpr int prep_smem = prepare_smem_bytes(DK), scan_smem = scan_smem_bytes(DK);
   CUtensorMap tmK, tmQ, tmV;
   const uint64_t kdims[3] = {(uint64_t)p->G * DK, (uint64_t)p->L, (uint64_t)p->B}, vdims[3] = {(uint64_t)p->H * p->dv, (uint64_t)p->L, (uint64_t)p->B};
   const uint64_t strides[2] = {(uint64_t)p->ld * 2, (uint64_t)p->L * p->ld * 2};
-  const uint32_t kbox[3] = {64, BT, 1}, vbox[3] = {CH, BT, 1};
+  // delta_single_kernel: two warps (32 channels) to eight per CTA, as few as fill the chip
+  int nw = 2;
+  while (nw < 8 && nw * 16 < p->dv && (int64_t)p->B * p->H * (p->dv / 16) > (int64_t)nw * device_sm_count()) nw *= 2;
+  const uint32_t kbox[3] = {64, BT, 1}, vbox[3] = {one ? (uint32_t)nw * 16 : CH, BT, 1};
   int rc;
   if ((rc = make_tmap_nd_bf16(&tmK, p->k, 3, kdims, strides, kbox, true)) || (rc = make_tmap_nd_bf16(&tmQ, p->q, 3, kdims, strides, kbox, true)) ||
-      (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, true))) return rc;
-  static unsigned long long done_prep = 0, done_scan = 0;
-  if ((rc = ensure_dyn_smem(delta_prepare_kernel<DK>, prep_smem, done_prep)) || (rc = ensure_dyn_smem(delta_scan_kernel<DK>, scan_smem, done_scan))) return rc;
+      (rc = make_tmap_nd_bf16(&tmV, p->v, 3, vdims, strides, vbox, !one))) return rc;
+  static unsigned long long done_prep = 0, done_scan = 0, done_single = 0;
+  if ((rc = ensure_dyn_smem(delta_prepare_kernel<DK>, prep_smem, done_prep)) || (rc = ensure_dyn_smem(delta_scan_kernel<DK>, scan_smem, done_scan)) ||
+      (rc = ensure_dyn_smem(delta_single_kernel<DK>, single_smem_bytes(DK, 8), done_single))) return rc;
   for (int64_t first = 0; first < s.blocks; first += s.slab) {
     a.first = first; a.n_blocks = (int)std::min<int64_t>(s.slab, s.blocks - first);
     a.zero_start = first == 0 && (p->zero_start || !p->state);
     a.store_state = p->state || s.state;
     delta_prepare_kernel<DK><<<dim3(a.n_blocks, a.H, a.B), 128, prep_smem, st>>>(a);
     if ((rc = check_launch("evo_gated_delta_fwd(prepare)"))) return rc;
+    if (one) {
+      delta_single_kernel<DK><<<dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), nw * 32, single_smem_bytes(DK, nw), st>>>(tmK, tmQ, tmV, a);
+      if ((rc = check_launch("evo_gated_delta_fwd(single)"))) return rc;
+      break;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.H, a.B, (a.dv + CH - 1) / CH); cfg.blockDim = dim3(SCAN_THREADS); cfg.dynamicSmemBytes = scan_smem; cfg.stream = st;
     cudaLaunchAttribute attrs[2] = {};
@@ -941,15 +1210,19 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
     attrs[1].id = cudaLaunchAttributeClusterDimension; attrs[1].val.clusterDim = {1, 1, 2};
     // Launched dependent, the scan's CTAs are set up while the last of delta_prepare_kernel's run, which is worth 2 to 4 us: normal / dependent (us) 1 x 300 tokens, 8 heads of 64 x 64
     // 28.8 / 26.7, 1 x 777, 32 heads of 128 x 128 62.9 / 60.4, 1 x 4096 253 / 249.  But CTAs that come to most of the SMs one by one are placed worse: 64 pairs, 128 CTAs, 4 x 4096 tokens
-    // 313 / 340, 4 x 1024 95 / 99; 128 pairs of 128 x 64 67.0 / 67.6.
-    const bool dependent = (int64_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z * 2 <= device_sm_count();
+    // 329 / 340, 4 x 1024 95 / 99; 128 pairs of 128 x 64 67.0 / 67.6.  For one or two blocks the early start is worth more than the place: 48 tokens, 128 pairs of 64 x 128 37.9 / 33.8,
+    // 160 of 64 x 32 33.8 / 31.6; 128 tokens, 128 pairs of 128 x 128 50 / 48, 1024 249 / 245.
+    const bool dependent = (int64_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z * 2 <= device_sm_count() || s.blocks <= 2;
     cfg.attrs = dependent ? attrs : attrs + 1; cfg.numAttrs = (dependent ? 1 : 0) + (a.pair ? 1 : 0);
     EVO_CUDA(cudaLaunchKernelEx(&cfg, delta_scan_kernel<DK>, tmK, tmQ, tmV, a));
     if ((rc = check_launch("evo_gated_delta_fwd(scan)"))) return rc;
   }
   if (a.norm) return 0;
   const int64_t rows = (int64_t)p->B * p->L, w = rows * p->H;
-  delta_norm_kernel<<<(unsigned)((w + 7) / 8), 256, 0, st>>>(a.y, a.gate, p->ldz, a.norm_w, a.out, p->ldo, rows, p->H, p->dv, p->eps);
+  const bool wide = a.wide && ((uintptr_t)p->norm_w & 7) == 0;
+  const auto norm = wide && p->dv == 128 ? delta_norm4_kernel<4> : (wide && p->dv == 32 ? delta_norm4_kernel<1> : delta_norm_kernel);
+  const int per_cta = norm == delta_norm_kernel ? 8 : 32;
+  norm<<<(unsigned)((w + per_cta - 1) / per_cta), 256, 0, st>>>(a.y, a.gate, p->ldz, a.norm_w, a.out, p->ldo, rows, p->H, p->dv, p->eps);
   return check_launch("evo_gated_delta_fwd(norm)");
 }
 
