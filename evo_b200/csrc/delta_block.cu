@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
       if (blk + 1 < n_blocks) { ok = wait(&full[ph ^ 1], ((blk + 1) >> 1) & 1); if (ok) publish(); }
     }
     const bool lost = __syncthreads_or(!ok);
-    if (lost) { if (tid == 0) *p.failed = 1u; }
+    if (lost) { if (tid == 0) { pdl_wait(); *p.failed = 1u; } }            // (delta_prepare_kernel, which clears the word, may still be running)
     else if (p.store_state && works && !skip) {
       asm volatile("" : "+l"(Sg));                       // (or the compiler keeps the addresses of the loads above, two registers each, over the whole recurrence)
 #pragma unroll

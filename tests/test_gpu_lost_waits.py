@@ -35,9 +35,10 @@ def _reported():
     check_lost_waits()                                               # reported once
 
 
-@pytest.mark.parametrize("L", [64, 200])
-def test_gated_delta(L):
-    B, H, dk, dv = 2, 2, 128, 64
+@pytest.mark.parametrize("B,H,dv,L", [(2, 2, 64, 64), (2, 2, 64, 200), (2, 2, 80, 200), (2, 2, 128, 64), (2, 2, 128, 200), (2, 2, 192, 200), (76, 2, 32, 64)])
+def test_gated_delta(B, H, dv, L):
+    """A CTA for a head, two that are a cluster, several that leave read-outs to a norm, and the kernel for calls of one block."""
+    dk = 128
     t = D._inputs(B, L, H, H, dk, dv)
     out, S, _ = D._run(t, B, L, H, H, dk, dv)
     with _no_tries():
