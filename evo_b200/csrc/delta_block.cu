@@ -13,8 +13,8 @@
 //     W^T = V^T - S^T K^T (x G rk);  Q^T-part = S^T Q^T;  U^T = W^T T^T;  O^T += U^T P^T;  S'^T = G S^T + (U Gam rk)^T K
 //   S, W, U are fp32 and enter as three bf16 parts; K and Q are bf16 as they stand (their norms scale the sums); T, P have three parts and meet W, U in the six products
 //   down to 2^-16 of the leading one.  K, Q, V, T, P of the next block arrive by bulk copies while one is in work; the read-outs are normed, weighted and gated by warps of their own.
-// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 313 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588), of
-// which the scan 224 (395 + 51) and delta_prepare_kernel 92 (135 with the norms summed apart, both matrices stored and read again, and the square of T by
+// Measured (B200): 4 x 4096 tokens, 16 heads of 128 x 128: 329 us (token by token 2774; the scan on mma.sync, one warp per 16 channels and a launch of its own for the head norm, 588);
+// the kernels by themselves: the scan 224 (395 + 51), delta_prepare_kernel 92 (135 with the norms summed apart, both matrices stored and read again, and the square of T by
 // multiply-adds from shared memory: 15.7 k instructions and 5.5 k shared-memory wavefronts an item then, 10.5 k and 2.3 k now; its four warps wait for one another at barriers; six CTAs per
 // SM, which spill: 135); 1 x 777 tokens, 32 heads: 60 us (516; 113).  A block takes 6.3 k cycles, 4.1 k of them products (120 of M 64 and 40 or 25
 // cycles, by clock stamps); what is left of the chain  state's parts - K S - W's parts - T W - U's parts - K U - state  is the splitting, bound by instructions (11 k warp instructions a
@@ -51,7 +51,7 @@ struct Args {
   float unit_eps, q_scale;
   uint8_t* blocks;                                      // (sequence, head, block of the slab)
   float* state; int zero_start, store_state;
-  float* y;                                             // (rows, H * dv) fp32 read-outs, where more than one CTA has a head's channels
+  float* y;                                             // (rows, H * dv) fp32 read-outs, where a norm of its own follows
   int norm, pair, wide;                                 // head norm, weight and gate here; with a second CTA; their rows start on four elements
   const bf16* gate; const bf16* norm_w; bf16* out; int64_t ldo; float eps;
   int B; int64_t L; int H, G, dv;
@@ -1117,12 +1117,13 @@ __global__ void __launch_bounds__(256) delta_norm4_kernel(const float* __restric
 // A longer call runs slab after slab, the state carried in between.
 constexpr int64_t SLAB_BYTES = 256ll << 20;
 
-// From how many tokens on the blocks are faster.  Three launches and a 64-token block take 25 us (8 pairs of head and sequence) to 300 (2048 pairs of 128 x 128) whether the block is
-// full or not; token by token a call takes 0.5 to 1 us per token while the pairs fit the SMs, in proportion to their number beyond.  Measured (us, token by token / blocks):
-// (the block figures are those of the mma.sync scan with a launch for the norm; the present one takes less, and the lines have been left where they were)
-//   heads of 64 x 64, 32 pairs: 32 tokens 23 / 26, 40 tokens 27 / 26, 48 tokens 31 / 26;  128 x 128, 128 pairs: 32 / 36, 39 / 37, 45 / 37;  64 x 128, 128 pairs: 25 / 32, 31 / 33, 33 / 33
-//   512 pairs, where token by token has more than a wave: 64 x 64: 32 tokens 52 / 51;  128 x 128: 125 / 86
-//   few value channels, whose token-by-token CTAs are nearly empty: 128 x 16, 32 pairs: 32 tokens 50 / 29;  but 1024 pairs: 48 tokens 97 / 120
+// From how many tokens on the blocks are taken.  A call of one block takes 22 us (8 pairs of head and sequence, 64 x 64) to 290 (2048 pairs of 128 x 128), nearly whatever its number of tokens;
+// token by token it takes 0.6 to 1.2 us per token while the pairs fit the SMs, in proportion to their number beyond.  Measured (us, cold L2, token by token / blocks):
+//   64 x 64, 8 to 128 pairs: 16 tokens 18 / 23, 24 tokens 25 / 23, 32 tokens 31 / 23, 47 tokens 41 / 23;  128 x 128, 32 pairs: 16: 25 / 29, 32: 39 / 30;  128 pairs: 24: 37 / 38, 32: 41 / 40,
+//   47: 55 / 40;  64 x 128, 128 pairs: 24: 29 / 32, 32: 33 / 32, 47: 43 / 34
+//   512 pairs, where token by token has more than a wave: 64 x 64: 16: 39 / 48, 32: 65 / 48;  128 x 128: 16: 84 / 81, 32: 141 / 85;  2048 pairs of 128 x 128: 32: 479 / 261
+//   few value channels, whose token-by-token CTAs are nearly empty: 128 x 16, 32 pairs: 16: 37 / 28;  1024 pairs: 24: 66 / 73, 32: 82 / 77, 47: 117 / 83;  64 x 16, 1024 pairs: 32: 70 / 67
+// The lines are those of the blocks' former kernels, which were slower: by these figures the blocks could be taken from 32 tokens on throughout.  What lies between would then be rounded elsewhere.
 int64_t block_tokens(const evo_gated_delta_params* p) {
   const int64_t pairs = (int64_t)p->B * p->H;
   if (p->dv >= 48) return pairs >= 512 ? 32 : 48;
@@ -1145,7 +1146,7 @@ Sizes sizes(const evo_gated_delta_params* p) {
   s.blocks = (p->L + BT - 1) / BT;
   s.slab = std::max<int64_t>(1, std::min<int64_t>(s.blocks, SLAB_BYTES / ((int64_t)BLOCK_BYTES * p->B * p->H)));
   const auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-  // the read-outs' place is asked for in any case, so that a call takes the workspace it always took (up to 128 channels the scan norms them itself and leaves it alone)
+  // The read-outs' place is asked for in any case, so that a call takes the workspace it always took.  Where the scan norms them itself (up to 128 channels, more than one block) it is left alone.
   s.y = up(sizeof(float) * (size_t)p->B * p->L * p->H * p->dv);
   s.tri = up((size_t)BLOCK_BYTES * s.slab * p->B * p->H);
   s.state = p->state || s.slab == s.blocks ? 0 : up(sizeof(float) * (size_t)p->B * p->H * p->dk * p->dv);

@@ -490,7 +490,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 8] = clock64(); g.trace[blockIdx.x * 16 + 15] = gtimer(); }
 }
 
-// Shared memory of the ring.  Two CTAs of neighbouring layers do not fit an SM together (168 registers a thread), so a CTA starts when that of the layer in front has ended there: in
+// Shared memory of the ring.  Two CTAs of neighbouring layers do not fit an SM together (256 threads of 168 to 255 registers), so a CTA starts when that of the layer in front has ended there: in
 // the tail in which memory idles, and what its ring holds by the time the sums are published is ahead of the stream.  One step of one request / of 16 (us): 104 KB 399 / 625,
 // 150 KB 389 / 616, 180 KB 385 / 614, 216 KB 388 / 615.  (Two to an SM, 128 registers and 104 KB: 410 / 642; the ring is then filled during the layer in front, which it slows.)
 int smem_budget_bytes() {
@@ -517,7 +517,7 @@ int launch_as(const evo_gemm_smallm_params* p, cudaStream_t st) {
   g.KB = (int)(p->K / BK);
   const int stage_bytes = R * WROWS * BK * 2 + Mb * BK * 2;
   const int tail = 2 * MAXST * 8 + 4 * 8 + 16;
-  // three row groups stage 48 KB of W per k-block: give the ring 160 KB (3 stages) instead of the default budget (2)
+  // (three row groups stage 48 KB of W per k-block: three stages of up to 48 rows, should the environment ask for a smaller ring)
   const int budget = R == 3 ? std::max(smem_budget_bytes(), 160 * 1024) : smem_budget_bytes();
   g.n_stages = std::max(2, std::min(MAXST, (budget - tail) / stage_bytes));
   const int smem_bytes = g.n_stages * stage_bytes + tail;

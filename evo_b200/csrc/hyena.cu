@@ -308,11 +308,12 @@ int pick_segments(const evo_hyena_params* p, int sms) {
 struct HyenaPlan { bool tc; int R, nseg; long long seg_len; int scan_variant; };
 
 // The tensor-core path does the work of 256 R tokens x 32 channels per tile and item in a time that hardly depends on how many of the tokens exist, and computes its
-// constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 64: scan 14.9, tensor
-// cores 20; 1 x 301: 42 / 23; 1 x 1999: 138 / 44; 4 x 1000: 123 / 76; 8 x 300: 44 / 76; 8 x 8193: 953 / 811.  D = 2048: 1 x 300: 42 / 21; 8 x 300: 42 / 48; 8 x 500: 64 / 51;
+// constants first; the modal scan costs 0.116 us per token of a sequence, whatever the number of CTAs that fit at once.  Measured (us, B x L, D = 4096): 1 x 65: scan 16.4, tensor
+// cores 19.5; 1 x 301: 42 / 20; 1 x 1999: 138 / 41.5; 4 x 1000: 123 / 76; 8 x 300: 45 / 75; 8 x 8193: 953 / 811.  D = 2048: 1 x 300: 42 / 21; 8 x 300: 42 / 48; 8 x 500: 64 / 51;
 // 2 x 4096: 117 / 70; 1 x 8193, both in segments: 126 / 134; 8 x 8193: 774 / 463.  D = 256, from 1000 tokens on in segments: 1 x 300: 42 / 21; 1 x 1999: 136 / 23; 8 x 8193: 126 / 133.
-// The smaller estimate decides; both sides are in us.  Over 1 to 8 sequences of 20 to 8193 tokens at the three widths it picks the faster side, or one within 5 % of it, with one
-// exception: narrow models' constants take less than estimated (a single tile 14.5 us at D = 256, 17 at 2048, 19 at 4096), so between about 75 and 110 tokens the scan's 16 to 19 are kept.
+// The smaller estimate decides; both sides are in us.  It was fitted to an operator that began behind its constants; now that it begins beside them a call of one tile takes 13 to 15 us at
+// D = 256, 17.4 at 2048 and 19.5 at 4096 where the estimate says 19.7, and the scan keeps some calls in which it is up to 4 us behind: one sequence of 4096 channels, 75 tokens (scan / tensor
+// cores) 18.5 / 19.5, 90 20.5 / 19.5, 109 22.5 / 19.5; with a state kept 65 19.5 / 19.5, 109 23.5 / 19.5; D = 2048, 75 18.4 / 17.4; D = 256, 65 16.4 / 15.1, 109 21.4 / 15.4.
 // Few items (narrow models, one sequence) are cut into segments: a pass over x1 and v then finds the states between them, at about half the price of the output pass.
 HyenaPlan make_plan(const evo_hyena_params* p) {
   const long long L = p->L;

@@ -16,7 +16,7 @@
 //                      steps with powers p^{16R}, p^{32R}, p^{64R}); then every block's c, rounded, + D x, back into the place of x
 // The fragment layouts of A operands and sums agree (a lane owns 4 consecutive tokens of rows g and g + 8), so B needs no shuffle besides the fold.
 // z is read once and y written once.
-// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 850 us sustained (modal scan on the CUDA cores 953), 1 x 1999 41.5 us (138), 4 x 1000 76 us (123), 1 x 301 20 us (42).
+// Measured (B200, D = 4096, constants included): 8 x 8193 tokens 834 us sustained (modal scan on the CUDA cores 953), 1 x 1999 41.5 us (138), 4 x 1000 76 us (123), 1 x 301 20 us (42).
 // A steady tile of 1024 tokens takes 24.5 k cycles, all of them the tensor-core warps' (tensor pipe 6.7 k, fp32 pipe 9 k, issue 10 k per scheduler): bound by the
 // latencies of its dependent steps with two such warps per scheduler (5.6 cycles per instruction each, by clock stamps; ncu on 1 x 8193: issue slots 59 % used, tensor pipe 23 %).  Register shares of 128 / 88 or 136 / 80
 // are 2 - 3 % slower: the element-wise warps then spill more (the output kernels spill 16 to 112 bytes as it is, -Xptxas -v).

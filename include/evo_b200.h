@@ -116,7 +116,7 @@ size_t evo_gemm_smallm_workspace(int64_t M, int64_t N, int64_t K, int epilogue);
 int evo_gemm_smallm(const evo_gemm_smallm_params* p, void* stream);
 /* Programmatic dependent launch for the decode step.  0 = off (default); 1 = every decode-step kernel is launched with
  * programmatic stream serialization; 2 = only evo_gemm_smallm is (its weight prefetch then overlaps the small kernel or
- * the GEMM tail in front of it); 3 = evo_gemm_smallm and the few-row evo_rmsnorm; 4 = those and
+ * the GEMM tail in front of it); 3 = evo_gemm_smallm, the few-row evo_rmsnorm, evo_decode_qkv_prep and evo_decode_attn with its merge; 4 = those and
  * evo_hyena_step (which fetches its filter parameters and states ahead of the wait).  Every decode-step kernel begins with griddepcontrol.launch_dependents and waits
  * (griddepcontrol.wait) before it first touches dependent data.  Process-wide switch; returns the previous value. */
 int evo_set_pdl(int level);
@@ -578,8 +578,9 @@ typedef struct {
   void* out; int64_t ldo; int dtype;
   int B; int64_t L; int H, G, dk, dv;
 } evo_gated_delta_params;
-/* workspace: evo_gated_delta_workspace() bytes (0 for a head whose tokens one CTA takes one by one; fp32 read-outs where its value channels are spread over several CTAs;
- * the blocks' matrices too where a prompt runs in 64-token blocks: at most 256 MB of them at a time, or 32 KB per head and sequence where that is more) */
+/* workspace: evo_gated_delta_workspace() bytes (0 for a head whose tokens one CTA takes one by one, fp32 read-outs where its value channels are spread over several CTAs;
+ * where a prompt runs in 64-token blocks: a place for fp32 read-outs in any case, although those of up to 128 channels only need it in a call of one block, and the blocks' matrices, at
+ * most 256 MB of them at a time, or 32 KB per head and sequence where that is more) */
 size_t evo_gated_delta_workspace(const evo_gated_delta_params* p);
 int evo_gated_delta_fwd(const evo_gated_delta_params* p, void* workspace, size_t workspace_bytes, void* stream);
 

@@ -281,8 +281,9 @@ def test_streamk_partition_invariants():
             c_first, c_last = cta_of(tile * KB, total, parts), cta_of((tile + 1) * KB - 1, total, parts)
             assert [c for (c, _, _, _) in v] == list(range(c_first, c_last + 1))
             assert sum(k1 - k0 for (_, k0, k1, _) in v) == KB
-            for (c, _, _, s) in v:                           # the finisher recomputes every contributor's slot the same way
-                assert s == 2 * c + (0 if range_start(c, total, parts) // KB == tile else 1)
+            first_begins_before = range_start(c_first, total, parts) < tile * KB
+            for (c, _, _, s) in v:                           # the finisher knows every contributor's slot from the first one's range
+                assert s == 2 * c + (1 if c == c_first and first_begins_before else 0)
 
 
 def test_generate_function_batches_equal_lengths_and_scores_like_the_reference(capsys):
