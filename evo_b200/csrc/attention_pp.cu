@@ -15,7 +15,9 @@
 //   pipe has PV_B(j) and QK_B(j+1) to do, and vice versa.
 //   The MMA warp stays converged and one lane issues: with a branch around the issuing code every product took that lane 90 to 130 cycles by clock
 //   stamps (64 on the tensor pipe), and the softmax waited for them (warm loop: 1 x 8193 tokens x 32 heads 534 -> 491 us, 2 x 4096 294 -> 271).
-//   Measured on B200: 1.01-1.12 PFLOP/s from 4096 tokens on in a warm loop, 0.95 for 1 x 8193 x 32 with cold L2 (576 us; P aliases S, so QK(j+1)
+//   P goes over in two halves, so that half of PV runs beside the other half's exponentials, with packed arithmetic and three-way maxima in front (1 x 8193 x 32 among other
+//   passes, so under the power cap: 580 us; packed and three-way 568; halves as well 561; one of 8 pairs exponentiated by a fifth-degree polynomial 559, two 572).
+//   Measured on B200: 1.01-1.12 PFLOP/s from 4096 tokens on in a warm loop, 0.98 for 1 x 8193 x 32 with cold L2 (561 us; P aliases S, so QK(j+1)
 //   queues behind PV(j)).  Tried and rejected: a second TMEM pass over S instead
 //   of holding the row in registers (0.50-0.57 PFLOP/s: tcgen05.ld bandwidth), a degree-3 FMA-pipe exp2 for half of
 //   the scores (0.82-0.96: issue slots, not MUFU, bind), 64-key tiles with double-buffered S (0.65-0.76).
@@ -102,7 +104,8 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint64_t* s_full = v_empty + KV_STAGES;           // 2 (per query tile)
   uint64_t* p_full = s_full + 2;                    // 2
   uint64_t* o_full = p_full + 2;                    // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t* p_half = o_full + 2;                    // 2: the first half of the keys
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_half + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (head, sequence) by (head, sequence), its longest query pair first; the last `tail` of them together, the longest pairs of all first (see the launcher)
@@ -123,7 +126,7 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
   if (warp == 9 && lane == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&o_full[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&s_full[i], 1); mbar_init(&p_half[i], 128); mbar_init(&p_full[i], 128); mbar_init(&o_full[i], 1); }
     for (int i = 0; i < KV_STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     fence_barrier_init();
   }
@@ -172,11 +175,15 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           if (j >= 0 && j < n) {
             const int st = j % KV_STAGES;
             mbar_wait(&v_full[st], (uint32_t)(j / KV_STAGES) & 1);
-            mbar_wait(&p_full[t], (uint32_t)j & 1);
+            mbar_wait(&p_half[t], (uint32_t)j & 1);
             tc_fence_after();
             const uint64_t vd = v_desc + st * (TILE_BYTES >> 4);
 #pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk) umma_ts_if(lead, o_tm, s_tm + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv, (j | kk) != 0);
+            for (int kk = 0; kk < BKV / 32; ++kk) umma_ts_if(lead, o_tm, s_tm + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv, (j | kk) != 0);
+            mbar_wait(&p_full[t], (uint32_t)j & 1);
+            tc_fence_after();
+#pragma unroll
+            for (int kk = BKV / 32; kk < BKV / 16; ++kk) umma_ts_if(lead, o_tm, s_tm + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv, 1);
             if (lead && (t == 1 || j >= n_kv[1])) umma_commit(&v_empty[st]);
             if (lead && j == n - 1) umma_commit(&o_full[t]);
           }
@@ -227,12 +234,15 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < BKV; ++i) if (key0 + i > pos) sc[i] = -INFINITY;
         }
-        float mxs[8];
+        float mxs[4];
 #pragma unroll
-        for (int q8 = 0; q8 < 8; ++q8) mxs[q8] = sc[q8];
+        for (int q4 = 0; q4 < 4; ++q4) mxs[q4] = max3(sc[q4], sc[4 + q4], sc[8 + q4]);
 #pragma unroll
-        for (int i = 8; i < BKV; ++i) mxs[i & 7] = fmaxf(mxs[i & 7], sc[i]);
-        float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7]))) * a.scale_log2;
+        for (int i = 12; i + 8 <= BKV; i += 8)
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) mxs[q4] = max3(mxs[q4], sc[i + q4], sc[i + 4 + q4]);
+        static_assert((BKV - 12) % 8 == 4, "four scores are left");
+        float mx = fmaxf(max3(max3(mxs[0], sc[BKV - 4], sc[BKV - 3]), max3(mxs[1], sc[BKV - 2], sc[BKV - 1]), mxs[2]), mxs[3]) * a.scale_log2;
         float alpha = 1.f;
         bool grow = mx > m_ref + 8.f;
         if (j == 0) { m_ref = (mx == -INFINITY) ? 0.f : mx; grow = false; }
@@ -250,43 +260,30 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           }
         }
         // ---- P = exp2(s*scale - m_ref) as bf16, written over the S columns (all of S is in registers by now)
-        float ls0 = 0.f, ls1 = 0.f, ls2 = 0.f, ls3 = 0.f;
-        if constexpr (NPOLY == 0) {
+        // packed arithmetic (one FFMA2 scales two scores, one FADD2 sums two probabilities); variant 3: NPOLY of every 8 pairs exponentiated on the FMA pipe, interleaved with the
+        // MUFU pairs so that both pipes stay busy inside one warp.  The products with the first half of the keys begin while the second half is worked on.
+        const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), nm2 = make_float2(-m_ref, -m_ref);
+        float2 la = make_float2(0.f, 0.f), lb = la;
 #pragma unroll
-          for (int c = 0; c < BKV; c += 32) {
-            uint32_t w[16];
+        for (int c = 0; c < BKV; c += 32) {
+          uint32_t w[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float p0 = ex2(fmaf(sc[c + 2 * i], a.scale_log2, -m_ref)), p1 = ex2(fmaf(sc[c + 2 * i + 1], a.scale_log2, -m_ref));
-              if (i & 1) { ls2 += p0; ls3 += p1; } else { ls0 += p0; ls1 += p1; }
-              w[i] = pack_bf16(p0, p1);
-            }
-            tmem_st_32x32_x16(s_addr + c / 2, w);
+          for (int i = 0; i < 16; ++i) {
+            const float2 x = __ffma2_rn(make_float2(sc[c + 2 * i], sc[c + 2 * i + 1]), scale2, nm2);
+            float2 p;
+            if (NPOLY && (i & 7) * NPOLY % 8 < NPOLY) p = exp2_poly2(x);      // NPOLY pairs of 8, spread evenly
+            else p = make_float2(ex2(x.x), ex2(x.y));
+            if (i & 1) lb = __fadd2_rn(lb, p); else la = __fadd2_rn(la, p);
+            w[i] = pack_bf16(p.x, p.y);
           }
-        } else {
-          // packed arithmetic (one FFMA2 scales two scores, one FADD2 sums two probabilities) and NPOLY of every 8 pairs
-          // exponentiated on the FMA pipe, interleaved with the MUFU pairs so that both pipes stay busy inside one warp
-          const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), nm2 = make_float2(-m_ref, -m_ref);
-          float2 la = make_float2(0.f, 0.f), lb = la;
-#pragma unroll
-          for (int c = 0; c < BKV; c += 32) {
-            uint32_t w[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float2 x = __ffma2_rn(make_float2(sc[c + 2 * i], sc[c + 2 * i + 1]), scale2, nm2);
-              float2 p;
-              if ((i & 7) * NPOLY % 8 < NPOLY) p = exp2_poly2(x);      // NPOLY pairs of 8, spread evenly
-              else p = make_float2(ex2(x.x), ex2(x.y));
-              if (i & 1) lb = __fadd2_rn(lb, p); else la = __fadd2_rn(la, p);
-              w[i] = pack_bf16(p.x, p.y);
-            }
-            tmem_st_32x32_x16(s_addr + c / 2, w);
+          tmem_st_32x32_x16(s_addr + c / 2, w);
+          if (c == BKV / 2 - 32) {
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(&p_half[t]);
           }
-          ls0 = la.x + lb.x; ls1 = la.y + lb.y;
         }
-        const float ls0_ = ls0 + ls2, ls1_ = ls1 + ls3;
-        ls0 = ls0_; ls1 = ls1_;
-        l += ls0 + ls1;
+        l += (la.x + lb.x) + (la.y + lb.y);
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&p_full[t]);

@@ -58,6 +58,8 @@ __device__ __forceinline__ float2 silu2_bf16(float2 v) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
   return __fmul2_rn(__fmul2_rn(v, quarter), r);
 }
+// the largest of three; a NaN gives way to a number, as in fmaxf
+__device__ __forceinline__ float max3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 // a warpgroup's registers per thread (the shares of a block add up to at most what it was launched with)
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
