@@ -262,81 +262,130 @@ __global__ void __launch_bounds__(256) sum_norm_row_kernel(const evo_sum_norm_pa
 }
 
 // ---- evo_conv_act: a thread owns one channel of one sequence over RT consecutive rows, its last taps inputs in registers
-constexpr int CONV_RT = 32, CONV_MAX_TAPS = 8, CONV_NB = 4;
+constexpr int CONV_RT = 32, CONV_MAX_TAPS = 8, CONV_CTAS = 4;
 
-// silu of two values
-template <typename T> __device__ __forceinline__ float2 silu2(float2 v) { return make_float2(silu_f(v.x), silu_f(v.y)); }
-template <> __device__ __forceinline__ float2 silu2<bf16>(float2 v) { return silu2_bf16(v); }
+// silu(4 v) of two values, as silu2_bf16 (common.cuh) does it, for sums whose weights were made a quarter beforehand (exact): the factor that keeps the reciprocal from being flushed
+// then costs nothing, and every constant is four times its own
+__device__ __forceinline__ float2 silu2_of_quarter(float2 v) {
+  constexpr float LOG2E = 1.44269502f, LOG2E_REST = 1.92596303e-8f, QUARTER_LN2 = 0.25f * 0.693147182f;
+  const float2 x = make_float2(fminf(v.x, 25.f), fminf(v.y, 25.f)), up = make_float2(-4.f * LOG2E, -4.f * LOG2E), quarter = make_float2(0.25f, 0.25f);
+  const float2 t = __fmul2_rn(x, up);
+  const float2 lo = __ffma2_rn(x, make_float2(-4.f * LOG2E_REST, -4.f * LOG2E_REST), __ffma2_rn(x, up, make_float2(-t.x, -t.y)));
+  float2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+  const float2 d = __ffma2_rn(e, __ffma2_rn(lo, make_float2(QUARTER_LN2, QUARTER_LN2), quarter), quarter);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+  return __fmul2_rn(v, r);
+}
+template <typename T, bool ACT> __device__ __forceinline__ float2 conv_finish(float2 v) {
+  if constexpr (!ACT) return v;
+  else if constexpr (sizeof(T) == 2) return silu2_of_quarter(v);
+  else return make_float2(silu_f(v.x), silu_f(v.y));
+}
 
-// four channels per thread (8- or 16-byte accesses), taps known at compile time.  Bound by instructions per element: 4 x 4096 rows of 6144 bf16 channels, 4 taps, SiLU take
-// 86 us (92 with cold L2 and carried inputs), 76 without the activation, where a plain copy of the same bytes takes 64; issue slots 74 % used, special functions 53 %, DRAM 50 %.
-// (168 with one row in flight, expf and IEEE division; 100 with expf beside the reciprocal instruction.  4 + 4 rows in flight beat 8 + 8, whose 118 registers halve the warps per
-// SM: 105.  Seven CTAs per SM, 72 registers: 86; left to the compiler, 94: 96; six 90; eight, which spills, 88.)
-template <typename T, int TAPS>
-__global__ void __launch_bounds__(128, sizeof(T) == 2 ? 7 : 1) conv_act4_kernel(evo_conv_act_params p, int write_carry) {
+// four channels per thread (8- or 16-byte accesses), taps and activation known at compile time.  Two special functions per element are 46 us for 4 x 4096 rows of 6144 channels, the
+// bytes 64 (a plain copy): 79 us with cold L2 (88 to 92 as CTAs of 32 rows with four rows in work and four under way).  What it takes: bytes under way -- eight bf16 rows in work and
+// eight under way, four CTAs per SM of 128 registers (four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows).  fp32 rows, four and four: 148 us (162).
+template <typename T, int TAPS, bool ACT>
+__global__ void __launch_bounds__(128, CONV_CTAS) conv_act4_kernel(evo_conv_act_params p, int write_carry, int rows_per) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= p.C) return;
-  constexpr int HALO = TAPS - 1;
+  constexpr int HALO = TAPS - 1, NB = sizeof(T) == 2 ? 8 : 4;
   const int b = blockIdx.z;
-  const int64_t t0 = (int64_t)blockIdx.y * CONV_RT, t1 = min(p.L, t0 + CONV_RT);
-  const T* in = (const T*)p.in + (int64_t)b * p.L * p.ld + c;
+  const int64_t t0 = (int64_t)blockIdx.y * rows_per, ld = p.ld, ldo = p.ldo;
+  const int rows = (int)min((int64_t)rows_per, p.L - t0);
+  const T* src = (const T*)p.in + ((int64_t)b * p.L + t0) * ld + c;
+  T* dst = (T*)p.out + ((int64_t)b * p.L + t0) * ldo + c;
   float* carry = p.carry ? p.carry + (int64_t)b * HALO * p.C + c : nullptr;
-  float2 w[2][TAPS];                                      // channel pairs: one packed multiply-add serves two channels
-  float win[HALO > 0 ? HALO : 1][4], bias[4] = {0.f, 0.f, 0.f, 0.f};
+  constexpr float SCALE = ACT && sizeof(T) == 2 ? 0.25f : 1.f;
+  float2 w[TAPS][2], bias[2];                             // channel pairs: one packed multiply-add serves two channels
+  {
+    // the four channels' taps lie one behind the other: 8 TAPS bytes, which start on 8 wherever the first channel's do
+    const bf16* wp = (const bf16*)p.weight + (int64_t)c * TAPS;
+    float f[4 * TAPS];
+    if (((uintptr_t)p.weight & 7) == 0) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+      for (int j = 0; j < TAPS; ++j) Vec4<bf16>::load(wp + 4 * j, f + 4 * j);
+    } else {
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j)
-      w[u][j] = make_float2(__bfloat162float(((const bf16*)p.weight)[(int64_t)(c + 2 * u) * TAPS + j]), __bfloat162float(((const bf16*)p.weight)[(int64_t)(c + 2 * u + 1) * TAPS + j]));
-  if (p.bias) Vec4<bf16>::load((const bf16*)p.bias + c, bias);
-  // rows travel packed, as they lie in memory: CONV_NB in work, CONV_NB under way (one row at a time left a single load in flight per thread)
-  Raw4<T> rows[CONV_NB], next[CONV_NB];
-#pragma unroll
-  for (int i = 0; i < CONV_NB; ++i)
-    if (t0 + i < t1) rows[i].load(in + (t0 + i) * p.ld);
-#pragma unroll
-  for (int j = 0; j < HALO; ++j) {
-    const int64_t s = t0 - HALO + j;
-    win[j][0] = win[j][1] = win[j][2] = win[j][3] = 0.f;
-    if (s >= 0) Vec4<T>::load(in + s * p.ld, win[j]);
-    else if (carry && !p.zero_start) Vec4<float>::load(carry + (int64_t)(HALO + s) * p.C, win[j]);
-  }
-  T* out = (T*)p.out + (int64_t)b * p.L * p.ldo + c;
-  for (int64_t tb = t0; tb < t1; tb += CONV_NB) {
-    // the next rows are under way while these are worked on
-#pragma unroll
-    for (int i = 0; i < CONV_NB; ++i)
-      if (tb + CONV_NB + i < t1) next[i].load(in + (tb + CONV_NB + i) * p.ld);
-#pragma unroll
-    for (int i = 0; i < CONV_NB; ++i) {
-      if (tb + i < t1) {
-        float cur[4], acc[4];
-        rows[i].get(cur);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          float2 a = __ffma2_rn(w[u][HALO], make_float2(cur[2 * u], cur[2 * u + 1]), make_float2(bias[2 * u], bias[2 * u + 1]));
-#pragma unroll
-          for (int j = 0; j < HALO; ++j) a = __ffma2_rn(w[u][j], make_float2(win[j][2 * u], win[j][2 * u + 1]), a);
-          if (p.act == 1) a = silu2<T>(a);
-          acc[2 * u] = a.x; acc[2 * u + 1] = a.y;
-        }
-        Vec4<T>::store(out + (tb + i) * p.ldo, acc);
-#pragma unroll
-        for (int j = 0; j + 1 < HALO; ++j)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) win[j][u] = win[j + 1][u];
-        if (HALO > 0) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) win[HALO - 1][u] = cur[u];
-        }
-      }
+      for (int j = 0; j < 4 * TAPS; ++j) f[j] = __bfloat162float(wp[j]);
     }
 #pragma unroll
-    for (int i = 0; i < CONV_NB; ++i) rows[i] = next[i];
-  }
-  if (write_carry && carry && t1 == p.L) {
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int j = 0; j < HALO; ++j) Vec4<float>::store(carry + (int64_t)j * p.C, win[j]);
+      for (int j = 0; j < TAPS; ++j) w[j][u] = make_float2(SCALE * f[2 * u * TAPS + j], SCALE * f[(2 * u + 1) * TAPS + j]);
+  }
+  bias[0] = bias[1] = make_float2(0.f, 0.f);
+  if (p.bias) {
+    float v[4];
+    Vec4<bf16>::load((const bf16*)p.bias + c, v);
+    bias[0] = make_float2(SCALE * v[0], SCALE * v[1]); bias[1] = make_float2(SCALE * v[2], SCALE * v[3]);
+  }
+  // rows travel packed, as they lie in memory: NB in work, NB under way
+  Raw4<T> next[NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (i < rows) next[i].load(src + i * ld);
+  float2 x[HALO + NB][2];                            // the inputs in front, and the rows in work
+#pragma unroll
+  for (int j = 0; j < HALO; ++j) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (t0 - HALO + j >= 0) Vec4<T>::load(src + (j - HALO) * ld, v);
+    else if (carry && !p.zero_start) Vec4<float>::load(carry + (t0 + j) * p.C, v);
+    x[j][0] = make_float2(v[0], v[1]); x[j][1] = make_float2(v[2], v[3]);
+  }
+  const auto take = [&](int i) {                          // row i of the group under way
+    float v[4];
+    next[i].get(v);
+    x[HALO + i][0] = make_float2(v[0], v[1]); x[HALO + i][1] = make_float2(v[2], v[3]);
+  };
+  const auto row = [&](int i) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float2 a = __ffma2_rn(w[HALO][u], x[HALO + i][u], bias[u]);
+#pragma unroll
+      for (int j = 0; j < HALO; ++j) a = __ffma2_rn(w[j][u], x[i + j][u], a);
+      a = conv_finish<T, ACT>(a);
+      v[2 * u] = a.x; v[2 * u + 1] = a.y;
+    }
+    Vec4<T>::store(dst + i * ldo, v);
+  };
+  int left = rows;
+  for (; left >= NB; left -= NB) {
+#pragma unroll
+    for (int i = 0; i < NB; ++i) take(i);
+    src += NB * ld;
+    // the next rows are under way while these are worked on
+    if (left >= 2 * NB) {
+#pragma unroll
+      for (int i = 0; i < NB; ++i) next[i].load(src + i * ld);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (NB + i < left) next[i].load(src + i * ld);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) row(i);
+    dst += NB * ldo;
+#pragma unroll
+    for (int j = 0; j < HALO; ++j) { x[j][0] = x[j + NB][0]; x[j][1] = x[j + NB][1]; }
+  }
+#pragma unroll
+  for (int i = 0; i + 1 < NB; ++i)                        // fewer than NB rows
+    if (i < left) { take(i); row(i); }
+  if (write_carry && carry && t0 + rows == p.L) {         // the last HALO inputs: x[left ..]
+#pragma unroll
+    for (int j = 0; j < HALO; ++j) {
+      float2 lo = x[j][0], hi = x[j][1];
+#pragma unroll
+      for (int i = 1; i < NB; ++i)
+        if (left == i) { lo = x[j + i][0]; hi = x[j + i][1]; }
+      const float v[4] = {lo.x, lo.y, hi.x, hi.y};
+      Vec4<float>::store(carry + (int64_t)j * p.C, v);
+    }
   }
 }
 
@@ -548,29 +597,43 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
   return check_launch("evo_sum_norm");
 }
 
+// Rows per CTA of the kernel with four channels per thread: one wave of CTAs that end together, each with its taps and the inputs in front fetched once, instead of many of 32 rows (4 x 4096 x 6144 with six CTAs per SM: 88 us by 32 rows, 83 so); where
+// sequences and channels alone are more than a wave, the split with the least of (waves x (rows + what a CTA's start takes, about 16 rows' time)).
+static int64_t conv_rows(const evo_conv_act_params* p) {
+  const int64_t slots = (int64_t)device_sm_count() * CONV_CTAS, per = ((p->C / 4 + 127) / 128) * (int64_t)p->B;
+  int64_t best = CONV_RT, cost = INT64_MAX;
+  for (int64_t n = 1; n <= 1024 && (n == 1 || p->L / n >= CONV_RT); ++n) {
+    const int64_t rows = std::min<int64_t>(1 << 20, std::max<int64_t>(CONV_RT, ((p->L + n - 1) / n + 3) / 4 * 4)), ctas = per * ((p->L + rows - 1) / rows), c = ((ctas + slots - 1) / slots) * (rows + 16);
+    if (c < cost) { cost = c; best = rows; }
+  }
+  return best;
+}
+
 extern "C" int evo_conv_act(const evo_conv_act_params* p, void* stream) {
   EVO_REQUIRE(p->in && p->weight && p->out && p->C > 0 && p->taps >= 1 && p->taps <= CONV_MAX_TAPS, "evo_conv_act: bad arguments (taps 1..%d)", CONV_MAX_TAPS);
   EVO_REQUIRE(p->ld >= p->C && p->ldo >= p->C && p->B >= 0 && p->L >= 0, "evo_conv_act: bad shape");
   if (p->B == 0 || p->L == 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  const unsigned chunks = (unsigned)((p->L + CONV_RT - 1) / CONV_RT);
+  const bool vec = p->C % 4 == 0 && p->ld % 4 == 0 && p->ldo % 4 == 0 && p->taps <= 4 && (!p->carry || ((uintptr_t)p->carry & 15) == 0) &&
+                   (!p->bias || aligned4<bf16>(p->bias)) &&
+                   (p->dtype ? aligned4<float>(p->in) && aligned4<float>(p->out) : aligned4<bf16>(p->in) && aligned4<bf16>(p->out));
+  const int64_t rows_per = vec ? conv_rows(p) : CONV_RT;
+  const unsigned chunks = (unsigned)((p->L + rows_per - 1) / rows_per);
   const dim3 grid((p->C + 127) / 128, chunks, p->B);
   // with one thread per (sequence, channel) that thread reads the carried inputs before it replaces them, and where none are read (zero_start) the thread of the last
   // rows may replace them; otherwise a second launch does
   const int own = chunks == 1 || p->zero_start;
-  const bool vec = p->C % 4 == 0 && p->ld % 4 == 0 && p->ldo % 4 == 0 && p->taps <= 4 && (!p->carry || ((uintptr_t)p->carry & 15) == 0) &&
-                   (!p->bias || aligned4<bf16>(p->bias)) &&
-                   (p->dtype ? aligned4<float>(p->in) && aligned4<float>(p->out) : aligned4<bf16>(p->in) && aligned4<bf16>(p->out));
   if (vec) {
     const dim3 g4((p->C / 4 + 127) / 128, chunks, p->B);
-#define EVO_CONV4(TT) \
+#define EVO_CONV4(TT, ACT) \
     switch (p->taps) { \
-      case 1: conv_act4_kernel<TT, 1><<<g4, 128, 0, st>>>(*p, own); break; \
-      case 2: conv_act4_kernel<TT, 2><<<g4, 128, 0, st>>>(*p, own); break; \
-      case 3: conv_act4_kernel<TT, 3><<<g4, 128, 0, st>>>(*p, own); break; \
-      default: conv_act4_kernel<TT, 4><<<g4, 128, 0, st>>>(*p, own); break; \
+      case 1: conv_act4_kernel<TT, 1, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
+      case 2: conv_act4_kernel<TT, 2, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
+      case 3: conv_act4_kernel<TT, 3, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
+      default: conv_act4_kernel<TT, 4, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
     }
-    if (p->dtype) { EVO_CONV4(float) } else { EVO_CONV4(bf16) }
+    if (p->dtype) { if (p->act == 1) { EVO_CONV4(float, true) } else { EVO_CONV4(float, false) } }
+    else if (p->act == 1) { EVO_CONV4(bf16, true) } else { EVO_CONV4(bf16, false) }
 #undef EVO_CONV4
   } else if (p->dtype) conv_act_kernel<float><<<grid, 128, 0, st>>>(*p, own); else conv_act_kernel<bf16><<<grid, 128, 0, st>>>(*p, own);
   int rc = check_launch("evo_conv_act");

@@ -81,6 +81,25 @@ def test_conv_act(dtype, B, L, C_, taps, carried):
         assert torch.equal(carry, z[:, L:].float())
 
 
+# CTAs of more than 32 rows that end in 1 to 7 rows, sequences that are more than a wave of CTAs, taps that start on two bytes, no activation, no bias
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,L,C_,taps,act,off,carried", [(40, 257, 2048, 4, 1, 0, True), (40, 262, 2048, 4, 0, 1, True), (37, 263, 2044, 3, 1, 1, False), (700, 43, 512, 2, 1, 0, True),
+                                                          (1, 39, 64, 4, 1, 3, True), (3, 46, 64, 1, 1, 1, False), (2, 8, 64, 4, 1, 0, True), (2, 5, 64, 3, 0, 0, True)])
+def test_conv_act_splits(dtype, B, L, C_, taps, act, off, carried):
+    g = torch.Generator(device=DEV).manual_seed(L)
+    x, buf = torch.randn(B * L, C_ + 4, generator=g, device=DEV).to(dtype), (0.5 * torch.randn(C_ * taps + 8, generator=g, device=DEV)).bfloat16()
+    w, carry = buf[off:off + C_ * taps].view(C_, taps), torch.randn(B, max(taps - 1, 1), C_, generator=g, device=DEV)
+    z = torch.cat([carry[:, :taps - 1].double() if carried else torch.zeros(B, taps - 1, C_, dtype=torch.float64, device=DEV), x.view(B, L, -1)[:, :, :C_].double()], 1)
+    want = sum(z[:, j:j + L] * w[:, j].double() for j in range(taps)).reshape(B * L, C_)
+    out = torch.empty(B * L, C_, dtype=dtype, device=DEV)
+    p = ConvActParams(inp=x.data_ptr(), ld=x.shape[1], weight=w.data_ptr(), carry=carry.data_ptr(), zero_start=int(not carried), out=out.data_ptr(), ldo=C_, B=B, L=L, C=C_, taps=taps,
+                      act=act, dtype=int(dtype == torch.float32))
+    check(_lib.lib().evo_conv_act(C.byref(p), _stream()), "evo_conv_act")
+    _near(out, torch.nn.functional.silu(want) if act else want, dtype)
+    if taps > 1:
+        assert torch.equal(carry, z[:, L:].float())
+
+
 def test_conv_act_limits():
     """SiLU far from zero and beyond: large negative inputs end at (minus) zero, infinities and NaN as in v / (1 + e^-v)."""
     v = torch.tensor([-1e38, -200.0, -89.0, -30.0, 0.0, 30.0, 200.0, 1e38, float("inf"), float("-inf"), float("nan"), -1.0], device=DEV).bfloat16().view(1, 12)
