@@ -14,7 +14,7 @@
 //   * programmatic dependent launch: the producer prefetches its first ring of W tiles (weights never depend
 //     on the previous kernel) BEFORE griddepcontrol.wait, so the pipeline fill overlaps the tail of whatever
 //     ran before; everything that reads activations / residuals or writes happens after the wait.
-// Roles: warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator, warps 4-7 epilogue (TMEM lane
+// Roles: warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator, warps 4-7 and 8-11 epilogue, a tile each in turn (TMEM lane
 // quarter = warp % 4; thread = one W row = one output column, Mb batch values in registers).
 // EVO_EPI_GELU_GATE: a tile is 256 packed rows [l1 | l2] (two MMA row groups into adjacent TMEM columns), the
 // epilogue thread holds l1[b] and l2[b] of its column: gelu(l1)*l2 is fused (the 128x64 tile needed a second kernel).
@@ -32,8 +32,17 @@ constexpr int BK = 64;              // bf16 per k-block = one 128-byte swizzle r
 constexpr int UK = 16;
 constexpr int WROWS = 128;          // W rows per MMA row group (UMMA M)
 constexpr int MAXST = 12;           // ring depth upper bound (barrier array size)
-constexpr int NTHREADS = 256;
 constexpr int EPI_WARP0 = 4;
+// Groups of four epilogue warps.  A CTA's range ends one tile and begins another, and with one group the second tile's sums waited until the first one's were published and, for its last
+// contributor, added up: 1.5 to 3 us at the end of a layer.  One step of one request 378 -> 356 us, of 16 604 -> 580.  Two groups leave a thread 168 registers; what needs more has
+// one: the Hyena step, whose threads hold a channel's filter and states, and the gated layers of many rows with their 128 sums in flight (three of 2816 x 1024 one behind the other,
+// 16 rows: 34 us, 40 with two groups; 11264 x 2048, 64 rows 85 / 89, though 22016 x 4096 163 / 159).  So do layers too small to give every SM eight k-blocks, whose CTAs gain nothing
+// and start later (768 x 256, one row, dependent: 3.6 / 4.1).
+template <int EPI, bool MANY> struct Epilogue {
+  static constexpr bool GATED = EPI == EVO_EPI_GELU_GATE || EPI == EVO_EPI_GELU_TANH_GATE;
+  static constexpr bool TWO = EPI != EVO_EPI_HYENA_STEP && !(GATED && MANY);
+  static constexpr int ONE_GROUP = (EPI_WARP0 + 4) * 32, THREADS = TWO ? ONE_GROUP + 128 : ONE_GROUP;
+};
 constexpr int MAX_MB = 64;
 
 struct SmArgs {
@@ -202,7 +211,7 @@ __device__ __forceinline__ void sum_rows(const SmArgs& g, int tile, int c_first,
   const long long n = (long long)tile * WROWS + col;
   const float* base = g.slots + col;
 #pragma unroll 1
-  for (int b0 = (threadIdx.x >> 5) - EPI_WARP0; b0 < g.M; b0 += 4 * NB) {
+  for (int b0 = (threadIdx.x >> 5) & 3; b0 < g.M; b0 += 4 * NB) {
     int b[NB];                                                         // (the last row again rather than none)
 #pragma unroll
     for (int i = 0; i < NB; ++i) b[i] = min(b0 + 4 * i, g.M - 1);
@@ -294,7 +303,7 @@ __device__ __forceinline__ void sum_columns(const SmArgs& g, int Mb, int tile, i
 }
 
 template <int EPI, bool MANY>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(Epilogue<EPI, MANY>::THREADS, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const SmArgs g) {
   constexpr int R = RowGroups<EPI>::R;                         // MMA row groups per tile
   constexpr bool COLUMNS = EPI == EPI_HYENA_STEP || (MANY && R == 2);
@@ -404,14 +413,17 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (lead) stamp(g, 4);                                            // all MMAs issued
     }
   } else if (warp >= EPI_WARP0) {
-    // ------------------------------------------------ epilogue / stream-K fix-up
+    // ------------------------------------------------ epilogue / stream-K fix-up: the groups take the CTA's tiles, and the two accumulators, in turn
+    const bool two = Epilogue<EPI, MANY>::TWO && blockDim.x > Epilogue<EPI, MANY>::ONE_GROUP;
+    const int group = (warp - EPI_WARP0) >> 2, lead = (EPI_WARP0 + 4 * group) * 32;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int q = warp - EPI_WARP0;
+    const int q = warp & 3;
     const int row = q * 32 + lane;                            // W row inside the row group == output column inside the tile
     const int slot_floats = acc_cols * WROWS;
-    int acc = 0; uint32_t acc_phase = 0;
+    int acc = group; uint32_t acc_phase = 0;
     int it = it_begin;
     const int my_first_tile = it_begin / KB;
+    if (group == 1) it = min(it_end, (my_first_tile + 1) * KB);
     while (it < it_end) {
       const int tile = it / KB, k0 = it - tile * KB;
       const int k1 = min(KB, k0 + (it_end - it));
@@ -422,7 +434,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       // (the tile's contributors, found while its products are under way)
       const int c_first = whole ? 0 : cta_of((uint32_t)tile * KB, total, parts), c_last = whole ? 0 : cta_of((uint32_t)(tile + 1) * KB - 1, total, parts);
       mbar_wait(&tfull[acc], acc_phase);
-      if (threadIdx.x == EPI_WARP0 * 32) stamp(g, it + (k1 - k0) >= it_end ? 5 : 9);   // (last) accumulator complete
+      if (threadIdx.x == lead) stamp(g, it + (k1 - k0) >= it_end ? 5 : 9);   // (last) accumulator complete
       tc_fence_after();
       const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * acc_cols);
       if (whole) {
@@ -458,27 +470,29 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);               // the accumulator is free once it has been read
-      acc ^= 1; if (acc == 0) acc_phase ^= 1;
+      if (two) acc_phase ^= 1;
+      else { acc ^= 1; if (acc == 0) acc_phase ^= 1; }
       if (!whole) {
         // publication: the CTA barrier orders every thread's partial stores before thread 0's acq_rel atomic (release
         // is cumulative), whose acquire half orders the finisher's slot reads after the other contributors' releases
-        named_bar(1, 128);
-        if (threadIdx.x == EPI_WARP0 * 32) {
+        named_bar(1 + group, 128);
+        if (threadIdx.x == lead) {
           int old;
           asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(g.counters + tile) : "memory");
-          *flag = old;
+          flag[group] = old;
         }
-        named_bar(1, 128);
-        const bool last = *flag == c_last - c_first;
-        if (threadIdx.x == EPI_WARP0 * 32) stamp(g, 6);       // partial published
+        named_bar(1 + group, 128);
+        const bool last = flag[group] == c_last - c_first;
+        if (threadIdx.x == lead) stamp(g, 6);       // partial published
         if (last) {
           const bool first_begins_before = range_start((uint32_t)c_first, total, parts) < (uint32_t)tile * KB;
           if constexpr (COLUMNS) sum_columns<EPI>(g, Mb, tile, row, c_first, c_last, first_begins_before, slot_floats);
           else sum_rows<EPI, MANY>(g, tile, c_first, c_last, first_begins_before, slot_floats);
-          if (threadIdx.x == EPI_WARP0 * 32) g.counters[tile] = 0;   // self-cleaning for the next launch
+          if (threadIdx.x == lead) g.counters[tile] = 0;   // self-cleaning for the next launch
         }
       }
       it += k1 - k0;
+      if (two) it = min(it_end, it + KB);               // the other group's tile
     }
   }
 
@@ -490,7 +504,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 8] = clock64(); g.trace[blockIdx.x * 16 + 15] = gtimer(); }
 }
 
-// Shared memory of the ring.  Two CTAs of neighbouring layers do not fit an SM together (256 threads of 168 to 255 registers), so a CTA starts when that of the layer in front has ended there: in
+// Shared memory of the ring.  Two CTAs of neighbouring layers do not fit an SM together (384 threads of up to 168 registers), so a CTA starts when that of the layer in front has ended there: in
 // the tail in which memory idles, and what its ring holds by the time the sums are published is ahead of the stream.  One step of one request / of 16 (us): 104 KB 399 / 625,
 // 150 KB 389 / 616, 180 KB 385 / 614, 216 KB 388 / 615.  (Two to an SM, 128 registers and 104 KB: 410 / 642; the ring is then filled during the layer in front, which it slows.)
 int smem_budget_bytes() {
@@ -516,7 +530,7 @@ int launch_as(const evo_gemm_smallm_params* p, cudaStream_t st) {
   g.n_tiles = (int)(p->N / (R * WROWS));
   g.KB = (int)(p->K / BK);
   const int stage_bytes = R * WROWS * BK * 2 + Mb * BK * 2;
-  const int tail = 2 * MAXST * 8 + 4 * 8 + 16;
+  const int tail = 2 * MAXST * 8 + 4 * 8 + 16;              // barriers; the address of TMEM and the groups' flags
   // (three row groups stage 48 KB of W per k-block: three stages of up to 48 rows, should the environment ask for a smaller ring)
   const int budget = R == 3 ? std::max(smem_budget_bytes(), 160 * 1024) : smem_budget_bytes();
   g.n_stages = std::max(2, std::min(MAXST, (budget - tail) / stage_bytes));
@@ -535,7 +549,7 @@ int launch_as(const evo_gemm_smallm_params* p, cudaStream_t st) {
   { int rc_ = ensure_dyn_smem(kern, 224 * 1024, attr_done); if (rc_) return rc_; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(NTHREADS);
+  cfg.blockDim = dim3(total < 8LL * device_sm_count() ? Epilogue<EPI, MANY>::ONE_GROUP : Epilogue<EPI, MANY>::THREADS);
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

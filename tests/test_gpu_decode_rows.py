@@ -57,3 +57,28 @@ def test_many_rows_are_the_first_rows_of_more(N, K, epi):
         full = _linear(a, w, widest, getattr(_lib, epi), bias, resid)
         for M in rows:
             assert torch.equal(_linear(a, w, M, getattr(_lib, epi), bias, resid), full[:M]), M
+
+
+@pytest.mark.parametrize("epi", ["EPI_BIAS_RESID", "EPI_NONE", "EPI_GELU_GATE", "EPI_SILU_COLS"])
+@pytest.mark.parametrize("N,K", [(37632, 256), (37888, 256), (40960, 256), (77824, 128), (9728, 1088)])
+def test_tiles_of_a_cta_in_turn(N, K, epi):
+    """CTAs whose range is part of a tile, whole tiles and part of a third or fifth, on both sides of the line between one and two groups of epilogue warps (eight k-blocks per SM)."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    n = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    a, w, bias, resid = n(16, K).to(BF), (n(N, K) / math.sqrt(K)).to(BF), n(N).to(BF), n(17, N).to(BF)
+    for M in (1, 16):
+        got = _linear(a, w, M, getattr(_lib, epi), bias, resid).double()
+        acc, r = a[:M].double() @ w.double().T, lambda x: x.to(BF).double()  # noqa: E731
+        slack = torch.zeros_like(got)
+        if epi == "EPI_NONE":
+            want = acc
+        elif epi == "EPI_BIAS_RESID":
+            want, slack = r(acc + bias.double()) + resid[:M].double(), 2.0 ** -7 * (acc + bias.double()).abs()        # the rounded product may be a step away
+        elif epi == "EPI_SILU_COLS":
+            want = torch.where(torch.arange(N, device=DEV) < N // 2, torch.nn.functional.silu(acc), acc)
+        else:
+            t = acc.view(M, -1, 2, 128)
+            want = (r(torch.nn.functional.gelu(r(t[:, :, 0]))) * r(t[:, :, 1])).reshape(M, -1)
+            slack = (2.0 ** -6 * (t[:, :, 0].abs() * t[:, :, 1].abs())).reshape(M, -1)                                # three rounded factors, each a step of 2^-7 away at most
+        # half a step of bf16 of the result, and 2^-16 of the sums' scale for K products in fp32
+        assert ((got - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + slack + 2.0 ** -16 * want.abs().max()).all(), (M, epi)
