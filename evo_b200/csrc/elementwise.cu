@@ -88,6 +88,34 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* __restrict__ 
   }
 }
 
+// pieces of a row held by a CTA of 256 threads
+__device__ __forceinline__ float square_sum(const uint4& v, float ss) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { const float a = bf_lo(w[j]), b = bf_hi(w[j]); ss = fmaf(a, a, ss); ss = fmaf(b, b, ss); }
+  return ss;
+}
+__device__ __forceinline__ float row_rinv(float ss, float (&red)[8], float inv_sqrt_d, float eps) {      // 1 / n of the note above
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) tot += red[w];
+  float n = rbf(sqrtf(tot));
+  n = rbf(n * inv_sqrt_d);
+  n = rbf(n + eps);
+  return __frcp_rn(n);
+}
+__device__ __forceinline__ uint4 normed(const uint4& v, const uint4& s, float rinv) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w}, sw[4] = {s.x, s.y, s.z, s.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[j] = pack_bf16(bf_lo(sw[j]) * rbf(bf_lo(w[j]) * rinv), bf_hi(sw[j]) * rbf(bf_hi(w[j]) * rinv));
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // Few rows (decode step): one 256-thread CTA per row instead of one warp per row -- the row and the scale are fetched
 // by 8 warps at once (the warp-per-row kernel is a 5 us latency chain on 2 CTAs at 16 rows).  Same rounding chain.
 __global__ void __launch_bounds__(256) rmsnorm_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ scale,
@@ -104,41 +132,58 @@ __global__ void __launch_bounds__(256) rmsnorm_row_kernel(const uint4* __restric
     if (idx < row_vec) { v[i] = __ldg(xr + idx); sc[i] = __ldg(scale + idx); }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (tid + i * 256 < row_vec) {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(&v[i]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { float a = bf_lo(w[j]), b = bf_hi(w[j]); ss = fmaf(a, a, ss); ss = fmaf(b, b, ss); }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if ((tid & 31) == 0) red[tid >> 5] = ss;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) tot += red[w];
-  float n = rbf(sqrtf(tot));
-  n = rbf(n * inv_sqrt_d);
-  n = rbf(n + eps);
-  const float rinv = __frcp_rn(n);
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < row_vec) ss = square_sum(v[i], ss);
+  const float rinv = row_rinv(ss, red, inv_sqrt_d, eps);
   uint4* orow = out + (int64_t)blockIdx.x * row_vec;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < row_vec) orow[tid + i * 256] = normed(v[i], sc[i], rinv);
+}
+
+// The beginning of a decode step in one launch: a CTA fetches its sequence's embedding row, leaves it as it is and normed (the chain above), and one thread notes the position.  Position,
+// ids, embedding and norm as a launch each took 13 us in front of a first layer, this one 6: a step of one request 359 -> 351 us, of sixteen 585 -> 575.
+template <typename IdT>
+__global__ void __launch_bounds__(256) embed_norm_kernel(const IdT* __restrict__ ids, const uint4* __restrict__ table, const uint4* __restrict__ scale, uint4* __restrict__ u,
+                                                         uint4* __restrict__ out, int row_vec, int vocab, float inv_sqrt_d, float eps, long long* __restrict__ pos, long long position) {
+  pdl_launch_dependents(); pdl_wait();
+  __shared__ float red[8];
+  const int tid = threadIdx.x;
+  long long id = (long long)ids[blockIdx.x];
+  id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
+  if (pos && blockIdx.x == 0 && tid == 0) *pos = position;
+  const uint4* xr = table + id * row_vec;
+  const int64_t row = (int64_t)blockIdx.x * row_vec;
+  uint4 v[4], sc[4];
+  float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int idx = tid + i * 256;
-    if (idx < row_vec) {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(&v[i]);
-      const uint32_t* sw = reinterpret_cast<const uint32_t*>(&sc[i]);
-      uint4 o;
-      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float y0 = rbf(bf_lo(w[j]) * rinv), y1 = rbf(bf_hi(w[j]) * rinv);
-        ow[j] = pack_bf16(bf_lo(sw[j]) * y0, bf_hi(sw[j]) * y1);
-      }
-      orow[idx] = o;
-    }
+    if (idx < row_vec) { v[i] = __ldg(xr + idx); sc[i] = __ldg(scale + idx); }
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (tid + i * 256 < row_vec) { u[row + tid + i * 256] = v[i]; ss = square_sum(v[i], ss); }
+  }
+  const float rinv = row_rinv(ss, red, inv_sqrt_d, eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (tid + i * 256 < row_vec) out[row + tid + i * 256] = normed(v[i], sc[i], rinv);
+}
+
+extern "C" int evo_embed_norm(const void* ids, int ids_are_i64, const void* table, const void* scale, void* u, void* out, int64_t rows, int D, int vocab, float eps, int64_t* pos,
+                              int64_t position, void* stream) {
+  EVO_REQUIRE(D % 256 == 0 && D <= 8192, "evo_embed_norm: D (%d) must be a multiple of 256 and <= 8192", D);
+  EVO_REQUIRE(rows > 0 && rows < (1ll << 31), "evo_embed_norm: rows (%lld)", (long long)rows);
+  // (not dependent where evo_hyena_step fetches its states ahead of its wait: between two of a layer's steps there has to be one launch that waits for all in front of it)
+  const float isd = (float)(1.0 / sqrt((double)D));
+  if (ids_are_i64)
+    EVO_CUDA(launch_pdl(embed_norm_kernel<long long>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const long long*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u,
+                              (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position));
+  else
+    EVO_CUDA(launch_pdl(embed_norm_kernel<int>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const int*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u,
+                              (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position));
+  return check_launch("evo_embed_norm");
 }
 
 extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t rows, int D, float eps, void* stream) {

@@ -535,16 +535,23 @@ class StripedHyena(KernelOps, nn.Module):
         self._tiled = t
         return t
 
-    def _decode_body(self, x, pos_dev, ipd, B):
-        """One token per sequence through all blocks; every launch reads the position from pos_dev."""
+    def _decode_begin(self, x, u, xn, B, pos_dev=None, pos=0):
+        """u = the embedding rows of x, xn = the first block's norm of them; pos_dev, if given, is set to pos: one launch."""
+        cfg = self.config
+        self._record("rmsnorm", 4.0 * B * cfg.hidden_size, lambda: check(_lib.lib().evo_embed_norm(
+            ptr(x), int(x.dtype == torch.int64), ptr(self.embedding_layer.weight), ptr(self.blocks[0].pre_norm.scale), ptr(u), ptr(xn), B, cfg.hidden_size, cfg.vocab_size,
+            float(cfg.eps), ptr(pos_dev), pos, self._stream()), "evo_embed_norm"))
+
+    def _decode_body(self, x, pos_dev, ipd, B, begun=None):
+        """One token per sequence through all blocks; every launch reads the position from pos_dev.  begun = (u, xn): _decode_begin has run."""
         lib = _lib.lib()
         prev = lib.evo_set_pdl(int(self.decode_pdl))
         try:
-            return self._decode_body_impl(x, pos_dev, ipd, B)
+            return self._decode_body_impl(x, pos_dev, ipd, B, begun)
         finally:
             lib.evo_set_pdl(prev)
 
-    def _decode_body_impl(self, x, pos_dev, ipd, B):
+    def _decode_body_impl(self, x, pos_dev, ipd, B, begun):
         cfg = self.config
         d, H, V = cfg.hidden_size, cfg.num_attention_heads, cfg.vocab_size
         hd = d // H
@@ -562,12 +569,15 @@ class StripedHyena(KernelOps, nn.Module):
             else:
                 self._gemm(a, w, out, B, N, K, epi, bias=bias, resid=resid, variant=G2)
 
-        u = torch.empty(B, d, dtype=torch.bfloat16, device=dev)
-        check(lib.evo_embed(ptr(x), int(x.dtype == torch.int64), ptr(self.embedding_layer.weight), ptr(u), B, d, V, self._stream()), "evo_embed")
+        if begun is None:
+            begun = torch.empty(B, d, dtype=torch.bfloat16, device=dev), torch.empty(B, d, dtype=torch.bfloat16, device=dev)
+            self._decode_begin(x, *begun, B)
+        u, xn = begun
         nsplit = max(1, min(16, -(-8 * torch.cuda.get_device_properties(dev).multi_processor_count // (H * B))))   # >= ~4 waves of 2 CTAs/SM
         for i, blk in enumerate(self.blocks):
-            xn = torch.empty_like(u)
-            self._rmsnorm(u, blk.pre_norm.scale, xn, B)
+            if i > 0:
+                xn = torch.empty_like(u)
+                self._rmsnorm(u, blk.pre_norm.scale, xn, B)
             u2 = torch.empty_like(u)
             if i in self._attn_idxs:
                 mha = blk.inner_mha_cls
@@ -735,19 +745,19 @@ class StripedHyena(KernelOps, nn.Module):
                 raise _lib.EvoError(f"sequence length {off + 1} exceeds the KV cache ({mha_ip.key_value_memory_dict[i].shape[1]}) (mha.py:367)")
         st = self._decode
         if st is None or st["key"] != key:
-            st = {"key": key, "graph": None, "x": torch.empty_like(x), "pos": torch.zeros(1, dtype=torch.int64, device=dev), "logits": None, "steps": 0}
+            new = lambda: torch.empty(B, self.config.hidden_size, dtype=torch.bfloat16, device=dev)  # noqa: E731
+            st = {"key": key, "graph": None, "begun": (new(), new()), "pos": torch.zeros(1, dtype=torch.int64, device=dev), "logits": None, "steps": 0}
             self._decode = st
-        st["pos"].fill_(off)
-        st["x"].copy_(x)
+        self._decode_begin(x, *st["begun"], B, st["pos"], off)        # in front of the graph: its ids are another tensor each time
         if not self.decode_graph or self._prof is not None or st["steps"] == 0:
             st["steps"] += 1
-            return self._decode_body(st["x"], st["pos"], ipd, B).view(B, 1, -1)
+            return self._decode_body(x, st["pos"], ipd, B, st["begun"]).view(B, 1, -1)
         if st["graph"] is None:
             g = torch.cuda.CUDAGraph()
             torch.cuda.synchronize()
             n0 = _lib.lib().evo_launch_count()
             with torch.cuda.graph(g):
-                st["logits"] = self._decode_body(st["x"], st["pos"], ipd, B)
+                st["logits"] = self._decode_body(x, st["pos"], ipd, B, st["begun"])
             st["graph"] = g
             st["launches"] = _lib.lib().evo_launch_count() - n0      # counted while capturing, when nothing ran: undo, then count per replay
             _lib.lib().evo_note_graph_replay(-st["launches"])

@@ -45,6 +45,9 @@ int evo_embed(const void* ids, int ids_are_i64, const void* table, void* out,
  * y = scale * x / (||x||_2 * D^-1/2 + eps), every intermediate rounded to bf16 as the
  * reference's bf16 tensor ops do.  x,out (rows, D) bf16; scale (D) bf16. */
 int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t rows, int D, float eps, void* stream);
+/* evo_embed (into u) and evo_rmsnorm (into out) of a few rows in one launch; pos, if given, becomes `position`: the beginning of a decode step. */
+int evo_embed_norm(const void* ids, int ids_are_i64, const void* table, const void* scale, void* u, void* out, int64_t rows, int D, int vocab, float eps, int64_t* pos, int64_t position,
+                   void* stream);
 
 /* ---- tensor-core linear layers (nn.Linear / ParallelGatedMLP / unembed) ----
  * C[M,N] = epilogue(A[M,K] . W[N,K]^T), bf16 in, fp32 accumulate (tcgen05, TMEM), bf16 out.

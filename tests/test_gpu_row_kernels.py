@@ -143,3 +143,27 @@ def test_rmsnorm_forms(rows, D):
     want = d / (d.norm(dim=-1, keepdim=True) * D ** -0.5 + 1e-6) * s.double()
     # five roundings to bf16 (norm, times D^-1/2, plus eps, quotient, product), each at most half a step of 2^-7
     assert ((out.double() - want).abs() <= 5 * 2.0 ** -8 * want.abs()).all()
+
+
+@pytest.mark.parametrize("ids_dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("rows,D", [(1, 256), (3, 4096), (16, 2304), (2, 8192), (300, 512)])
+def test_embed_norm_is_embed_and_rmsnorm(rows, D, ids_dtype):
+    """The beginning of a decode step in one launch: the bits of the two it stands for, ids out of range included, and the position."""
+    g = torch.Generator(device=DEV).manual_seed(D + rows)
+    table, scale = torch.randn(512, D, generator=g, device=DEV).bfloat16(), (1 + 0.1 * torch.randn(D, generator=g, device=DEV)).bfloat16()
+    ids = torch.randint(-3, 520, (rows,), generator=g, device=DEV).to(ids_dtype)
+    lib, new = _lib.lib(), lambda: torch.full((rows, D), 9.0, dtype=torch.bfloat16, device=DEV)  # noqa: E731
+    u, xn, u2, xn2 = new(), new(), new(), new()
+    wide, pos = int(ids_dtype == torch.int64), torch.tensor([-1, 77], device=DEV)
+    check(lib.evo_embed(C.c_void_p(ids.data_ptr()), wide, C.c_void_p(table.data_ptr()), C.c_void_p(u.data_ptr()), rows, D, 512, _stream()), "evo_embed")
+    check(lib.evo_rmsnorm(C.c_void_p(u.data_ptr()), C.c_void_p(scale.data_ptr()), C.c_void_p(xn.data_ptr()), rows, D, 1e-6, _stream()), "evo_rmsnorm")
+    check(lib.evo_embed_norm(C.c_void_p(ids.data_ptr()), wide, C.c_void_p(table.data_ptr()), C.c_void_p(scale.data_ptr()), C.c_void_p(u2.data_ptr()), C.c_void_p(xn2.data_ptr()), rows, D, 512,
+                             1e-6, C.c_void_p(pos.data_ptr()), 1234567, _stream()), "evo_embed_norm")
+    assert torch.equal(u, u2) and pos.tolist() == [1234567, 77]
+    if rows <= 64:                                   # (beyond, evo_rmsnorm may sum a row's squares in another order)
+        assert torch.equal(xn, xn2)
+    else:
+        assert ((xn.float() - xn2.float()).abs() <= 2.0 ** -6 * xn.float().abs()).all()
+    with pytest.raises(_lib.EvoError):
+        check(lib.evo_embed_norm(C.c_void_p(ids.data_ptr()), wide, C.c_void_p(table.data_ptr()), C.c_void_p(scale.data_ptr()), C.c_void_p(u2.data_ptr()), C.c_void_p(xn2.data_ptr()), rows, 8448,
+                                 512, 1e-6, None, 0, _stream()), "evo_embed_norm")
