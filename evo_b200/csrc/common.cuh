@@ -341,6 +341,17 @@ inline cudaError_t launch_pdl_at(int min_level_extra, void (*kern)(KArgs...), di
   }
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
+// always with the attribute: for kernels that wait (pdl_wait) before they touch anything
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_light(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   return launch_pdl_at(3, kern, grid, block, smem, st, args...);

@@ -198,8 +198,8 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
   // 2048 wide: 1024 rows 7.9 / 8.0, 2048 rows 8.4 / 8.0, 8192 rows 22.7 / 18.6 (too few bytes per CTA), narrower the same; 8192 wide: 903 rows 8.4 / 15.1, 32768 rows 156 / 268
   // (a warp would hold 32 vectors per lane)
   if (D > 4096 || rows <= (D >= 4096 ? 12288 : 1024)) {
-    EVO_CUDA(launch_pdl(rmsnorm_row_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
-                        D / 8, (float)(1.0 / sqrt((double)D)), eps));
+    EVO_CUDA(launch_dependent(rmsnorm_row_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
+                              D / 8, (float)(1.0 / sqrt((double)D)), eps));
     return check_launch("evo_rmsnorm");
   }
   int nvec = D / 256;

@@ -259,6 +259,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();   // every CTA of this launch has its TMEM before one of the next launch can ask for some
+  pdl_wait();                // launched dependent (see launch()): nothing in front of this reads or writes what a kernel before may write or read
 
   // Tile walk of this CTA (pair): tiles w_first, w_first + w_step, ... < n_tiles of the row-blocks [m_lo, m_lo + m_cnt).
   // Die-aware (CG == 2, full grid): each die works on its own contiguous share of the row-blocks, so the streamed operand's
@@ -508,7 +510,7 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = C_::SMEM_BYTES;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   g.die_tab = nullptr; g.die_claim = nullptr; g.m_split = 0; g.die_pairs0 = g.die_pairs1 = 0; g.die_collide = 0;
   if (CG == 2) {
     int pairs = min(n_tiles, sms / 2);
@@ -538,9 +540,17 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
     cfg.gridDim = dim3(pairs * 2);
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.numAttrs = 1;
   } else {
     cfg.gridDim = dim3(min(n_tiles, sms * C_::CTAS_PER_SM));
+  }
+  cfg.attrs = attr;
+  // Launched dependent, but for the die-aware form, whose claims are cleared in front of it: barriers, TMEM and tensor maps are ready when the kernel in front ends.
+  // The two layers of a feed-forward of 3002 rows 652 -> 641 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606.
+  if (g.die_tab == nullptr) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
   }
   EVO_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, g));
   return check_launch("evo_gemm");
