@@ -135,6 +135,7 @@ attn_pp_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();              // launched dependent: nothing in front of this touches what a kernel before may write or read
 
   if (warp == 8) {
     // ------------------------------------------------ TMA producer
@@ -348,10 +349,10 @@ int evo_attn_pp_launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUt
   dim3 grid((unsigned)(heads * pairs));
   if (npoly == 0) {
     { int rc_ = ensure_dyn_smem(attn_pp_kernel<0>, SMEM, done0); if (rc_) return rc_; }
-    attn_pp_kernel<0><<<grid, THREADS, SMEM, st>>>(tmQ, tmK, tmV, a);
+    EVO_CUDA(launch_dependent(attn_pp_kernel<0>, grid, dim3(THREADS), SMEM, st, tmQ, tmK, tmV, a));
   } else {
     { int rc_ = ensure_dyn_smem(attn_pp_kernel<3>, SMEM, done3); if (rc_) return rc_; }
-    attn_pp_kernel<3><<<grid, THREADS, SMEM, st>>>(tmQ, tmK, tmV, a);
+    EVO_CUDA(launch_dependent(attn_pp_kernel<3>, grid, dim3(THREADS), SMEM, st, tmQ, tmK, tmV, a));
   }
   return check_launch("evo_attn_fwd(pp)");
 }

@@ -63,6 +63,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ---- evo_sum_norm: one CTA per row; the new row of x is kept in shared memory between the passes
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) sum_norm_kernel(evo_sum_norm_params p) {
+  pdl_wait();
   extern __shared__ float xs[];          // [D] + 33
   float* red = xs + p.D;
   const int64_t r = blockIdx.x;
@@ -180,6 +181,7 @@ template <> struct Raw4<bf16> {
 
 template <typename T, int NV, int NB>
 __global__ void __launch_bounds__(256) sum_norm_row_kernel(const evo_sum_norm_params p) {
+  pdl_wait();
   __shared__ __align__(16) float red[4][8];
   const int64_t r = blockIdx.x;
   const int64_t src = p.gather ? p.gather[r] : r;
@@ -290,6 +292,7 @@ template <typename T, bool ACT> __device__ __forceinline__ float2 conv_finish(fl
 // eight under way, four CTAs per SM of 128 registers (four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows).  fp32 rows, four and four: 148 us (162).
 template <typename T, int TAPS, bool ACT>
 __global__ void __launch_bounds__(128, CONV_CTAS) conv_act4_kernel(evo_conv_act_params p, int write_carry, int rows_per) {
+  pdl_wait();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= p.C) return;
   constexpr int HALO = TAPS - 1, NB = sizeof(T) == 2 ? 8 : 4;
@@ -391,6 +394,7 @@ __global__ void __launch_bounds__(128, CONV_CTAS) conv_act4_kernel(evo_conv_act_
 
 template <typename T>
 __global__ void __launch_bounds__(128) conv_act_kernel(evo_conv_act_params p, int write_carry) {
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int b = blockIdx.z, taps = p.taps, halo = taps - 1;
@@ -439,6 +443,7 @@ __global__ void __launch_bounds__(128) conv_act_kernel(evo_conv_act_params p, in
 // the carried inputs of a call whose rows were spread over several threads per channel: written after every row has been read
 template <typename T>
 __global__ void __launch_bounds__(128) conv_carry_kernel(evo_conv_act_params p) {
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int b = blockIdx.z, halo = p.taps - 1;
@@ -581,10 +586,10 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
     // rows in registers: (groups of four per thread) x (branches)
 #define EVO_SUM_NORM(TT, NV) \
     switch (p->n_branches) { \
-      case 0: sum_norm_row_kernel<TT, NV, 0><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
-      case 1: sum_norm_row_kernel<TT, NV, 1><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
-      case 2: sum_norm_row_kernel<TT, NV, 2><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
-      default: sum_norm_row_kernel<TT, NV, 3><<<(unsigned)p->rows, 256, 0, st>>>(*p); break; \
+      case 0: EVO_CUDA(launch_dependent(sum_norm_row_kernel<TT, NV, 0>, dim3((unsigned)p->rows), dim3(256), 0, st, *p)); break; \
+      case 1: EVO_CUDA(launch_dependent(sum_norm_row_kernel<TT, NV, 1>, dim3((unsigned)p->rows), dim3(256), 0, st, *p)); break; \
+      case 2: EVO_CUDA(launch_dependent(sum_norm_row_kernel<TT, NV, 2>, dim3((unsigned)p->rows), dim3(256), 0, st, *p)); break; \
+      default: EVO_CUDA(launch_dependent(sum_norm_row_kernel<TT, NV, 3>, dim3((unsigned)p->rows), dim3(256), 0, st, *p)); break; \
     }
     if (p->dtype) { if (p->D <= 1024) { EVO_SUM_NORM(float, 1) } else if (p->D <= 2048) { EVO_SUM_NORM(float, 2) } else { EVO_SUM_NORM(float, 4) } }
     else { if (p->D <= 1024) { EVO_SUM_NORM(bf16, 1) } else if (p->D <= 2048) { EVO_SUM_NORM(bf16, 2) } else { EVO_SUM_NORM(bf16, 4) } }
@@ -593,7 +598,7 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
   }
   auto kern = p->dtype ? (vec ? sum_norm_kernel<float, true> : sum_norm_kernel<float, false>) : (vec ? sum_norm_kernel<bf16, true> : sum_norm_kernel<bf16, false>);
   if (smem > 48 * 1024) EVO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<(unsigned)p->rows, 256, smem, st>>>(*p);
+  EVO_CUDA(launch_dependent(kern, dim3((unsigned)p->rows), dim3(256), smem, st, *p));
   return check_launch("evo_sum_norm");
 }
 
@@ -627,19 +632,19 @@ extern "C" int evo_conv_act(const evo_conv_act_params* p, void* stream) {
     const dim3 g4((p->C / 4 + 127) / 128, chunks, p->B);
 #define EVO_CONV4(TT, ACT) \
     switch (p->taps) { \
-      case 1: conv_act4_kernel<TT, 1, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
-      case 2: conv_act4_kernel<TT, 2, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
-      case 3: conv_act4_kernel<TT, 3, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
-      default: conv_act4_kernel<TT, 4, ACT><<<g4, 128, 0, st>>>(*p, own, (int)rows_per); break; \
+      case 1: EVO_CUDA(launch_dependent(conv_act4_kernel<TT, 1, ACT>, g4, dim3(128), 0, st, *p, own, (int)rows_per)); break; \
+      case 2: EVO_CUDA(launch_dependent(conv_act4_kernel<TT, 2, ACT>, g4, dim3(128), 0, st, *p, own, (int)rows_per)); break; \
+      case 3: EVO_CUDA(launch_dependent(conv_act4_kernel<TT, 3, ACT>, g4, dim3(128), 0, st, *p, own, (int)rows_per)); break; \
+      default: EVO_CUDA(launch_dependent(conv_act4_kernel<TT, 4, ACT>, g4, dim3(128), 0, st, *p, own, (int)rows_per)); break; \
     }
     if (p->dtype) { if (p->act == 1) { EVO_CONV4(float, true) } else { EVO_CONV4(float, false) } }
     else if (p->act == 1) { EVO_CONV4(bf16, true) } else { EVO_CONV4(bf16, false) }
 #undef EVO_CONV4
-  } else if (p->dtype) conv_act_kernel<float><<<grid, 128, 0, st>>>(*p, own); else conv_act_kernel<bf16><<<grid, 128, 0, st>>>(*p, own);
+  } else EVO_CUDA(launch_dependent(p->dtype ? conv_act_kernel<float> : conv_act_kernel<bf16>, grid, dim3(128), 0, st, *p, own));
   int rc = check_launch("evo_conv_act");
   if (rc || own || !p->carry || p->taps == 1) return rc;
   const dim3 g2((p->C + 127) / 128, 1, p->B);
-  if (p->dtype) conv_carry_kernel<float><<<g2, 128, 0, st>>>(*p); else conv_carry_kernel<bf16><<<g2, 128, 0, st>>>(*p);
+  EVO_CUDA(launch_dependent(p->dtype ? conv_carry_kernel<float> : conv_carry_kernel<bf16>, g2, dim3(128), 0, st, *p));
   return check_launch("evo_conv_act");
 }
 

@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const Args p) {
   float* beta = rq + BT;
   float* lh = beta + BT;                                     // running log decay, high and low float
   float* ll = lh + BT;
+  pdl_wait();                                                // itself launched dependent: what it writes may still be read, and what the scan reads before its own wait must be there
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (p.H / p.G);
@@ -842,6 +843,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 1) delta_scan_kernel(const __gri
 // several of which share an SM; the state is in registers, the read-outs are left to a norm of their own.  single() says where it is taken.
 template <int DK>
 __global__ void __launch_bounds__(256, 1) delta_single_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmV, const Args p) {
+  pdl_wait();
   constexpr int KT = DK / 16, BOX = BT * 128, ROWS_BYTES = DK / 64 * BOX;      // keys and queries: boxes of 64 columns, 16-byte pieces of a row swizzled by row & 7
   extern __shared__ __align__(16) uint8_t sm_raw[];
   uint8_t* ks = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~(uintptr_t)1023);
@@ -1197,10 +1199,10 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
     a.first = first; a.n_blocks = (int)std::min<int64_t>(s.slab, s.blocks - first);
     a.zero_start = first == 0 && (p->zero_start || !p->state);
     a.store_state = p->state || s.state;
-    delta_prepare_kernel<DK><<<dim3(a.n_blocks, a.H, a.B), 128, prep_smem, st>>>(a);
+    EVO_CUDA(launch_dependent(delta_prepare_kernel<DK>, dim3(a.n_blocks, a.H, a.B), dim3(128), prep_smem, st, a));
     if ((rc = check_launch("evo_gated_delta_fwd(prepare)"))) return rc;
     if (one) {
-      delta_single_kernel<DK><<<dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), nw * 32, single_smem_bytes(DK, nw), st>>>(tmK, tmQ, tmV, a);
+      EVO_CUDA(launch_dependent(delta_single_kernel<DK>, dim3(a.H, a.B, (a.dv / 16 + nw - 1) / nw), dim3(nw * 32), single_smem_bytes(DK, nw), st, tmK, tmQ, tmV, a));
       if ((rc = check_launch("evo_gated_delta_fwd(single)"))) return rc;
       break;
     }

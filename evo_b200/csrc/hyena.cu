@@ -408,8 +408,6 @@ static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, voi
   if ((rc = ensure_dyn_smem(hyena_tc_kernel<R, false>, smem, done_o))) return rc;
   bf16* fir_out = fir_state_over_halo(p) ? nullptr : (bf16*)p->fir_state_out;
   const int copies = fir_out ? (int)(((long long)p->B * 3 * p->D + PREP_WARPS * 32 - 1) / (PREP_WARPS * 32)) : 0;
-  hyena_tc_constants_kernel<<<p->D / PREP_WARPS + copies, PREP_WARPS * 32, 0, st>>>(p->poles, p->residues, consts, seg_pow, p->D, R, nseg > 1 ? seg_len : 0, a.z, a.halo, fir_out, p->B, p->L);
-  if ((rc = check_launch("hyena_tc_constants"))) return rc;
   const int per_seg = p->D / CH * p->B, sms = device_sm_count();
   const bool states = p->state_only || (nseg > 1 && !p->reuse_segment_states);
   // A dependent launch takes about 4 us off a call, but its CTAs do not start together, and long calls lose more by that: neighbouring channels' CTAs then no longer read a token's row at
@@ -417,6 +415,10 @@ static int launch_tc(const evo_hyena_params* p, int nseg, long long seg_len, voi
   // 8 x 8193 850 / 867.  The line: 16 k tokens that a CTA walks.
   const long long walked = (long long)((per_seg * nseg + sms - 1) / sms) * std::min<long long>(seg_len, p->L);
   const bool soon = walked <= (16 << 10) + 1024;
+  // (the constants, in front, the same: 1 x 1999 41.8 / 39.8, 8 x 8193 831 / 833)
+  EVO_CUDA(launch_after(soon, hyena_tc_constants_kernel, dim3(p->D / PREP_WARPS + copies), dim3(PREP_WARPS * 32), 0, st, p->poles, p->residues, consts, seg_pow, p->D, R,
+                        nseg > 1 ? seg_len : 0, a.z, a.halo, fir_out, p->B, p->L));
+  if ((rc = check_launch("hyena_tc_constants"))) return rc;
   if (states) {
     a.items = per_seg * (p->state_only ? nseg : nseg - 1);
     EVO_CUDA(launch_after(soon, hyena_tc_kernel<R, true>, dim3(std::min(a.items, sms)), dim3(evo_hytc::THREADS), smem, st, tmZ, a));

@@ -106,6 +106,7 @@ constexpr int PREP_WARPS = 4;
 __global__ void __launch_bounds__(PREP_WARPS * 32) hyena_tc_constants_kernel(const float* __restrict__ poles, const float* __restrict__ residues, uint8_t* __restrict__ consts,
                                                                              float2* __restrict__ seg_pow, int D, int R, long long seg_len, const bf16* __restrict__ z,
                                                                              const bf16* __restrict__ halo, bf16* __restrict__ fir_out, int B, long long L) {
+  pdl_wait();                                               // itself launched dependent: what it writes may still be read, and what the operator reads before its own wait must be there
   pdl_launch_dependents();
   if ((int)blockIdx.x >= D / PREP_WARPS) {
     const long long idx = (long long)(blockIdx.x - D / PREP_WARPS) * (PREP_WARPS * 32) + threadIdx.x;

@@ -99,6 +99,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  pdl_wait();              // launched dependent: nothing in front of this touches what a kernel before may write or read
 
   if (warp >= WARPS) {
     regs_down<OTHER_REGS>();
@@ -385,7 +386,7 @@ int launch(const evo_window_attn_params* p, cudaStream_t st) {
   constexpr int smem = BQ * HD * 2 * (2 + 2 * KV_STAGES) + 1024;
   static unsigned long long done = 0;
   if ((rc = ensure_dyn_smem(window_attn_tc_kernel<HD>, smem, done))) return rc;
-  window_attn_tc_kernel<HD><<<(unsigned)(heads * pairs), THREADS, smem, st>>>(tmQ, tmK, tmV, a);
+  EVO_CUDA(launch_dependent(window_attn_tc_kernel<HD>, dim3((unsigned)(heads * pairs)), dim3(THREADS), smem, st, tmQ, tmK, tmV, a));
   return check_launch("evo_window_attn_fwd");
 }
 
