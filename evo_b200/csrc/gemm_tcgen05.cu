@@ -578,6 +578,24 @@ int dispatch_epi(const evo_gemm_params* p, cudaStream_t st) {
   return -1;
 }
 
+// Variant 0's tiles: a sum's order does not depend on them (the results are the same bits), so the shape decides.  Few rows leave most of the pairs of SMs without a 256 x 256 tile, or the
+// last wave nearly empty.  By pairs / by 128 x 256 / by 128 x 64 (us, cold L2):
+//   128 x 64 while all its tiles fit at once, two to an SM, and K is not so long that their small operands' loads cost more than the SMs gained: 4096 x 4096, 300 rows 36.9 / 41 / 32.8,
+//   514 rows (320 tiles) 38.9 / 41 / 51; 2048 x 2048, 903 rows 26.6 / 28.7 / 22.5, 1300 (352) 28.7 / 28.7 / 30.7; 2048 x 5504, 200 rows 41.0 / 45 / 34.8; 4096 x 11008, 66 rows 65.6 /
+//   80 / 67.6, 400 rows 71.7 / 84 / 73.7
+//   128 x 256 where it takes a wave less (few waves: one is 5 to 8 % longer): 12288 x 4096, 300 rows 59.4 / 47.1 / 57.3, 400 rows 59.4 / 68.4; gated 22016 x 4096, 128 rows 67.6 / 55.2,
+//   141 rows 67.6 / 73.7, 300 rows 81.9 / 73.7, 514 rows 98.3 / 92.2
+int pick_tile(const evo_gemm_params* p) {
+  const char* env = getenv("EVO_B200_GEMM_TILE");                    // comparisons: 0, 1 or 2; read per call
+  const bool plain = p->n_c_peers == 0 && (p->epilogue == EVO_EPI_NONE || p->epilogue == EVO_EPI_BIAS || p->epilogue == EVO_EPI_BIAS_RESID || p->epilogue == EVO_EPI_RESID ||
+                                           p->epilogue == EVO_EPI_SILU_COLS);
+  if (env) return atoi(env) == 2 ? (plain ? 2 : 1) : atoi(env);
+  const int64_t sms = device_sm_count(), rows128 = (p->M + 127) / 128, n256 = p->N / 256;
+  if (plain && p->K <= 6144 && rows128 * n256 * 4 <= 2 * sms) return 2;
+  const int64_t pairs = ((p->M + 255) / 256) * n256, waves = (pairs + sms / 2 - 1) / (sms / 2);
+  return waves <= 4 && (rows128 * n256 + sms - 1) / sms < waves ? 1 : 0;
+}
+
 }  // namespace
 
 extern "C" int evo_gemm(const evo_gemm_params* p, void* stream) {
@@ -600,8 +618,9 @@ extern "C" int evo_gemm(const evo_gemm_params* p, void* stream) {
     EVO_REQUIRE(p->variant == 0 || p->variant == 1, "evo_gemm: peer scatter needs the 256-column tiles");
   }
   if (p->M == 0) return 0;
-  if (p->variant == 2 || p->variant == 3) return dispatch_epi<1, BN_SMALL>(p, (cudaStream_t)stream);
-  if (p->variant == 1) return dispatch_epi<1, BN_BIG>(p, (cudaStream_t)stream);
+  const int tile = p->variant == 0 ? pick_tile(p) : p->variant;
+  if (tile == 2 || tile == 3) return dispatch_epi<1, BN_SMALL>(p, (cudaStream_t)stream);
+  if (tile == 1) return dispatch_epi<1, BN_BIG>(p, (cudaStream_t)stream);
   return dispatch_epi<2, BN_BIG>(p, (cudaStream_t)stream);
 }
 

@@ -79,7 +79,7 @@ typedef struct {
   const void* residual; int64_t ldr;
   int64_t M, N, K;
   int epilogue;
-  int variant;                   /* 0 = 2-CTA 256x256 tiles; 1 = 1-CTA 128x256 tiles; 2 = 1-CTA 128x64 weight-streaming tiles (small M);
+  int variant;                   /* 0 = tiles by shape: 2-CTA 256x256, or one of the next two where these would leave SMs idle (the same results); 1 = 1-CTA 128x256 tiles; 2 = 1-CTA 128x64 weight-streaming tiles (small M);
                                     3 = like 2 with W given tile-major: (N/64, K/64, 64, 64), i.e. W.view(N/64,64,K/64,64).permute(0,2,1,3) */
   const void* rope_cos; const void* rope_sin;   /* EVO_EPI_BIAS_ROPE: (positions, 64) bf16 tables (evo_rope_tables) */
   int64_t rope_L;                /* tokens per sequence: row m uses table row m % rope_L */

@@ -1,0 +1,40 @@
+"""The tiles that evo_gemm picks for a shape leave the bits of a result as they are: around the lines of the rule, and its three forms against one another."""
+import math
+
+import pytest
+import torch
+
+import evo_b200._lib as _lib
+from evo_b200.engine import KernelOps
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda:0", torch.bfloat16
+
+
+class _Ops(KernelOps):
+    _prof, gemm_variant, gemm_variant_gate = None, 0, 0
+
+
+# one row block and several; 296 small tiles and more; a wave less in narrow tiles; one row behind and in front of a block's end; K past the small tile's line
+@pytest.mark.parametrize("M,N,K", [(65, 512, 64), (127, 4096, 256), (129, 256, 4096), (384, 6144, 128), (385, 6144, 128), (300, 12288, 256), (513, 4096, 320), (141, 2048, 6208), (640, 11008, 128),
+                                   (1, 256, 64), (2368, 1024, 64), (2369, 1024, 64)])
+def test_picked_tiles_are_the_same_bits(M, N, K, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a, w = torch.randn(M, K, generator=g, device=DEV).to(BF), (torch.randn(N, K, generator=g, device=DEV) / math.sqrt(K)).to(BF)
+    bias, resid = torch.randn(N, generator=g, device=DEV).to(BF), torch.randn(M, N, generator=g, device=DEV).to(BF)
+    for epi in (_lib.EPI_NONE, _lib.EPI_BIAS, _lib.EPI_BIAS_RESID, _lib.EPI_RESID, _lib.EPI_SILU_COLS, _lib.EPI_GELU_GATE, _lib.EPI_GELU_TANH_GATE):
+        gate = epi in (_lib.EPI_GELU_GATE, _lib.EPI_GELU_TANH_GATE)
+        outs = []
+        for tile in (None, "0", "1", "2"):
+            monkeypatch.delenv("EVO_B200_GEMM_TILE", raising=False)
+            if tile is not None:
+                monkeypatch.setenv("EVO_B200_GEMM_TILE", tile)
+            out = torch.full((M + 1, N // 2 if gate else N), 7.0, dtype=BF, device=DEV)
+            _Ops()._gemm(a, w, out, M, N, K, epi, bias=bias, resid=resid, ldc=out.shape[1], act_cols=N // 2)
+            assert (out[M] == 7.0).all()
+            outs.append(out)
+        assert all(torch.equal(outs[0], o) for o in outs[1:]), epi
+        if epi == _lib.EPI_NONE:
+            want = a.double() @ w.double().T
+            # half a step of bf16, and K products in fp32
+            assert ((outs[0][:M].double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2.0 ** -16 * want.abs().max()).all()
