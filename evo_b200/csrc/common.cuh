@@ -326,6 +326,12 @@ int pdl_level();         // evo_set_pdl(): 0 off, 1 all decode-step kernels, 2 w
 // first reads data written by (or writes data read by) the previous kernel; both are no-ops in a normal launch.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the beginning of a kernel that is launched both in a decode step, where its successor may start at once, and over whole sequences, where it may when all that is in front of this kernel is through
+template <bool STEP> __device__ __forceinline__ void pdl_enter() {
+  if constexpr (STEP) pdl_launch_dependents();
+  pdl_wait();
+  if constexpr (!STEP) pdl_launch_dependents();
+}
 
 // host: kernel launch that adds the programmatic-serialization attribute when evo_set_pdl(1) is active (or, for a kernel launched
 // through launch_pdl_light, at level 3 as well)
@@ -341,7 +347,8 @@ inline cudaError_t launch_pdl_at(int min_level_extra, void (*kern)(KArgs...), di
   }
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
-// always with the attribute: for kernels that wait (pdl_wait) before they touch anything
+// always with the attribute: for kernels that wait (pdl_wait) before they touch anything and before they let a successor start, which may fetch what a kernel in front of both wrote ahead of
+// its own wait (evo_hyena_step, evo_gemm_smallm)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};

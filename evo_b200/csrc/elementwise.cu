@@ -118,9 +118,10 @@ __device__ __forceinline__ uint4 normed(const uint4& v, const uint4& s, float ri
 
 // Few rows (decode step): one 256-thread CTA per row instead of one warp per row -- the row and the scale are fetched
 // by 8 warps at once (the warp-per-row kernel is a 5 us latency chain on 2 CTAs at 16 rows).  Same rounding chain.
+template <bool STEP>
 __global__ void __launch_bounds__(256) rmsnorm_row_kernel(const uint4* __restrict__ x, const uint4* __restrict__ scale,
                                                           uint4* __restrict__ out, int row_vec, float inv_sqrt_d, float eps) {
-  pdl_launch_dependents(); pdl_wait();
+  pdl_enter<STEP>();
   __shared__ float red[8];
   const int tid = threadIdx.x;
   const uint4* xr = x + (int64_t)blockIdx.x * row_vec;
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(256) rmsnorm_row_kernel(const uint4* __restric
 template <typename IdT>
 __global__ void __launch_bounds__(256) embed_norm_kernel(const IdT* __restrict__ ids, const uint4* __restrict__ table, const uint4* __restrict__ scale, uint4* __restrict__ u,
                                                          uint4* __restrict__ out, int row_vec, int vocab, float inv_sqrt_d, float eps, long long* __restrict__ pos, long long position) {
-  pdl_launch_dependents(); pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[8];
   const int tid = threadIdx.x;
   long long id = (long long)ids[blockIdx.x];
@@ -175,14 +176,13 @@ extern "C" int evo_embed_norm(const void* ids, int ids_are_i64, const void* tabl
                               int64_t position, void* stream) {
   EVO_REQUIRE(D % 256 == 0 && D <= 8192, "evo_embed_norm: D (%d) must be a multiple of 256 and <= 8192", D);
   EVO_REQUIRE(rows > 0 && rows < (1ll << 31), "evo_embed_norm: rows (%lld)", (long long)rows);
-  // (not dependent where evo_hyena_step fetches its states ahead of its wait: between two of a layer's steps there has to be one launch that waits for all in front of it)
+  // an ordinary launch at every level: evo_hyena_step fetches its states ahead of its wait, so that between two of a layer's steps one launch has to wait for all in front of it, and this one does
   const float isd = (float)(1.0 / sqrt((double)D));
+  cudaStream_t st = (cudaStream_t)stream;
   if (ids_are_i64)
-    EVO_CUDA(launch_pdl(embed_norm_kernel<long long>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const long long*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u,
-                              (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position));
+    embed_norm_kernel<long long><<<(unsigned)rows, 256, 0, st>>>((const long long*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u, (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position);
   else
-    EVO_CUDA(launch_pdl(embed_norm_kernel<int>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const int*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u,
-                              (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position));
+    embed_norm_kernel<int><<<(unsigned)rows, 256, 0, st>>>((const int*)ids, (const uint4*)table, (const uint4*)scale, (uint4*)u, (uint4*)out, D / 8, vocab, isd, eps, (long long*)pos, (long long)position);
   return check_launch("evo_embed_norm");
 }
 
@@ -190,7 +190,7 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
   EVO_REQUIRE(D % 256 == 0 && D <= 8192, "evo_rmsnorm: D (%d) must be a multiple of 256 and <= 8192", D);
   if (rows == 0) return 0;
   if (rows <= 64) {
-    EVO_CUDA(launch_pdl_light(rmsnorm_row_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
+    EVO_CUDA(launch_pdl_light(rmsnorm_row_kernel<true>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
                         D / 8, (float)(1.0 / sqrt((double)D)), eps));
     return check_launch("evo_rmsnorm");
   }
@@ -198,7 +198,7 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
   // 2048 wide: 1024 rows 7.9 / 8.0, 2048 rows 8.4 / 8.0, 8192 rows 22.7 / 18.6 (too few bytes per CTA), narrower the same; 8192 wide: 903 rows 8.4 / 15.1, 32768 rows 156 / 268
   // (a warp would hold 32 vectors per lane)
   if (D > 4096 || rows <= (D >= 4096 ? 12288 : 1024)) {
-    EVO_CUDA(launch_dependent(rmsnorm_row_kernel, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
+    EVO_CUDA(launch_dependent(rmsnorm_row_kernel<false>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
                               D / 8, (float)(1.0 / sqrt((double)D)), eps));
     return check_launch("evo_rmsnorm");
   }

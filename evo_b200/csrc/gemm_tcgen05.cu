@@ -259,8 +259,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_launch_dependents();   // every CTA of this launch has its TMEM before one of the next launch can ask for some
-  pdl_wait();                // launched dependent (see launch()): nothing in front of this reads or writes what a kernel before may write or read
+  // Launched dependent (see launch()): nothing in front of this reads or writes what a kernel before may write or read.  The successor starts only when the last CTA has ended: evo_hyena_step
+  // fetches its states, and evo_gemm_smallm its weights, ahead of their waits, and a GEMM between them and the kernel that wrote those is what orders the two.
+  pdl_wait();
 
   // Tile walk of this CTA (pair): tiles w_first, w_first + w_step, ... < n_tiles of the row-blocks [m_lo, m_lo + m_cnt).
   // Die-aware (CG == 2, full grid): each die works on its own contiguous share of the row-blocks, so the streamed operand's
@@ -546,7 +547,8 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
   }
   cfg.attrs = attr;
   // Launched dependent, but for the die-aware form, whose claims are cleared in front of it: barriers, TMEM and tensor maps are ready when the kernel in front ends.
-  // The two layers of a feed-forward of 3002 rows 652 -> 641 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606.
+  // The two layers of a feed-forward of 3002 rows 645 -> 637 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606 (when a GEMM's successor could
+  // start beside it; without that, as now, the feed-forward is 631 / 637 and the call 1579 / 1577).
   if (g.die_tab == nullptr) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;

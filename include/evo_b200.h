@@ -159,7 +159,11 @@ size_t evo_hyena_fwd_workspace(const evo_hyena_params* p);
 int evo_hyena_fwd(const evo_hyena_params* p, void* workspace, size_t workspace_bytes, void* stream);
 
 /* decode step: engine.step_fir + step_iir.  u (B, 3D) bf16 -> y (B, D) bf16;
- * fir_state (B, 3D, 2) bf16 and state (B, D, S, 2) fp32 are updated in place. */
+ * fir_state (B, 3D, 2) bf16 and state (B, D, S, 2) fp32 are updated in place.
+ * Where evo_set_pdl has it launched dependent (levels 1 and 4), it fetches the filter and both states ahead of its wait.  Two steps on the same states, and a step and whatever else
+ * writes its filter or states, then need a launch between them that is through only when all in front of it is, and that lets its successor start only then: evo_gemm, evo_embed_norm, a
+ * kernel or copy of another library, or any function of this header that is no part of a decode step.  evo_gemm_smallm, evo_rmsnorm of up to 64 rows, evo_hyena_step itself,
+ * evo_decode_qkv_prep, evo_decode_attn and, at level 1, evo_embed, evo_rmsnorm and the sampler's functions are not such launches.  evo_gemm_smallm's W is under the same rule at levels 1 to 4. */
 int evo_hyena_step(const void* u, void* y, void* fir_state, float* state,
                    const void* fir_w, const void* fir_b, const void* Dskip,
                    const float* poles, const float* residues,
