@@ -323,7 +323,6 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   int* flag = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if ((smem_u32(smem) & 1023u) != 0) __trap();
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 0] = gtimer(); g.trace[blockIdx.x * 16 + 1] = clock64(); }
 
@@ -350,6 +349,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Only now: evo_gemm, whose small tiles fit an SM beside a short ring of this kernel, is launched dependent at every level, and must not take the TMEM that a CTA of this launch still asks for.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) stamp(g, 2);                          // setup done
 
   if (warp == 0) {

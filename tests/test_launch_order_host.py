@@ -57,6 +57,18 @@ def test_every_dependent_launch_is_listed():
             assert file in DEPENDENT or file == "gemm_smallm.cu", file
 
 
+def test_tmem_is_held_before_a_successor_may_ask_for_some():
+    """A successor that takes the TMEM which a CTA of the kernel in front still asks for, and then waits for that kernel, would wait for good."""
+    found = 0
+    for name, body in _bodies().items():
+        alloc, start = body.find("tmem_alloc<"), re.search(START, body)
+        if alloc >= 0 and start is not None:
+            found += 1
+            barrier = body.find("__syncthreads()", alloc)
+            assert 0 <= barrier < start.start(), name
+    assert found == 1                                        # gemm_smallm_kernel
+
+
 def test_the_first_launch_of_a_decode_step_is_ordinary():
     """evo_embed_norm is the launch that waits for everything of the step in front."""
     s = _text(os.path.join(CSRC, "elementwise.cu"))
