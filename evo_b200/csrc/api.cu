@@ -10,7 +10,7 @@ namespace evo {
 
 static thread_local char g_err[512] = "";
 static std::atomic<int64_t> g_launches{0};
-static std::atomic<int> g_pdl{0};
+static std::atomic<int> g_pdl{-1};
 int pdl_level() { return g_pdl.load(std::memory_order_relaxed); }
 
 // One word of host memory that every device can write and the host reads without a stream; allocated by the first launch that may need it, which may be under capture.
@@ -133,5 +133,5 @@ int evo_set_wait_polls(int polls) {
   evo::g_polls = polls < 0 ? evo::WAIT_POLLS : polls;
   return before;
 }
-int evo_set_pdl(int level) { return evo::g_pdl.exchange(level < 0 ? 0 : (level > 4 ? 4 : level)); }
+int evo_set_pdl(int level) { return evo::g_pdl.exchange(level < 0 ? -1 : (level > 4 ? 4 : level)); }
 }

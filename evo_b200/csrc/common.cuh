@@ -320,7 +320,7 @@ inline int ensure_dyn_smem(K kern, int bytes, unsigned long long& mask) {
   }
   return 0;
 }
-int pdl_level();         // evo_set_pdl(): 0 off, 1 all decode-step kernels, 2 weight-streaming GEMM only, 3 + the row-norm kernel, 4 + hyena_step
+int pdl_level();         // evo_set_pdl(): -1 (at first) kernels of whole sequences only, 0 off, and beside those 1 all decode-step kernels, 2 weight-streaming GEMM only, 3 + the row-norm kernel, 4 + hyena_step
 
 // Programmatic dependent launch: every kernel that may be launched with the attribute calls pdl_wait() before it
 // first reads data written by (or writes data read by) the previous kernel; both are no-ops in a normal launch.
@@ -347,8 +347,9 @@ inline cudaError_t launch_pdl_at(int min_level_extra, void (*kern)(KArgs...), di
   }
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
-// always with the attribute: for kernels that wait (pdl_wait) before they touch anything and before they let a successor start, which may fetch what a kernel in front of both wrote ahead of
-// its own wait (evo_hyena_step, evo_gemm_smallm)
+inline bool pdl_off() { return pdl_level() == 0; }
+// with the attribute at every level but 0: for kernels that wait (pdl_wait) before they touch anything and before they let a successor start, which may fetch what a kernel in front of both
+// wrote ahead of its own wait (evo_hyena_step, evo_gemm_smallm)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -356,7 +357,7 @@ inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_off() ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 template <typename... KArgs, typename... Args>

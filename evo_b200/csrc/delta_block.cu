@@ -1215,7 +1215,7 @@ int run(const evo_gated_delta_params* p, const Sizes& s, uint8_t* ws, cudaStream
     // 28.8 / 26.7, 1 x 777, 32 heads of 128 x 128 62.9 / 60.4, 1 x 4096 253 / 249.  But CTAs that come to most of the SMs one by one are placed worse: 64 pairs, 128 CTAs, 4 x 4096 tokens
     // 329 / 340, 4 x 1024 95 / 99; 128 pairs of 128 x 64 67.0 / 67.6.  For one or two blocks the early start is worth more than the place: 48 tokens, 128 pairs of 64 x 128 37.9 / 33.8,
     // 160 of 64 x 32 33.8 / 31.6; 128 tokens, 128 pairs of 128 x 128 50 / 48, 1024 249 / 245.
-    const bool dependent = (int64_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z * 2 <= device_sm_count() || s.blocks <= 2;
+    const bool dependent = !pdl_off() && ((int64_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z * 2 <= device_sm_count() || s.blocks <= 2);
     cfg.attrs = dependent ? attrs : attrs + 1; cfg.numAttrs = (dependent ? 1 : 0) + (a.pair ? 1 : 0);
     EVO_CUDA(cudaLaunchKernelEx(&cfg, delta_scan_kernel<DK>, tmK, tmQ, tmV, a));
     if ((rc = check_launch("evo_gated_delta_fwd(scan)"))) return rc;

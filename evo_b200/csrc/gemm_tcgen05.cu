@@ -549,7 +549,7 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
   // Launched dependent, but for the die-aware form, whose claims are cleared in front of it: barriers, TMEM and tensor maps are ready when the kernel in front ends.
   // The two layers of a feed-forward of 3002 rows 645 -> 637 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606 (when a GEMM's successor could
   // start beside it; without that, as now, the feed-forward is 631 / 637 and the call 1579 / 1577).
-  if (g.die_tab == nullptr) {
+  if (g.die_tab == nullptr && !pdl_off()) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;

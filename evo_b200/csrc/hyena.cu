@@ -370,7 +370,7 @@ static cudaError_t launch_after(bool dependent, void (*kern)(KArgs...), dim3 gri
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization; attr.val.programmaticStreamSerializationAllowed = 1;
-  if (dependent) { cfg.attrs = &attr; cfg.numAttrs = 1; }
+  if (dependent && !pdl_off()) { cfg.attrs = &attr; cfg.numAttrs = 1; }
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 

@@ -117,11 +117,16 @@ typedef struct {
 } evo_gemm_smallm_params;
 size_t evo_gemm_smallm_workspace(int64_t M, int64_t N, int64_t K, int epilogue);
 int evo_gemm_smallm(const evo_gemm_smallm_params* p, void* stream);
-/* Programmatic dependent launch for the decode step.  0 = off (default); 1 = every decode-step kernel is launched with
- * programmatic stream serialization; 2 = only evo_gemm_smallm is (its weight prefetch then overlaps the small kernel or
- * the GEMM tail in front of it); 3 = evo_gemm_smallm, the few-row evo_rmsnorm, evo_decode_qkv_prep and evo_decode_attn with its merge; 4 = those and
- * evo_hyena_step (which fetches its filter parameters and states ahead of the wait).  Every decode-step kernel begins with griddepcontrol.launch_dependents and waits
- * (griddepcontrol.wait) before it first touches dependent data.  Process-wide switch; returns the previous value. */
+/* Programmatic dependent launch: a kernel may be set up while the one in front of it in the stream still runs.  It waits (griddepcontrol.wait) before it first touches dependent data, so
+ * the results are the same bits at every level.
+ *   negative (the library's start): the kernels that go over whole sequences -- evo_gemm (but for its die-aware form), evo_rmsnorm of 65 rows up to where a warp takes a row,
+ *       evo_sum_norm, evo_conv_act, evo_attn_fwd_ws variants 2 and 3, evo_window_attn_fwd on tcgen05, and kernels inside evo_hyena_fwd and evo_gated_delta_fwd.  They let a successor
+ *       start only when all in front of them is through.
+ *   0 = off: every launch waits for the one in front of it.
+ *   1 to 4: the same kernels, and of a decode step 1 = every kernel; 2 = only evo_gemm_smallm (its weight prefetch then overlaps the kernel in front of it); 3 = evo_gemm_smallm,
+ *       evo_rmsnorm of up to 64 rows, evo_decode_qkv_prep and evo_decode_attn with its merge; 4 = those and evo_hyena_step (which fetches its filter parameters and states ahead of the
+ *       wait: see there).  These let their successor start before they wait themselves.
+ * Process-wide switch; returns the previous value. */
 int evo_set_pdl(int level);
 /* Waits inside the kernels of evo_hyena_fwd, evo_gated_delta_fwd and evo_window_attn_fwd have a limit: one that runs out ends its CTA without writing a state, and the
  * call's outputs are incomplete although it returned 0 (launches are asynchronous).  evo_lost_waits returns 1 if that has happened, on any device of the process, since the

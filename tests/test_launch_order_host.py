@@ -7,7 +7,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "evo_b200", "csrc")
-# launched dependent whatever evo_set_pdl says, by the file that launches them
+# launched dependent at every level of evo_set_pdl but 0, by the file that launches them
 DEPENDENT = {
     "gemm_tcgen05.cu": {"gemm_tcgen05_kernel"}, "elementwise.cu": {"rmsnorm_row_kernel<false>"}, "attention_pp.cu": {"attn_pp_kernel"}, "window_attention_tc.cu": {"window_attn_tc_kernel"},
     "branch_ops.cu": {"sum_norm_kernel", "sum_norm_row_kernel", "conv_act4_kernel", "conv_act_kernel", "conv_carry_kernel"},
@@ -75,3 +75,12 @@ def test_the_first_launch_of_a_decode_step_is_ordinary():
     entry = s[s.index("int evo_embed_norm("):]
     entry = entry[:entry.index("\n}")]
     assert "embed_norm_kernel<long long><<<" in entry and "launch_pdl" not in entry and "launch_dependent" not in entry
+
+
+def test_level_zero_reaches_every_dependent_launch():
+    """evo_set_pdl(0) is off for each launch that carries the attribute."""
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        s = _text(path)
+        for m in re.finditer(r"ProgrammaticStreamSerialization;", s):
+            start, end = s.rfind("\n}", 0, m.start()), s.find("\n}", m.start())        # the function around it
+            assert re.search(r"pdl_off\(\)|pdl_level\(\) (==|>=) 1", s[start:end]), (os.path.basename(path), s.count("\n", 0, m.start()) + 1)
