@@ -55,6 +55,7 @@ struct GemmArgs {
   const bf16* resid; long long ldr;
   long long M, N, K;
   int m_blocks, n_blocks, group_m;
+  bool early;            // the successor may start beside this kernel
   int b_tiled;           // small-M tile only: W is tile-major [N/64][K/64][64][64] (contiguous 8 KB tiles: every DRAM page opened is fully used)
   int a_rows, n_stages, ksub;  // small-M tile only: rows of A staged per k-block, ring depth, 64-column k-blocks per ring stage
   // peer-scattered output (sequence-parallel Ulysses re-shard fused into the Wqkv epilogue): column n of row m goes to
@@ -259,9 +260,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Launched dependent (see launch()): nothing in front of this reads or writes what a kernel before may write or read.  The successor starts only when the last CTA has ended: evo_hyena_step
-  // fetches its states, and evo_gemm_smallm its weights, ahead of their waits, and a GEMM between them and the kernel that wrote those is what orders the two.
+  // Launched dependent (see launch()): nothing in front of this reads or writes what a kernel before may write or read.  Every CTA has its TMEM before one of the next launch can ask for some.
   pdl_wait();
+  if (g.early) pdl_launch_dependents();
 
   // Tile walk of this CTA (pair): tiles w_first, w_first + w_step, ... < n_tiles of the row-blocks [m_lo, m_lo + m_cnt).
   // Die-aware (CG == 2, full grid): each die works on its own contiguous share of the row-blocks, so the streamed operand's
@@ -547,8 +548,10 @@ int launch(const evo_gemm_params* p, cudaStream_t st, const long long* targets =
   }
   cfg.attrs = attr;
   // Launched dependent, but for the die-aware form, whose claims are cleared in front of it: barriers, TMEM and tensor maps are ready when the kernel in front ends.
-  // The two layers of a feed-forward of 3002 rows 645 -> 637 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606 (when a GEMM's successor could
-  // start beside it; without that, as now, the feed-forward is 631 / 637 and the call 1579 / 1577).
+  // The two layers of a feed-forward of 3002 rows 645 -> 637 us; a call on 3 x 301 tokens through four blocks, its norms launched so as well, 1671 -> 1606.  The successor starts beside it, but
+  // behind its wait, where no kernel fetches ahead of its own: 637 -> 633, few rows 140 -> 137.  At levels 1 to 4 evo_hyena_step fetches its states so, and evo_gemm_smallm its weights, and
+  // a GEMM between them and the kernel that wrote those, or which wrote those itself, is what orders the two.
+  g.early = pdl_level() < 0;
   if (g.die_tab == nullptr && !pdl_off()) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;

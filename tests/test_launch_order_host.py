@@ -66,7 +66,7 @@ def test_tmem_is_held_before_a_successor_may_ask_for_some():
             found += 1
             barrier = body.find("__syncthreads()", alloc)
             assert 0 <= barrier < start.start(), name
-    assert found == 1                                        # gemm_smallm_kernel
+    assert found == 2                                        # gemm_smallm_kernel, gemm_tcgen05_kernel
 
 
 def test_the_first_launch_of_a_decode_step_is_ordinary():
