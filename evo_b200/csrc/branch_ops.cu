@@ -5,6 +5,7 @@
 //   evo_gated_group_norm  y * silu(gate), RMS norm in equal parts of the row, weight
 // Sums of squares, norms and the stream are fp32 whatever the activation type.
 #include "common.cuh"
+#include "conv_rows.h"
 #include "../../include/evo_b200.h"
 #include <math.h>
 #include <algorithm>
@@ -289,7 +290,7 @@ template <typename T, bool ACT> __device__ __forceinline__ float2 conv_finish(fl
 
 // four channels per thread (8- or 16-byte accesses), taps and activation known at compile time.  Two special functions per element are 46 us for 4 x 4096 rows of 6144 channels, the
 // bytes 64 (a plain copy): 79 us with cold L2 (88 to 92 as CTAs of 32 rows with four rows in work and four under way).  What it takes: bytes under way -- eight bf16 rows in work and
-// eight under way, four CTAs per SM of 128 registers (four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows).  fp32 rows, four and four: 148 us (162).
+// eight under way, four CTAs per SM of 128 registers (four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows.h).  fp32 rows, four and four: 148 us (162).
 template <typename T, int TAPS, bool ACT>
 __global__ void __launch_bounds__(128, CONV_CTAS) conv_act4_kernel(evo_conv_act_params p, int write_carry, int rows_per) {
   pdl_wait();
@@ -602,18 +603,6 @@ extern "C" int evo_sum_norm(const evo_sum_norm_params* p, void* stream) {
   return check_launch("evo_sum_norm");
 }
 
-// Rows per CTA of the kernel with four channels per thread: one wave of CTAs that end together, each with its taps and the inputs in front fetched once, instead of many of 32 rows (4 x 4096 x 6144 with six CTAs per SM: 88 us by 32 rows, 83 so); where
-// sequences and channels alone are more than a wave, the split with the least of (waves x (rows + what a CTA's start takes, about 16 rows' time)).
-static int64_t conv_rows(const evo_conv_act_params* p) {
-  const int64_t slots = (int64_t)device_sm_count() * CONV_CTAS, per = ((p->C / 4 + 127) / 128) * (int64_t)p->B;
-  int64_t best = CONV_RT, cost = INT64_MAX;
-  for (int64_t n = 1; n <= 1024 && (n == 1 || p->L / n >= CONV_RT); ++n) {
-    const int64_t rows = std::min<int64_t>(1 << 20, std::max<int64_t>(CONV_RT, ((p->L + n - 1) / n + 3) / 4 * 4)), ctas = per * ((p->L + rows - 1) / rows), c = ((ctas + slots - 1) / slots) * (rows + 16);
-    if (c < cost) { cost = c; best = rows; }
-  }
-  return best;
-}
-
 extern "C" int evo_conv_act(const evo_conv_act_params* p, void* stream) {
   EVO_REQUIRE(p->in && p->weight && p->out && p->C > 0 && p->taps >= 1 && p->taps <= CONV_MAX_TAPS, "evo_conv_act: bad arguments (taps 1..%d)", CONV_MAX_TAPS);
   EVO_REQUIRE(p->ld >= p->C && p->ldo >= p->C && p->B >= 0 && p->L >= 0, "evo_conv_act: bad shape");
@@ -622,7 +611,7 @@ extern "C" int evo_conv_act(const evo_conv_act_params* p, void* stream) {
   const bool vec = p->C % 4 == 0 && p->ld % 4 == 0 && p->ldo % 4 == 0 && p->taps <= 4 && (!p->carry || ((uintptr_t)p->carry & 15) == 0) &&
                    (!p->bias || aligned4<bf16>(p->bias)) &&
                    (p->dtype ? aligned4<float>(p->in) && aligned4<float>(p->out) : aligned4<bf16>(p->in) && aligned4<bf16>(p->out));
-  const int64_t rows_per = vec ? conv_rows(p) : CONV_RT;
+  const int64_t rows_per = vec ? conv_rows(p->L, (p->C / 4 + 127) / 128 * (int64_t)p->B, (int64_t)device_sm_count() * CONV_CTAS, CONV_RT) : CONV_RT;
   const unsigned chunks = (unsigned)((p->L + rows_per - 1) / rows_per);
   const dim3 grid((p->C + 127) / 128, chunks, p->B);
   // with one thread per (sequence, channel) that thread reads the carried inputs before it replaces them, and where none are read (zero_start) the thread of the last
