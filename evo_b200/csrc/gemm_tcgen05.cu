@@ -586,15 +586,17 @@ int dispatch_epi(const evo_gemm_params* p, cudaStream_t st) {
 // Variant 0's tiles: a sum's order does not depend on them (the results are the same bits), so the shape decides.  Few rows leave most of the pairs of SMs without a 256 x 256 tile, or the
 // last wave nearly empty.  By pairs / by 128 x 256 / by 128 x 64 (us, cold L2):
 //   128 x 64 while all its tiles fit at once, two to an SM, and K is not so long that their small operands' loads cost more than the SMs gained: 4096 x 4096, 300 rows 36.9 / 41 / 32.8,
-//   514 rows (320 tiles) 38.9 / 41 / 51; 2048 x 2048, 903 rows 26.6 / 28.7 / 22.5, 1300 (352) 28.7 / 28.7 / 30.7; 2048 x 5504, 200 rows 41.0 / 45 / 34.8; 4096 x 11008, 66 rows 65.6 /
-//   80 / 67.6, 400 rows 71.7 / 84 / 73.7
+//   514 rows (320 tiles) 38.9 / 41 / 51; 2048 x 2048, 903 rows 26.6 / 28.7 / 22.5, 1300 (352) 28.7 / 28.7 / 30.7; 2048 x 5504, 200 rows 41.0 / 45 / 34.8.  Tall and narrow the same, 256 wide,
+//   9472 rows: K = 256 18.4 / 16.4 / 14.3, 4096 41.0 / 47 / 38.9, 5504 49.2 / 57 / 49.2.  Where the two meet depends on the rows: 4096 wide, 66 / 296 rows, pairs / 128 x 64: K = 6144
+//   43.0 / 41.0, 46.9 / 45.1, 7168 49.1 / 47.1, 51.2 / 50.2, 8192 53.2 / 51.3, 55.3 / 55.3, 11008 65.5 / 67.6, 68.5 / 71.6; 256 wide, 128 / 9472 rows: 6144 42.9 / 36.9, 51.3 / 51.2,
+//   8192 51.2 / 47.1, 63.5 / 63.5, 11008 63.5 / 59.4, 75.8 / 77.9.  6144 is the longest K up to which no shape measured was slower than pairs; up to 8192 few rows would gain 0 to 9 % more.
 //   128 x 256 where it takes a wave less (few waves: one is 5 to 8 % longer): 12288 x 4096, 300 rows 59.4 / 47.1 / 57.3, 400 rows 59.4 / 68.4; gated 22016 x 4096, 128 rows 67.6 / 55.2,
 //   141 rows 67.6 / 73.7, 300 rows 81.9 / 73.7, 514 rows 98.3 / 92.2
 int pick_tile(const evo_gemm_params* p) {
-  const char* env = getenv("EVO_B200_GEMM_TILE");                    // comparisons: 0, 1 or 2; read per call
+  const char* env = getenv("EVO_B200_GEMM_TILE");                    // comparisons: 0, 1 or 2, anything else is as if unset; read per call
   const bool plain = p->n_c_peers == 0 && (p->epilogue == EVO_EPI_NONE || p->epilogue == EVO_EPI_BIAS || p->epilogue == EVO_EPI_BIAS_RESID || p->epilogue == EVO_EPI_RESID ||
                                            p->epilogue == EVO_EPI_SILU_COLS);
-  if (env) return atoi(env) == 2 ? (plain ? 2 : 1) : atoi(env);
+  if (env && env[0] >= '0' && env[0] <= '2' && env[1] == 0) return env[0] == '2' && !plain ? 1 : env[0] - '0';
   const int64_t sms = device_sm_count(), rows128 = (p->M + 127) / 128, n256 = p->N / 256;
   if (plain && p->K <= 6144 && rows128 * n256 * 4 <= 2 * sms) return 2;
   const int64_t pairs = ((p->M + 255) / 256) * n256, waves = (pairs + sms / 2 - 1) / (sms / 2);

@@ -38,3 +38,20 @@ def test_picked_tiles_are_the_same_bits(M, N, K, monkeypatch):
             want = a.double() @ w.double().T
             # half a step of bf16, and K products in fp32
             assert ((outs[0][:M].double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + 2.0 ** -16 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("setting", ["3", "-1", "12", "two", ""])
+def test_an_unknown_tile_is_no_tile(setting, monkeypatch):
+    """EVO_B200_GEMM_TILE names a tile with 0, 1 or 2; anything else leaves the choice to the rule, for the epilogues that the 128 x 64 tile does not have as well."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    M, N, K = 100, 512, 192
+    a, w = torch.randn(M, K, generator=g, device=DEV).to(BF), (torch.randn(N, K, generator=g, device=DEV) / math.sqrt(K)).to(BF)
+    for epi in (_lib.EPI_NONE, _lib.EPI_GELU_GATE, _lib.EPI_GELU_TANH_GATE):
+        outs = []
+        for value in (None, setting):
+            monkeypatch.delenv("EVO_B200_GEMM_TILE", raising=False)
+            if value is not None:
+                monkeypatch.setenv("EVO_B200_GEMM_TILE", value)
+            outs.append(torch.zeros(M, N if epi == _lib.EPI_NONE else N // 2, dtype=BF, device=DEV))
+            _Ops()._gemm(a, w, outs[-1], M, N, K, epi, ldc=outs[-1].shape[1])
+        assert torch.equal(*outs) and outs[0].abs().max() > 0
