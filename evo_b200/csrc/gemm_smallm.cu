@@ -34,7 +34,8 @@ constexpr int WROWS = 128;          // W rows per MMA row group (UMMA M)
 constexpr int MAXST = 12;           // ring depth upper bound (barrier array size)
 constexpr int EPI_WARP0 = 4;
 // Groups of four epilogue warps.  A CTA's range ends one tile and begins another, and with one group the second tile's sums waited until the first one's were published and, for its last
-// contributor, added up: 1.5 to 3 us at the end of a layer.  One step of one request 378 -> 356 us, of 16 604 -> 580.  Two groups leave a thread 168 registers; what needs more has
+// contributor, added up: 1.5 to 3 us at the end of a layer.  One step of one request 378 -> 356 us, of 16 604 -> 580; three layers one behind the other, 17 / 32 / 64 rows: 12288 x 4096
+// 89 -> 79, 91 -> 81, 107 -> 91, 4096 x 4096 52 -> 48, 54 -> 50, 71 -> 67, 2048 x 5632 48 -> 44, 54 -> 50, 77 -> 71.  Two groups leave a thread 168 registers; what needs more has
 // one: the Hyena step, whose threads hold a channel's filter and states, and the gated layers of many rows with their 128 sums in flight (three of 2816 x 1024 one behind the other,
 // 16 rows: 34 us, 40 with two groups; 11264 x 2048, 64 rows 85 / 89, though 22016 x 4096 163 / 159).  So do layers too small to give every SM eight k-blocks, whose CTAs gain nothing
 // and start later (768 x 256, one row, dependent: 3.6 / 4.1).
@@ -416,7 +417,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   } else if (warp >= EPI_WARP0) {
     // ------------------------------------------------ epilogue / stream-K fix-up: the groups take the CTA's tiles, and the two accumulators, in turn
     const bool two = Epilogue<EPI, MANY>::TWO && blockDim.x > Epilogue<EPI, MANY>::ONE_GROUP;
-    const int group = (warp - EPI_WARP0) >> 2, lead = (EPI_WARP0 + 4 * group) * 32;
+    // (the group's barrier by a register: as constants behind a branch they take a step of sixteen requests 579 -> 580.5 us, though fewer of a CTA's sixteen then count as used)
+    const int group = (warp - EPI_WARP0) >> 2, lead = (EPI_WARP0 + 4 * group) * 32, bar = Epilogue<EPI, MANY>::TWO ? 1 + group : 1;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int q = warp & 3;
     const int row = q * 32 + lane;                            // W row inside the row group == output column inside the tile
@@ -476,15 +478,15 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (!whole) {
         // publication: the CTA barrier orders every thread's partial stores before thread 0's acq_rel atomic (release
         // is cumulative), whose acquire half orders the finisher's slot reads after the other contributors' releases
-        named_bar(1 + group, 128);
+        named_bar(bar, 128);
         if (threadIdx.x == lead) {
           int old;
           asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(old) : "l"(g.counters + tile) : "memory");
           flag[group] = old;
         }
-        named_bar(1 + group, 128);
+        named_bar(bar, 128);
         const bool last = flag[group] == c_last - c_first;
-        if (threadIdx.x == lead) stamp(g, 6);       // partial published
+        if (threadIdx.x == lead) stamp(g, it + (k1 - k0) >= it_end ? 6 : 10);   // (last) partial published
         if (last) {
           const bool first_begins_before = range_start((uint32_t)c_first, total, parts) < (uint32_t)tile * KB;
           if constexpr (COLUMNS) sum_columns<EPI>(g, Mb, tile, row, c_first, c_last, first_begins_before, slot_floats);
@@ -497,10 +499,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   }
 
-  if (threadIdx.x == EPI_WARP0 * 32) stamp(g, 7);             // epilogue done
   __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) stamp(g, 7);                          // epilogue done
   if (warp == 2) tmem_dealloc<1>(tmem_base, tmem_cols);
   if (g.trace && threadIdx.x == 0) { g.trace[blockIdx.x * 16 + 8] = clock64(); g.trace[blockIdx.x * 16 + 15] = gtimer(); }
 }
