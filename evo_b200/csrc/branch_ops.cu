@@ -290,7 +290,7 @@ template <typename T, bool ACT> __device__ __forceinline__ float2 conv_finish(fl
 
 // four channels per thread (8- or 16-byte accesses), taps and activation known at compile time.  Two special functions per element are 46 us for 4 x 4096 rows of 6144 channels, the
 // bytes 64 (a plain copy): 79 us with cold L2 (88 to 92 as CTAs of 32 rows with four rows in work and four under way).  What it takes: bytes under way -- eight bf16 rows in work and
-// eight under way, four CTAs per SM of 128 registers (four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows.h).  fp32 rows, four and four: 148 us (162).
+// eight under way, four CTAs per SM of 128 registers (with SiLU and two to four taps 8 to 16 bytes of a thread spill; four rows and six CTAs 83, five 90, four 97) -- and one wave of CTAs (conv_rows.h).  fp32 rows, four and four: 148 us (162).
 template <typename T, int TAPS, bool ACT>
 __global__ void __launch_bounds__(128, CONV_CTAS) conv_act4_kernel(evo_conv_act_params p, int write_carry, int rows_per) {
   pdl_wait();

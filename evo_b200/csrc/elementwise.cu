@@ -196,7 +196,8 @@ extern "C" int evo_rmsnorm(const void* x, const void* scale, void* out, int64_t 
   }
   // one CTA per row, or one warp per row (eight to a CTA).  Us, CTA / warp: 4096 wide: 903 rows 7.8 / 10.4, 8193 rows 29.1 / 32.4, 12288 rows 41.1 / 42.6, 16384 rows 53.3 / 52.1;
   // 2048 wide: 1024 rows 7.9 / 8.0, 2048 rows 8.4 / 8.0, 8192 rows 22.7 / 18.6 (too few bytes per CTA), narrower the same; 8192 wide: 903 rows 8.4 / 15.1, 32768 rows 156 / 268
-  // (a warp would hold 32 vectors per lane)
+  // (a warp would hold 32 vectors per lane).  Only the former is launched dependent at every level: 3 x 301 tokens' norms are part of the figure at evo_gemm's launch; a warp per row, from 12289
+  // rows or 1025 narrow ones on, was not measured so.
   if (D > 4096 || rows <= (D >= 4096 ? 12288 : 1024)) {
     EVO_CUDA(launch_dependent(rmsnorm_row_kernel<false>, dim3((unsigned)rows), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, (const uint4*)scale, (uint4*)out,
                               D / 8, (float)(1.0 / sqrt((double)D)), eps));

@@ -55,3 +55,29 @@ def test_an_unknown_tile_is_no_tile(setting, monkeypatch):
             outs.append(torch.zeros(M, N if epi == _lib.EPI_NONE else N // 2, dtype=BF, device=DEV))
             _Ops()._gemm(a, w, outs[-1], M, N, K, epi, ldc=outs[-1].shape[1])
         assert torch.equal(*outs) and outs[0].abs().max() > 0
+
+
+@pytest.mark.parametrize("tile", ["0", "1"])
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (16, 12288, 4096), (65, 768, 256), (129, 512, 4096), (257, 256, 64), (300, 1024, 256)])
+def test_big_tiles_on_few_rows(M, N, K, tile, monkeypatch):
+    """Pairs and 128 x 256 tiles where the rule takes smaller ones: every epilogue against products in 64 bits."""
+    monkeypatch.setenv("EVO_B200_GEMM_TILE", tile)
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    n = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    a, w, bias, resid = n(M, K).to(BF), (n(N, K) / math.sqrt(K)).to(BF), n(N).to(BF), n(M, N).to(BF)
+    F, r = torch.nn.functional, lambda x: x.to(BF).double()  # noqa: E731
+    acc = a.double() @ w.double().T
+    t = acc.view(M, -1, 2, 128)
+    l1, l2 = t[:, :, 0].reshape(M, -1), t[:, :, 1].reshape(M, -1)
+    cols = torch.arange(N, device=DEV) < N // 2
+    # what is expected, and by how much a sum that rounds to the other neighbour moves it (steps of 2^-8 of each rounded factor)
+    want = {_lib.EPI_NONE: (acc, 0 * acc), _lib.EPI_BIAS: (acc + bias.double(), 0 * acc),
+            _lib.EPI_BIAS_RESID: (r(acc + bias.double()) + resid.double(), 2.0 ** -7 * (acc + bias.double()).abs()), _lib.EPI_RESID: (r(acc) + resid.double(), 2.0 ** -7 * acc.abs()),
+            _lib.EPI_SILU_COLS: (torch.where(cols, F.silu(acc), acc), 0 * acc), _lib.EPI_GELU_GATE: (r(F.gelu(r(l1))) * r(l2), 2.0 ** -6 * (l1 * l2).abs()),
+            _lib.EPI_GELU_TANH_GATE: (F.gelu(l1, approximate="tanh") * l2, 0 * l1)}
+    for epi, (ref, slack) in want.items():
+        out = torch.full((M + 1, ref.shape[1]), 7.0, dtype=BF, device=DEV)
+        _Ops()._gemm(a, w, out, M, N, K, epi, bias=bias, resid=resid, ldc=out.shape[1], act_cols=N // 2)
+        assert (out[M] == 7.0).all()
+        # half a step of bf16 of the result, and 2^-16 of the sums' scale for K products in fp32
+        assert ((out[:M].double() - ref).abs() <= 1.01 * 2.0 ** -8 * ref.abs() + slack + 2.0 ** -16 * max(1.0, ref.abs().max().item())).all(), epi
