@@ -123,7 +123,7 @@ int evo_gemm_smallm(const evo_gemm_smallm_params* p, void* stream);
  *       evo_sum_norm, evo_conv_act, evo_attn_fwd_ws variants 2 and 3, evo_window_attn_fwd on tcgen05, and kernels inside evo_hyena_fwd and evo_gated_delta_fwd.  They let a successor
  *       start only when all in front of them is through (evo_gemm: and, at levels 0 to 4, when it has ended itself).
  *   0 = off: every launch waits for the one in front of it.
- *   1 to 4: the same kernels, and of a decode step 1 = every kernel; 2 = only evo_gemm_smallm (its weight prefetch then overlaps the kernel in front of it); 3 = evo_gemm_smallm,
+ *   1 to 4: the same kernels, and of a decode step 1 = every kernel but evo_embed_norm; 2 = only evo_gemm_smallm (its weight prefetch then overlaps the kernel in front of it); 3 = evo_gemm_smallm,
  *       evo_rmsnorm of up to 64 rows, evo_decode_qkv_prep and evo_decode_attn with its merge; 4 = those and evo_hyena_step (which fetches its filter parameters and states ahead of the
  *       wait: see there).  These let their successor start before they wait themselves.
  * Process-wide switch; returns the previous value.  Raise it from 0 or below in front of a launch that is ordinary then (evo_embed_norm, a copy): see evo_hyena_step. */
